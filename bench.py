@@ -161,11 +161,6 @@ NARROW_BYTES = {"pt": 824, "ee": 872}
 # launches (k_contact_hessian_sorted) of one step: one-pass ncu capture of each
 # full workload
 NARROW_DRAM_BYTES_PER_STEP = {"rod_bundle": 464.2e6, "screw_nut": 169.6e6}
-# DRAM bytes (read + write) of the CCD edge-edge query per step -- k_ee_collect
-# (both passes), k_cand_bound, k_cand_bucket, k_cand_solve -- from one ncu pass
-# of dram__bytes_read.sum + dram__bytes_write.sum on the full workload (caches
-# flushed before each launch, so an upper bound on the in-step traffic)
-CCD_DRAM_BYTES_PER_STEP = {"rod_bundle": 41.6e6, "screw_nut": 342.1e6}
 
 
 def stage_times(pipe, dx, reps, torch):
@@ -186,13 +181,16 @@ def stage_times(pipe, dx, reps, torch):
     n_ee, n_pt = pipe.n_contacts, pipe.n_contacts_pt
     t = pipe.collision_triplets
     for _ in range(reps):
+        N.call("ipcb_add_dx", ctypes.byref(pipe.soup.c_struct()), N.ptr(dx), N.ptr(pipe.ccd_x1), N.stream_handle())
+        pipe.ccd_toi.fill_(1.0)
+        pipe._status.zero_()
         marks = [("start", ev())]
-        pipe.update_bvh()
-        marks.append(("refit", ev()))
-        pipe._launch_dcd("ee")
-        marks.append(("dcd_ee", ev()))
-        pipe._launch_dcd("pt")
-        marks.append(("dcd_pt", ev()))
+        # box refit and the walk that finds the discrete records and stages
+        # the pairs that can touch within the step
+        pipe._both_queries("ee", pipe._toi_ws)
+        marks.append(("query_ee", ev()))
+        pipe._both_queries("pt", pipe._toi_ws_pt)
+        marks.append(("query_pt", ev()))
         pipe.b.zero_()
         contact_hessian_ee(None, pipe.soup, pipe.contacts_new, t, pipe.b, pipe.contact_stiffness, n=n_ee,
                            ws=pipe._ws_ee)
@@ -207,29 +205,10 @@ def stage_times(pipe, dx, reps, torch):
         marks.append(("bsr", ev()))
         pipe.compute_collision_energy(detect=False)
         marks.append(("energy", ev()))
-        # the CCD of collision_free_step, stage by stage: swept boxes + refit,
-        # then each query (candidate collection + candidate solve, one call)
-        soup = ctypes.byref(pipe.soup.c_struct())
-        s = N.stream_handle()
-        N.call("ipcb_add_dx", soup, N.ptr(dx), N.ptr(pipe.ccd_x1), s)
-        N.call("ipcb_swept_edge_aabbs", soup, N.ptr(pipe.ccd_x1), 1e-7, N.ptr(pipe.ccd_edge_lower),
-               N.ptr(pipe.ccd_edge_upper), s)
-        pipe.ccd_edge_bvh.refit(pipe.ccd_edge_lower, pipe.ccd_edge_upper)
-        pipe.ccd_toi.fill_(1.0)
-        pipe._status.zero_()
-        marks.append(("ccd_boxes_ee", ev()))
-        N.call("ipcb_edge_edge_toi", soup, N.ptr(pipe.ccd_x1), ctypes.byref(pipe.ccd_edge_bvh.c),
-               N.ptr(pipe.ccd_edge_lower), N.ptr(pipe.ccd_edge_upper), int(pipe.disable_self_collision),
-               N.ptr(pipe.ccd_toi), N.ptr(pipe._status), N.ptr(pipe._toi_ws), pipe._toi_ws.numel(), s)
-        marks.append(("ccd_query_ee", ev()))
-        N.call("ipcb_swept_triangle_aabbs", soup, N.ptr(pipe.ccd_x1), 1e-7, N.ptr(pipe.ccd_triangle_lower),
-               N.ptr(pipe.ccd_triangle_upper), s)
-        pipe.ccd_triangle_bvh.refit(pipe.ccd_triangle_lower, pipe.ccd_triangle_upper)
-        marks.append(("ccd_boxes_pt", ev()))
-        N.call("ipcb_point_triangle_toi", soup, N.ptr(pipe.ccd_x1), ctypes.byref(pipe.ccd_triangle_bvh.c), 1e-7,
-               int(pipe.disable_self_collision), N.ptr(pipe.ccd_toi), N.ptr(pipe._status), N.ptr(pipe._toi_ws_pt),
-               pipe._toi_ws_pt.numel(), s)
-        marks.append(("ccd_query_pt", ev()))
+        pipe._solve_staged("ee", pipe._toi_ws)
+        marks.append(("ccd_solve_ee", ev()))
+        pipe._solve_staged("pt", pipe._toi_ws_pt)
+        marks.append(("ccd_solve_pt", ev()))
         torch.cuda.synchronize()
         for (a, ea), (b, eb) in zip(marks[:-1], marks[1:]):
             acc[b] = acc.get(b, 0.0) + ea.elapsed_time(eb) / reps
@@ -605,24 +584,23 @@ def measure(name, args, dev, world, rank, torch, dist, full: bool):
     narrow_roof = {"kernel": "k_contact_hessian_sorted (EE + PT, with its two ordering kernels)", "bound": "hbm",
                    "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                    "frac": achieved / peak, "traffic": NARROW_DRAM_BYTES_PER_STEP[name], "algorithmic_bytes": algo}
-    # CCD edge-edge query: 56 B per query edge (its box and ids) + 112 B per
-    # staged candidate (pair, 8 positions at t0 and t1), per the survey's
-    # per-unit figures; it is the largest stage on the screw and nut
-    ccd_algo = 56 * pipe.soup.n_edges + 112 * ws[0]
-    ccd_achieved = ccd_algo / (st["ccd_query_ee"] * 1e-3) / 1e9
-    ccd_roof = {"kernel": "k_ee_collect + k_cand_toi (CCD edge-edge query)", "bound": "hbm",
-                "achieved": ccd_achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
-                "frac": ccd_achieved / peak, "traffic": CCD_DRAM_BYTES_PER_STEP[name], "algorithmic_bytes": ccd_algo,
-                "note": "bound by the double-precision root isolation and the dependent position gathers, "
-                        "not by DRAM"}
-    dominant = "ccd" if st["ccd_query_ee"] > narrow_ms else "narrow"
+    # edge-edge query (box refit and walk): per edge its ids and 4 positions in
+    # (56 B) and its packed box out and in (64 B); 36 B per record; per staged
+    # pair its ids and bound (12 B)
+    q_algo = 120 * pipe.soup.n_edges + 36 * n_ee + 12 * ws[0]
+    q_achieved = q_algo / (st["query_ee"] * 1e-3) / 1e9
+    query_roof = {"kernel": "k_tree + k_ee_collect (discrete and CCD edge-edge query in one walk)", "bound": "hbm",
+                  "achieved": q_achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
+                  "frac": q_achieved / peak, "algorithmic_bytes": q_algo,
+                  "note": "bound by instruction issue over the box tests of the walk, not by DRAM"}
+    dominant = "query" if st["query_ee"] > narrow_ms else "narrow"
     cpu_pairs, cpu_sec = cpu_pipeline(sc, dx_np, 3)
     out.update({
-        "ccd_candidates": ws[0] + ws[1],
+        "ccd_staged_pairs": ws[0] + ws[1],
         "stage_ms": {k: round(v, 4) for k, v in st.items()},
-        "roofline": ccd_roof if dominant == "ccd" else narrow_roof,
+        "roofline": query_roof if dominant == "query" else narrow_roof,
         "roofline_narrow": narrow_roof,
-        "roofline_ccd": ccd_roof,
+        "roofline_query": query_roof,
         "cpu_baseline": {"value": cpu_pairs / cpu_sec, "unit": "pairs/s", "cores": os.cpu_count(), "kind": "port",
                          "sample": "full workload, 3 passes of the C++ oracle pipeline (DCD+narrow+energy+BSR+CCD)"},
         "gpu_launches": n_launch * args.steps, "kernels": names,
@@ -717,14 +695,14 @@ def run_ours(args):
         wrecking = None if args.no_newton else wrecking_balls_steps(dev, torch)
         sc = head.pop("sc")
         cfg = workload_config(args.workload, sc, head["pairs"])
-        details = {"n_ee": head["n_ee"], "n_pt": head["n_pt"], "ccd_candidates": head["ccd_candidates"],
+        details = {"n_ee": head["n_ee"], "n_pt": head["n_pt"], "ccd_staged_pairs": head["ccd_staged_pairs"],
                    "parallelism": f"replicas x{world}", "stage_ms": head["stage_ms"]}
         out = {
             "metric": METRIC, "value": head["value"], "unit": "pairs/s",
             "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": head["ms_per_step"],
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic", "config": cfg, "details": details, "roofline": head["roofline"],
-            "roofline_narrow": head["roofline_narrow"], "roofline_ccd": head["roofline_ccd"],
+            "roofline_narrow": head["roofline_narrow"], "roofline_query": head["roofline_query"],
             "cpu_baseline": head["cpu_baseline"],
             "e2e": head["e2e"], "gpu_launches": head["gpu_launches"], "kernels": head["kernels"], "clocks": clocks,
             "newton_step": newton, "wrecking_balls": wrecking,

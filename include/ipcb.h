@@ -79,7 +79,8 @@ typedef struct {
   int* sorted;    /* int32[capacity]: primitive of each leaf slot (Morton order) */
   unsigned* keys; /* uint32[capacity]: sorted Morton codes */
   unsigned* flags;/* uint32[capacity]: refit arrival counters (zero between calls) */
-  void* wide;     /* float4[8*max(capacity-1,1)]: 4-wide view rebuilt by build/refit (queries use it) */
+  void* wide;     /* float4[8*max(capacity-1,1)]: 4-wide view rebuilt by build/refit; followed in the block by
+                   * the packed 32-ary boxes over the same leaf order, which the DCD and CCD queries use */
 } ipcb_lbvh;
 
 int ipcb_version(void);
@@ -142,6 +143,13 @@ int ipcb_swept_edge_aabbs(const ipcb_soup* soup, const void* x1, double pad, flo
                           ipcb_stream s);
 int ipcb_swept_triangle_aabbs(const ipcb_soup* soup, const void* x1, double pad, float* lower, float* upper,
                               ipcb_stream s);
+
+/* The packed boxes of a hierarchy over the soup's edges / triangles, formed
+ * from x4 (padded by pad) in one pass: what the queries below read.  The
+ * binary and 4-wide nodes keep the boxes of the last build or
+ * ipcb_lbvh_refit (which refits the packed boxes too). */
+int ipcb_lbvh_refit_edges(const ipcb_soup* soup, const float* x4, float pad, const ipcb_lbvh* bvh, ipcb_stream s);
+int ipcb_lbvh_refit_triangles(const ipcb_soup* soup, const float* x4, float pad, const ipcb_lbvh* bvh, ipcb_stream s);
 
 /* ---- DCD broad phase (contact.py:199-228 edge_edge_collision, 304-336 point_triangle_collision) ----
  * Appends every pair with float32 closest distance < 2*thickness that passes
@@ -222,6 +230,38 @@ int ipcb_edge_edge_toi(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* s
                        ipcb_stream s);
 int ipcb_point_triangle_toi(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* swept_tri_bvh, double pad,
                             int exclude_same_body, void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s);
+/* The CCD queries of one step from the positions alone: the packed boxes of
+ * the hierarchy are refit to the swept boxes of (x, x1) and queried.  seeds
+ * (may be null): a contact list whose pairs (e0e1; its count read on the
+ * device) are tried first; the boxes then only span the step up to the TOI
+ * they give, so the query meets far fewer pairs.  The TOI is that of
+ * ipcb_edge_edge_toi / ipcb_point_triangle_toi on the whole step.  first,
+ * count: the queries as in the _range calls; query_order: as in ipcb_dcd_pt. */
+int ipcb_edge_edge_step(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                        const ipcb_contacts* seeds, int exclude_same_body, int first, int count, void* toi, int* status,
+                        void* ws, size_t ws_bytes, ipcb_stream s);
+int ipcb_point_triangle_step(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                             const int* query_order, const ipcb_contacts* seeds, int exclude_same_body, int first,
+                             int count, void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s);
+/* The discrete and the CCD query of one kind in one walk, for a host that has
+ * the direction when it detects (the contact iteration): the packed boxes are
+ * refit to the union of both queries' boxes (edges: padded by box_pad; the
+ * points' discrete reach is query_pad), the discrete records go to out (the
+ * caller zeroes its count) exactly as ipcb_dcd_ee / _pt would append them, and
+ * the pairs that can touch within the step are staged in ws; the _solve call
+ * (same arguments, before the hierarchy is refit again) lowers toi by them as
+ * ipcb_edge_edge_toi / _point_triangle_toi would. */
+int ipcb_edge_edge_both(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh, float thickness,
+                        float box_pad, int exclude_same_body, ipcb_contacts* out, void* toi, int* status, void* ws,
+                        size_t ws_bytes, ipcb_stream s);
+int ipcb_edge_edge_solve(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                         int exclude_same_body, void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s);
+int ipcb_point_triangle_both(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh, float thickness,
+                             float query_pad, const int* query_order, int exclude_same_body, ipcb_contacts* out,
+                             void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s);
+int ipcb_point_triangle_solve(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                              const int* query_order, int exclude_same_body, void* toi, int* status, void* ws,
+                              size_t ws_bytes, ipcb_stream s);
 /* The CCD queries restricted to a range of queries, as ipcb_dcd_ee_range /
  * ipcb_dcd_pt_range (EE: Morton ranks of swept_edge_bvh; PT: vertices). */
 int ipcb_edge_edge_toi_range(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* swept_edge_bvh,

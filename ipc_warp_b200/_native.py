@@ -111,6 +111,8 @@ SIGNATURES = {
     "ipcb_lbvh_build_workspace": (c_size_t, [c_int]),
     "ipcb_lbvh_build": (c_int, [BP, P, P, c_int, P, c_size_t, P]),
     "ipcb_lbvh_refit": (c_int, [BP, P, P, P]),
+    "ipcb_lbvh_refit_edges": (c_int, [SP, P, c_float, BP, P]),
+    "ipcb_lbvh_refit_triangles": (c_int, [SP, P, c_float, BP, P]),
     "ipcb_lbvh_build_noalloc_scratch_bytes": (c_size_t, []),
     "ipcb_lbvh_build_noalloc": (c_int, [BP, P, P, c_int, P]),
     "ipcb_pack_positions": (c_int, [SP, P, P]),
@@ -132,6 +134,12 @@ SIGNATURES = {
     "ipcb_toi_workspace": (c_size_t, [c_int]),
     "ipcb_edge_edge_toi": (c_int, [SP, P, BP, P, P, c_int, P, P, P, c_size_t, P]),
     "ipcb_point_triangle_toi": (c_int, [SP, P, BP, c_double, c_int, P, P, P, c_size_t, P]),
+    "ipcb_edge_edge_step": (c_int, [SP, P, c_double, BP, CP, c_int, c_int, c_int, P, P, P, c_size_t, P]),
+    "ipcb_point_triangle_step": (c_int, [SP, P, c_double, BP, P, CP, c_int, c_int, c_int, P, P, P, c_size_t, P]),
+    "ipcb_edge_edge_both": (c_int, [SP, P, c_double, BP, c_float, c_float, c_int, CP, P, P, P, c_size_t, P]),
+    "ipcb_edge_edge_solve": (c_int, [SP, P, c_double, BP, c_int, P, P, P, c_size_t, P]),
+    "ipcb_point_triangle_both": (c_int, [SP, P, c_double, BP, c_float, c_float, P, c_int, CP, P, P, P, c_size_t, P]),
+    "ipcb_point_triangle_solve": (c_int, [SP, P, c_double, BP, P, c_int, P, P, P, c_size_t, P]),
     "ipcb_edge_edge_toi_range": (c_int, [SP, P, BP, P, P, c_int, c_int, c_int, P, P, P, c_size_t, P]),
     "ipcb_point_triangle_toi_range": (c_int, [SP, P, BP, c_double, c_int, c_int, c_int, P, P, P, c_size_t, P]),
     "ipcb_collision_time": (c_int, [c_int, c_int, P, P, P, P, P]),

@@ -152,6 +152,10 @@ class ContactSolverBase:
             self.ccd_triangle_lower = torch.zeros((n_tris, 3), **f32)
             self.ccd_triangle_upper = torch.zeros((n_tris, 3), **f32)
             self.ccd_triangle_bvh = self.tri_mesh
+            # visiting order of the point queries: a warp's 32 vertices are
+            # neighbours on the Morton curve (built once, like the hierarchies)
+            points = self.x4[:, :3].contiguous()
+            self._point_order = Bvh(points, points).sorted.clone()
         self.contacts_new = Contacts(contact_volume, dtype, dev)
         self.contacts_pt = Contacts(contact_volume, dtype, dev)
         self.contacts_list_new = self.contacts_new
@@ -206,6 +210,26 @@ class ContactSolverBase:
             else:
                 self.tri_mesh.refit()
 
+    def _refit_edges(self):
+        """The boxes the edge query reads, from x4 (after _pack)."""
+        N.call("ipcb_lbvh_refit_edges", ctypes.byref(self.soup.c_struct()), N.ptr(self.x4),
+               float(_thickness + buffer), ctypes.byref(self.bvh_edges.c), N.stream_handle())
+
+    def _refit_triangles(self):
+        """The boxes the point-triangle query reads, from x4 (after _pack)."""
+        N.call("ipcb_lbvh_refit_triangles", ctypes.byref(self.soup.c_struct()), N.ptr(self.x4), 0.0,
+               ctypes.byref(self.tri_mesh.c), N.stream_handle())
+
+    def _refit_queries(self):
+        """What the queries need of update_bvh: the packed boxes only (the
+        binary nodes and the box arrays keep update_bvh's last values)."""
+        if getattr(self, "bvh_rebuild_interval", 0):
+            return self.update_bvh()
+        self._pack()
+        self._refit_edges()
+        if self.has_triangles:
+            self._refit_triangles()
+
     # ----------------------------------------------------------------- DCD
     def _grow_contact_list(self, contacts: Contacts, required: int, point_triangle: bool = False):
         """contact.py:523-537: grow to the next power of two."""
@@ -228,8 +252,8 @@ class ContactSolverBase:
         else:
             self.contacts_pt.cnt.zero_()
             N.call("ipcb_dcd_pt", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.tri_mesh.c),
-                   float(_thickness), float(2.0 * (_thickness + buffer)), int(self.disable_self_collision), None,
-                   ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self._status), s)
+                   float(_thickness), float(2.0 * (_thickness + buffer)), int(self.disable_self_collision),
+                   N.ptr(self._point_order), ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self._status), s)
 
     def _read_counts(self):
         """One host read of both list counts and the query status word (kept
@@ -251,7 +275,7 @@ class ContactSolverBase:
         self.compute_V(ret=False)
         self._status.zero_()
         with self.profile_timer("collision BVH refit"):
-            self.update_bvh()
+            self._refit_queries()
         with self.profile_timer("EE collision query"):
             self._launch_dcd("ee")
         if self.has_triangles:
@@ -306,24 +330,65 @@ class ContactSolverBase:
         reset_status is False)."""
         soup = self.soup.c_struct()
         s = N.stream_handle()
-        pad = 1e-7
         N.call("ipcb_add_dx", ctypes.byref(soup), N.ptr(dx), N.ptr(self.ccd_x1), s)
-        N.call("ipcb_swept_edge_aabbs", ctypes.byref(soup), N.ptr(self.ccd_x1), pad, N.ptr(self.ccd_edge_lower),
-               N.ptr(self.ccd_edge_upper), s)
-        self.ccd_edge_bvh.refit(self.ccd_edge_lower, self.ccd_edge_upper)
         self.ccd_toi.fill_(1.0)
         if reset_status:
             self._status.zero_()
-        N.call("ipcb_edge_edge_toi", ctypes.byref(soup), N.ptr(self.ccd_x1), ctypes.byref(self.ccd_edge_bvh.c),
-               N.ptr(self.ccd_edge_lower), N.ptr(self.ccd_edge_upper), int(self.disable_self_collision),
-               N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(self._toi_ws), self._toi_ws.numel(), s)
+        self._ccd_query("ee", 0, self.soup.n_edges, self._toi_ws)
         if self.has_triangles:
-            N.call("ipcb_swept_triangle_aabbs", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   N.ptr(self.ccd_triangle_lower), N.ptr(self.ccd_triangle_upper), s)
-            self.ccd_triangle_bvh.refit(self.ccd_triangle_lower, self.ccd_triangle_upper)
-            N.call("ipcb_point_triangle_toi", ctypes.byref(soup), N.ptr(self.ccd_x1),
-                   ctypes.byref(self.ccd_triangle_bvh.c), pad, int(self.disable_self_collision),
-                   N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(self._toi_ws), self._toi_ws.numel(), s)
+            self._ccd_query("pt", 0, self.soup.n_verts, self._toi_ws)
+
+    def _ccd_query(self, which: str, first: int, count: int, ws: torch.Tensor):
+        """One CCD query of the step x -> ccd_x1 on the current stream: boxes
+        and TOI.  The contact list of the kind is tried first (whatever
+        positions it was found at, its pairs are pairs of the query): the
+        TOI it gives bounds the sweep the query has to look at."""
+        soup = self.soup.c_struct()
+        pad = 1e-7
+        excl = int(self.disable_self_collision)
+        s = N.stream_handle()
+        if which == "ee":
+            N.call("ipcb_edge_edge_step", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
+                   ctypes.byref(self.ccd_edge_bvh.c), ctypes.byref(self.contacts_new.c_struct()), excl, first, count,
+                   N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(ws), ws.numel(), s)
+        else:
+            N.call("ipcb_point_triangle_step", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
+                   ctypes.byref(self.ccd_triangle_bvh.c), N.ptr(self._point_order),
+                   ctypes.byref(self.contacts_pt.c_struct()), excl, first, count, N.ptr(self.ccd_toi),
+                   N.ptr(self._status), N.ptr(ws), ws.numel(), s)
+
+    def _both_queries(self, which: str, ws: torch.Tensor):
+        """The discrete and the CCD query of one kind in one walk of its
+        hierarchy (direction in ccd_x1): records into the contact list, the
+        pairs that can touch within the step into ``ws``."""
+        soup = self.soup.c_struct()
+        pad = 1e-7
+        excl = int(self.disable_self_collision)
+        s = N.stream_handle()
+        if which == "ee":
+            self.contacts_new.cnt.zero_()
+            N.call("ipcb_edge_edge_both", ctypes.byref(soup), N.ptr(self.ccd_x1), pad, ctypes.byref(self.bvh_edges.c),
+                   float(_thickness), float(_thickness + buffer), excl, ctypes.byref(self.contacts_new.c_struct()),
+                   N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(ws), ws.numel(), s)
+        else:
+            self.contacts_pt.cnt.zero_()
+            N.call("ipcb_point_triangle_both", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
+                   ctypes.byref(self.tri_mesh.c), float(_thickness), float(2.0 * (_thickness + buffer)),
+                   N.ptr(self._point_order), excl, ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self.ccd_toi),
+                   N.ptr(self._status), N.ptr(ws), ws.numel(), s)
+
+    def _solve_staged(self, which: str, ws: torch.Tensor):
+        """The TOI of the pairs _both_queries staged."""
+        soup = self.soup.c_struct()
+        pad = 1e-7
+        excl = int(self.disable_self_collision)
+        tail = (excl, N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(ws), ws.numel(), N.stream_handle())
+        if which == "ee":
+            N.call("ipcb_edge_edge_solve", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
+                   ctypes.byref(self.ccd_edge_bvh.c), *tail)
+        else:
+            N.call("ipcb_point_triangle_solve", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
+                   ctypes.byref(self.ccd_triangle_bvh.c), N.ptr(self._point_order), *tail)
 
     def new_intersections(self, x0: torch.Tensor, x1: torch.Tensor) -> float:
         """contact.py:587-670 (the augmented-Lagrangian solver's CCD): every

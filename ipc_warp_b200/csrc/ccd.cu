@@ -3,13 +3,14 @@
 // in double.  This file is compiled with -fmad=false: every operation rounds
 // on its own, in source order, so the TOI is reproducible bit for bit by a
 // plain IEEE evaluation.
-#include <cooperative_groups.h>
+#include <type_traits>
 
 #include "bodies.cuh"
 #include "common.cuh"
+#include "geom.cuh"
 #include "lbvh.cuh"
-
-namespace cg = cooperative_groups;
+#include "records.cuh"
+#include "tree.cuh"
 
 namespace ipcb {
 int check_launch(const char* where);
@@ -486,7 +487,7 @@ IPCB_D double pt_pair_time(const S* __restrict__ x0, const S* __restrict__ x1, i
   return collision_time<1>(p0, p1, st);
 }
 
-constexpr int kQueue = 32;  // per-thread queue of filtered leaf hits
+constexpr int kQueue = 32;  // per-thread queue of filtered leaf hits (fixed bodies)
 
 IPCB_D int warp_max(int v) {
 #pragma unroll
@@ -510,142 +511,463 @@ IPCB_D bool push_converged(const CandList& L, bool has, int a, int b) {
   return !has;
 }
 
-// Traversal applies the cheap filters and queues leaves; the warp then pushes
-// the queued pairs converged (divergent pushes would serialise on the count).
-// FAST: stage pairs only (a lane whose queue is full pushes on its own); a
-// pair that does not fit in the list raises cand.overflow instead of being
-// solved here, which keeps the cubic solver out of this kernel (56 instead of
-// 255 registers).  !FAST (run only when *gate is set, with a zero-capacity
-// list): every pair solved in place.
-template <class S, bool FAST>
-__global__ void __launch_bounds__(128) k_ee_collect(const S* __restrict__ x0, const S* __restrict__ x1,
-                                                    const int* __restrict__ edges, const int* __restrict__ body,
-                                                    const float4* __restrict__ nodes, const int* __restrict__ order,
-                                                    int n, int first, int count, const float* __restrict__ lo,
-                                                    const float* __restrict__ hi, int exclude, CandList cand, S* toi,
-                                                    int* status, Sink sink, const int* gate) {
-  if (gate && *gate == 0) return;
-  bool dropped = false;
-  // queries: the edges of Morton rank first .. first + count - 1
-  int t = first + blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = t < first + count;
-  int i = active ? __ldg(order + t) : 0;
-  int2 ea = __ldg(reinterpret_cast<const int2*>(edges) + i);
-  int bi = exclude ? __ldg(body + ea.x) : 0;
-  int st = 0;
-  int q[kQueue];
-  int nq = 0;
-  if (active) {
-    f3 qlo = mk3(__ldg(lo + 3 * i), __ldg(lo + 3 * i + 1), __ldg(lo + 3 * i + 2));
-    f3 qhi = mk3(__ldg(hi + 3 * i), __ldg(hi + 3 * i + 1), __ldg(hi + 3 * i + 2));
-    // thread t queries the edge of Morton rank t in its own hierarchy: only
-    // leaves of higher rank are visited, so each pair is met once; it is then
-    // taken as the reference's (lower id, higher id) pair
-    bool ok = traverse4_after(nodes, n, t, qlo, qhi, [&](int j, int) {
-      int2 eb = __ldg(reinterpret_cast<const int2*>(edges) + j);
-      if (ea.x == eb.x || ea.x == eb.y || ea.y == eb.x || ea.y == eb.y) return;
-      if (exclude && bi == __ldg(body + eb.x)) return;
-      if (nq < kQueue) {
-        q[nq++] = j;
-      } else if (FAST) {  // lane queue full: stage this pair directly
-        const int slot = atomicAdd(cand.count, 1);
-        if (slot < cand.capacity) cand.pairs[slot] = make_int2(min(i, j), max(i, j));
-        else dropped = true;
-      } else {
-        const bool fwd = i < j;
-        const int2 e_lo = fwd ? ea : eb, e_hi = fwd ? eb : ea;
-        double tt = ee_pair_time(x0, x1, e_lo, e_hi, st);
-        if (tt < 1.0) {
-          store_toi(toi, tt);
-          sink_append<S>(sink, make_int4(e_lo.x, e_lo.y, e_hi.x, e_hi.y), min(i, j), max(i, j), tt);
-        }
-      }
-    });
-    if (!ok) st |= IPCB_STATUS_STACK;
+// Swept boxes over [0, t_end] of the step (tree.cuh functor): over the whole
+// step (t_end null or 1) exactly k_swept's.  Only the minimum TOI matters to a
+// query without a sink, and a pair whose root is below the TOI stored so far
+// is within the touch margin (see touch_time_bound) by that time, so boxes
+// over [0, stored TOI] grown by that margin still meet for every pair that can
+// lower it: the result is the same minimum, from far fewer pairs when the
+// step is much longer than the first contact.
+template <class S, int NV>
+IPCB_D void swept_box(const S* __restrict__ x0, const S* __restrict__ x1, const int* ids, double pad, double t, f3& lo,
+                      f3& hi) {
+  double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const d3 a = ld(x0, ids[v]);
+    d3 b = ld(x1, ids[v]);
+    if (t < 1.0) b = a + (b - a) * t;
+    mn[0] = dmin(mn[0], dmin(a.x, b.x)); mx[0] = dmax(mx[0], dmax(a.x, b.x));
+    mn[1] = dmin(mn[1], dmin(a.y, b.y)); mx[1] = dmax(mx[1], dmax(a.y, b.y));
+    mn[2] = dmin(mn[2], dmin(a.z, b.z)); mx[2] = dmax(mx[2], dmax(a.z, b.z));
   }
-  int rounds = warp_max(nq);
-  for (int k = 0; k < rounds; ++k) {
-    bool has = k < nq;
-    int j = has ? q[k] : 0;
-    if (!push_converged(cand, has, min(i, j), max(i, j))) {
-      if (FAST) {
-        dropped = true;
-        continue;
-      }
-      int2 eb = __ldg(reinterpret_cast<const int2*>(edges) + j);
-      const bool fwd = i < j;
-      const int2 e_lo = fwd ? ea : eb, e_hi = fwd ? eb : ea;
-      double tt = ee_pair_time(x0, x1, e_lo, e_hi, st);
-      if (tt < 1.0) {
-        store_toi(toi, tt);
-        sink_append<S>(sink, make_int4(e_lo.x, e_lo.y, e_hi.x, e_hi.y), min(i, j), max(i, j), tt);
-      }
-    }
+  if (t < 1.0) {
+    double ext = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) ext = dmax(ext, dmax(fabs(mn[k]), fabs(mx[k])));
+    pad += 1e-6 * (1.0 + ext);
   }
-  if (dropped) *cand.overflow = 1;
-  if (st) atomicOr(status, st);
+  lo = mk3(__double2float_rd(mn[0] - pad), __double2float_rd(mn[1] - pad), __double2float_rd(mn[2] - pad));
+  hi = mk3(__double2float_ru(mx[0] + pad), __double2float_ru(mx[1] + pad), __double2float_ru(mx[2] + pad));
 }
 
-template <class S, bool FAST>
-__global__ void __launch_bounds__(128) k_pt_collect(const S* __restrict__ x0, const S* __restrict__ x1,
-                                                    const int* __restrict__ tris, const int* __restrict__ body,
-                                                    const float4* __restrict__ nodes, int n_tris, int first, int count,
-                                                    double pad, int exclude, CandList cand, S* toi, int* status,
-                                                    Sink sink, const int* gate) {
-  if (gate && *gate == 0) return;
-  bool dropped = false;
-  // queries: the vertices first .. first + count - 1
-  int i0 = first + blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = i0 < first + count;
-  int i = active ? i0 : 0;
-  d3 a = ld(x0, i), b = ld(x1, i);
-  int bi = exclude ? __ldg(body + i) : 0;
-  int st = 0;
-  int q[kQueue];
-  int nq = 0;
-  if (active) {
-    f3 qlo = mk3(__double2float_rd(dmin(a.x, b.x) - pad), __double2float_rd(dmin(a.y, b.y) - pad),
-                 __double2float_rd(dmin(a.z, b.z) - pad));
-    f3 qhi = mk3(__double2float_ru(dmax(a.x, b.x) + pad), __double2float_ru(dmax(a.y, b.y) + pad),
-                 __double2float_ru(dmax(a.z, b.z) + pad));
-    bool ok = traverse4(nodes, n_tris, qlo, qhi, [&](int j) {
-      int3 tj = make_int3(__ldg(tris + 3 * j), __ldg(tris + 3 * j + 1), __ldg(tris + 3 * j + 2));
-      if (i == tj.x || i == tj.y || i == tj.z) return;
-      if (exclude && bi == __ldg(body + tj.x)) return;
-      if (nq < kQueue) {
-        q[nq++] = j;
-      } else if (FAST) {  // lane queue full: stage this pair directly
-        const int slot = atomicAdd(cand.count, 1);
-        if (slot < cand.capacity) cand.pairs[slot] = make_int2(i, j);
-        else dropped = true;
-      } else {
-        double tt = pt_pair_time(x0, x1, i, tj, st);
-        if (tt < 1.0) {
-          store_toi(toi, tt);
-          sink_append<S>(sink, make_int4(i, tj.x, tj.y, tj.z), i, j, tt);
-        }
-      }
-    });
-    if (!ok) st |= IPCB_STATUS_STACK;
+IPCB_D double current_toi(const float* toi) { return (double)__ldcg(toi); }
+IPCB_D double current_toi(const double* toi) { return __ldcg(toi); }
+
+template <class S, int NV>
+struct SweptBox {
+  const S* x0;
+  const S* x1;
+  const int* prims;
+  double pad;
+  const S* t_end;
+  IPCB_D void operator()(int p, f3& lo, f3& hi) const {
+    int ids[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) ids[k] = __ldg(prims + NV * p + k);
+    swept_box<S, NV>(x0, x1, ids, pad, t_end ? current_toi(t_end) : 1.0, lo, hi);
   }
-  int rounds = warp_max(nq);
-  for (int k = 0; k < rounds; ++k) {
-    bool has = k < nq;
-    int j = has ? q[k] : 0;
-    if (!push_converged(cand, has, i, j)) {
-      if (FAST) {
-        dropped = true;
-        continue;
-      }
-      int3 tj = make_int3(__ldg(tris + 3 * j), __ldg(tris + 3 * j + 1), __ldg(tris + 3 * j + 2));
-      double tt = pt_pair_time(x0, x1, i, tj, st);
-      if (tt < 1.0) {
-        store_toi(toi, tt);
-        sink_append<S>(sink, make_int4(i, tj.x, tj.y, tj.z), i, j, tt);
-      }
+};
+
+// The swept box of the whole step joined with the discrete query's box (x in
+// float, padded by reach): one tree for both queries.
+template <class S, int NV>
+struct BothBox {
+  const S* x0;
+  const S* x1;
+  const int* prims;
+  double pad;
+  float reach;
+  IPCB_D void operator()(int p, f3& lo, f3& hi) const {
+    int ids[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) ids[k] = __ldg(prims + NV * p + k);
+    swept_box<S, NV>(x0, x1, ids, pad, 1.0, lo, hi);
+    f3 a = to_f(load3(x0, ids[0])), b = a;
+#pragma unroll
+    for (int k = 1; k < NV; ++k) {
+      const f3 q = to_f(load3(x0, ids[k]));
+      a = mk3(fminf(a.x, q.x), fminf(a.y, q.y), fminf(a.z, q.z));
+      b = mk3(fmaxf(b.x, q.x), fmaxf(b.y, q.y), fmaxf(b.z, q.z));
+    }
+    lo = mk3(fminf(lo.x, a.x - reach), fminf(lo.y, a.y - reach), fminf(lo.z, a.z - reach));
+    hi = mk3(fmaxf(hi.x, b.x + reach), fmaxf(hi.y, b.y + reach), fmaxf(hi.z, b.z + reach));
+  }
+};
+
+// ---- ordered candidate solve (no record sink): the collect pass computes
+// each pair's touch-time bound, drops the pairs that cannot touch within the
+// step or before the TOI stored so far, and counts the rest in 32 buckets over
+// [0, 1]; the solve then takes the pairs in bucket order, so the pairs that
+// can touch earliest set the TOI first, and a pair whose bound is at or above
+// the TOI stored so far is skipped (it cannot lower the minimum: the result is
+// the same minimum, bit for bit); a warp that meets a bucket starting at or
+// above the stored TOI stops.  Divergence between pruned and solved pairs and
+// the cubic solver's registers stay out of the collect pass.
+constexpr int kBuckets = 32;
+struct CandOrder {
+  int* bcount;   // pairs per bucket
+  int* bcursor;  // fill cursors
+  int* work;     // next position of the ordered solve
+  float* tlb;    // per staged pair: touch-time bound rounded down
+  int* order;    // staged pair indices in bucket order
+};
+
+IPCB_D int bucket_of(float tl) { return min(kBuckets - 1, (int)(tl * (float)kBuckets)); }
+
+template <int KIND>
+IPCB_D int4 pair_ids(const int* __restrict__ prims, int2 pr) {
+  if (KIND == 0) {
+    const int2 ea = __ldg(reinterpret_cast<const int2*>(prims) + pr.x);
+    const int2 eb = __ldg(reinterpret_cast<const int2*>(prims) + pr.y);
+    return make_int4(ea.x, ea.y, eb.x, eb.y);
+  }
+  return make_int4(pr.x, __ldg(prims + 3 * pr.y), __ldg(prims + 3 * pr.y + 1), __ldg(prims + 3 * pr.y + 2));
+}
+
+// Lower bound on the time at which a pair can touch, in float: the distance
+// along the axis n of the closest points at t = 0 (r = closest point of a -
+// closest point of b, d = |r|).  n . (a_i - b_j) is linear in t for every
+// vertex pair, and as long as all of them exceed the margin n separates the
+// primitives by it: the earliest time one falls to the margin is the bound (a
+// verified root needs the primitives within 1e-6 (1 + extent), see
+// touch_time_bound).  Only the closing speed along n counts, where the
+// distance-over-speed bound charges sliding motion too: a loaded thread flank
+// sliding 8e-3 at a gap of 2e-5 keeps a bound near its true touch time.  The
+// margin covers the float rounding of the (locally formed) dots, and for
+// double positions their rounding to float.
+template <class S, int KIND>
+IPCB_D float touch_bound(const f3* p, const f3* v, f3 r, float d) {
+  if (!(d > 0.f)) return 0.f;
+  const float q = 1.0f / d;
+  const f3 n = mk3(r.x * q, r.y * q, r.z * q);
+  constexpr int NA = KIND == 0 ? 2 : 1;
+  float s[4], w[4], size = 0.f, ext = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const f3 l = mk3(p[k].x - p[0].x, p[k].y - p[0].y, p[k].z - p[0].z);
+    s[k] = fmaf(n.x, l.x, fmaf(n.y, l.y, n.z * l.z));
+    w[k] = fmaf(n.x, v[k].x, fmaf(n.y, v[k].y, n.z * v[k].z));
+    const float av = fabsf(v[k].x) + fabsf(v[k].y) + fabsf(v[k].z);
+    size += fabsf(l.x) + fabsf(l.y) + fabsf(l.z) + av;
+    ext = fmaxf(ext, fmaxf(fabsf(p[k].x), fmaxf(fabsf(p[k].y), fabsf(p[k].z))) + av);
+  }
+  const float margin = 1.05e-6f * (1.0f + ext) + 1e-6f * size + (sizeof(S) == 8 ? 5e-7f * ext : 0.f);
+  float t = 4.0f;
+#pragma unroll
+  for (int i = 0; i < NA; ++i)
+#pragma unroll
+    for (int j = NA; j < 4; ++j) {
+      const float c = s[i] - s[j] - margin, u = w[j] - w[i];
+      if (!(c > 0.f)) t = 0.f;
+      else if (u > 0.f) t = fminf(t, c / u);
+    }
+  return t * 0.9999f;
+}
+
+// Closest points at t = 0 (the discrete predicate's float operations): their
+// distance, and the difference r.
+template <int KIND>
+IPCB_D float closest_difference(const f3* p, f3& r) {
+  if (KIND == 0) {
+    const CPEE c = closest_point_edge_edge(p[0], p[1], p[2], p[3], 1.0e-6f);
+    r = (p[0] - p[2]) + (p[1] - p[0]) * c.s - (p[3] - p[2]) * c.t;
+    return c.d;
+  }
+  const CPT c = closest_point_triangle(p[0], p[1], p[2], p[3]);
+  r = (p[0] - p[1]) - (p[2] - p[1]) * c.v - (p[3] - p[1]) * (1.0f - c.u - c.v);
+  return c.d;
+}
+
+// Whether the boxes of the whole step (k_swept's) meet: the query's own test,
+// applied to the few pairs that are solved (the tree's boxes may be larger).
+template <class S, int KIND>
+IPCB_D bool swept_boxes_meet(const S* __restrict__ x0, const S* __restrict__ x1, int4 ids, double pad) {
+  const int v[4] = {ids.x, ids.y, ids.z, ids.w};
+  constexpr int NA = KIND == 0 ? 2 : 1;
+  f3 alo, ahi, blo, bhi;
+  swept_box<S, NA>(x0, x1, v, pad, 1.0, alo, ahi);
+  swept_box<S, 4 - NA>(x0, x1, v + NA, pad, 1.0, blo, bhi);
+  return alo.x <= bhi.x && blo.x <= ahi.x && alo.y <= bhi.y && blo.y <= ahi.y && alo.z <= bhi.z && blo.z <= ahi.z;
+}
+
+template <class S>
+IPCB_D void load_motion(const S* __restrict__ x0, const S* __restrict__ x1, int i, f3& p, f3& v) {
+  const d3 a = ld(x0, i), b = ld(x1, i);
+  p = mk3((float)a.x, (float)a.y, (float)a.z);
+  v = mk3((float)(b.x - a.x), (float)(b.y - a.y), (float)(b.z - a.z));
+}
+IPCB_D void load_motion(const float* __restrict__ x0, const float* __restrict__ x1, int i, f3& p, f3& v) {
+  p = load3(x0, i);
+  const f3 b = load3(x1, i);
+  v = mk3(b.x - p.x, b.y - p.y, b.z - p.z);
+}
+
+// What a query does with its pairs.
+enum Mode {
+  kStage,   // CCD: stage the pairs that can lower the TOI
+  kInline,  // CCD: solve them in place (the staging list overflowed)
+  kBoth     // the discrete test and record, and CCD staging
+};
+
+// One queued pair a lane (has), converged over the warp: the closest points
+// (the discrete predicate's exact float operations, so kBoth appends what the
+// discrete query appends), the touch bound along their axis, and the pair is
+// staged or solved.
+template <class S, int KIND, int MODE>
+IPCB_D void take_pairs(const S* __restrict__ x0, const S* __restrict__ x1, const int* __restrict__ prims, bool has,
+                       int2 pr, double pad, float l0f, S l0, const ipcb_contacts& out, const CandList& cand,
+                       const CandOrder& o, int* hist, S* toi, const Sink& sink, int& st) {
+  const unsigned lane = threadIdx.x & 31;
+  bool want = false, accept = false;
+  float tl = 4.0f;
+  int4 ids = make_int4(0, 0, 0, 0);
+  if (has) {
+    ids = pair_ids<KIND>(prims, pr);
+    f3 p[4], v[4], r;
+    load_motion(x0, x1, ids.x, p[0], v[0]);
+    load_motion(x0, x1, ids.y, p[1], v[1]);
+    load_motion(x0, x1, ids.z, p[2], v[2]);
+    load_motion(x0, x1, ids.w, p[3], v[3]);
+    const float d = closest_difference<KIND>(p, r);
+    if (MODE == kBoth) accept = d < l0f;
+    tl = touch_bound<S, KIND>(p, v, r, sqrtf(dot(r, r)));
+    // cannot touch within the step, or (only the minimum wanted) cannot lower it
+    want = tl <= 1.0f && (sink.on || (double)tl < current_toi(toi));
+  }
+  if (MODE == kBoth) {
+    const int slot = warp_reserve(out.cnt, accept);
+    if (accept) {
+      if (KIND == 0) write_record<S>(out, slot, ids.x, ids.y, ids.z, ids.w, pr.x, pr.y, l0);
+      else write_record<S>(out, slot, ids.x, ids.z, ids.y, ids.w, pr.x, pr.y, l0);  // (p, tri[1], tri[0], tri[2])
     }
   }
-  if (dropped) *cand.overflow = 1;
+  if (MODE == kInline) {
+    if (want && (pad < 0.0 || swept_boxes_meet<S, KIND>(x0, x1, ids, pad))) {
+      const d3 p0[4] = {ld(x0, ids.x), ld(x0, ids.y), ld(x0, ids.z), ld(x0, ids.w)};
+      const d3 p1[4] = {ld(x1, ids.x), ld(x1, ids.y), ld(x1, ids.z), ld(x1, ids.w)};
+      const double tt = collision_time<KIND>(p0, p1, st);
+      if (tt < 1.0) {
+        store_toi(toi, tt);
+        sink_append<S>(sink, ids, pr.x, pr.y, tt);
+      }
+    }
+    return;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  if (!m) return;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(cand.count, __popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (want) {
+    const int slot = base + __popc(m & ((1u << lane) - 1u));
+    if (slot < cand.capacity) {
+      cand.pairs[slot] = pr;
+      o.tlb[slot] = tl;
+      atomicAdd(hist + bucket_of(tl), 1);
+    } else {
+      *cand.overflow = 1;  // the inline pass redoes the query
+    }
+  }
+}
+
+// The CCD edge-edge query over the packed tree of swept boxes: a warp per
+// block of 32 edges in Morton order (tree.cuh); pairs that survive the box and
+// topology tests are bounded on full warps and staged.  kInline (run only when
+// *gate is set: the staging list overflowed) solves every pair in place.
+// lo / hi: the queries' boxes, or null for the tree's own leaf boxes.
+// 64 registers (8 blocks a SM; 96 unbounded): the walk issues about 5,000
+// instructions a block in short dependent runs, and the spills (72 B, around
+// the flush) cost less than the missing warps (screw and nut iteration 1.59 ->
+// 1.45 ms, from 3.37 with a traversal per thread).
+template <class S, int MODE>
+__global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_ee_collect(
+    const S* __restrict__ x0, const S* __restrict__ x1, const int* __restrict__ edges, const int* __restrict__ body,
+    const __grid_constant__ tree::View v, const int* __restrict__ order, int first, int count, int nsub, int items,
+    const float* __restrict__ lo, const float* __restrict__ hi, double pad, int exclude, float thickness,
+    ipcb_contacts out, CandList cand, CandOrder o, S* toi, int* status, Sink sink, const int* gate) {
+  __shared__ tree::Block blocks[tree::kWarps];
+  __shared__ int hist[kBuckets];
+  if (MODE == kInline && *gate == 0) return;
+  if (threadIdx.x < kBuckets) hist[threadIdx.x] = 0;
+  __syncthreads();
+  tree::Block& B = blocks[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const float l0f = xmul(thickness, 2.0f);
+  const S l0 = S(thickness) * S(2.0);
+  int st = 0;
+  for (int item = blockIdx.x * tree::kWarps + (threadIdx.x >> 5); item < items; item += gridDim.x * tree::kWarps) {
+    const int qb = (first >> 5) + item / nsub, sub = item % nsub;
+    const int t = qb * 32 + lane;
+    // queries: the edges of Morton rank first .. first + count - 1
+    const bool active = t >= first && t < first + count;
+    const int i = active ? __ldg(order + t) : 0;
+    const int2 ea = __ldg(reinterpret_cast<const int2*>(edges) + i);
+    f3 qlo = mk3(tree::kBig, tree::kBig, tree::kBig), qhi = mk3(-tree::kBig, -tree::kBig, -tree::kBig);
+    if (active) {
+      if (lo) {
+        qlo = mk3(__ldg(lo + 3 * i), __ldg(lo + 3 * i + 1), __ldg(lo + 3 * i + 2));
+        qhi = mk3(__ldg(hi + 3 * i), __ldg(hi + 3 * i + 1), __ldg(hi + 3 * i + 2));
+      } else {
+        const float4 l = __ldg(v.lv[0] + 2 * (size_t)t), h = __ldg(v.lv[0] + 2 * (size_t)t + 1);
+        qlo = mk3(l.x, l.y, l.z);
+        qhi = mk3(h.x, h.y, h.z);
+      }
+    }
+    const int bi = exclude ? __ldg(body + ea.x) : 0;
+    __syncwarp();
+    B.qlo[lane] = make_float4(qlo.x, qlo.y, qlo.z, __int_as_float(i));
+    B.qhi[lane] = make_float4(qhi.x, qhi.y, qhi.z, __int_as_float(bi));
+    B.ev[lane] = ea;
+    __syncwarp();
+      int nq = 0;
+    auto flush = [&](int n) {
+      const bool has = lane < n;
+      const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);
+      const int a = __float_as_int(B.qlo[pr.x].w);
+      // the reference's (lower id, higher id) pair
+      take_pairs<S, 0, MODE>(x0, x1, edges, has, make_int2(min(a, pr.y), max(a, pr.y)), pad, l0f, l0, out, cand, o,
+                             hist, toi, sink, st);
+    };
+    tree::for_segments(active, qlo, qhi, [&](bool in, f3 glo, f3 ghi) {
+    tree::for_block_pairs<true>(v, glo, ghi, qb, sub, nsub, B.stack, [&](int tb) {
+      tree::block_pair<true>(
+          v, B, qb, tb, in, qlo, qhi, glo, ghi, nq,
+          [&](int j) {
+            int3 e = make_int3(-1, -1, 0);
+            if (j >= 0) {
+              const int2 w = __ldg(reinterpret_cast<const int2*>(edges) + j);
+              e = make_int3(w.x, w.y, exclude ? __ldg(body + w.x) : 0);
+            }
+            return e;
+          },
+          [&](int q, int3 e) {
+            const int2 w = B.ev[q];
+            if (w.x == e.x || w.x == e.y || w.y == e.x || w.y == e.y) return false;
+            return !(exclude && __float_as_int(B.qhi[q].w) == e.z);
+          },
+          flush);
+    });
+    });
+    __syncwarp();
+    if (nq) flush(nq);
+  }
+  if (st) atomicOr(status, st);
+  if (MODE == kInline) return;
+  __syncthreads();
+  if (threadIdx.x < kBuckets && hist[threadIdx.x]) atomicAdd(o.bcount + threadIdx.x, hist[threadIdx.x]);
+}
+
+// The CCD point-triangle query: blocks of 32 vertices of the visiting order.
+template <class S, int MODE>
+__global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_pt_collect(
+    const S* __restrict__ x0, const S* __restrict__ x1, const int* __restrict__ tris, const int* __restrict__ body,
+    const __grid_constant__ tree::View v, const int* __restrict__ order, int first, int count, int nsub, int items,
+    double pad, float qpad, int exclude, float thickness, ipcb_contacts out, CandList cand, CandOrder o, S* toi,
+    int* status, Sink sink, const int* gate) {
+  __shared__ tree::Block blocks[tree::kWarps];
+  __shared__ int hist[kBuckets];
+  if (MODE == kInline && *gate == 0) return;
+  if (threadIdx.x < kBuckets) hist[threadIdx.x] = 0;
+  __syncthreads();
+  tree::Block& B = blocks[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const float l0f = xmul(thickness, 2.0f);
+  const S l0 = S(thickness) * S(2.0);
+  int st = 0;
+  // boxes up to the TOI stored so far (see swept_box)
+  const double t_end = sink.on ? 1.0 : dmin(1.0, current_toi(toi));
+  for (int item = blockIdx.x * tree::kWarps + (threadIdx.x >> 5); item < items; item += gridDim.x * tree::kWarps) {
+    const int sub = item % nsub;
+    // queries: the vertices first .. first + count - 1 of the visiting order
+    const int t = (item / nsub) * 32 + lane;
+    const bool active = t < count;
+    const int i = active ? (order ? __ldg(order + first + t) : first + t) : 0;
+    f3 qlo = mk3(tree::kBig, tree::kBig, tree::kBig), qhi = mk3(-tree::kBig, -tree::kBig, -tree::kBig);
+    if (active) {
+      swept_box<S, 1>(x0, x1, &i, pad, t_end, qlo, qhi);
+      if (MODE == kBoth) {  // and the discrete query's box
+        const f3 p = to_f(load3(x0, i));
+        qlo = mk3(fminf(qlo.x, p.x - qpad), fminf(qlo.y, p.y - qpad), fminf(qlo.z, p.z - qpad));
+        qhi = mk3(fmaxf(qhi.x, p.x + qpad), fmaxf(qhi.y, p.y + qpad), fmaxf(qhi.z, p.z + qpad));
+      }
+    }
+    const int bi = exclude ? __ldg(body + i) : 0;
+    __syncwarp();
+    B.qlo[lane] = make_float4(qlo.x, qlo.y, qlo.z, __int_as_float(i));
+    B.qhi[lane] = make_float4(qhi.x, qhi.y, qhi.z, __int_as_float(bi));
+    __syncwarp();
+      int nq = 0;
+    auto flush = [&](int n) {
+      const bool has = lane < n;
+      const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);
+      const int a = __float_as_int(B.qlo[pr.x].w);
+      take_pairs<S, 1, MODE>(x0, x1, tris, has, make_int2(a, pr.y), pad, l0f, l0, out, cand, o, hist, toi, sink, st);
+    };
+    tree::for_segments(active, qlo, qhi, [&](bool in, f3 glo, f3 ghi) {
+    tree::for_block_pairs<false>(v, glo, ghi, 0, sub, nsub, B.stack, [&](int tb) {
+      tree::block_pair<false>(
+          v, B, 0, tb, in, qlo, qhi, glo, ghi, nq,
+          [&](int j) {
+            int4 e = make_int4(-1, -1, -1, 0);
+            if (j >= 0) {
+              e = make_int4(__ldg(tris + 3 * j), __ldg(tris + 3 * j + 1), __ldg(tris + 3 * j + 2), 0);
+              if (exclude) e.w = __ldg(body + e.x);
+            }
+            return e;
+          },
+          [&](int q, int4 e) {
+            const int a = __float_as_int(B.qlo[q].w);
+            if (a == e.x || a == e.y || a == e.z) return false;
+            return !(exclude && __float_as_int(B.qhi[q].w) == e.w);
+          },
+          flush);
+    });
+    });
+    __syncwarp();
+    if (nq) flush(nq);
+  }
+  if (st) atomicOr(status, st);
+  if (MODE == kInline) return;
+  __syncthreads();
+  if (threadIdx.x < kBuckets && hist[threadIdx.x]) atomicAdd(o.bcount + threadIdx.x, hist[threadIdx.x]);
+}
+
+// An early upper bound on the TOI: pairs of a contact list (the discrete
+// query's) that the CCD query would meet too -- the same filters, and boxes
+// over the whole step that overlap -- are solved before the boxes are formed.
+// Each lane takes up to kSeedPairs spread over the list and solves the one
+// with the smallest touch-time bound.  Every solved pair is one of the
+// query's, so the minimum is unchanged; the list may be of any age.
+constexpr int kSeedPairs = 4, kSeedLanes = 8192;
+
+template <class S, int KIND>
+__global__ void __launch_bounds__(64) k_seed(const S* __restrict__ x0, const S* __restrict__ x1,
+                                             const int* __restrict__ prims, const int* __restrict__ body, int n_a,
+                                             int n_b, int exclude, double pad, ipcb_contacts list, S* toi,
+                                             int* status) {
+  const int n = min(*list.cnt, list.capacity);
+  const int m = min(n, kSeedPairs * kSeedLanes);
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  float best = 2.0f;
+  int4 ids = make_int4(0, 0, 0, 0);
+  for (int q = 0; q < kSeedPairs; ++q) {
+    const int k = q * kSeedLanes + g;
+    if (k >= m) break;
+    int2 pr = reinterpret_cast<const int2*>(list.e0e1)[(long long)k * n / m];
+    if (KIND == 0) pr = make_int2(min(pr.x, pr.y), max(pr.x, pr.y));
+    if (pr.x < 0 || pr.y < 0 || pr.x >= n_a || pr.y >= n_b) continue;
+    const int4 w = pair_ids<KIND>(prims, pr);
+    if (w.x == w.z || w.x == w.w || (KIND == 0 ? (w.y == w.z || w.y == w.w) : w.x == w.y)) continue;
+    if (exclude && __ldg(body + w.x) == __ldg(body + (KIND == 0 ? w.z : w.y))) continue;
+    f3 p[4], v[4], r;
+    load_motion(x0, x1, w.x, p[0], v[0]);
+    load_motion(x0, x1, w.y, p[1], v[1]);
+    load_motion(x0, x1, w.z, p[2], v[2]);
+    load_motion(x0, x1, w.w, p[3], v[3]);
+    closest_difference<KIND>(p, r);
+    const float tl = touch_bound<S, KIND>(p, v, r, sqrtf(dot(r, r)));
+    if (tl < best) {
+      best = tl;
+      ids = w;
+    }
+  }
+  if (!(best <= 1.0f) || (double)best >= current_toi(toi) || !swept_boxes_meet<S, KIND>(x0, x1, ids, pad)) return;
+  const d3 p0[4] = {ld(x0, ids.x), ld(x0, ids.y), ld(x0, ids.z), ld(x0, ids.w)};
+  const d3 p1[4] = {ld(x1, ids.x), ld(x1, ids.y), ld(x1, ids.z), ld(x1, ids.w)};
+  int st = 0;
+  const double tt = collision_time<KIND>(p0, p1, st);
+  if (tt < 1.0) store_toi(toi, tt);
   if (st) atomicOr(status, st);
 }
 
@@ -655,9 +977,6 @@ __global__ void __launch_bounds__(128) k_pt_collect(const S* __restrict__ x0, co
 // (re-read from L2 for every pair; it only decreases) cannot lower it, so its
 // cubic is not solved -- the result is the same minimum, bit for bit.  With
 // a sink every pair that can touch within the step is solved.
-IPCB_D double current_toi(float* toi) { return (double)__ldcg(toi); }
-IPCB_D double current_toi(double* toi) { return __ldcg(toi); }
-
 template <class S, int KIND>
 __global__ void __launch_bounds__(128) k_cand_toi(const S* __restrict__ x0, const S* __restrict__ x1,
                                                   const int* __restrict__ prims, CandList cand, S* toi,
@@ -667,14 +986,7 @@ __global__ void __launch_bounds__(128) k_cand_toi(const S* __restrict__ x0, cons
   int st = 0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     const int2 pr = cand.pairs[k];
-    int4 ids;
-    if (KIND == 0) {
-      const int2 ea = __ldg(reinterpret_cast<const int2*>(prims) + pr.x);
-      const int2 eb = __ldg(reinterpret_cast<const int2*>(prims) + pr.y);
-      ids = make_int4(ea.x, ea.y, eb.x, eb.y);
-    } else {
-      ids = make_int4(pr.x, __ldg(prims + 3 * pr.y), __ldg(prims + 3 * pr.y + 1), __ldg(prims + 3 * pr.y + 2));
-    }
+    const int4 ids = pair_ids<KIND>(prims, pr);
     d3 p0[4] = {ld(x0, ids.x), ld(x0, ids.y), ld(x0, ids.z), ld(x0, ids.w)};
     d3 p1[4] = {ld(x1, ids.x), ld(x1, ids.y), ld(x1, ids.z), ld(x1, ids.w)};
     const double lb = touch_time_bound<KIND>(p0, p1);
@@ -689,95 +1001,37 @@ __global__ void __launch_bounds__(128) k_cand_toi(const S* __restrict__ x0, cons
   if (st) atomicOr(status, st);
 }
 
-// ---- ordered candidate solve (no record sink): the staged pairs' touch-time
-// bounds are computed first by a light kernel and the pairs bucketed by them
-// (32 buckets over [0, 1]; a pair that cannot touch within the step is
-// dropped); the solve then takes the pairs in bucket order, so the pairs that
-// can touch earliest set the TOI first, and a pair whose bound is at or above
-// the TOI stored so far is skipped (it cannot lower the minimum: the result is
-// the same minimum, bit for bit); a warp that meets a bucket starting at or
-// above the stored TOI stops.  Divergence between pruned and solved pairs and
-// the cubic solver's registers stay out of the bound pass.
-constexpr int kBuckets = 32;
-struct CandOrder {
-  int* bcount;   // pairs per bucket
-  int* bcursor;  // fill cursors
-  int* work;     // next position of the ordered solve
-  float* tlb;    // per staged pair: touch-time bound rounded down, or 2 (cannot touch)
-  int* order;    // staged pair indices in bucket order
-};
-
-IPCB_D int bucket_of(float tl) { return min(kBuckets - 1, (int)(tl * (float)kBuckets)); }
-
-// 3 blocks per SM (at most 85 registers; 88 unbounded): the pass waits on
-// gathers of the pair's positions, and the extra warps hide them (screw and
-// nut edge-edge query 1.21 -> 1.14 ms)
-template <class S, int KIND>
-__global__ void __launch_bounds__(256, 3) k_cand_bound(const S* __restrict__ x0, const S* __restrict__ x1,
-                                                    const int* __restrict__ prims, CandList cand, CandOrder o,
-                                                    const int* skip_if) {
-  __shared__ int sb[kBuckets];
-  if (skip_if && *skip_if) return;  // the inline pass redoes every pair
-  const int n = min(*cand.count, cand.capacity);
-  if ((int)(blockIdx.x * blockDim.x) >= n) return;
-  if (threadIdx.x < kBuckets) sb[threadIdx.x] = 0;
-  __syncthreads();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) {
-    const int2 pr = cand.pairs[k];
-    int4 ids;
-    if (KIND == 0) {
-      const int2 ea = __ldg(reinterpret_cast<const int2*>(prims) + pr.x);
-      const int2 eb = __ldg(reinterpret_cast<const int2*>(prims) + pr.y);
-      ids = make_int4(ea.x, ea.y, eb.x, eb.y);
-    } else {
-      ids = make_int4(pr.x, __ldg(prims + 3 * pr.y), __ldg(prims + 3 * pr.y + 1), __ldg(prims + 3 * pr.y + 2));
-    }
-    d3 p0[4] = {ld(x0, ids.x), ld(x0, ids.y), ld(x0, ids.z), ld(x0, ids.w)};
-    d3 p1[4] = {ld(x1, ids.x), ld(x1, ids.y), ld(x1, ids.z), ld(x1, ids.w)};
-    const double lb = touch_time_bound<KIND>(p0, p1);
-    float tl = 2.0f;
-    if (lb <= 1.0) {
-      tl = __double2float_rd(lb);  // not above the bound
-      atomicAdd(&sb[bucket_of(tl)], 1);
-    }
-    o.tlb[k] = tl;
-  }
-  __syncthreads();
-  if (threadIdx.x < kBuckets && sb[threadIdx.x]) atomicAdd(o.bcount + threadIdx.x, sb[threadIdx.x]);
-}
-
+// The staged pairs' indices in bucket order.
 __global__ void __launch_bounds__(256) k_cand_bucket(CandList cand, CandOrder o, const int* skip_if) {
   __shared__ int sb[kBuckets], sbase[kBuckets];
-  if (skip_if && *skip_if) return;
+  if (*skip_if) return;
   const int n = min(*cand.count, cand.capacity);
-  if ((int)(blockIdx.x * blockDim.x) >= n) return;
-  if (threadIdx.x < kBuckets) sb[threadIdx.x] = 0;
-  __syncthreads();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  int b = -1, local = 0;
-  if (k < n) {
-    const float tl = o.tlb[k];
-    if (tl <= 1.0f) {
-      b = bucket_of(tl);
+  for (int first = blockIdx.x * blockDim.x; first < n; first += gridDim.x * blockDim.x) {
+    if (threadIdx.x < kBuckets) sb[threadIdx.x] = 0;
+    __syncthreads();
+    const int k = first + threadIdx.x;
+    int b = -1, local = 0;
+    if (k < n) {
+      b = bucket_of(o.tlb[k]);
       local = atomicAdd(&sb[b], 1);
     }
+    __syncthreads();
+    if (threadIdx.x < kBuckets) {
+      const int q = threadIdx.x;
+      int start = 0;
+      for (int c = 0; c < q; ++c) start += o.bcount[c];
+      sbase[q] = sb[q] ? start + atomicAdd(o.bcursor + q, sb[q]) : 0;
+    }
+    __syncthreads();
+    if (b >= 0) o.order[sbase[b] + local] = k;
+    __syncthreads();
   }
-  __syncthreads();
-  if (threadIdx.x < kBuckets) {
-    const int q = threadIdx.x;
-    int start = 0;
-    for (int c = 0; c < q; ++c) start += o.bcount[c];
-    sbase[q] = sb[q] ? start + atomicAdd(o.bcursor + q, sb[q]) : 0;
-  }
-  __syncthreads();
-  if (b >= 0) o.order[sbase[b] + local] = k;
 }
 
 template <class S, int KIND>
 __global__ void __launch_bounds__(128) k_cand_solve(const S* __restrict__ x0, const S* __restrict__ x1,
-                                                    const int* __restrict__ prims, CandList cand, CandOrder o, S* toi,
-                                                    int* status, const int* skip_if) {
+                                                    const int* __restrict__ prims, double pad, CandList cand,
+                                                    CandOrder o, S* toi, int* status, const int* skip_if) {
   if (skip_if && *skip_if) return;
   int total = 0;
 #pragma unroll 1
@@ -800,14 +1054,8 @@ __global__ void __launch_bounds__(128) k_cand_solve(const S* __restrict__ x0, co
     if ((double)bucket_of(first) / kBuckets >= cur) break;
     if (k < 0 || (double)tl >= cur) continue;
     const int2 pr = cand.pairs[k];
-    int4 ids;
-    if (KIND == 0) {
-      const int2 ea = __ldg(reinterpret_cast<const int2*>(prims) + pr.x);
-      const int2 eb = __ldg(reinterpret_cast<const int2*>(prims) + pr.y);
-      ids = make_int4(ea.x, ea.y, eb.x, eb.y);
-    } else {
-      ids = make_int4(pr.x, __ldg(prims + 3 * pr.y), __ldg(prims + 3 * pr.y + 1), __ldg(prims + 3 * pr.y + 2));
-    }
+    const int4 ids = pair_ids<KIND>(prims, pr);
+    if (pad >= 0.0 && !swept_boxes_meet<S, KIND>(x0, x1, ids, pad)) continue;
     d3 p0[4] = {ld(x0, ids.x), ld(x0, ids.y), ld(x0, ids.z), ld(x0, ids.w)};
     d3 p1[4] = {ld(x1, ids.x), ld(x1, ids.y), ld(x1, ids.z), ld(x1, ids.w)};
     const double tt = collision_time<KIND>(p0, p1, st);
@@ -1044,24 +1292,6 @@ inline CandOrder cand_order(void* ws, const CandList& c) {
   return o;
 }
 
-template <class S, int KIND>
-void solve_candidates(const S* x0, const S* x1, const int* prims, void* ws, const CandList& c, S* toi, int* status,
-                      const Sink& sink, cudaStream_t st) {
-  if (!c.capacity) return;
-  if (sink.on) {  // every pair that collides is a record: solve them all
-    const dim3 gc(min(div_up(c.capacity, 128), 2048));
-    k_cand_toi<S, KIND><<<gc, 128, 0, st>>>(x0, x1, prims, c, toi, status, sink, c.overflow);
-    return;
-  }
-  const CandOrder o = cand_order(ws, c);
-  cudaMemsetAsync(o.bcount, 0, (2 * kBuckets + 1) * sizeof(int), st);
-  const dim3 g256(div_up(c.capacity, 256));
-  k_cand_bound<S, KIND><<<g256, 256, 0, st>>>(x0, x1, prims, c, o, c.overflow);
-  k_cand_bucket<<<g256, 256, 0, st>>>(c, o, c.overflow);
-  k_cand_solve<S, KIND><<<148 * 3, 128, 0, st>>>(x0, x1, prims, c, o, toi, status, c.overflow);
-}
-
-
 __global__ void k_pair_time(int kind, int n, const double* __restrict__ a, const double* __restrict__ b,
                             double* __restrict__ t, int* status) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1091,46 +1321,145 @@ __global__ void k_cubic(int n, const double* __restrict__ coef, double x0, doubl
   if (st) atomicOr(status, st);
 }
 
-// The CCD query of one kind: a staging-only collect pass, the per-candidate
-// TOI pass, and (only when the first pass dropped pairs) an inline pass that
-// solves every pair of the query in place.
+// One CCD query of one kind (KIND 0: edges first .. first + count - 1 in
+// Morton rank; 1: the vertices of those places of the visiting order).
 template <class S>
-void run_ee(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, const float* lower, const float* upper,
-            int exclude, CandList c, void* toi, int* status, Sink sink, cudaStream_t st, int first, int count) {
-  const int n = soup->n_edges;
-  const dim3 g(div_up(count, 64));  // 64-thread blocks, as the discrete queries
-  cudaMemsetAsync(c.count, 0, 2 * sizeof(int), st);
-  k_ee_collect<S, true><<<g, 64, 0, st>>>((const S*)soup->x, (const S*)x1, soup->edges, soup->body,
-                                           (const float4*)bvh->wide, bvh->sorted, n, first, count, lower, upper,
-                                           exclude, c, (S*)toi, status, sink, nullptr);
-  solve_candidates<S, 0>((const S*)soup->x, (const S*)x1, soup->edges, c.count, c, (S*)toi, status, sink, st);
-  CandList none = c;
-  none.capacity = 0;
-  k_ee_collect<S, false><<<g, 64, 0, st>>>((const S*)soup->x, (const S*)x1, soup->edges, soup->body,
-                                            (const float4*)bvh->wide, bvh->sorted, n, first, count, lower, upper,
-                                            exclude, none, (S*)toi, status, sink, c.overflow);
+struct Query {
+  const ipcb_soup* soup;
+  const S* x1;
+  const ipcb_lbvh* bvh;
+  const float *lower, *upper;  // EE: query boxes (null: the tree's leaf boxes)
+  double pad;                  // of the swept boxes; < 0: the caller's boxes decide
+  float reach, thickness;      // kBoth: the discrete query's
+  const int* order;            // PT: visiting order or null
+  int exclude, first, count;
+  ipcb_contacts out;           // kBoth: records
+  void* ws;
+  CandList cand;
+  S* toi;
+  int* status;
+  Sink sink;
+  cudaStream_t st;
+};
+
+constexpr int kInlineBlocks = 148 * 2;
+
+template <class S, int KIND, int MODE>
+void collect(const Query<S>& q) {
+  const S* x0 = (const S*)q.soup->x;
+  const tree::View v = tree::view(q.bvh);
+  const CandOrder o = cand_order(q.ws, q.cand);
+  const int blocks = KIND == 0 ? ((q.first + q.count - 1) >> 5) - (q.first >> 5) + 1 : div_up(q.count, 32);
+  const int nsub = tree::share(blocks), items = blocks * nsub;
+  int grid = div_up(items, tree::kWarps);
+  if (MODE == kInline) grid = min(grid, kInlineBlocks);
+  const int* gate = MODE == kInline ? q.cand.overflow : nullptr;
+  if (KIND == 0)
+    k_ee_collect<S, MODE><<<grid, 32 * tree::kWarps, 0, q.st>>>(
+        x0, q.x1, q.soup->edges, q.soup->body, v, q.bvh->sorted, q.first, q.count, nsub, items, q.lower, q.upper,
+        q.pad, q.exclude, q.thickness, q.out, q.cand, o, q.toi, q.status, q.sink, gate);
+  else
+    k_pt_collect<S, MODE><<<grid, 32 * tree::kWarps, 0, q.st>>>(
+        x0, q.x1, q.soup->triangles, q.soup->body, v, q.order, q.first, q.count, nsub, items, q.pad, q.reach,
+        q.exclude, q.thickness, q.out, q.cand, o, q.toi, q.status, q.sink, gate);
+}
+
+inline void clear_header(void* ws, cudaStream_t st) {
+  cudaMemsetAsync(ws, 0, (2 + 2 * kBuckets + 1) * sizeof(int), st);
+}
+
+// The staged pairs (in bucket order without a sink), then -- a small grid that
+// returns at once unless the staging list overflowed -- every pair in place.
+template <class S, int KIND>
+void solve(const Query<S>& q) {
+  const S* x0 = (const S*)q.soup->x;
+  const int* prims = KIND == 0 ? q.soup->edges : q.soup->triangles;
+  const CandList& c = q.cand;
+  if (c.capacity && q.sink.on) {  // every pair that collides is a record: solve them all
+    k_cand_toi<S, KIND><<<min(div_up(c.capacity, 128), 2048), 128, 0, q.st>>>(x0, q.x1, prims, c, q.toi, q.status,
+                                                                              q.sink, c.overflow);
+  } else if (c.capacity) {
+    const CandOrder o = cand_order(q.ws, c);
+    k_cand_bucket<<<min(div_up(c.capacity, 256), 148 * 4), 256, 0, q.st>>>(c, o, c.overflow);
+    k_cand_solve<S, KIND><<<148 * 3, 128, 0, q.st>>>(x0, q.x1, prims, q.pad, c, o, q.toi, q.status, c.overflow);
+  }
+  collect<S, KIND, kInline>(q);
+}
+
+// Boxes given (EE: also the query boxes): stage and solve.
+template <class S, int KIND>
+void run_boxes(const Query<S>& q) {
+  clear_header(q.ws, q.st);
+  collect<S, KIND, kStage>(q);
+  solve<S, KIND>(q);
+}
+
+// Boxes formed here, over the step up to the TOI the seeds give.
+template <class S, int KIND>
+void run_step(const Query<S>& q, const ipcb_contacts* seeds) {
+  const S* x0 = (const S*)q.soup->x;
+  const int* prims = KIND == 0 ? q.soup->edges : q.soup->triangles;
+  clear_header(q.ws, q.st);
+  if (seeds)
+    k_seed<S, KIND><<<kSeedLanes / 64, 64, 0, q.st>>>(x0, q.x1, prims, q.soup->body,
+                                                      KIND == 0 ? q.soup->n_edges : q.soup->n_verts,
+                                                      KIND == 0 ? q.soup->n_edges : q.soup->n_tris, q.exclude, q.pad,
+                                                      *seeds, q.toi, q.status);
+  tree::refit(q.bvh, SweptBox<S, KIND == 0 ? 2 : 3>{x0, q.x1, prims, q.pad, q.toi}, q.st);
+  collect<S, KIND, kStage>(q);
+  solve<S, KIND>(q);
+}
+
+// Boxes of both queries; the discrete records and the staged CCD pairs (solve
+// takes those).
+template <class S, int KIND>
+void run_both(const Query<S>& q, float box_reach) {
+  const int* prims = KIND == 0 ? q.soup->edges : q.soup->triangles;
+  clear_header(q.ws, q.st);
+  tree::refit(q.bvh, BothBox<S, KIND == 0 ? 2 : 3>{(const S*)q.soup->x, q.x1, prims, q.pad, box_reach}, q.st);
+  collect<S, KIND, kBoth>(q);
 }
 
 template <class S>
-void run_pt(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, double pad, int exclude, CandList c,
-            void* toi, int* status, Sink sink, cudaStream_t st, int first, int count) {
-  const dim3 g(div_up(count, 64));
-  cudaMemsetAsync(c.count, 0, 2 * sizeof(int), st);
-  k_pt_collect<S, true><<<g, 64, 0, st>>>((const S*)soup->x, (const S*)x1, soup->triangles, soup->body,
-                                           (const float4*)bvh->wide, soup->n_tris, first, count, pad, exclude, c,
-                                           (S*)toi, status, sink, nullptr);
-  solve_candidates<S, 1>((const S*)soup->x, (const S*)x1, soup->triangles, c.count, c, (S*)toi, status, sink, st);
-  CandList none = c;
-  none.capacity = 0;
-  k_pt_collect<S, false><<<g, 64, 0, st>>>((const S*)soup->x, (const S*)x1, soup->triangles, soup->body,
-                                            (const float4*)bvh->wide, soup->n_tris, first, count, pad, exclude, none,
-                                            (S*)toi, status, sink, c.overflow);
+Query<S> make_query(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, double pad, int exclude, int first,
+                    int count, void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
+  Query<S> q{};
+  q.soup = soup;
+  q.x1 = (const S*)x1;
+  q.bvh = bvh;
+  q.pad = pad;
+  q.exclude = exclude;
+  q.first = first;
+  q.count = count;
+  q.ws = ws;
+  q.cand = cand_list(ws, ws_bytes);
+  q.toi = (S*)toi;
+  q.status = status;
+  q.st = (cudaStream_t)s;
+  return q;
+}
+
+inline bool query_ok(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, const void* toi, const int* status,
+                     const void* ws, size_t ws_bytes, int prims) {
+  return x1 && bvh && toi && status && ws && ws_bytes >= kCandHeader && bvh->n == prims;
+}
+
+inline bool range_ok(int first, int count, int n) {
+  return first >= 0 && count >= 0 && first <= n && count <= n - first;
+}
+
+// f(Query<S>) in the soup's scalar
+template <class F>
+void in_scalar(const ipcb_soup* soup, F&& f) {
+  if (soup->fp64) f((double*)nullptr);
+  else f((float*)nullptr);
 }
 
 }  // namespace
 }  // namespace ipcb
 
 using namespace ipcb;
+
 
 extern "C" {
 
@@ -1180,19 +1509,17 @@ size_t ipcb_toi_workspace(int capacity) { return kCandHeader + (size_t)(capacity
 int ipcb_edge_edge_toi_range(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, const float* lower,
                              const float* upper, int exclude_same_body, int first, int count, void* toi, int* status,
                              void* ws, size_t ws_bytes, ipcb_stream s) {
-  if (!soup || !x1 || !bvh || !lower || !upper || !toi || !status || !ws || ws_bytes < kCandHeader ||
-      bvh->n != soup->n_edges)
+  if (!soup || !lower || !upper || !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_edges) ||
+      !range_ok(first, count, soup->n_edges))
     return IPCB_E_ARG;
-  const int n = soup->n_edges;
-  if (first < 0 || count < 0 || first > n || count > n - first) return IPCB_E_ARG;
   if (count == 0) return IPCB_OK;
-  const CandList c = cand_list(ws, ws_bytes);
-  if (soup->fp64)
-    run_ee<double>(soup, x1, bvh, lower, upper, exclude_same_body, c, toi, status, Sink{}, (cudaStream_t)s, first,
-                   count);
-  else
-    run_ee<float>(soup, x1, bvh, lower, upper, exclude_same_body, c, toi, status, Sink{}, (cudaStream_t)s, first,
-                  count);
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    Query<S> q = make_query<S>(soup, x1, bvh, -1.0, exclude_same_body, first, count, toi, status, ws, ws_bytes, s);
+    q.lower = lower;
+    q.upper = upper;
+    run_boxes<S, 0>(q);
+  });
   return check_launch("ipcb_edge_edge_toi");
 }
 
@@ -1207,16 +1534,14 @@ int ipcb_edge_edge_toi(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* b
 int ipcb_point_triangle_toi_range(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, double pad,
                                   int exclude_same_body, int first, int count, void* toi, int* status, void* ws,
                                   size_t ws_bytes, ipcb_stream s) {
-  if (!soup || !x1 || !bvh || !toi || !status || !ws || ws_bytes < kCandHeader || bvh->n != soup->n_tris)
+  if (!soup || !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_tris) ||
+      !range_ok(first, count, soup->n_verts))
     return IPCB_E_ARG;
-  const int nv = soup->n_verts;
-  if (first < 0 || count < 0 || first > nv || count > nv - first) return IPCB_E_ARG;
   if (count == 0 || soup->n_tris == 0) return IPCB_OK;
-  const CandList c = cand_list(ws, ws_bytes);
-  if (soup->fp64)
-    run_pt<double>(soup, x1, bvh, pad, exclude_same_body, c, toi, status, Sink{}, (cudaStream_t)s, first, count);
-  else
-    run_pt<float>(soup, x1, bvh, pad, exclude_same_body, c, toi, status, Sink{}, (cudaStream_t)s, first, count);
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    run_boxes<S, 1>(make_query<S>(soup, x1, bvh, pad, exclude_same_body, first, count, toi, status, ws, ws_bytes, s));
+  });
   return check_launch("ipcb_point_triangle_toi");
 }
 
@@ -1228,39 +1553,133 @@ int ipcb_point_triangle_toi(const ipcb_soup* soup, const void* x1, const ipcb_lb
                                        ws_bytes, s);
 }
 
+static bool list_ok(const ipcb_contacts* l) {
+  return l && l->cnt && (l->capacity <= 0 || (l->a1a2b1b2 && l->e0e1 && l->l0 && l->alpha && l->lam));
+}
+static bool seeds_ok(const ipcb_contacts* seeds) {
+  return !seeds || (seeds->cnt && (seeds->capacity <= 0 || seeds->e0e1));
+}
+
+int ipcb_edge_edge_step(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                        const ipcb_contacts* seeds, int exclude_same_body, int first, int count, void* toi, int* status,
+                        void* ws, size_t ws_bytes, ipcb_stream s) {
+  if (!soup || !(pad >= 0.0) || !seeds_ok(seeds) ||
+      !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_edges) || !range_ok(first, count, soup->n_edges))
+    return IPCB_E_ARG;
+  if (count == 0) return IPCB_OK;
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    run_step<S, 0>(make_query<S>(soup, x1, bvh, pad, exclude_same_body, first, count, toi, status, ws, ws_bytes, s),
+                   seeds);
+  });
+  return check_launch("ipcb_edge_edge_step");
+}
+
+int ipcb_point_triangle_step(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                             const int* query_order, const ipcb_contacts* seeds, int exclude_same_body, int first,
+                             int count, void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
+  if (!soup || !(pad >= 0.0) || !seeds_ok(seeds) ||
+      !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_tris) || !range_ok(first, count, soup->n_verts))
+    return IPCB_E_ARG;
+  if (count == 0 || soup->n_tris == 0) return IPCB_OK;
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    Query<S> q = make_query<S>(soup, x1, bvh, pad, exclude_same_body, first, count, toi, status, ws, ws_bytes, s);
+    q.order = query_order;
+    run_step<S, 1>(q, seeds);
+  });
+  return check_launch("ipcb_point_triangle_step");
+}
+
+int ipcb_edge_edge_both(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh, float thickness,
+                        float box_pad, int exclude_same_body, ipcb_contacts* out, void* toi, int* status, void* ws,
+                        size_t ws_bytes, ipcb_stream s) {
+  if (!soup || !(pad >= 0.0) || !list_ok(out) || !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_edges))
+    return IPCB_E_ARG;
+  if (soup->n_edges == 0) return IPCB_OK;
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    Query<S> q = make_query<S>(soup, x1, bvh, pad, exclude_same_body, 0, soup->n_edges, toi, status, ws, ws_bytes, s);
+    q.thickness = thickness;
+    q.out = *out;
+    run_both<S, 0>(q, box_pad);
+  });
+  return check_launch("ipcb_edge_edge_both");
+}
+
+int ipcb_point_triangle_both(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh, float thickness,
+                             float query_pad, const int* query_order, int exclude_same_body, ipcb_contacts* out,
+                             void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
+  if (!soup || !(pad >= 0.0) || !list_ok(out) || !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_tris))
+    return IPCB_E_ARG;
+  if (soup->n_verts == 0 || soup->n_tris == 0) return IPCB_OK;
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    Query<S> q = make_query<S>(soup, x1, bvh, pad, exclude_same_body, 0, soup->n_verts, toi, status, ws, ws_bytes, s);
+    q.order = query_order;
+    q.thickness = thickness;
+    q.reach = query_pad;
+    q.out = *out;
+    run_both<S, 1>(q, 0.f);
+  });
+  return check_launch("ipcb_point_triangle_both");
+}
+
+int ipcb_edge_edge_solve(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                         int exclude_same_body, void* toi, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
+  if (!soup || !(pad >= 0.0) || !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_edges)) return IPCB_E_ARG;
+  if (soup->n_edges == 0) return IPCB_OK;
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    solve<S, 0>(
+        make_query<S>(soup, x1, bvh, pad, exclude_same_body, 0, soup->n_edges, toi, status, ws, ws_bytes, s));
+  });
+  return check_launch("ipcb_edge_edge_solve");
+}
+
+int ipcb_point_triangle_solve(const ipcb_soup* soup, const void* x1, double pad, const ipcb_lbvh* bvh,
+                              const int* query_order, int exclude_same_body, void* toi, int* status, void* ws,
+                              size_t ws_bytes, ipcb_stream s) {
+  if (!soup || !(pad >= 0.0) || !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_tris)) return IPCB_E_ARG;
+  if (soup->n_verts == 0 || soup->n_tris == 0) return IPCB_OK;
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    Query<S> q = make_query<S>(soup, x1, bvh, pad, exclude_same_body, 0, soup->n_verts, toi, status, ws, ws_bytes, s);
+    q.order = query_order;
+    solve<S, 1>(q);
+  });
+  return check_launch("ipcb_point_triangle_solve");
+}
+
 int ipcb_edge_edge_intersections(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, const float* lower,
                                  const float* upper, int exclude_same_body, double thickness, void* toi,
                                  const ipcb_contacts* out, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
-  if (!soup || !x1 || !bvh || !lower || !upper || !toi || !out || !out->cnt || !status || !ws || ws_bytes < kCandHeader ||
-      bvh->n != soup->n_edges)
+  if (!soup || !lower || !upper || !list_ok(out) ||
+      !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_edges))
     return IPCB_E_ARG;
-  if (out->capacity > 0 && (!out->a1a2b1b2 || !out->e0e1 || !out->l0 || !out->alpha || !out->lam)) return IPCB_E_ARG;
   if (soup->n_edges == 0) return IPCB_OK;
-  const CandList c = cand_list(ws, ws_bytes);
-  const Sink sink{*out, thickness * 2.0, 1};
-  const int n = soup->n_edges;
-  if (soup->fp64)
-    run_ee<double>(soup, x1, bvh, lower, upper, exclude_same_body, c, toi, status, sink, (cudaStream_t)s, 0, n);
-  else
-    run_ee<float>(soup, x1, bvh, lower, upper, exclude_same_body, c, toi, status, sink, (cudaStream_t)s, 0, n);
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    Query<S> q = make_query<S>(soup, x1, bvh, -1.0, exclude_same_body, 0, soup->n_edges, toi, status, ws, ws_bytes, s);
+    q.lower = lower;
+    q.upper = upper;
+    q.sink = Sink{*out, thickness * 2.0, 1};
+    run_boxes<S, 0>(q);
+  });
   return check_launch("ipcb_edge_edge_intersections");
 }
 
 int ipcb_point_triangle_intersections(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh, double pad,
                                       int exclude_same_body, double thickness, void* toi, const ipcb_contacts* out,
                                       int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
-  if (!soup || !x1 || !bvh || !toi || !out || !out->cnt || !status || !ws || ws_bytes < kCandHeader ||
-      bvh->n != soup->n_tris)
-    return IPCB_E_ARG;
-  if (out->capacity > 0 && (!out->a1a2b1b2 || !out->e0e1 || !out->l0 || !out->alpha || !out->lam)) return IPCB_E_ARG;
+  if (!soup || !list_ok(out) || !query_ok(soup, x1, bvh, toi, status, ws, ws_bytes, soup->n_tris)) return IPCB_E_ARG;
   if (soup->n_verts == 0 || soup->n_tris == 0) return IPCB_OK;
-  const CandList c = cand_list(ws, ws_bytes);
-  const Sink sink{*out, thickness * 2.0, 1};
-  const int nv = soup->n_verts;
-  if (soup->fp64)
-    run_pt<double>(soup, x1, bvh, pad, exclude_same_body, c, toi, status, sink, (cudaStream_t)s, 0, nv);
-  else
-    run_pt<float>(soup, x1, bvh, pad, exclude_same_body, c, toi, status, sink, (cudaStream_t)s, 0, nv);
+  in_scalar(soup, [&](auto* scalar) {
+    using S = std::remove_pointer_t<decltype(scalar)>;
+    Query<S> q = make_query<S>(soup, x1, bvh, pad, exclude_same_body, 0, soup->n_verts, toi, status, ws, ws_bytes, s);
+    q.sink = Sink{*out, thickness * 2.0, 1};
+    run_boxes<S, 1>(q);
+  });
   return check_launch("ipcb_point_triangle_intersections");
 }
 

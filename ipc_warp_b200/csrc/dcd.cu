@@ -6,6 +6,8 @@
 #include "common.cuh"
 #include "geom.cuh"
 #include "lbvh.cuh"
+#include "records.cuh"
+#include "tree.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -50,17 +52,6 @@ __global__ void k_tri_aabbs(const float4* __restrict__ x4, const int* __restrict
 
 constexpr int kQueue = 32;  // per-thread queue of filtered leaf hits
 
-template <class S>
-IPCB_D void write_record(const ipcb_contacts& c, int slot, int a1, int a2, int b1, int b2, int e0, int e1, S l0) {
-  if (slot < c.capacity) {
-    reinterpret_cast<int4*>(c.a1a2b1b2)[slot] = make_int4(a1, a2, b1, b2);
-    reinterpret_cast<int2*>(c.e0e1)[slot] = make_int2(e0, e1);
-    static_cast<S*>(c.l0)[slot] = l0;
-    static_cast<S*>(c.alpha)[slot] = S(1e-6);
-    static_cast<S*>(c.lam)[slot] = S(0);
-  }
-}
-
 // Append from inside divergent code (rare path: a full queue).
 template <class S>
 IPCB_D void append_divergent(const ipcb_contacts& c, int a1, int a2, int b1, int b2, int e0, int e1, S l0) {
@@ -70,128 +61,179 @@ IPCB_D void append_divergent(const ipcb_contacts& c, int a1, int a2, int b1, int
   write_record<S>(c, g.shfl(base, 0) + (int)g.thread_rank(), a1, a2, b1, b2, e0, e1, l0);
 }
 
-// Append from converged code: one ballot and one atomicAdd per warp.
-IPCB_D int warp_reserve(int* cnt, bool accept) {
-  const unsigned lane = threadIdx.x & 31;
-  unsigned m = __ballot_sync(0xffffffffu, accept);
-  int base = 0;
-  if (lane == 0 && m) base = atomicAdd(cnt, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  return base + __popc(m & ((1u << lane) - 1u));
-}
-
 IPCB_D int warp_max(int v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
 
-// One thread per edge, visiting edges in the BVH leaf (Morton) order so a
-// warp's queries walk neighbouring subtrees.  Traversal only applies the cheap
-// filters and queues the surviving leaves; the exact closest-point test and
-// the append run afterwards with the warp converged.
-// 64-thread blocks, 14 per SM (at most 73 registers; 80 unbounded): more
-// warps in flight over the dependent node loads (screw and nut 0.568 ->
-// 0.539 ms; 64 registers spill and were slower)
+// Box functors of the packed tree (tree.cuh): padded boxes of x4.
+struct EdgeBox {
+  const float4* x4;
+  const int* edges;
+  float pad;
+  IPCB_D void operator()(int p, f3& lo, f3& hi) const {
+    const int2 e = __ldg(reinterpret_cast<const int2*>(edges) + p);
+    const f3 a = load4(x4, e.x), b = load4(x4, e.y);
+    lo = mk3(fminf(a.x, b.x) - pad, fminf(a.y, b.y) - pad, fminf(a.z, b.z) - pad);
+    hi = mk3(fmaxf(a.x, b.x) + pad, fmaxf(a.y, b.y) + pad, fmaxf(a.z, b.z) + pad);
+  }
+};
+struct TriBox {
+  const float4* x4;
+  const int* tris;
+  float pad;
+  IPCB_D void operator()(int p, f3& lo, f3& hi) const {
+    const f3 a = load4(x4, __ldg(tris + 3 * p)), b = load4(x4, __ldg(tris + 3 * p + 1)),
+             c = load4(x4, __ldg(tris + 3 * p + 2));
+    lo = mk3(fminf(fminf(a.x, b.x), c.x) - pad, fminf(fminf(a.y, b.y), c.y) - pad, fminf(fminf(a.z, b.z), c.z) - pad);
+    hi = mk3(fmaxf(fmaxf(a.x, b.x), c.x) + pad, fmaxf(fmaxf(a.y, b.y), c.y) + pad, fmaxf(fmaxf(a.z, b.z), c.z) + pad);
+  }
+};
+
+// Edge-edge query: a warp per block of 32 edges in Morton order (nsub warps
+// when there are few), walking the packed tree once for the block (tree.cuh);
+// the surviving pairs are queued and the exact closest-point test and the
+// append run on full warps.  A block only meets blocks of its own and higher
+// rank, so each pair is met once, by its lower-ranked edge; it is then stated
+// as the reference's (lower id, higher id).
 template <class S>
-__global__ void __launch_bounds__(64, 14) k_dcd_ee(const float4* __restrict__ x4, const int* __restrict__ edges,
-                                                const int* __restrict__ body, const float4* __restrict__ nodes,
-                                                const int* __restrict__ order, int n, int first, int count,
-                                                float thickness, float qpad, int exclude, ipcb_contacts out,
-                                                int* status) {
+__global__ void __launch_bounds__(32 * tree::kWarps) k_dcd_ee(const float4* __restrict__ x4,
+                                                              const int* __restrict__ edges,
+                                                              const int* __restrict__ body, const __grid_constant__ tree::View v,
+                                                              const int* __restrict__ order, int first, int count,
+                                                              int nsub, float thickness, float qpad, int exclude,
+                                                              ipcb_contacts out) {
+  __shared__ tree::Block blocks[tree::kWarps];
+  tree::Block& B = blocks[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int item = blockIdx.x * tree::kWarps + (threadIdx.x >> 5);
+  const int qb = (first >> 5) + item / nsub, sub = item % nsub;
+  const int t = qb * 32 + lane;
   // queries: the edges of Morton rank first .. first + count - 1
-  int t = first + blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = t < first + count;
-  int i = active ? __ldg(order + t) : 0;
-  int2 ea = active ? __ldg(reinterpret_cast<const int2*>(edges) + i) : make_int2(0, 0);
-  f3 p1 = load4(x4, ea.x), p2 = load4(x4, ea.y);
-  int bi = exclude ? __ldg(body + ea.x) : 0;
+  const bool active = t >= first && t < first + count;
+  if (!__any_sync(0xffffffffu, active)) return;
+  const int i = active ? __ldg(order + t) : 0;
+  const int2 ea = active ? __ldg(reinterpret_cast<const int2*>(edges) + i) : make_int2(0, 0);
+  const f3 p1 = load4(x4, ea.x), p2 = load4(x4, ea.y);
+  f3 qlo = mk3(fminf(p1.x, p2.x) - qpad, fminf(p1.y, p2.y) - qpad, fminf(p1.z, p2.z) - qpad);
+  f3 qhi = mk3(fmaxf(p1.x, p2.x) + qpad, fmaxf(p1.y, p2.y) + qpad, fmaxf(p1.z, p2.z) + qpad);
+  if (!active) {
+    qlo = mk3(tree::kBig, tree::kBig, tree::kBig);
+    qhi = mk3(-tree::kBig, -tree::kBig, -tree::kBig);
+  }
+  const int bi = exclude ? __ldg(body + ea.x) : 0;
+  B.qlo[lane] = make_float4(qlo.x, qlo.y, qlo.z, __int_as_float(i));
+  B.qhi[lane] = make_float4(qhi.x, qhi.y, qhi.z, __int_as_float(bi));
+  B.ev[lane] = ea;
+  __syncwarp();
   const float l0f = xmul(thickness, 2.0f);
   const S l0 = S(thickness) * S(2.0);
-  int q[kQueue];
   int nq = 0;
-  if (active) {
-    f3 qlo = mk3(fminf(p1.x, p2.x) - qpad, fminf(p1.y, p2.y) - qpad, fminf(p1.z, p2.z) - qpad);
-    f3 qhi = mk3(fmaxf(p1.x, p2.x) + qpad, fmaxf(p1.y, p2.y) + qpad, fmaxf(p1.z, p2.z) + qpad);
-    // the hierarchy is over the queries themselves: thread t is the edge of
-    // Morton rank t, so only leaves of higher rank are visited and each pair
-    // is met once; it is then stated as the reference's (lower id, higher id)
-    bool ok = traverse4_after(nodes, n, t, qlo, qhi, [&](int j, int) {
-      int2 eb = __ldg(reinterpret_cast<const int2*>(edges) + j);
-      if (ea.x == eb.x || ea.x == eb.y || ea.y == eb.x || ea.y == eb.y) return;
-      if (exclude && bi == __ldg(body + eb.x)) return;
-      if (nq < kQueue) {
-        q[nq++] = j;
-      } else if (i < j) {
-        CPEE r = closest_point_edge_edge(p1, p2, load4(x4, eb.x), load4(x4, eb.y), 1.0e-6f);
-        if (r.d < l0f) append_divergent<S>(out, ea.x, ea.y, eb.x, eb.y, i, j, l0);
-      } else {
-        CPEE r = closest_point_edge_edge(load4(x4, eb.x), load4(x4, eb.y), p1, p2, 1.0e-6f);
-        if (r.d < l0f) append_divergent<S>(out, eb.x, eb.y, ea.x, ea.y, j, i, l0);
-      }
-    });
-    if (!ok) atomicOr(status, IPCB_STATUS_STACK);
-  }
-  int rounds = warp_max(nq);
-  for (int k = 0; k < rounds; ++k) {
-    bool has = k < nq;
-    int j = has ? q[k] : 0;
-    int2 eb = has ? __ldg(reinterpret_cast<const int2*>(edges) + j) : make_int2(0, 0);
+  auto flush = [&](int n) {
+    const bool has = lane < n;
+    const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);
+    const int a = __float_as_int(B.qlo[pr.x].w), j = pr.y;
+    const int2 e1 = B.ev[pr.x], e2 = has ? __ldg(reinterpret_cast<const int2*>(edges) + j) : make_int2(0, 0);
     // (lower id, higher id): the reference's orientation and argument order
-    const bool fwd = i < j;
-    const int lo_id = fwd ? i : j, hi_id = fwd ? j : i;
-    const int2 e_lo = fwd ? ea : eb, e_hi = fwd ? eb : ea;
+    const bool fwd = a < j;
+    const int2 el = fwd ? e1 : e2, eh = fwd ? e2 : e1;
     bool accept = false;
     if (has)
-      accept = closest_point_edge_edge(load4(x4, e_lo.x), load4(x4, e_lo.y), load4(x4, e_hi.x), load4(x4, e_hi.y),
+      accept = closest_point_edge_edge(load4(x4, el.x), load4(x4, el.y), load4(x4, eh.x), load4(x4, eh.y),
                                        1.0e-6f).d < l0f;
-    int slot = warp_reserve(out.cnt, accept);
-    if (accept) write_record<S>(out, slot, e_lo.x, e_lo.y, e_hi.x, e_hi.y, lo_id, hi_id, l0);
-  }
+    const int slot = warp_reserve(out.cnt, accept);
+    if (accept) write_record<S>(out, slot, el.x, el.y, eh.x, eh.y, fwd ? a : j, fwd ? j : a, l0);
+  };
+  tree::for_segments(active, qlo, qhi, [&](bool in, f3 glo, f3 ghi) {
+  tree::for_block_pairs<true>(v, glo, ghi, qb, sub, nsub, B.stack, [&](int tb) {
+    tree::block_pair<true>(
+        v, B, qb, tb, in, qlo, qhi, glo, ghi, nq,
+        [&](int j) {
+          int3 e = make_int3(-1, -1, 0);
+          if (j >= 0) {
+            const int2 w = __ldg(reinterpret_cast<const int2*>(edges) + j);
+            e = make_int3(w.x, w.y, exclude ? __ldg(body + w.x) : 0);
+          }
+          return e;
+        },
+        [&](int q, int3 e) {
+          const int2 w = B.ev[q];
+          if (w.x == e.x || w.x == e.y || w.y == e.x || w.y == e.y) return false;
+          return !(exclude && __float_as_int(B.qhi[q].w) == e.z);
+        },
+        flush);
+  });
+  });
+  __syncwarp();
+  if (nq) flush(nq);
 }
 
+// Point-triangle query: the same over blocks of 32 vertices of the visiting
+// order (Morton order keeps a block's box small) against the triangles.
 template <class S>
-__global__ void __launch_bounds__(64, 14) k_dcd_pt(const float4* __restrict__ x4, const int* __restrict__ tris,
-                                                const int* __restrict__ body, const float4* __restrict__ nodes,
-                                                int n_tris, const int* __restrict__ order, int first, int count,
-                                                float thickness, float qpad, int exclude, ipcb_contacts out,
-                                                int* status) {
+__global__ void __launch_bounds__(32 * tree::kWarps) k_dcd_pt(const float4* __restrict__ x4,
+                                                              const int* __restrict__ tris,
+                                                              const int* __restrict__ body, const __grid_constant__ tree::View v,
+                                                              const int* __restrict__ order, int first, int count,
+                                                              int nsub, float thickness, float qpad, int exclude,
+                                                              ipcb_contacts out) {
+  __shared__ tree::Block blocks[tree::kWarps];
+  tree::Block& B = blocks[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int item = blockIdx.x * tree::kWarps + (threadIdx.x >> 5);
+  const int sub = item % nsub;
   // queries: the vertices first .. first + count - 1 of the visiting order
-  int t = first + blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = t < first + count;
-  int i = active ? (order ? __ldg(order + t) : t) : 0;
-  f3 p = load4(x4, i);
-  int bi = exclude ? __ldg(body + i) : 0;
+  const int t = (item / nsub) * 32 + lane;
+  const bool active = t < count;
+  if (!__any_sync(0xffffffffu, active)) return;
+  const int i = active ? (order ? __ldg(order + first + t) : first + t) : 0;
+  const f3 p = load4(x4, i);
+  f3 qlo = mk3(p.x - qpad, p.y - qpad, p.z - qpad), qhi = mk3(p.x + qpad, p.y + qpad, p.z + qpad);
+  if (!active) {
+    qlo = mk3(tree::kBig, tree::kBig, tree::kBig);
+    qhi = mk3(-tree::kBig, -tree::kBig, -tree::kBig);
+  }
+  const int bi = exclude ? __ldg(body + i) : 0;
+  B.qlo[lane] = make_float4(qlo.x, qlo.y, qlo.z, __int_as_float(i));
+  B.qhi[lane] = make_float4(qhi.x, qhi.y, qhi.z, __int_as_float(bi));
+  __syncwarp();
   const float l0f = xmul(thickness, 2.0f);
   const S l0 = S(thickness) * S(2.0);
-  int q[kQueue];
   int nq = 0;
-  if (active) {
-    f3 qlo = mk3(p.x - qpad, p.y - qpad, p.z - qpad), qhi = mk3(p.x + qpad, p.y + qpad, p.z + qpad);
-    bool ok = traverse4(nodes, n_tris, qlo, qhi, [&](int j) {
-      int t0 = __ldg(tris + 3 * j), t1 = __ldg(tris + 3 * j + 1), t2 = __ldg(tris + 3 * j + 2);
-      if (t0 == i || t1 == i || t2 == i) return;
-      if (exclude && bi == __ldg(body + t0)) return;
-      if (nq < kQueue) {
-        q[nq++] = j;
-      } else {
-        CPT r = closest_point_triangle(p, load4(x4, t0), load4(x4, t1), load4(x4, t2));
-        if (r.d < l0f) append_divergent<S>(out, i, t1, t0, t2, i, j, l0);
-      }
-    });
-    if (!ok) atomicOr(status, IPCB_STATUS_STACK);
-  }
-  int rounds = warp_max(nq);
-  for (int k = 0; k < rounds; ++k) {
-    bool has = k < nq;
-    int j = has ? q[k] : 0;
-    int t0 = has ? __ldg(tris + 3 * j) : 0, t1 = has ? __ldg(tris + 3 * j + 1) : 0,
-        t2 = has ? __ldg(tris + 3 * j + 2) : 0;
+  auto flush = [&](int n) {
+    const bool has = lane < n;
+    const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);
+    const int a = __float_as_int(B.qlo[pr.x].w), j = pr.y;
+    const int t0 = has ? __ldg(tris + 3 * j) : 0, t1 = has ? __ldg(tris + 3 * j + 1) : 0,
+              t2 = has ? __ldg(tris + 3 * j + 2) : 0;
     bool accept = false;
-    if (has) accept = closest_point_triangle(p, load4(x4, t0), load4(x4, t1), load4(x4, t2)).d < l0f;
-    int slot = warp_reserve(out.cnt, accept);
-    if (accept) write_record<S>(out, slot, i, t1, t0, t2, i, j, l0);  // (p, tri[1], tri[0], tri[2])
-  }
+    if (has) accept = closest_point_triangle(load4(x4, a), load4(x4, t0), load4(x4, t1), load4(x4, t2)).d < l0f;
+    const int slot = warp_reserve(out.cnt, accept);
+    if (accept) write_record<S>(out, slot, a, t1, t0, t2, a, j, l0);  // (p, tri[1], tri[0], tri[2])
+  };
+  tree::for_segments(active, qlo, qhi, [&](bool in, f3 glo, f3 ghi) {
+  tree::for_block_pairs<false>(v, glo, ghi, 0, sub, nsub, B.stack, [&](int tb) {
+    tree::block_pair<false>(
+        v, B, 0, tb, in, qlo, qhi, glo, ghi, nq,
+        [&](int j) {
+          int4 e = make_int4(-1, -1, -1, 0);
+          if (j >= 0) {
+            e = make_int4(__ldg(tris + 3 * j), __ldg(tris + 3 * j + 1), __ldg(tris + 3 * j + 2), 0);
+            if (exclude) e.w = __ldg(body + e.x);
+          }
+          return e;
+        },
+        [&](int q, int4 e) {
+          const int a = __float_as_int(B.qlo[q].w);
+          if (a == e.x || a == e.y || a == e.z) return false;
+          return !(exclude && __float_as_int(B.qhi[q].w) == e.w);
+        },
+        flush);
+  });
+  });
+  __syncwarp();
+  if (nq) flush(nq);
 }
 
 // ---------------------------------------------------------------- fixed bodies
@@ -384,6 +426,18 @@ int ipcb_triangle_aabbs(const ipcb_soup* soup, const float* x4, float pad, float
   return check_launch("ipcb_triangle_aabbs");
 }
 
+int ipcb_lbvh_refit_edges(const ipcb_soup* soup, const float* x4, float pad, const ipcb_lbvh* bvh, ipcb_stream s) {
+  if (!soup || !x4 || !bvh || bvh->n != soup->n_edges) return IPCB_E_ARG;
+  tree::refit(bvh, EdgeBox{(const float4*)x4, soup->edges, pad}, (cudaStream_t)s);
+  return check_launch("ipcb_lbvh_refit_edges");
+}
+
+int ipcb_lbvh_refit_triangles(const ipcb_soup* soup, const float* x4, float pad, const ipcb_lbvh* bvh, ipcb_stream s) {
+  if (!soup || !x4 || !bvh || bvh->n != soup->n_tris) return IPCB_E_ARG;
+  tree::refit(bvh, TriBox{(const float4*)x4, soup->triangles, pad}, (cudaStream_t)s);
+  return check_launch("ipcb_lbvh_refit_triangles");
+}
+
 int ipcb_dcd_ee_range(const ipcb_soup* soup, const float* x4, const ipcb_lbvh* bvh, float thickness,
                       float query_pad, int exclude_same_body, int first, int count, ipcb_contacts* out, int* status,
                       ipcb_stream s) {
@@ -391,17 +445,17 @@ int ipcb_dcd_ee_range(const ipcb_soup* soup, const float* x4, const ipcb_lbvh* b
   int n = soup->n_edges;
   if (first < 0 || count < 0 || first > n || count > n - first) return IPCB_E_ARG;
   if (count == 0) return IPCB_OK;
-  // 64-thread blocks: queries end at different depths, and a small block
-  // frees its slot sooner (measured a few percent faster than 128)
-  dim3 grid(div_up(count, 64));
+  const tree::View v = tree::view(bvh);
+  const int blocks = ((first + count - 1) >> 5) - (first >> 5) + 1, nsub = tree::share(blocks);
+  const dim3 grid(div_up((long long)blocks * nsub, tree::kWarps));
   if (soup->fp64)
-    k_dcd_ee<double><<<grid, 64, 0, (cudaStream_t)s>>>((const float4*)x4, soup->edges, soup->body,
-                                                        (const float4*)bvh->wide, bvh->sorted, n, first, count,
-                                                        thickness, query_pad, exclude_same_body, *out, status);
+    k_dcd_ee<double><<<grid, 32 * tree::kWarps, 0, (cudaStream_t)s>>>((const float4*)x4, soup->edges, soup->body, v,
+                                                                      bvh->sorted, first, count, nsub, thickness,
+                                                                      query_pad, exclude_same_body, *out);
   else
-    k_dcd_ee<float><<<grid, 64, 0, (cudaStream_t)s>>>((const float4*)x4, soup->edges, soup->body,
-                                                       (const float4*)bvh->wide, bvh->sorted, n, first, count,
-                                                       thickness, query_pad, exclude_same_body, *out, status);
+    k_dcd_ee<float><<<grid, 32 * tree::kWarps, 0, (cudaStream_t)s>>>((const float4*)x4, soup->edges, soup->body, v,
+                                                                     bvh->sorted, first, count, nsub, thickness,
+                                                                     query_pad, exclude_same_body, *out);
   return check_launch("ipcb_dcd_ee");
 }
 
@@ -418,15 +472,17 @@ int ipcb_dcd_pt_range(const ipcb_soup* soup, const float* x4, const ipcb_lbvh* b
   int nv = soup->n_verts;
   if (first < 0 || count < 0 || first > nv || count > nv - first) return IPCB_E_ARG;
   if (count == 0 || soup->n_tris == 0) return IPCB_OK;
-  dim3 grid(div_up(count, 64));
+  const tree::View v = tree::view(bvh);
+  const int blocks = div_up(count, 32), nsub = tree::share(blocks);
+  const dim3 grid(div_up((long long)blocks * nsub, tree::kWarps));
   if (soup->fp64)
-    k_dcd_pt<double><<<grid, 64, 0, (cudaStream_t)s>>>((const float4*)x4, soup->triangles, soup->body,
-                                                        (const float4*)bvh->wide, soup->n_tris, query_order, first,
-                                                        count, thickness, query_pad, exclude_same_body, *out, status);
+    k_dcd_pt<double><<<grid, 32 * tree::kWarps, 0, (cudaStream_t)s>>>((const float4*)x4, soup->triangles, soup->body,
+                                                                      v, query_order, first, count, nsub, thickness,
+                                                                      query_pad, exclude_same_body, *out);
   else
-    k_dcd_pt<float><<<grid, 64, 0, (cudaStream_t)s>>>((const float4*)x4, soup->triangles, soup->body,
-                                                       (const float4*)bvh->wide, soup->n_tris, query_order, first,
-                                                       count, thickness, query_pad, exclude_same_body, *out, status);
+    k_dcd_pt<float><<<grid, 32 * tree::kWarps, 0, (cudaStream_t)s>>>((const float4*)x4, soup->triangles, soup->body, v,
+                                                                     query_order, first, count, nsub, thickness,
+                                                                     query_pad, exclude_same_body, *out);
   return check_launch("ipcb_dcd_pt");
 }
 

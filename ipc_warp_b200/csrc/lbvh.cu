@@ -6,6 +6,7 @@
 #include "common.cuh"
 #include "lbvh.cuh"
 #include "sort.cuh"
+#include "tree.cuh"
 
 namespace ipcb {
 
@@ -342,7 +343,8 @@ size_t ipcb_lbvh_bytes(int capacity) {
   if (capacity < 1) capacity = 1;
   size_t c = (size_t)capacity;
   size_t nn = c > 1 ? c - 1 : 1;
-  return al256(nn * 4 * 16) + al256(2 * c * 4) + al256(c * 4) + al256(c * 4) + al256(c * 4) + al256(nn * 8 * 16);
+  return al256(nn * 4 * 16) + al256(2 * c * 4) + al256(c * 4) + al256(c * 4) + al256(c * 4) + al256(nn * 8 * 16) +
+         tree::bytes(capacity);
 }
 
 int ipcb_lbvh_bind(ipcb_lbvh* bvh, void* mem, int capacity) {
@@ -396,6 +398,7 @@ int ipcb_lbvh_build(ipcb_lbvh* bvh, const float* lower, const float* upper, int 
                                                   bvh->capacity);
   k_refit<<<div_up(n, 32 * kRefitWarps), 32 * kRefitWarps, 0, st>>>(lower, upper, n, bvh->sorted, bvh->parent, bvh->capacity,
                                            (float4*)bvh->nodes, bvh->flags, (float4*)bvh->wide);
+  tree::refit(bvh, tree::BoxArray{lower, upper}, st);
   return check_launch("ipcb_lbvh_build");
 }
 
@@ -406,6 +409,7 @@ int ipcb_lbvh_refit(const ipcb_lbvh* bvh, const float* lower, const float* upper
   k_refit<<<div_up(bvh->n, 32 * kRefitWarps), 32 * kRefitWarps, 0, (cudaStream_t)s>>>(lower, upper, bvh->n, bvh->sorted, bvh->parent,
                                                             bvh->capacity, (float4*)bvh->nodes, bvh->flags,
                                                             (float4*)bvh->wide);
+  tree::refit(bvh, tree::BoxArray{lower, upper}, (cudaStream_t)s);
   return check_launch("ipcb_lbvh_refit");
 }
 

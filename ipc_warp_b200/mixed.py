@@ -518,7 +518,7 @@ class MixedSolver(ContactBarrierMixin):
         h2 = self.h * self.h
         kappa = float(self.contact_stiffness)
         if detect:
-            self.update_bvh()
+            self._refit_queries()
             self._launch_dcd("ee")
             if self.has_triangles:
                 self._launch_dcd("pt")

@@ -397,7 +397,7 @@ class FEMContactSolver(ContactBarrierMixin):
         self.b.zero_()
         self.compute_V(ret=False)
         self._status.zero_()
-        self.update_bvh()
+        self._refit_queries()
         self._launch_dcd("ee")
         if self.has_triangles:
             self._launch_dcd("pt")
@@ -737,7 +737,7 @@ class FEMContactSolver(ContactBarrierMixin):
         fp64 = int(self.dtype == torch.float64)
         kappa = float(self.contact_stiffness)
         if detect:
-            self.update_bvh()
+            self._refit_queries()
             self._launch_dcd("ee")
             if self.has_triangles:
                 self._launch_dcd("pt")
@@ -754,28 +754,6 @@ class FEMContactSolver(ContactBarrierMixin):
         N.call("ipcb_ls_inertia", fp64, self.soup.n_verts, N.ptr(self.states.x), N.ptr(self.states.x0),
                N.ptr(self.states.xdot), ls["gravity"], self.h, N.ptr(self.mass),
                N.ptr(ls["fixed"]) if ls["any_fixed"] else None, N.ptr(self.x_target), self.k_att, base + 16, s)
-
-    def _ccd_launches(self, dx: torch.Tensor):
-        """collision_free_step without its read: the TOI stays in ccd_toi."""
-        soup = self.soup.c_struct()
-        s = N.stream_handle()
-        pad = 1e-7
-        N.call("ipcb_add_dx", ctypes.byref(soup), N.ptr(dx), N.ptr(self.ccd_x1), s)
-        N.call("ipcb_swept_edge_aabbs", ctypes.byref(soup), N.ptr(self.ccd_x1), pad, N.ptr(self.ccd_edge_lower),
-               N.ptr(self.ccd_edge_upper), s)
-        self.ccd_edge_bvh.refit(self.ccd_edge_lower, self.ccd_edge_upper)
-        self.ccd_toi.fill_(1.0)
-        self._status.zero_()
-        N.call("ipcb_edge_edge_toi", ctypes.byref(soup), N.ptr(self.ccd_x1), ctypes.byref(self.ccd_edge_bvh.c),
-               N.ptr(self.ccd_edge_lower), N.ptr(self.ccd_edge_upper), int(self.disable_self_collision),
-               N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(self._toi_ws), self._toi_ws.numel(), s)
-        if self.has_triangles:
-            N.call("ipcb_swept_triangle_aabbs", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   N.ptr(self.ccd_triangle_lower), N.ptr(self.ccd_triangle_upper), s)
-            self.ccd_triangle_bvh.refit(self.ccd_triangle_lower, self.ccd_triangle_upper)
-            N.call("ipcb_point_triangle_toi", ctypes.byref(soup), N.ptr(self.ccd_x1),
-                   ctypes.byref(self.ccd_triangle_bvh.c), pad, int(self.disable_self_collision),
-                   N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(self._toi_ws), self._toi_ws.numel(), s)
 
     def _ls_buffers(self):
         if self._ls is None:
@@ -869,7 +847,7 @@ class FEMContactSolver(ContactBarrierMixin):
             ls["acc0"].zero_()
             self._energy_launches(ls["acc0"], detect=not fresh)
         self._lists_at_x = False
-        self._ccd_launches(self.states.dx)
+        self._launch_ccd(self.states.dx)
         eps = 1.1920928955078125e-7 if self.dtype == torch.float32 else 2.220446049250313e-16
         N.call("ipcb_ls_begin", N.ptr(ls["state"]), N.ptr(self.ccd_toi), fp64, N.ptr(self._status),
                N.ptr(ls["acc0"]), h2, eps, 64,

@@ -164,12 +164,17 @@ class ContactPipeline(ContactBarrierMixin):
     def _enqueue(self):
         """All stages of iteration(), ending with the copies of counts,
         status, energy and TOI into pinned host memory, on four streams: the
-        triangle side (box refit, PT query, PT records) beside the edge side,
-        and each CCD query (swept boxes, refit, TOI; own candidate workspace)
-        as soon as the discrete query on its hierarchy is done, beside the
-        narrow phase, the contact BSR and the energy.  Nothing after the
-        discrete queries reads the hierarchies, so the CCD refits cannot
-        disturb them; every stream joins the first before the read."""
+        triangle side (PT query, PT records) beside the edge side, and the
+        CCD of each kind as soon as its query is done, beside the narrow
+        phase, the contact BSR and the energy.  With the direction on the
+        device, the discrete and the CCD query of a kind are one walk of its
+        hierarchy (_both_queries: on the screw and nut the swept boxes meet
+        12% more pairs than the discrete ones alone, and a second walk and
+        refit are saved) and only the staged pairs are solved beside the rest;
+        from host memory the CCD queries wait for the direction's copy and
+        walk on their own, bounded by the contacts just found.  Nothing else
+        reads the hierarchies; every stream joins the first before the
+        read."""
         if getattr(self, "bvh_rebuild_interval", 0) or not self.has_triangles:
             return self._enqueue_serial()
         ee, pt = self.contacts_new, self.contacts_pt
@@ -177,8 +182,6 @@ class ContactPipeline(ContactBarrierMixin):
         side, ccd_e, ccd_t = self._side, self._ccd_e, self._ccd_t
         soup = ctypes.byref(self.soup.c_struct())
         kappa = float(self.contact_stiffness)
-        excl = int(self.disable_self_collision)
-        pad = 1e-7
         cap = ee.capacity + pt.capacity
         t = self.collision_triplets
         if t is None or t.rows.shape[0] < 16 * cap:
@@ -189,7 +192,6 @@ class ContactPipeline(ContactBarrierMixin):
         if io is not None:
             self.soup.x_transformed.copy_(io[0], non_blocking=True)
         self.compute_V(ret=False)
-        self._pack()
         self.b.zero_()
         self.ccd_toi.fill_(1.0)
         self._status.zero_()
@@ -202,39 +204,35 @@ class ContactPipeline(ContactBarrierMixin):
                 self._dx_buf.copy_(io[1], non_blocking=True)
                 N.call("ipcb_add_dx", soup, N.ptr(self._dx_buf), N.ptr(self.ccd_x1), N.stream_handle())
                 self._x1_done.record(cin)
+            self._pack()
         side.wait_stream(main)
         with torch.cuda.stream(side):
-            self._triangle_aabbs()
-            self.tri_mesh.refit()
-            self._launch_dcd("pt")
+            if io is None:
+                self._both_queries("pt", self._toi_ws_pt)
+            else:
+                self._refit_triangles()
+                self._launch_dcd("pt")
             self._pt_done.record(side)
-        N.call("ipcb_edge_aabbs", soup, N.ptr(self.x4), float(contact._thickness + contact.buffer),
-               N.ptr(self.bvh_edges_lower), N.ptr(self.bvh_edges_upper), N.stream_handle())
-        self.bvh_edges.refit()
-        self._launch_dcd("ee")
+        if io is None:
+            self._both_queries("ee", self._toi_ws)
+        else:
+            self._refit_edges()
+            self._launch_dcd("ee")
         self._ee_done.record(main)
         with torch.cuda.stream(ccd_e):
             ccd_e.wait_event(self._ee_done)
-            if io is not None:
+            if io is None:
+                self._solve_staged("ee", self._toi_ws)
+            else:
                 ccd_e.wait_event(self._x1_done)
-            s1 = N.stream_handle()
-            N.call("ipcb_swept_edge_aabbs", soup, N.ptr(self.ccd_x1), pad, N.ptr(self.ccd_edge_lower),
-                   N.ptr(self.ccd_edge_upper), s1)
-            self.ccd_edge_bvh.refit(self.ccd_edge_lower, self.ccd_edge_upper)
-            N.call("ipcb_edge_edge_toi", soup, N.ptr(self.ccd_x1), ctypes.byref(self.ccd_edge_bvh.c),
-                   N.ptr(self.ccd_edge_lower), N.ptr(self.ccd_edge_upper), excl, N.ptr(self.ccd_toi),
-                   N.ptr(self._status), N.ptr(self._toi_ws), self._toi_ws.numel(), s1)
+                self._ccd_query("ee", 0, self.soup.n_edges, self._toi_ws)
         with torch.cuda.stream(ccd_t):
             ccd_t.wait_event(self._pt_done)
-            if io is not None:
+            if io is None:
+                self._solve_staged("pt", self._toi_ws_pt)
+            else:
                 ccd_t.wait_event(self._x1_done)
-            s2 = N.stream_handle()
-            N.call("ipcb_swept_triangle_aabbs", soup, N.ptr(self.ccd_x1), pad, N.ptr(self.ccd_triangle_lower),
-                   N.ptr(self.ccd_triangle_upper), s2)
-            self.ccd_triangle_bvh.refit(self.ccd_triangle_lower, self.ccd_triangle_upper)
-            N.call("ipcb_point_triangle_toi", soup, N.ptr(self.ccd_x1), ctypes.byref(self.ccd_triangle_bvh.c), pad,
-                   excl, N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(self._toi_ws_pt),
-                   self._toi_ws_pt.numel(), s2)
+                self._ccd_query("pt", 0, self.soup.n_verts, self._toi_ws_pt)
         contact_hessian_ee(self.states, self.soup, ee, t, self.b, kappa, n=-1, ws=self._ws_ee)
         with torch.cuda.stream(side):
             side.wait_event(self._ee_done)  # the PT records follow the EE count
@@ -277,7 +275,7 @@ class ContactPipeline(ContactBarrierMixin):
             self._dx_buf.copy_(io[1], non_blocking=True)
         self.compute_V(ret=False)
         self._status.zero_()
-        self.update_bvh()
+        self._refit_queries()
         self._launch_dcd("ee")
         if self.has_triangles:
             self._launch_dcd("pt")

@@ -117,33 +117,19 @@ class ShardedContactPipeline(ContactBarrierMixin):
             self.contacts_pt.cnt.zero_()
             first, count = self.pt_range
             N.call("ipcb_dcd_pt_range", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.tri_mesh.c), th,
-                   float(2.0 * (contact._thickness + contact.buffer)), int(self.disable_self_collision), None, first,
+                   float(2.0 * (contact._thickness + contact.buffer)), int(self.disable_self_collision), N.ptr(self._point_order), first,
                    count, ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self._status), s)
 
     def _launch_ccd(self, dx: torch.Tensor, reset_status: bool = True):
         soup = self.soup.c_struct()
         s = N.stream_handle()
-        pad = 1e-7
-        excl = int(self.disable_self_collision)
         N.call("ipcb_add_dx", ctypes.byref(soup), N.ptr(dx), N.ptr(self.ccd_x1), s)
         self.ccd_toi.fill_(1.0)
         if reset_status:
             self._status.zero_()
-        N.call("ipcb_swept_edge_aabbs", ctypes.byref(soup), N.ptr(self.ccd_x1), pad, N.ptr(self.ccd_edge_lower),
-               N.ptr(self.ccd_edge_upper), s)
-        self.ccd_edge_bvh.refit(self.ccd_edge_lower, self.ccd_edge_upper)
-        first, count = self.ee_range
-        N.call("ipcb_edge_edge_toi_range", ctypes.byref(soup), N.ptr(self.ccd_x1), ctypes.byref(self.ccd_edge_bvh.c),
-               N.ptr(self.ccd_edge_lower), N.ptr(self.ccd_edge_upper), excl, first, count, N.ptr(self.ccd_toi),
-               N.ptr(self._status), N.ptr(self._toi_ws), self._toi_ws.numel(), s)
+        self._ccd_query("ee", *self.ee_range, self._toi_ws)
         if self.has_triangles:
-            N.call("ipcb_swept_triangle_aabbs", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   N.ptr(self.ccd_triangle_lower), N.ptr(self.ccd_triangle_upper), s)
-            self.ccd_triangle_bvh.refit(self.ccd_triangle_lower, self.ccd_triangle_upper)
-            first, count = self.pt_range
-            N.call("ipcb_point_triangle_toi_range", ctypes.byref(soup), N.ptr(self.ccd_x1),
-                   ctypes.byref(self.ccd_triangle_bvh.c), pad, excl, first, count, N.ptr(self.ccd_toi),
-                   N.ptr(self._status), N.ptr(self._toi_ws), self._toi_ws.numel(), s)
+            self._ccd_query("pt", *self.pt_range, self._toi_ws)
 
     # --------------------------------------------------------- iteration
     def iteration(self, dx: torch.Tensor) -> ShardResult:

@@ -1,0 +1,96 @@
+"""The packed tree the queries walk (csrc/tree.cuh): candidate sets and TOI
+against the oracle at sizes around its block, group and level edges (32, 1024
+and 32768 leaves), for the discrete query, the CCD query with and without a
+contact list to start from, and both in one walk (gpu)."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import sort_records
+from ipc_warp_b200.pipeline import ContactPipeline
+from ipc_warp_b200.scenes import Scene
+from oracle import pyoracle as po
+
+pytestmark = pytest.mark.gpu
+
+
+def loose_triangles(n, seed, dhat=0.02):
+    """n separate triangles (3n edges, 3n vertices) in a box that keeps a few
+    neighbours per triangle; a third of them far away, so that blocks of the
+    Morton order span the gap."""
+    rng = np.random.default_rng(seed)
+    side = max(0.35, 0.22 * n ** (1 / 3))
+    c = rng.uniform(0, side, size=(n, 1, 3))
+    c[: n // 3] += 40.0 * side
+    x = (c + rng.uniform(-0.1, 0.1, size=(n, 3, 3))).reshape(-1, 3)
+    t = np.arange(3 * n).reshape(n, 3)
+    edges = np.concatenate([t[:, [0, 1]], t[:, [1, 2]], t[:, [0, 2]]])
+    return Scene(name="loose", x=x, xcs=x.copy(), edges=edges.astype(np.int32).ravel(),
+                 triangles=t.astype(np.int32).ravel(), body=np.repeat(np.arange(n) % 3, 3).astype(np.int32),
+                 tets=np.zeros((0, 4), np.int32), dhat=dhat, kappa=1.0)
+
+
+@pytest.mark.parametrize("n", [1, 10, 11, 341, 342, 10922, 10923])
+@pytest.mark.parametrize("fp64", [False, True])
+def test_tree_queries_match_oracle(cuda, n, fp64):
+    sc = loose_triangles(n, seed=n)
+    dtype = torch.float64 if fp64 else torch.float32
+    excl = n % 2 == 0
+    pipe = ContactPipeline.from_scene(sc, dtype=dtype, device=cuda, exclude_same_body=excl)
+    rng = np.random.default_rng(n + 1)
+    dx = torch.tensor(rng.normal(scale=0.01, size=sc.x.shape), dtype=dtype, device=cuda)
+    x0 = pipe.soup.x_transformed.cpu().numpy()
+    x32 = x0.astype(np.float32)
+    th = np.float32(sc.thickness)
+    kw = dict(exclude_same_body=excl)
+    ee = sort_records(po.dcd_ee(x32, sc.edges, sc.body, th, **kw))
+    pt = sort_records(po.dcd_pt(x32, sc.triangles, sc.body, th, **kw))
+    x1 = (x0 - dx.cpu().numpy())
+    toi, st = po.scene_toi(x0, x1, sc.edges, sc.triangles, sc.body, fp64=fp64, **kw)
+    assert st == 0
+    if n >= 341:
+        assert len(ee) and len(pt) and toi < 1.0
+
+    def check(bound):
+        assert np.array_equal(sort_records(pipe.contacts_new.records(pipe.n_contacts).cpu().numpy()), ee)
+        assert np.array_equal(sort_records(pipe.contacts_pt.records(pipe.n_contacts_pt).cpu().numpy()), pt)
+        got = float(pipe.ccd_toi.item())
+        assert got <= toi and toi - got <= 1e-6
+        assert bound == (0.9 * got if got < 1.0 else 1.0)
+        return got
+
+    alone = None
+    bound = pipe.collision_free_step(dx)  # no contact list yet
+    pipe.detect_collision()
+    alone = check(bound)
+    assert check(pipe.collision_free_step(dx)) == alone  # started from the list
+    for _ in range(2):  # eager, then the replayed graph: one walk for both queries
+        r = pipe.iteration(dx)
+        assert r.status == 0 and (r.n_ee, r.n_pt) == (len(ee), len(pt))
+        assert check(r.alpha) == alone
+    pipe.iteration(-dx)  # the lists now belong to the same positions, another direction
+    assert check(pipe.collision_free_step(dx)) == alone
+    # the lists may be of other positions: only their pairs are tried
+    x = pipe.soup.x_transformed.clone()
+    pipe.soup.x_transformed.add_(torch.tensor(rng.normal(scale=0.05, size=sc.x.shape), dtype=dtype, device=cuda))
+    pipe.detect_collision()
+    pipe.soup.x_transformed.copy_(x)
+    assert pipe.collision_free_step(dx) == bound
+
+
+def test_both_queries_with_a_small_staging_list(cuda):
+    """Pairs that do not fit the staging list send the staged CCD to the pass
+    that solves in place; the discrete records are not affected."""
+    from ipc_warp_b200 import _native as N
+
+    sc = loose_triangles(342, seed=5)
+    pipe = ContactPipeline.from_scene(sc, dtype=torch.float32, device=cuda)
+    pipe.use_graph = False
+    rng = np.random.default_rng(6)
+    dx = torch.tensor(rng.normal(scale=0.01, size=sc.x.shape), dtype=torch.float32, device=cuda)
+    full = pipe.iteration(dx)
+    for cap in (16, 0):
+        pipe._toi_ws = torch.empty(N.size("ipcb_toi_workspace", cap), dtype=torch.uint8, device=cuda)
+        pipe._toi_ws_pt = torch.empty_like(pipe._toi_ws)
+        small = pipe.iteration(dx)
+        assert (small.n_ee, small.n_pt, small.alpha, small.status) == (full.n_ee, full.n_pt, full.alpha, 0)

@@ -184,6 +184,8 @@ def stage_times(pipe, dx, reps, torch):
         N.call("ipcb_add_dx", ctypes.byref(pipe.soup.c_struct()), N.ptr(dx), N.ptr(pipe.ccd_x1), N.stream_handle())
         pipe.ccd_toi.fill_(1.0)
         pipe._status.zero_()
+        pipe.contacts_new.cnt.zero_()
+        pipe.contacts_pt.cnt.zero_()
         marks = [("start", ev())]
         # box refit and the walk that finds the discrete records and stages
         # the pairs that can touch within the step

@@ -174,6 +174,17 @@ int ipcb_dcd_pt_range(const ipcb_soup* soup, const float* x4, const ipcb_lbvh* t
                       float query_pad, int exclude_same_body, const int* query_order, int first, int count,
                       ipcb_contacts* out, int* status, ipcb_stream s);
 
+/* The two ends of a contact iteration, one launch each.  begin: b = 0, x1 =
+ * x - dx (dx may be null: x1 untouched), both list counts, both status words
+ * and the energy 0, toi 1.  results: the counts, the two status words
+ * (counts_out[0..3]), the energy and the TOI written to memory the device can
+ * reach (pinned host memory). */
+int ipcb_iteration_begin(const ipcb_soup* soup, const void* dx, void* x1, void* b, int* ee_cnt, int* pt_cnt,
+                         int* status, int* bsr_status, double* energy, void* toi, ipcb_stream s);
+int ipcb_iteration_results(int fp64, const int* ee_cnt, const int* pt_cnt, const int* bsr_status, const int* status,
+                           const double* energy, const void* toi, int* counts_out, double* energy_out, void* toi_out,
+                           ipcb_stream s);
+
 /* ---- narrow phase (dynamic_contacts.py:152-246 contact_hessian_ee/pt, 375-398 energy) ----
  * kind 0 = EE list, 1 = PT list.  n >= 0: number of records; n < 0: read
  * min(*list->cnt, capacity) on the device (graph-capturable).
@@ -656,6 +667,14 @@ size_t ipcb_contact_bsr_workspace(int n_records, int n_verts);
 int ipcb_contact_bsr(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, int n_verts,
                      const void* vals, const unsigned short* block_mask, int fp64, int* offsets, int* columns,
                      void* values, int* nnz, int* status, void* ws, size_t ws_bytes, ipcb_stream s);
+/* ipcb_contact_bsr in its two parts on one workspace: the records bucketed by
+ * row, which needs the lists only and can run beside the narrow phase, then
+ * the pattern and the blocks. */
+int ipcb_contact_bsr_rows(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, int n_verts, void* ws,
+                          size_t ws_bytes, ipcb_stream s);
+int ipcb_contact_bsr_blocks(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, int n_verts,
+                            const void* vals, const unsigned short* block_mask, int fp64, int* offsets, int* columns,
+                            void* values, int* nnz, int* status, void* ws, size_t ws_bytes, ipcb_stream s);
 /* y = alpha*A*x + beta*y for a 3x3 BSR (bsr_mv) */
 int ipcb_bsr_mv(int nrow, const int* offsets, const int* columns, const void* values, int fp64, const void* x,
                 void* y, double alpha, double beta, ipcb_stream s);

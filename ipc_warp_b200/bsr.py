@@ -79,34 +79,51 @@ def bsr_from_triplets(nrow: int, ncol: int, rows: torch.Tensor, cols: torch.Tens
     return out
 
 
+def contact_bsr_buffers(n_records: int, n_verts: int, dtype, device, out: BsrMatrix | None = None) -> BsrMatrix:
+    """``out``, or a new matrix, with room (and workspace) for the contact
+    matrix of n_records records."""
+    cap = max(16 * n_records, 1)
+    if out is None or out.columns.shape[0] < cap or out.nrow != n_verts or out.dtype != dtype:
+        out = BsrMatrix(n_verts, n_verts, cap, dtype, device)
+    nbytes = N.size("ipcb_contact_bsr_workspace", n_records, n_verts)
+    if out._ws is None or out._ws.numel() < nbytes:
+        out._ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    return out
+
+
 def contact_bsr(ee, n_ee: int | None, pt, n_pt: int | None, n_verts: int, trip: Triplets,
                 out: BsrMatrix | None = None, status: torch.Tensor | None = None,
-                read_status: bool = True) -> tuple[BsrMatrix, int | None]:
+                read_status: bool = True, part: str = "all") -> tuple[BsrMatrix, int | None]:
     """BSR of the contact Hessian from the EE/PT lists and their triplets
     (16 blocks per record, EE first, with block masks).  Returns (matrix, status);
     status has IPCB_STATUS_ROW_OVERFLOW (4) set when a row had too many
     distinct columns for the fast path (the matrix is then incomplete).
     n_ee / n_pt None: the lists' counts are read on the device (sizes follow
     the capacities).  read_status=False: no host read; the status stays in
-    ``status`` (device) and None is returned in its place."""
+    ``status`` (device) and None is returned in its place.
+    part "rows", then "blocks" (with the matrix "rows" returned): the same in
+    two calls; "rows" needs the lists only and can run beside the narrow
+    phase, "blocks" takes ``status`` as it is (the caller has zeroed it)."""
     vals = trip.vals
     dtype, dev = vals.dtype, vals.device
     ne = ee.capacity if n_ee is None else n_ee
     npt = pt.capacity if n_pt is None else n_pt
-    cap = max(16 * (ne + npt), 1)
-    if out is None or out.columns.shape[0] < cap or out.nrow != n_verts or out.dtype != dtype:
-        out = BsrMatrix(n_verts, n_verts, cap, dtype, dev)
-    st = torch.zeros(1, dtype=torch.int32, device=dev) if status is None else status.zero_()
-    nbytes = N.size("ipcb_contact_bsr_workspace", ne + npt, n_verts)
-    ws = getattr(out, "_ws", None)
-    if ws is None or ws.numel() < nbytes:
-        ws = out._ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    out = contact_bsr_buffers(ne + npt, n_verts, dtype, dev, out)
+    ws = out._ws
+    if part == "all":
+        st = torch.zeros(1, dtype=torch.int32, device=dev) if status is None else status.zero_()
+    else:
+        st = status
     import ctypes
 
-    N.call("ipcb_contact_bsr", ctypes.byref(ee.c_struct()), -1 if n_ee is None else n_ee,
-           ctypes.byref(pt.c_struct()), -1 if n_pt is None else n_pt, n_verts,
-           N.ptr(vals), N.ptr(trip.mask), int(dtype == torch.float64), N.ptr(out.offsets), N.ptr(out.columns),
-           N.ptr(out.values), N.ptr(out.nnz_dev), N.ptr(st), N.ptr(ws), ws.numel(), N.stream_handle())
+    lists = (ctypes.byref(ee.c_struct()), -1 if n_ee is None else n_ee, ctypes.byref(pt.c_struct()),
+             -1 if n_pt is None else n_pt, n_verts)
+    if part == "rows":
+        N.call("ipcb_contact_bsr_rows", *lists, N.ptr(ws), ws.numel(), N.stream_handle())
+        return out, None
+    N.call("ipcb_contact_bsr" if part == "all" else "ipcb_contact_bsr_blocks", *lists, N.ptr(vals), N.ptr(trip.mask),
+           int(dtype == torch.float64), N.ptr(out.offsets), N.ptr(out.columns), N.ptr(out.values),
+           N.ptr(out.nnz_dev), N.ptr(st), N.ptr(ws), ws.numel(), N.stream_handle())
     return out, (int(st.item()) if read_status else None)
 
 

@@ -360,18 +360,17 @@ class ContactSolverBase:
     def _both_queries(self, which: str, ws: torch.Tensor):
         """The discrete and the CCD query of one kind in one walk of its
         hierarchy (direction in ccd_x1): records into the contact list, the
-        pairs that can touch within the step into ``ws``."""
+        pairs that can touch within the step into ``ws``.  The caller has
+        zeroed the list's count."""
         soup = self.soup.c_struct()
         pad = 1e-7
         excl = int(self.disable_self_collision)
         s = N.stream_handle()
         if which == "ee":
-            self.contacts_new.cnt.zero_()
             N.call("ipcb_edge_edge_both", ctypes.byref(soup), N.ptr(self.ccd_x1), pad, ctypes.byref(self.bvh_edges.c),
                    float(_thickness), float(_thickness + buffer), excl, ctypes.byref(self.contacts_new.c_struct()),
                    N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(ws), ws.numel(), s)
         else:
-            self.contacts_pt.cnt.zero_()
             N.call("ipcb_point_triangle_both", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
                    ctypes.byref(self.tri_mesh.c), float(_thickness), float(2.0 * (_thickness + buffer)),
                    N.ptr(self._point_order), excl, ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self.ccd_toi),

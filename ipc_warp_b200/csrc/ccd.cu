@@ -1364,9 +1364,7 @@ void collect(const Query<S>& q) {
         q.exclude, q.thickness, q.out, q.cand, o, q.toi, q.status, q.sink, gate);
 }
 
-inline void clear_header(void* ws, cudaStream_t st) {
-  cudaMemsetAsync(ws, 0, (2 + 2 * kBuckets + 1) * sizeof(int), st);
-}
+constexpr int kHeaderWords = 2 + 2 * kBuckets + 1;  // zero when a query starts staging
 
 // The staged pairs (in bucket order without a sink), then -- a small grid that
 // returns at once unless the staging list overflowed -- every pair in place.
@@ -1389,7 +1387,7 @@ void solve(const Query<S>& q) {
 // Boxes given (EE: also the query boxes): stage and solve.
 template <class S, int KIND>
 void run_boxes(const Query<S>& q) {
-  clear_header(q.ws, q.st);
+  cudaMemsetAsync(q.ws, 0, kHeaderWords * sizeof(int), q.st);
   collect<S, KIND, kStage>(q);
   solve<S, KIND>(q);
 }
@@ -1399,13 +1397,13 @@ template <class S, int KIND>
 void run_step(const Query<S>& q, const ipcb_contacts* seeds) {
   const S* x0 = (const S*)q.soup->x;
   const int* prims = KIND == 0 ? q.soup->edges : q.soup->triangles;
-  clear_header(q.ws, q.st);
   if (seeds)
     k_seed<S, KIND><<<kSeedLanes / 64, 64, 0, q.st>>>(x0, q.x1, prims, q.soup->body,
                                                       KIND == 0 ? q.soup->n_edges : q.soup->n_verts,
                                                       KIND == 0 ? q.soup->n_edges : q.soup->n_tris, q.exclude, q.pad,
                                                       *seeds, q.toi, q.status);
-  tree::refit(q.bvh, SweptBox<S, KIND == 0 ? 2 : 3>{x0, q.x1, prims, q.pad, q.toi}, q.st);
+  tree::refit(q.bvh, SweptBox<S, KIND == 0 ? 2 : 3>{x0, q.x1, prims, q.pad, q.toi}, q.st, (int*)q.ws,
+              kHeaderWords);
   collect<S, KIND, kStage>(q);
   solve<S, KIND>(q);
 }
@@ -1415,8 +1413,8 @@ void run_step(const Query<S>& q, const ipcb_contacts* seeds) {
 template <class S, int KIND>
 void run_both(const Query<S>& q, float box_reach) {
   const int* prims = KIND == 0 ? q.soup->edges : q.soup->triangles;
-  clear_header(q.ws, q.st);
-  tree::refit(q.bvh, BothBox<S, KIND == 0 ? 2 : 3>{(const S*)q.soup->x, q.x1, prims, q.pad, box_reach}, q.st);
+  tree::refit(q.bvh, BothBox<S, KIND == 0 ? 2 : 3>{(const S*)q.soup->x, q.x1, prims, q.pad, box_reach}, q.st,
+              (int*)q.ws, kHeaderWords);
   collect<S, KIND, kBoth>(q);
 }
 

@@ -7,8 +7,8 @@
 // vertices).  A row's distinct columns are few (tens), so:
 //   1. thread per record: count the quads of each row and take each quad's
 //      arrival slot in its row (atomics; a row's first arrival also appends
-//      the row to the list of touched rows); scan the counts; scatter the
-//      quad ids to their rows (arrival order)
+//      the row to the list of touched rows); hand each touched row a range of
+//      quad slots; scatter the quad ids to their rows (arrival order)
 //   2. pass A, warp per row: sort the row's quad ids (so the order, and every
 //      sum below, is the same on every run), insert the columns of the
 //      non-zero blocks (the narrow phase's per-record block masks) into a
@@ -46,15 +46,23 @@ IPCB_D int4 record_ids(const int* __restrict__ ee, int n_ee, const int* __restri
 }
 IPCB_D int comp(int4 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); }
 
-// nrec = {EE records, PT records}: host values, or min(*cnt, capacity) of
-// the lists read on the device (graph-capturable; no host read of the counts)
-// nrec[2]: touched rows; nrec[3], nrec[4]: the work counters of passes A, B
-__global__ void k_counts(const int* __restrict__ ee_cnt, int ee_n, const int* __restrict__ pt_cnt, int pt_n,
-                         int* __restrict__ nrec) {
-  nrec[0] = ee_cnt ? min(max(*ee_cnt, 0), ee_n) : ee_n;
-  nrec[1] = pt_cnt ? min(max(*pt_cnt, 0), pt_n) : pt_n;
-  nrec[2] = nrec[3] = nrec[4] = 0;
-}
+// The lists' record counts: host values, or min(*cnt, capacity) read on the
+// device (graph-capturable; no host read of the counts).
+struct Counts {
+  const int* ee_cnt;
+  const int* pt_cnt;
+  int ee_n, pt_n;
+  IPCB_D int ee() const { return ee_cnt ? min(max(*ee_cnt, 0), ee_n) : ee_n; }
+  IPCB_D int pt() const { return pt_cnt ? min(max(*pt_cnt, 0), pt_n) : pt_n; }
+};
+
+// Counters of one assembly, zero at its start (cleared with the row counts).
+struct Work {
+  int rows;    // touched rows
+  int quads;   // quad slots handed out
+  int next_a;  // work counters of passes A, B
+  int next_b;
+};
 
 IPCB_D int arrive(int* __restrict__ row_cnt, int row, int* __restrict__ rows, int* __restrict__ nrows) {
   const int s = atomicAdd(row_cnt + row, 1);
@@ -62,16 +70,17 @@ IPCB_D int arrive(int* __restrict__ row_cnt, int row, int* __restrict__ rows, in
   return s;
 }
 
-__global__ void k_rec_slots(int* __restrict__ nrec, const int* __restrict__ ee, const int* __restrict__ pt,
-                            int4* __restrict__ slots, int* __restrict__ row_cnt, int* __restrict__ rows) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x, n_ee = nrec[0];
-  if (p >= n_ee + nrec[1]) return;
+__global__ void k_rec_slots(Counts C, Work* __restrict__ work, const int* __restrict__ ee,
+                            const int* __restrict__ pt, int4* __restrict__ slots, int* __restrict__ row_cnt,
+                            int* __restrict__ rows) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, n_ee = C.ee();
+  if (p >= n_ee + C.pt()) return;
   const int4 v = record_ids(ee, n_ee, pt, p);
   int4 s;
-  s.x = arrive(row_cnt, v.x, rows, nrec + 2);
-  s.y = arrive(row_cnt, v.y, rows, nrec + 2);
-  s.z = arrive(row_cnt, v.z, rows, nrec + 2);
-  s.w = arrive(row_cnt, v.w, rows, nrec + 2);
+  s.x = arrive(row_cnt, v.x, rows, &work->rows);
+  s.y = arrive(row_cnt, v.y, rows, &work->rows);
+  s.z = arrive(row_cnt, v.z, rows, &work->rows);
+  s.w = arrive(row_cnt, v.w, rows, &work->rows);
   slots[p] = s;
 }
 
@@ -83,10 +92,27 @@ IPCB_D int next_row(int* __restrict__ work, const int* __restrict__ rows, int nr
   return r < nrows ? __ldg(rows + r) : -1;
 }
 
-__global__ void k_rec_scatter(const int* __restrict__ nrec, const int* __restrict__ ee, const int* __restrict__ pt,
+// Each touched row's range of quad slots, in any order (a row's quads are
+// sorted in pass A, and no result depends on where its range lies): one warp
+// reservation per 32 rows, where a prefix sum would run over every vertex.
+__global__ void k_row_ranges(Work* __restrict__ work, const int* __restrict__ rows, const int* __restrict__ row_cnt,
+                             int* __restrict__ qstart) {
+  const int lane = threadIdx.x & 31, n = work->rows;
+  for (int first = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; first < n; first += gridDim.x * blockDim.x) {
+    const int row = first + lane < n ? __ldg(rows + first + lane) : -1;
+    const int c = row >= 0 ? row_cnt[row] : 0;
+    const int incl = scan::warp_inclusive(c, lane);
+    int base = 0;
+    if (lane == 31) base = atomicAdd(&work->quads, incl);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (row >= 0) qstart[row] = base + incl - c;
+  }
+}
+
+__global__ void k_rec_scatter(Counts C, const int* __restrict__ ee, const int* __restrict__ pt,
                               const int4* __restrict__ slots, const int* __restrict__ qstart, int* __restrict__ qids) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x, n_ee = nrec[0];
-  if (p >= n_ee + nrec[1]) return;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x, n_ee = C.ee();
+  if (p >= n_ee + C.pt()) return;
   const int4 v = record_ids(ee, n_ee, pt, p), s = slots[p];
   qids[qstart[v.x] + s.x] = 4 * p;
   qids[qstart[v.y] + s.y] = 4 * p + 1;
@@ -195,8 +221,9 @@ IPCB_D unsigned quad_mask(const unsigned short* __restrict__ bmask, int q) {
 // sorted, and every quad gets its 4 column positions through a slot ->
 // position table.
 __global__ void __launch_bounds__(kWarps * 32, 12)
-    k_row_columns(const int* __restrict__ rows, const int* __restrict__ qstart, int* __restrict__ qids,
-                  const int* __restrict__ ee, int* __restrict__ nrec, const int* __restrict__ pt,
+    k_row_columns(Counts C, Work* __restrict__ work, const int* __restrict__ rows, const int* __restrict__ qstart,
+                  const int* __restrict__ row_cnt, int* __restrict__ qids, const int* __restrict__ ee,
+                  const int* __restrict__ pt,
                   const unsigned short* __restrict__ bmask, int* __restrict__ tmpcols, unsigned* __restrict__ qpos,
                   int* __restrict__ row_nnz, int* __restrict__ status) {
   __shared__ int sq[kWarps][kSmemQuads];
@@ -204,10 +231,11 @@ __global__ void __launch_bounds__(kWarps * 32, 12)
   __shared__ int scol[kWarps][kHash];
   __shared__ unsigned char slot_pos[kWarps][kHash];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_ee = nrec[0], nrows = nrec[2];
-  for (int row = next_row(nrec + 3, rows, nrows, lane); row >= 0; row = next_row(nrec + 3, rows, nrows, lane)) {
+  const int n_ee = C.ee(), nrows = work->rows;
+  int* next = &work->next_a;
+  for (int row = next_row(next, rows, nrows, lane); row >= 0; row = next_row(next, rows, nrows, lane)) {
   __syncwarp();  // the previous row's shared-memory reads are done
-  const int b = qstart[row], n = qstart[row + 1] - b;
+  const int b = qstart[row], n = row_cnt[row];
   // the row's quads in quad-id order
   int nq2 = 32;
   while (nq2 < n) nq2 <<= 1;
@@ -311,8 +339,9 @@ __global__ void __launch_bounds__(kWarps * 32, 12)
 // within a batch a fixed tree over the group's lanes), so the result is
 // deterministic, and each column takes one shared-memory add per batch.
 template <class S>
-__global__ void __launch_bounds__(kWarps * 32) k_row_values(const int* __restrict__ rows, int* __restrict__ nrec,
+__global__ void __launch_bounds__(kWarps * 32) k_row_values(Work* __restrict__ work, const int* __restrict__ rows,
                                                             const int* __restrict__ qstart,
+                                                            const int* __restrict__ row_cnt,
                                                             const int* __restrict__ qids,
                                                             const unsigned* __restrict__ qpos,
                                                             const S* __restrict__ vals,
@@ -326,10 +355,11 @@ __global__ void __launch_bounds__(kWarps * 32) k_row_values(const int* __restric
   constexpr int kVec = 36 * (int)sizeof(S) / 16;  // 16-byte vectors per quad
   const unsigned full = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nrows = nrec[2];
-  for (int row = next_row(nrec + 4, rows, nrows, lane); row >= 0; row = next_row(nrec + 4, rows, nrows, lane)) {
+  const int nrows = work->rows;
+  int* next = &work->next_b;
+  for (int row = next_row(next, rows, nrows, lane); row >= 0; row = next_row(next, rows, nrows, lane)) {
   __syncwarp();  // the previous row's shared-memory reads are done
-  int b = qstart[row], e = qstart[row + 1];
+  const int b = qstart[row], e = b + row_cnt[row];
   const int out = offsets[row], cnt = min(offsets[row + 1] - out, kHash);
   if (cnt == 0) continue;  // a row whose blocks are all zero
   for (int k = lane; k < cnt; k += 32) {
@@ -395,43 +425,60 @@ __global__ void __launch_bounds__(kWarps * 32) k_row_values(const int* __restric
   }
 }
 
-__global__ void k_total(int nrow, int* __restrict__ offsets, const int* __restrict__ total, int* __restrict__ nnz) {
-  offsets[nrow] = *total;
-  *nnz = *total;
+// The workspace of an assembly.
+struct Layout {
+  int4* slots;     // per record: its quads' arrival slots
+  int* qids;       // quad ids row by row
+  unsigned* qpos;  // per quad: its 4 column positions
+  Work* work;      // followed by row_cnt (cleared together)
+  int* row_cnt;
+  int* qstart;
+  int* rows;
+  int* tmpcols;
+  void* scratch;
+};
+
+Layout layout(void* ws, int records, int nv) {
+  const size_t NQ = 4 * (size_t)(records > 0 ? records : 1), R = (size_t)(nv > 0 ? nv : 0) + 1;
+  char* p = (char*)ws;
+  Layout l;
+  l.slots = (int4*)p; p += al(NQ * 4);
+  l.qids = (int*)p; p += al(NQ * 4);
+  l.qpos = (unsigned*)p; p += al(NQ * 4);
+  l.work = (Work*)p;
+  l.row_cnt = (int*)(p + sizeof(Work)); p += al(sizeof(Work) + R * 4);
+  l.qstart = (int*)p; p += al(R * 4);
+  l.rows = (int*)p; p += al(R * 4);
+  l.tmpcols = (int*)p; p += al(NQ * 4 * 4);
+  l.scratch = p;
+  return l;
+}
+
+// The quads bucketed by row: needs the lists only, so it can run beside the
+// narrow phase.
+void bucket_rows(const Counts& C, int nv, const int* ee, const int* pt, const Layout& l, cudaStream_t st) {
+  const int P = C.ee_n + C.pt_n;
+  cudaMemsetAsync(l.work, 0, sizeof(Work) + (size_t)nv * sizeof(int), st);
+  k_rec_slots<<<div_up(P, 256), 256, 0, st>>>(C, l.work, ee, pt, l.slots, l.row_cnt, l.rows);
+  const long long max_rows = std::min<long long>(nv, 4LL * P);
+  k_row_ranges<<<(int)std::min<long long>(148 * 4, div_up(max_rows, 256)), 256, 0, st>>>(l.work, l.rows, l.row_cnt,
+                                                                                         l.qstart);
+  k_rec_scatter<<<div_up(P, 256), 256, 0, st>>>(C, ee, pt, l.slots, l.qstart, l.qids);
 }
 
 template <class S>
-int assemble(int n_ee, int n_pt, const int* ee_cnt, const int* pt_cnt, int nv, const int* ee, const int* pt,
-             const S* vals, const unsigned short* bmask, int* offsets, int* columns, S* values, int* nnz, int* status,
-             void* ws, cudaStream_t st) {
-  const int P = n_ee + n_pt;  // records, or their bound when the counts are read on the device
-  size_t NQ = 4 * (size_t)P, R = (size_t)nv + 1;
-  char* p = (char*)ws;
-  int4* slots = (int4*)p; p += al(NQ * 4);
-  int* qids = (int*)p; p += al(NQ * 4);
-  unsigned* qpos = (unsigned*)p; p += al(NQ * 4);
-  int* qstart = (int*)p; p += al(R * 4);
-  int* rows = (int*)p; p += al(R * 4);
-  int* tmpcols = (int*)p; p += al(NQ * 4 * 4);
-  int* total = (int*)p; p += 256;
-  int* nrec = (int*)p; p += 256;
-  void* scratch = p;
-  cudaMemsetAsync(qstart, 0, R * sizeof(int), st);
+void row_blocks(const Counts& C, int nv, const int* ee, const int* pt, const S* vals, const unsigned short* bmask,
+                int* offsets, int* columns, S* values, int* nnz, int* status, const Layout& l, cudaStream_t st) {
   cudaMemsetAsync(offsets, 0, (size_t)nv * sizeof(int), st);  // rows without contact: no blocks
-  k_counts<<<1, 1, 0, st>>>(ee_cnt, n_ee, pt_cnt, n_pt, nrec);
-  k_rec_slots<<<div_up(P, 256), 256, 0, st>>>(nrec, ee, pt, slots, qstart, rows);
-  scan::exclusive<int>(qstart, (int)R, scratch, total, st);
-  k_rec_scatter<<<div_up(P, 256), 256, 0, st>>>(nrec, ee, pt, slots, qstart, qids);
   // persistent warps over the touched rows (at most min(nv, 4 P) of them)
-  const long long max_rows = std::min<long long>(nv, NQ);
+  const long long max_rows = std::min<long long>(nv, 4LL * (C.ee_n + C.pt_n));
   const int ga = (int)std::min<long long>(148 * 12, div_up(max_rows, kWarps));
   const int gb = (int)std::min<long long>(148 * 8, div_up(max_rows, kWarps));
-  k_row_columns<<<ga, kWarps * 32, 0, st>>>(rows, qstart, qids, ee, nrec, pt, bmask, tmpcols, qpos, offsets, status);
-  scan::exclusive<int>(offsets, nv, scratch, total, st);
-  k_total<<<1, 1, 0, st>>>(nv, offsets, total, nnz);
-  k_row_values<S><<<gb, kWarps * 32, 0, st>>>(rows, nrec, qstart, qids, qpos, vals, tmpcols, offsets, columns,
-                                              values);
-  return check_launch("ipcb_contact_bsr");
+  k_row_columns<<<ga, kWarps * 32, 0, st>>>(C, l.work, l.rows, l.qstart, l.row_cnt, l.qids, ee, pt, bmask, l.tmpcols,
+                                            l.qpos, offsets, status);
+  scan::exclusive<int>(offsets, nv, l.scratch, offsets + nv, st, nnz);
+  k_row_values<S><<<gb, kWarps * 32, 0, st>>>(l.work, l.rows, l.qstart, l.row_cnt, l.qids, l.qpos, vals, l.tmpcols,
+                                              offsets, columns, values);
 }
 
 }  // namespace
@@ -443,34 +490,65 @@ extern "C" {
 
 size_t ipcb_contact_bsr_workspace(int n_records, int n_verts) {
   size_t NQ = 4 * (size_t)(n_records > 0 ? n_records : 1), R = (size_t)(n_verts > 0 ? n_verts : 0) + 1;
-  return al(NQ * 4) * 3 + 2 * al(R * 4) + al(NQ * 16) + 512 + scan::scratch_bytes((int)R);
+  return al(NQ * 4) * 3 + al(sizeof(Work) + R * 4) + 2 * al(R * 4) + al(NQ * 16) + scan::scratch_bytes((int)R);
 }
 
-int ipcb_contact_bsr(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, int n_verts,
-                     const void* vals, const unsigned short* block_mask, int fp64, int* offsets, int* columns,
-                     void* values, int* nnz, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
-  if (!ee || !pt || n_verts < 0 || !offsets || !nnz || !status) return IPCB_E_ARG;
-  // a negative count: min(*cnt, capacity) of that list, read on the device
-  const int* ee_cnt = n_ee < 0 ? ee->cnt : nullptr;
-  const int* pt_cnt = n_pt < 0 ? pt->cnt : nullptr;
-  if ((n_ee < 0 && !ee_cnt) || (n_pt < 0 && !pt_cnt)) return IPCB_E_ARG;
-  if (n_ee < 0) n_ee = ee->capacity;
-  if (n_pt < 0) n_pt = pt->capacity;
-  if (n_ee > ee->capacity || n_pt > pt->capacity || (long long)4 * (n_ee + n_pt) > 0x7fffffff) return IPCB_E_ARG;
+// a negative count: min(*cnt, capacity) of that list, read on the device
+static bool counts_of(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, Counts& C) {
+  if (!ee || !pt) return false;
+  C.ee_cnt = n_ee < 0 ? ee->cnt : nullptr;
+  C.pt_cnt = n_pt < 0 ? pt->cnt : nullptr;
+  if ((n_ee < 0 && !C.ee_cnt) || (n_pt < 0 && !C.pt_cnt)) return false;
+  C.ee_n = n_ee < 0 ? ee->capacity : n_ee;
+  C.pt_n = n_pt < 0 ? pt->capacity : n_pt;
+  return C.ee_n <= ee->capacity && C.pt_n <= pt->capacity && (long long)4 * (C.ee_n + C.pt_n) <= 0x7fffffff;
+}
+
+int ipcb_contact_bsr_rows(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, int n_verts, void* ws,
+                          size_t ws_bytes, ipcb_stream s) {
+  Counts C;
+  if (n_verts < 0 || !counts_of(ee, n_ee, pt, n_pt, C)) return IPCB_E_ARG;
+  if (C.ee_n + C.pt_n == 0 || n_verts == 0) return IPCB_OK;
+  if (!ws || ws_bytes < ipcb_contact_bsr_workspace(C.ee_n + C.pt_n, n_verts)) return IPCB_E_ARG;
+  bucket_rows(C, n_verts, ee->a1a2b1b2, pt->a1a2b1b2, layout(ws, C.ee_n + C.pt_n, n_verts), (cudaStream_t)s);
+  return check_launch("ipcb_contact_bsr_rows");
+}
+
+int ipcb_contact_bsr_blocks(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, int n_verts,
+                            const void* vals, const unsigned short* block_mask, int fp64, int* offsets, int* columns,
+                            void* values, int* nnz, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
+  Counts C;
+  if (n_verts < 0 || !offsets || !nnz || !status || !counts_of(ee, n_ee, pt, n_pt, C)) return IPCB_E_ARG;
   cudaStream_t st = (cudaStream_t)s;
-  if (n_ee + n_pt == 0 || n_verts == 0) {
+  if (C.ee_n + C.pt_n == 0 || n_verts == 0) {
     cudaMemsetAsync(offsets, 0, (size_t)(n_verts + 1) * sizeof(int), st);
     cudaMemsetAsync(nnz, 0, sizeof(int), st);
     return check_launch("ipcb_contact_bsr");
   }
   if (!vals || !block_mask || !columns || !values || !ws ||
-      ws_bytes < ipcb_contact_bsr_workspace(n_ee + n_pt, n_verts))
+      ws_bytes < ipcb_contact_bsr_workspace(C.ee_n + C.pt_n, n_verts))
     return IPCB_E_ARG;
+  const Layout l = layout(ws, C.ee_n + C.pt_n, n_verts);
   if (fp64)
-    return assemble<double>(n_ee, n_pt, ee_cnt, pt_cnt, n_verts, ee->a1a2b1b2, pt->a1a2b1b2, (const double*)vals,
-                            block_mask, offsets, columns, (double*)values, nnz, status, ws, st);
-  return assemble<float>(n_ee, n_pt, ee_cnt, pt_cnt, n_verts, ee->a1a2b1b2, pt->a1a2b1b2, (const float*)vals,
-                         block_mask, offsets, columns, (float*)values, nnz, status, ws, st);
+    row_blocks<double>(C, n_verts, ee->a1a2b1b2, pt->a1a2b1b2, (const double*)vals, block_mask, offsets, columns,
+                       (double*)values, nnz, status, l, st);
+  else
+    row_blocks<float>(C, n_verts, ee->a1a2b1b2, pt->a1a2b1b2, (const float*)vals, block_mask, offsets, columns,
+                      (float*)values, nnz, status, l, st);
+  return check_launch("ipcb_contact_bsr");
+}
+
+int ipcb_contact_bsr(const ipcb_contacts* ee, int n_ee, const ipcb_contacts* pt, int n_pt, int n_verts,
+                     const void* vals, const unsigned short* block_mask, int fp64, int* offsets, int* columns,
+                     void* values, int* nnz, int* status, void* ws, size_t ws_bytes, ipcb_stream s) {
+  Counts C;
+  if (n_verts < 0 || !offsets || !nnz || !status || !counts_of(ee, n_ee, pt, n_pt, C)) return IPCB_E_ARG;
+  // every argument of the second part is checked before anything is launched
+  if (C.ee_n + C.pt_n > 0 && n_verts > 0 && (!vals || !block_mask || !columns || !values)) return IPCB_E_ARG;
+  const int rc = ipcb_contact_bsr_rows(ee, n_ee, pt, n_pt, n_verts, ws, ws_bytes, s);
+  if (rc != IPCB_OK) return rc;
+  return ipcb_contact_bsr_blocks(ee, n_ee, pt, n_pt, n_verts, vals, block_mask, fp64, offsets, columns, values, nnz,
+                                 status, ws, ws_bytes, s);
 }
 
 }  // extern "C"

@@ -1,5 +1,8 @@
-// Device-wide exclusive prefix sum of int32/uint32 in three launches:
-// block-local scan -> scan of the block totals (one block, looping) -> add.
+// Device-wide exclusive prefix sum of int32/uint32: a block-local scan, then
+// an add whose blocks each sum the totals before their own (two launches; a
+// launch of a tenth of the work costs as much as it does).  Above kMaxBlocks
+// blocks the totals are scanned by a launch of their own, as each block would
+// read too many of them.
 #pragma once
 #include "common.cuh"
 
@@ -53,7 +56,8 @@ __global__ void __launch_bounds__(kBlock) k_local(int n, T* __restrict__ a, T* _
 }
 
 template <class T>
-__global__ void __launch_bounds__(kBlock) k_sums(int nb, T* __restrict__ sums, T* __restrict__ total) {
+__global__ void __launch_bounds__(kBlock) k_sums(int nb, T* __restrict__ sums, T* __restrict__ total,
+                                                 T* __restrict__ total2) {
   __shared__ T s[32];
   T carry = T(0);
   for (int base = 0; base < nb; base += kBlock) {
@@ -65,6 +69,7 @@ __global__ void __launch_bounds__(kBlock) k_sums(int nb, T* __restrict__ sums, T
     carry += tot;
   }
   if (threadIdx.x == 0 && total) *total = carry;
+  if (threadIdx.x == 0 && total2) *total2 = carry;
 }
 
 template <class T>
@@ -73,15 +78,37 @@ __global__ void k_add(int n, T* __restrict__ a, const T* __restrict__ sums) {
   if (t < n) a[t] += sums[blockIdx.x];
 }
 
-// exclusive scan of a[0..n) in place; *total (device, may be null) = sum.
-// scratch: scratch_bytes(n) bytes.
+constexpr int kMaxBlocks = 2048;
+
 template <class T>
-inline void exclusive(T* a, int n, void* scratch, T* total, cudaStream_t st) {
+__global__ void __launch_bounds__(kBlock) k_add_totals(int n, T* __restrict__ a, const T* __restrict__ sums,
+                                                       T* __restrict__ total, T* __restrict__ total2) {
+  __shared__ T s[32];
+  T before = T(0);
+  for (int t = threadIdx.x; t < (int)blockIdx.x; t += kBlock) before += sums[t];
+  T sum;
+  block_exclusive(before, s, sum);
+  const int t = blockIdx.x * kBlock + threadIdx.x;
+  if (t < n) a[t] += sum;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    if (total) *total = sum + sums[blockIdx.x];
+    if (total2) *total2 = sum + sums[blockIdx.x];
+  }
+}
+
+// exclusive scan of a[0..n) in place; *total, *total2 (device, may be null) =
+// sum.  scratch: scratch_bytes(n) bytes.
+template <class T>
+inline void exclusive(T* a, int n, void* scratch, T* total, cudaStream_t st, T* total2 = nullptr) {
   if (n <= 0) return;
   int nb = blocks(n);
   T* sums = (T*)scratch;
   k_local<T><<<nb, kBlock, 0, st>>>(n, a, sums);
-  k_sums<T><<<1, kBlock, 0, st>>>(nb, sums, total);
+  if (nb <= kMaxBlocks) {
+    k_add_totals<T><<<nb, kBlock, 0, st>>>(n, a, sums, total, total2);
+    return;
+  }
+  k_sums<T><<<1, kBlock, 0, st>>>(nb, sums, total, total2);
   k_add<T><<<nb, kBlock, 0, st>>>(n, a, sums);
 }
 

@@ -97,13 +97,16 @@ constexpr float kBig = 3.4e38f;
 // A block of 256 threads forms 1024 leaves (four a thread, so four gathers are
 // in flight), their 32 level-1 boxes and one level-2 box; the block that
 // finishes last (a counter it resets) reduces the levels above.  Box is a
-// functor: box(primitive, lo, hi).
+// functor: box(primitive, lo, hi).  clear: up to 256 words zeroed on the way
+// (a memset of its own costs a launch).
 template <class Box>
 __global__ void __launch_bounds__(256) k_tree(Box box, const int* __restrict__ order,
-                                              const __grid_constant__ View v, unsigned* counter) {
+                                              const __grid_constant__ View v, unsigned* counter,
+                                              int* clear, int n_clear) {
   __shared__ f3 slo[32], shi[32];
   __shared__ unsigned arrived;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && (int)threadIdx.x < n_clear) clear[threadIdx.x] = 0;
   int prim[4];
   f3 lo[4], hi[4];
 #pragma unroll
@@ -173,10 +176,10 @@ __global__ void __launch_bounds__(256) k_tree(Box box, const int* __restrict__ o
 }
 
 template <class Box>
-inline void refit(const ipcb_lbvh* b, Box box, cudaStream_t s) {
+inline void refit(const ipcb_lbvh* b, Box box, cudaStream_t s, int* clear = nullptr, int n_clear = 0) {
   if (b->n <= 0) return;
   // flags[n - 1] is not a node's arrival counter (internal nodes end at n - 2)
-  k_tree<Box><<<div_up(b->n, 1024), 256, 0, s>>>(box, b->sorted, view(b), b->flags + (b->n - 1));
+  k_tree<Box><<<div_up(b->n, 1024), 256, 0, s>>>(box, b->sorted, view(b), b->flags + (b->n - 1), clear, n_clear);
 }
 
 struct BoxArray {  // boxes given as float[3n] lower / upper

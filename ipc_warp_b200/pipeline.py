@@ -22,7 +22,7 @@ import torch
 from . import _native as N
 from . import contact
 from .contact import Soup
-from .bsr import Triplets, contact_bsr
+from .bsr import Triplets, contact_bsr, contact_bsr_buffers
 from .dynamic_contacts import (ContactBarrierMixin, contact_energy_ee, contact_energy_pt, contact_hessian_ee,
                                contact_hessian_pt_after, hessian_workspace)
 
@@ -66,11 +66,13 @@ class ContactPipeline(ContactBarrierMixin):
             self._side = torch.cuda.Stream(device=dev)
             self._ccd_e = torch.cuda.Stream(device=dev)
             self._ccd_t = torch.cuda.Stream(device=dev)
+            self._rows = torch.cuda.Stream(device=dev)
             self._copy_in = torch.cuda.Stream(device=dev)
             self._copy_out = torch.cuda.Stream(device=dev)
             self._x1_done = torch.cuda.Event()
             self._ee_done = torch.cuda.Event()
             self._pt_done = torch.cuda.Event()
+            self._rows_done = torch.cuda.Event()
             self._toi_ws_pt = torch.empty_like(self._toi_ws)
         self._dx_buf = torch.zeros_like(soup.x_transformed)
         self._host_io = None  # (x, dx, b) pinned host tensors during iteration_host
@@ -163,7 +165,7 @@ class ContactPipeline(ContactBarrierMixin):
 
     def _enqueue(self):
         """All stages of iteration(), ending with the copies of counts,
-        status, energy and TOI into pinned host memory, on four streams: the
+        status, energy and TOI into pinned host memory, on five streams: the
         triangle side (PT query, PT records) beside the edge side, and the
         CCD of each kind as soon as its query is done, beside the narrow
         phase, the contact BSR and the energy.  With the direction on the
@@ -179,7 +181,7 @@ class ContactPipeline(ContactBarrierMixin):
             return self._enqueue_serial()
         ee, pt = self.contacts_new, self.contacts_pt
         main = torch.cuda.current_stream()
-        side, ccd_e, ccd_t = self._side, self._ccd_e, self._ccd_t
+        side, ccd_e, ccd_t, rows = self._side, self._ccd_e, self._ccd_t, self._rows
         soup = ctypes.byref(self.soup.c_struct())
         kappa = float(self.contact_stiffness)
         cap = ee.capacity + pt.capacity
@@ -188,16 +190,16 @@ class ContactPipeline(ContactBarrierMixin):
             t = self.collision_triplets = Triplets.zeros(16 * cap, self.soup.xcs.dtype, self.device)
         self._ws_ee = hessian_workspace(ee, getattr(self, "_ws_ee", None))
         self._ws_pt = hessian_workspace(pt, getattr(self, "_ws_pt", None))
+        H = self.collision_hessian = contact_bsr_buffers(cap, self.soup.n_verts, self.soup.xcs.dtype, self.device,
+                                                         self.collision_hessian)
         io = self._host_io
         if io is not None:
             self.soup.x_transformed.copy_(io[0], non_blocking=True)
         self.compute_V(ret=False)
-        self.b.zero_()
-        self.ccd_toi.fill_(1.0)
-        self._status.zero_()
-        if io is None:
-            N.call("ipcb_add_dx", soup, N.ptr(self._dx_buf), N.ptr(self.ccd_x1), N.stream_handle())
-        else:  # the direction crosses the bus beside the discrete queries
+        N.call("ipcb_iteration_begin", soup, N.ptr(self._dx_buf) if io is None else None, N.ptr(self.ccd_x1),
+               N.ptr(self.b), N.ptr(ee.cnt), N.ptr(pt.cnt), N.ptr(self._status), N.ptr(self._bsr_status),
+               N.ptr(self._energy), N.ptr(self.ccd_toi), N.stream_handle())
+        if io is not None:  # the direction crosses the bus beside the discrete queries
             cin = self._copy_in
             cin.wait_stream(main)
             with torch.cuda.stream(cin):
@@ -233,6 +235,15 @@ class ContactPipeline(ContactBarrierMixin):
             else:
                 ccd_t.wait_event(self._x1_done)
                 self._ccd_query("pt", 0, self.soup.n_verts, self._toi_ws_pt)
+        # the records bucketed by row, and the energy: of the lists only
+        with torch.cuda.stream(rows):
+            rows.wait_event(self._ee_done)
+            rows.wait_event(self._pt_done)
+            contact_bsr(ee, None, pt, None, self.soup.n_verts, t, out=H, status=self._bsr_status, read_status=False,
+                        part="rows")
+            self._rows_done.record(rows)
+            contact_energy_ee(self.states, self.soup, ee, self._energy, kappa, n=-1)
+            contact_energy_pt(self.states, self.soup, pt, self._energy, kappa, n=-1)
         contact_hessian_ee(self.states, self.soup, ee, t, self.b, kappa, n=-1, ws=self._ws_ee)
         with torch.cuda.stream(side):
             side.wait_event(self._ee_done)  # the PT records follow the EE count
@@ -243,28 +254,23 @@ class ContactPipeline(ContactBarrierMixin):
             cout.wait_stream(main)
             with torch.cuda.stream(cout):
                 io[2].copy_(self.b, non_blocking=True)
-        H, _ = contact_bsr(ee, None, pt, None, self.soup.n_verts, t, out=self.collision_hessian,
-                           status=self._bsr_status, read_status=False)
-        self.collision_hessian = H
-        e = self._energy.zero_()
-        contact_energy_ee(self.states, self.soup, ee, e, kappa, n=-1)
-        contact_energy_pt(self.states, self.soup, pt, e, kappa, n=-1)
+        main.wait_event(self._rows_done)
+        contact_bsr(ee, None, pt, None, self.soup.n_verts, t, out=H, status=self._bsr_status, read_status=False,
+                    part="blocks")
+        main.wait_stream(rows)
         main.wait_stream(ccd_e)
         main.wait_stream(ccd_t)
         if io is not None:
             main.wait_stream(self._copy_in)
             main.wait_stream(self._copy_out)
-        self._copy_results(e)
+        self._copy_results(self._energy)
 
     def _copy_results(self, e):
-        ee, pt = self.contacts_new, self.contacts_pt
+        """Counts, statuses, the energy e and the TOI into the pinned words."""
         h = self._readback
-        h["counts"][0:1].copy_(ee.cnt, non_blocking=True)
-        h["counts"][1:2].copy_(pt.cnt, non_blocking=True)
-        h["counts"][2:3].copy_(self._bsr_status, non_blocking=True)
-        h["counts"][3:4].copy_(self._status, non_blocking=True)
-        h["energy"].copy_(e, non_blocking=True)
-        h["toi"].copy_(self.ccd_toi, non_blocking=True)
+        N.call("ipcb_iteration_results", int(self.soup.xcs.dtype == torch.float64), N.ptr(self.contacts_new.cnt),
+               N.ptr(self.contacts_pt.cnt), N.ptr(self._bsr_status), N.ptr(self._status), N.ptr(e),
+               N.ptr(self.ccd_toi), N.ptr(h["counts"]), N.ptr(h["energy"]), N.ptr(h["toi"]), N.stream_handle())
 
     def _enqueue_serial(self):
         """_enqueue on one stream (periodic BVH rebuilds, or no triangles)."""

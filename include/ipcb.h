@@ -562,6 +562,17 @@ int ipcb_newton_values(int fp64, const int* nnz, int capacity, const int* c_rows
                        const int* src_b, const int* gather_off, const int* gather_idx, const void* tet_vals,
                        double tet_scale, const void* diag, const void* contact_vals, double contact_scale,
                        void* values, ipcb_stream s);
+/* The same when the elastic values were gathered before (ipcb_newton_values
+ * on the fixed pattern alone): values = a_vals[src_a] + b_scale * b_vals[src_b]
+ * (an absent source counts 0). */
+int ipcb_union_values(int fp64, const int* nnz, int capacity, const int* src_a, const void* a_vals, const int* src_b,
+                      const void* b_vals, double b_scale, void* values, ipcb_stream s);
+/* rhs = -h^2 b + m (x - (x0 + h xdot + h^2 g)) + h^2 k_att (x - target) on the
+ * fixed vertices (compute_rhs, time_integrator_base.py:82-91, 428-438), formed
+ * in double; gravity: double[3] on the device, fixed: one byte a vertex. */
+int ipcb_newton_rhs(int fp64, int n, const void* b, const void* x, const void* x0, const void* xdot,
+                    const double* gravity, double h, const double* mass, const unsigned char* fixed,
+                    const void* target, double k_att, void* rhs, ipcb_stream s);
 
 /* ---- Device-side line search (time_integrator_base.py:514-546) ----
  * State of one backtracking search in device memory.  ipcb_ls_begin: E0 from

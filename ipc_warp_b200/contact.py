@@ -19,7 +19,7 @@ from __future__ import annotations
 
 import ctypes
 import warnings
-from contextlib import nullcontext
+from contextlib import contextmanager, nullcontext
 from dataclasses import dataclass
 
 import torch
@@ -169,6 +169,23 @@ class ContactSolverBase:
         cap = max(1 << 20, 4 * max(n_edges, n_nodes))
         self._toi_ws = torch.empty(N.size("ipcb_toi_workspace", cap), dtype=torch.uint8, device=dev)
         self._counts_host = torch.zeros(3, dtype=torch.int32).pin_memory() if dev.type == "cuda" else None
+
+    # ------------------------------------------------------------- branches
+    @contextmanager
+    def _branch(self, k: int):
+        """Launches on side stream k, after what the current stream has
+        queued; _join(k) makes the current stream wait for them.  Works inside
+        stream capture (the branches become parallel paths of the graph)."""
+        streams = self.__dict__.setdefault("_branches", {})
+        if k not in streams:
+            streams[k] = torch.cuda.Stream(device=self.device)
+        streams[k].wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(streams[k]):
+            yield streams[k]
+
+    def _join(self, *ks: int):
+        for k in ks:
+            torch.cuda.current_stream().wait_stream(self._branches[k])
 
     # --------------------------------------------------------------- hooks
     def profile_timer(self, name):
@@ -334,9 +351,14 @@ class ContactSolverBase:
         self.ccd_toi.fill_(1.0)
         if reset_status:
             self._status.zero_()
+        if self.has_triangles:  # the two queries side by side, each with its own staging list
+            if getattr(self, "_toi_ws_pt", None) is None:
+                self._toi_ws_pt = torch.empty_like(self._toi_ws)
+            with self._branch(0):
+                self._ccd_query("pt", 0, self.soup.n_verts, self._toi_ws_pt)
         self._ccd_query("ee", 0, self.soup.n_edges, self._toi_ws)
         if self.has_triangles:
-            self._ccd_query("pt", 0, self.soup.n_verts, self._toi_ws)
+            self._join(0)
 
     def _ccd_query(self, which: str, first: int, count: int, ws: torch.Tensor):
         """One CCD query of the step x -> ccd_x1 on the current stream: boxes

@@ -210,6 +210,44 @@ __global__ void k_newton_values(const int* __restrict__ nnz, int capacity, const
   }
 }
 
+// values = a's values (placed by src_a) + b_scale * b's values (by src_b): the
+// union's values when a's were gathered before (the elastic part, formed
+// beside the contact queries).  One thread per (slot, component).
+template <class S>
+__global__ void __launch_bounds__(256) k_union_values(const int* __restrict__ nnz, int capacity,
+                                                      const int* __restrict__ src_a, const S* __restrict__ a_vals,
+                                                      const int* __restrict__ src_b, const S* __restrict__ b_vals,
+                                                      S b_scale, S* __restrict__ vals) {
+  const long long n = 9LL * min(*nnz, capacity);
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const int p = (int)(t / 9), c = (int)(t - 9LL * p);
+    const int sa = __ldg(src_a + p), sb = __ldg(src_b + p);
+    S v = sa >= 0 ? __ldg(a_vals + 9LL * sa + c) : S(0);
+    if (sb >= 0) v += b_scale * __ldg(b_vals + 9LL * sb + c);
+    vals[t] = v;
+  }
+}
+
+// gradient of the incremental potential (time_integrator_base.py:82-91,
+// 428-438): every operation rounds on its own in double, in the order
+// -h^2 b + m (x - ((x0 + h v) + h^2 g)) + (h^2 k) f (x - target)
+template <class S>
+__global__ void __launch_bounds__(256) k_newton_rhs(int n, const S* __restrict__ b, const S* __restrict__ x,
+                                                    const S* __restrict__ x0, const S* __restrict__ xdot,
+                                                    const double* __restrict__ gravity, double h,
+                                                    const double* __restrict__ mass,
+                                                    const unsigned char* __restrict__ fixed,
+                                                    const S* __restrict__ target, double k_att, S* __restrict__ out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * n) return;
+  const int i = t / 3, c = t - 3 * i;
+  const double h2 = xmul(h, h), xi = (double)x[t];
+  const double xt = xadd(xadd((double)x0[t], xmul(h, (double)xdot[t])), xmul(h2, gravity[c]));
+  double g = xadd(xmul(-h2, (double)b[t]), xmul(mass[i], xsub(xi, xt)));
+  if (fixed[i]) g = xadd(g, xmul(xmul(h2, k_att), xsub(xi, (double)target[t])));
+  out[t] = (S)g;
+}
+
 }  // namespace
 }  // namespace ipcb
 
@@ -310,6 +348,37 @@ int ipcb_newton_values(int fp64, const int* nnz, int capacity, const int* c_rows
                                                  (const float*)tet_vals, (float)tet_scale, (const float*)diag,
                                                  (const float*)contact_vals, (float)contact_scale, (float*)values);
   return check_launch("ipcb_newton_values");
+}
+
+int ipcb_union_values(int fp64, const int* nnz, int capacity, const int* src_a, const void* a_vals, const int* src_b,
+                      const void* b_vals, double b_scale, void* values, ipcb_stream s) {
+  if (!nnz || capacity < 0 || !src_a || !a_vals || !src_b || !b_vals || !values) return IPCB_E_ARG;
+  if (capacity == 0) return IPCB_OK;
+  const int grid = 148 * 8;
+  if (fp64)
+    k_union_values<double><<<grid, 256, 0, (cudaStream_t)s>>>(nnz, capacity, src_a, (const double*)a_vals, src_b,
+                                                              (const double*)b_vals, b_scale, (double*)values);
+  else
+    k_union_values<float><<<grid, 256, 0, (cudaStream_t)s>>>(nnz, capacity, src_a, (const float*)a_vals, src_b,
+                                                             (const float*)b_vals, (float)b_scale, (float*)values);
+  return check_launch("ipcb_union_values");
+}
+
+int ipcb_newton_rhs(int fp64, int n, const void* b, const void* x, const void* x0, const void* xdot,
+                    const double* gravity, double h, const double* mass, const unsigned char* fixed,
+                    const void* target, double k_att, void* rhs, ipcb_stream s) {
+  if (n < 0 || !b || !x || !x0 || !xdot || !gravity || !mass || !fixed || !target || !rhs) return IPCB_E_ARG;
+  if (n == 0) return IPCB_OK;
+  const int grid = div_up(3LL * n, 256);
+  if (fp64)
+    k_newton_rhs<double><<<grid, 256, 0, (cudaStream_t)s>>>(n, (const double*)b, (const double*)x, (const double*)x0,
+                                                            (const double*)xdot, gravity, h, mass, fixed,
+                                                            (const double*)target, k_att, (double*)rhs);
+  else
+    k_newton_rhs<float><<<grid, 256, 0, (cudaStream_t)s>>>(n, (const float*)b, (const float*)x, (const float*)x0,
+                                                           (const float*)xdot, gravity, h, mass, fixed,
+                                                           (const float*)target, k_att, (float*)rhs);
+  return check_launch("ipcb_newton_rhs");
 }
 
 }  // extern "C"

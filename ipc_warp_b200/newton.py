@@ -27,7 +27,7 @@ import torch
 from . import _native as N
 from . import contact as contact_mod
 from .autotune import Autotuner, bucket
-from .bsr import BsrMatrix, Triplets, bsr_from_triplets, bsr_mv, contact_bsr
+from .bsr import BsrMatrix, Triplets, bsr_from_triplets, bsr_mv, contact_bsr, contact_bsr_buffers
 from .contact import QUERY_FAILED, Soup
 from .dynamic_contacts import (ContactBarrierMixin, contact_hessian_ee, contact_hessian_pt, contact_hessian_pt_after,
                                hessian_workspace)
@@ -378,57 +378,85 @@ class FEMContactSolver(ContactBarrierMixin):
             A = self.A = BsrMatrix(V, V, cap, self.dtype, self.device)
             for k in ("a_rows", "src_a", "src_b"):
                 st[k] = torch.empty(cap, dtype=torch.int32, device=self.device)
+        # here and not while capturing: a new matrix's zero fill would be
+        # captured, and replayed with every call
+        self._C = contact_bsr_buffers(cap_rec, V, self.dtype, self.device, getattr(self, "_C", None))
+        self._sorted_workspaces()
+        if "s_vals" not in st:
+            st["s_vals"] = torch.empty((st["nnz"], 3, 3), dtype=self.dtype, device=self.device)
         if "graph_read" not in st:
             st["graph_read"] = torch.zeros(4, dtype=torch.int32, pin_memory=True)
         return min(A.columns.shape[0], st["a_rows"].shape[0])
 
     def _enqueue_A(self, cfg, cap: int):
         """compute_A's launches with every count read on the device: box
-        refits and the discrete queries, the per-iteration terms on schedule
-        ``cfg``, the contact BSR of the lists' capacities, the union with the
-        elastic pattern and its values; ends with the copy of the two list
-        counts and the two status words into pinned host memory."""
+        refits and the discrete queries (the two kinds side by side), the
+        per-iteration terms on schedule ``cfg`` (per-kind: the tets, with
+        their gather into the elastic pattern, beside the queries), the
+        contact BSR of the lists' capacities, the union with the elastic
+        pattern and its values; ends with the copy of the two list counts and
+        the two status words into pinned host memory."""
         st = self._static
         h2 = self.h * self.h
         V = self.soup.n_verts
+        fp64 = int(self.dtype == torch.float64)
         ee, pt = self.contacts_new, self.contacts_pt
         t = self.collision_triplets
-        s = N.stream_handle()
+        kappa = float(self.contact_stiffness)
+        S, A = st["S"], self.A
+        C = self._C
+
+        def elastic_values():  # the elastic part on its own pattern
+            N.call("ipcb_newton_values", fp64, N.ptr(S.nnz_dev), st["nnz"], N.ptr(st["rows"]), N.ptr(S.columns),
+                   N.ptr(st["own"]), N.ptr(st["none"]), N.ptr(st["g_off"]), N.ptr(st["g_idx"]), N.ptr(st["tet_vals"]),
+                   h2, N.ptr(st["diag"]), None, 0.0, N.ptr(st["s_vals"]), N.stream_handle())
+
         self.b.zero_()
         self.compute_V(ret=False)
         self._status.zero_()
-        self._refit_queries()
+        st["status"].zero_()
+        separate = cfg[0] == "separate"
+        if separate:
+            with self._branch(1):
+                N.call("ipcb_tet_hessian", self.material, fp64, N.ptr(self.states.x), N.ptr(self.tets), self.n_tets,
+                       N.ptr(self.Bm), N.ptr(self.W), self.mu, self.lam, None, None, N.ptr(st["tet_vals"]),
+                       N.ptr(self.b), N.stream_handle())
+                elastic_values()
+        self._pack()
+        with self._branch(0):
+            if self.has_triangles:
+                self._refit_triangles()
+                self._launch_dcd("pt")
+            else:
+                pt.cnt.zero_()
+        self._refit_edges()
         self._launch_dcd("ee")
-        if self.has_triangles:
-            self._launch_dcd("pt")
-        else:
-            pt.cnt.zero_()
-        kappa = float(self.contact_stiffness)
-        if cfg[0] == "separate":
-            self._ws_ee = hessian_workspace(ee, getattr(self, "_ws_ee", None))
-            self._ws_pt = hessian_workspace(pt, getattr(self, "_ws_pt", None))
+        self._join(0)
+        with self._branch(2):  # of the lists only
+            contact_bsr(ee, None, pt, None, V, t, out=C, status=st["status"], read_status=False, part="rows")
+        if separate:
+            with self._branch(0):
+                contact_hessian_pt_after(None, self.soup, pt, t, self.b, ee, kappa, ws=self._ws_pt)
             contact_hessian_ee(None, self.soup, ee, t, self.b, kappa, n=-1, ws=self._ws_ee)
-            contact_hessian_pt_after(None, self.soup, pt, t, self.b, ee, kappa, ws=self._ws_pt)
-            N.call("ipcb_tet_hessian", self.material, int(self.dtype == torch.float64), N.ptr(self.states.x),
-                   N.ptr(self.tets), self.n_tets, N.ptr(self.Bm), N.ptr(self.W), self.mu, self.lam, None, None,
-                   N.ptr(st["tet_vals"]), N.ptr(self.b), s)
+            self._join(0)
         else:
-            Tc = N.Terms(int(self.dtype == torch.float64), N.ptr(self.states.x), N.ptr(self.soup.xcs),
-                         ee.c_struct(), pt.c_struct(), kappa, N.ptr(t.rows), N.ptr(t.cols), N.ptr(t.vals),
-                         N.ptr(t.mask), self.material, N.ptr(self.tets), self.n_tets, N.ptr(self.Bm), N.ptr(self.W),
-                         self.mu, self.lam, None, None, N.ptr(st["tet_vals"]), N.ptr(self.b), N.ptr(st["queue"]),
-                         *self._sorted_workspaces())
+            Tc = N.Terms(fp64, N.ptr(self.states.x), N.ptr(self.soup.xcs), ee.c_struct(), pt.c_struct(), kappa,
+                         N.ptr(t.rows), N.ptr(t.cols), N.ptr(t.vals), N.ptr(t.mask), self.material, N.ptr(self.tets),
+                         self.n_tets, N.ptr(self.Bm), N.ptr(self.W), self.mu, self.lam, None, None,
+                         N.ptr(st["tet_vals"]), N.ptr(self.b), N.ptr(st["queue"]), N.ptr(self._ws_ee),
+                         N.ptr(self._ws_pt))
             launch_terms(Tc, cfg, self._n_sm)
-        C, _ = contact_bsr(ee, None, pt, None, V, t, out=getattr(self, "_C", None), status=st["status"],
-                           read_status=False)
-        self._C = C
-        S, A = st["S"], self.A
+            with self._branch(1):
+                elastic_values()
+        self._join(2)
+        contact_bsr(ee, None, pt, None, V, t, out=C, status=st["status"], read_status=False, part="blocks")
+        s = N.stream_handle()
         N.call("ipcb_bsr_union", V, N.ptr(S.offsets), N.ptr(S.columns), N.ptr(C.offsets), N.ptr(C.columns),
                N.ptr(A.offsets), N.ptr(st["a_rows"]), N.ptr(A.columns), N.ptr(st["src_a"]), N.ptr(st["src_b"]), cap,
                N.ptr(A.nnz_dev), N.ptr(st["status"]), N.ptr(st["ws"]), st["ws"].numel(), s)
-        N.call("ipcb_newton_values", int(self.dtype == torch.float64), N.ptr(A.nnz_dev), cap, N.ptr(st["a_rows"]),
-               N.ptr(A.columns), N.ptr(st["src_a"]), N.ptr(st["src_b"]), N.ptr(st["g_off"]), N.ptr(st["g_idx"]),
-               N.ptr(st["tet_vals"]), h2, N.ptr(st["diag"]), N.ptr(C.values), h2, N.ptr(A.values), s)
+        self._join(1)
+        N.call("ipcb_union_values", fp64, N.ptr(A.nnz_dev), cap, N.ptr(st["src_a"]), N.ptr(st["s_vals"]),
+               N.ptr(st["src_b"]), N.ptr(C.values), h2, N.ptr(A.values), s)
         r = st["graph_read"]
         r[0:1].copy_(ee.cnt, non_blocking=True)
         r[1:2].copy_(pt.cnt, non_blocking=True)
@@ -539,6 +567,13 @@ class FEMContactSolver(ContactBarrierMixin):
                             queue=torch.zeros(1, dtype=torch.int32, device=dev),
                             status=torch.zeros(1, dtype=torch.int32, device=dev),
                             ws=torch.empty(N.size("ipcb_bsr_union_workspace", V), dtype=torch.uint8, device=dev))
+        # the fixed pattern as a source of its own union: its values can be
+        # gathered beside the contact queries
+        counts = (S.offsets[1:] - S.offsets[:-1]).long()
+        self._static.update(
+            rows=torch.repeat_interleave(torch.arange(V, dtype=torch.int32, device=dev), counts, output_size=nnz),
+            own=torch.arange(nnz, dtype=torch.int32, device=dev),
+            none=torch.full((nnz,), -1, dtype=torch.int32, device=dev))
         n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
         self._n_sm = n_sm
         self._tuner = Autotuner("terms", terms_candidates())
@@ -626,12 +661,11 @@ class FEMContactSolver(ContactBarrierMixin):
 
     def compute_rhs(self) -> torch.Tensor:
         """time_integrator_base.py:82-91,428-438: gradient of the total energy."""
-        h2 = self.h * self.h
-        x = self.states.x.double()
-        g = -h2 * self.b.double() + self.mass[:, None] * (x - self.x_tilde())
-        if bool(self.fixed.any()):
-            g = g + (h2 * self.k_att) * self.fixed.double()[:, None] * (x - self.x_target.double())
-        self.rhs = g.to(self.dtype)
+        st = self.states
+        self.rhs = torch.empty_like(self.b)
+        N.call("ipcb_newton_rhs", int(self.dtype == torch.float64), self.soup.n_verts, N.ptr(self.b), N.ptr(st.x),
+               N.ptr(st.x0), N.ptr(st.xdot), N.ptr(self.gravity), self.h, N.ptr(self.mass), N.ptr(self.fixed),
+               N.ptr(self.x_target), self.k_att, N.ptr(self.rhs), N.stream_handle())
         return self.rhs
 
     def _direct(self):
@@ -733,27 +767,43 @@ class FEMContactSolver(ContactBarrierMixin):
         at the current x into acc: [0] elastic Psi, [1] barrier, [2] inertia +
         attachment.  Contact lists are refilled by the DCD (their counts stay
         on the device), or, with detect=False, taken as they are."""
-        s = N.stream_handle()
         fp64 = int(self.dtype == torch.float64)
         kappa = float(self.contact_stiffness)
-        if detect:
-            self._refit_queries()
-            self._launch_dcd("ee")
-            if self.has_triangles:
-                self._launch_dcd("pt")
         soup = self.soup.c_struct()
         base = acc.data_ptr()
-        N.call("ipcb_contact_energy", 0, ctypes.byref(soup), ctypes.byref(self.contacts_new.c_struct()), -1, kappa,
-               base + 8, s)
-        if self.has_triangles:
-            N.call("ipcb_contact_energy", 1, ctypes.byref(soup), ctypes.byref(self.contacts_pt.c_struct()), -1,
-                   kappa, base + 8, s)
-        N.call("ipcb_tet_energy", self.material, fp64, N.ptr(self.states.x), N.ptr(self.tets), self.n_tets,
-               N.ptr(self.Bm), N.ptr(self.W), self.mu, self.lam, base, s)
         ls = self._ls
-        N.call("ipcb_ls_inertia", fp64, self.soup.n_verts, N.ptr(self.states.x), N.ptr(self.states.x0),
-               N.ptr(self.states.xdot), ls["gravity"], self.h, N.ptr(self.mass),
-               N.ptr(ls["fixed"]) if ls["any_fixed"] else None, N.ptr(self.x_target), self.k_att, base + 16, s)
+        # the tets and the inertia beside the contacts, the two kinds of
+        # contact side by side
+        with self._branch(1):
+            s = N.stream_handle()
+            N.call("ipcb_tet_energy", self.material, fp64, N.ptr(self.states.x), N.ptr(self.tets), self.n_tets,
+                   N.ptr(self.Bm), N.ptr(self.W), self.mu, self.lam, base, s)
+            N.call("ipcb_ls_inertia", fp64, self.soup.n_verts, N.ptr(self.states.x), N.ptr(self.states.x0),
+                   N.ptr(self.states.xdot), ls["gravity"], self.h, N.ptr(self.mass),
+                   N.ptr(ls["fixed"]) if ls["any_fixed"] else None, N.ptr(self.x_target), self.k_att, base + 16, s)
+        rebuild = getattr(self, "bvh_rebuild_interval", 0)
+        if detect:
+            if rebuild:
+                self.update_bvh()
+            else:
+                self._pack()
+        if self.has_triangles:
+            with self._branch(0):
+                if detect:
+                    if not rebuild:
+                        self._refit_triangles()
+                    self._launch_dcd("pt")
+                N.call("ipcb_contact_energy", 1, ctypes.byref(soup), ctypes.byref(self.contacts_pt.c_struct()), -1,
+                       kappa, base + 8, N.stream_handle())
+        if detect:
+            if not rebuild:
+                self._refit_edges()
+            self._launch_dcd("ee")
+        N.call("ipcb_contact_energy", 0, ctypes.byref(soup), ctypes.byref(self.contacts_new.c_struct()), -1, kappa,
+               base + 8, N.stream_handle())
+        if self.has_triangles:
+            self._join(0)
+        self._join(1)
 
     def _ls_buffers(self):
         if self._ls is None:
@@ -824,6 +874,46 @@ class FEMContactSolver(ContactBarrierMixin):
             if end_rc != 0:
                 raise N.NativeError("ipcb_graph_while_end failed: " + (N.lib().ipcb_last_error() or b"").decode())
 
+    def _ls_prelude(self, mode: str):
+        """Everything before the trials: x kept, E0, the CCD bound, the search
+        state.  Replayed from a graph from the second search on (per mode and
+        buffer set): the launches alone take the host longer than the GPU."""
+        ls = self._ls
+        key = (mode, self._ls_key(), self._toi_ws.data_ptr(), self.ccd_toi.data_ptr(), contact_mod._thickness,
+               contact_mod.buffer, self.disable_self_collision, float(self.contact_stiffness), self.h, self.material,
+               self.mu, self.lam, self.k_att)
+        graphs = ls.setdefault("prelude", {})
+        if len(graphs) > 8:  # buffers that came and went
+            graphs.clear()
+        g = graphs.get(key)
+        if isinstance(g, torch.cuda.CUDAGraph):
+            g.replay()
+            return
+        if g is None or getattr(self, "bvh_rebuild_interval", 0):
+            graphs[key] = 1
+            self._ls_prelude_launches(mode)
+            return
+        graph = torch.cuda.CUDAGraph()
+        with N.no_collection(), torch.cuda.graph(graph):
+            self._ls_prelude_launches(mode)
+        graphs[key] = graph
+        graph.replay()
+
+    def _ls_prelude_launches(self, mode: str):
+        ls = self._ls
+        fp64 = int(self.dtype == torch.float64)
+        ls["x_tmp"].copy_(self.states.x)
+        if mode == "cached":
+            ls["acc0"].copy_(ls["acc"])
+        else:
+            ls["acc0"].zero_()
+            self._energy_launches(ls["acc0"], detect=mode == "detect")
+        self._launch_ccd(self.states.dx)
+        eps = 1.1920928955078125e-7 if self.dtype == torch.float32 else 2.220446049250313e-16
+        N.call("ipcb_ls_begin", N.ptr(ls["state"]), N.ptr(self.ccd_toi), fp64, N.ptr(self._status),
+               N.ptr(ls["acc0"]), self.h * self.h, eps, 64, ctypes.byref(self.contacts_new.c_struct()),
+               ctypes.byref(self.contacts_pt.c_struct()), N.stream_handle())
+
     def _line_search_device(self) -> float:
         """The reference's search (same E0, bound, halving and accept test)
         with the trial loop on the device: E0 and the CCD bound are launched,
@@ -832,26 +922,16 @@ class FEMContactSolver(ContactBarrierMixin):
         lists and reruns it on the host."""
         ls = self._ls_buffers()
         fp64 = int(self.dtype == torch.float64)
-        h2 = self.h * self.h
         s = N.stream_handle()
-        ls["x_tmp"].copy_(self.states.x)
-        if getattr(self, "_ls_cache", False):
-            # inside a step, x is the point the previous search accepted: its
-            # energy terms are the accepted trial's (as the ABD search caches E0)
-            ls["acc0"].copy_(ls["acc"])
-        else:
-            # within newton_iteration, compute_A has just detected the contacts
-            # at this x: E0 uses its lists (the reference detects again, with
-            # the same result)
-            fresh = getattr(self, "_lists_at_x", False)
-            ls["acc0"].zero_()
-            self._energy_launches(ls["acc0"], detect=not fresh)
+        # E0: inside a step, x is the point the previous search accepted, and
+        # its energy terms are the accepted trial's (as the ABD search caches
+        # E0); within newton_iteration, compute_A has just detected the
+        # contacts at this x, and its lists are used (the reference detects
+        # again, with the same result)
+        mode = "cached" if getattr(self, "_ls_cache", False) else \
+            ("fresh" if getattr(self, "_lists_at_x", False) else "detect")
         self._lists_at_x = False
-        self._launch_ccd(self.states.dx)
-        eps = 1.1920928955078125e-7 if self.dtype == torch.float32 else 2.220446049250313e-16
-        N.call("ipcb_ls_begin", N.ptr(ls["state"]), N.ptr(self.ccd_toi), fp64, N.ptr(self._status),
-               N.ptr(ls["acc0"]), h2, eps, 64,
-               ctypes.byref(self.contacts_new.c_struct()), ctypes.byref(self.contacts_pt.c_struct()), s)
+        self._ls_prelude(mode)
         graph = self._ls_graph()
         N.call("ipcb_graph_launch", graph, s)
         N.call("ipcb_ls_finish", N.ptr(ls["state"]), fp64, self.soup.n_verts, N.ptr(ls["x_tmp"]),

@@ -183,29 +183,39 @@ __global__ void k_union_fill(int nrow, const int* __restrict__ a_off, const int*
   }
 }
 
-// one thread per (slot, component)
-template <class S>
-__global__ void k_newton_values(const int* __restrict__ nnz, int capacity, const int* __restrict__ c_rows,
-                                const int* __restrict__ c_cols, const int* __restrict__ src_a,
-                                const int* __restrict__ src_b, const int* __restrict__ g_off,
-                                const int* __restrict__ g_idx, const S* __restrict__ t_vals, S t_scale,
-                                const S* __restrict__ diag, const S* __restrict__ b_vals, S b_scale,
-                                S* __restrict__ vals) {
-  const long long n = 9LL * min(*nnz, capacity);
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int p = (int)(t / 9), c = (int)(t - 9LL * p);
+// One thread per (slot, component).  I: unsigned while 9 capacity fits it (a
+// 64-bit division by 9 costs more than the rest of a slot's work).  Two
+// gathered blocks are in flight; they are added one by one in list order.
+template <class S, class I>
+__global__ void __launch_bounds__(256) k_newton_values(const int* __restrict__ nnz, int capacity,
+                                                       const int* __restrict__ c_rows, const int* __restrict__ c_cols,
+                                                       const int* __restrict__ src_a, const int* __restrict__ src_b,
+                                                       const int* __restrict__ g_off, const int* __restrict__ g_idx,
+                                                       const S* __restrict__ t_vals, S t_scale,
+                                                       const S* __restrict__ diag, const S* __restrict__ b_vals,
+                                                       S b_scale, S* __restrict__ vals) {
+  const I n = (I)9 * (I)min(*nnz, capacity);
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (I)gridDim.x * blockDim.x) {
+    const int p = (int)(t / 9), c = (int)(t - (I)9 * p);
     S v = S(0);
-    const int sa = __ldg(src_a + p);
+    const int sa = __ldg(src_a + p), sb = __ldg(src_b + p);
+    const S bv = sb >= 0 ? __ldg(b_vals + 9LL * sb + c) : S(0);
     if (sa >= 0) {
       S acc = S(0);
       const int k1 = __ldg(g_off + sa + 1);
-      for (int k = __ldg(g_off + sa); k < k1; ++k) acc += __ldg(t_vals + 9LL * __ldg(g_idx + k) + c);
+      int k = __ldg(g_off + sa);
+      for (; k + 2 <= k1; k += 2) {
+        const int i0 = __ldg(g_idx + k), i1 = __ldg(g_idx + k + 1);
+        const S v0 = __ldg(t_vals + 9LL * i0 + c), v1 = __ldg(t_vals + 9LL * i1 + c);
+        acc += v0;
+        acc += v1;
+      }
+      if (k < k1) acc += __ldg(t_vals + 9LL * __ldg(g_idx + k) + c);
       v = t_scale * acc;
       const int r = __ldg(c_rows + p);
       if (diag && c % 4 == 0 && __ldg(c_cols + p) == r) v += __ldg(diag + r);
     }
-    const int sb = __ldg(src_b + p);
-    if (sb >= 0) v += b_scale * __ldg(b_vals + 9LL * sb + c);
+    if (sb >= 0) v += b_scale * bv;
     vals[t] = v;
   }
 }
@@ -213,14 +223,14 @@ __global__ void k_newton_values(const int* __restrict__ nnz, int capacity, const
 // values = a's values (placed by src_a) + b_scale * b's values (by src_b): the
 // union's values when a's were gathered before (the elastic part, formed
 // beside the contact queries).  One thread per (slot, component).
-template <class S>
+template <class S, class I>
 __global__ void __launch_bounds__(256) k_union_values(const int* __restrict__ nnz, int capacity,
                                                       const int* __restrict__ src_a, const S* __restrict__ a_vals,
                                                       const int* __restrict__ src_b, const S* __restrict__ b_vals,
                                                       S b_scale, S* __restrict__ vals) {
-  const long long n = 9LL * min(*nnz, capacity);
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int p = (int)(t / 9), c = (int)(t - 9LL * p);
+  const I n = (I)9 * (I)min(*nnz, capacity);
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (I)gridDim.x * blockDim.x) {
+    const int p = (int)(t / 9), c = (int)(t - (I)9 * p);
     const int sa = __ldg(src_a + p), sb = __ldg(src_b + p);
     S v = sa >= 0 ? __ldg(a_vals + 9LL * sa + c) : S(0);
     if (sb >= 0) v += b_scale * __ldg(b_vals + 9LL * sb + c);
@@ -246,6 +256,19 @@ __global__ void __launch_bounds__(256) k_newton_rhs(int n, const S* __restrict__
   double g = xadd(xmul(-h2, (double)b[t]), xmul(mass[i], xsub(xi, xt)));
   if (fixed[i]) g = xadd(g, xmul(xmul(h2, k_att), xsub(xi, (double)target[t])));
   out[t] = (S)g;
+}
+
+// f(scalar, index): the index type that holds 9 capacity and a grid beyond it
+template <class F>
+void with_index(int fp64, int capacity, F&& f) {
+  const bool small = capacity <= (0x7fffffff / 9);
+  if (fp64) {
+    if (small) f(0.0, 0u);
+    else f(0.0, 0ull);
+  } else {
+    if (small) f(0.0f, 0u);
+    else f(0.0f, 0ull);
+  }
 }
 
 }  // namespace
@@ -337,16 +360,14 @@ int ipcb_newton_values(int fp64, const int* nnz, int capacity, const int* c_rows
     return IPCB_E_ARG;
   if (capacity == 0) return IPCB_OK;
   cudaStream_t st = (cudaStream_t)s;
-  const int grid = 148 * 8;
-  if (fp64)
-    k_newton_values<double><<<grid, 256, 0, st>>>(nnz, capacity, c_rows, c_cols, src_a, src_b, gather_off,
-                                                  gather_idx, (const double*)tet_vals, tet_scale,
-                                                  (const double*)diag, (const double*)contact_vals, contact_scale,
-                                                  (double*)values);
-  else
-    k_newton_values<float><<<grid, 256, 0, st>>>(nnz, capacity, c_rows, c_cols, src_a, src_b, gather_off, gather_idx,
-                                                 (const float*)tet_vals, (float)tet_scale, (const float*)diag,
-                                                 (const float*)contact_vals, (float)contact_scale, (float*)values);
+  auto run = [&](auto zero, auto index) {
+    using S = decltype(zero);
+    using I = decltype(index);
+    k_newton_values<S, I><<<148 * 8, 256, 0, st>>>(nnz, capacity, c_rows, c_cols, src_a, src_b, gather_off, gather_idx,
+                                                   (const S*)tet_vals, (S)tet_scale, (const S*)diag,
+                                                   (const S*)contact_vals, (S)contact_scale, (S*)values);
+  };
+  with_index(fp64, capacity, run);
   return check_launch("ipcb_newton_values");
 }
 
@@ -354,13 +375,13 @@ int ipcb_union_values(int fp64, const int* nnz, int capacity, const int* src_a, 
                       const void* b_vals, double b_scale, void* values, ipcb_stream s) {
   if (!nnz || capacity < 0 || !src_a || !a_vals || !src_b || !b_vals || !values) return IPCB_E_ARG;
   if (capacity == 0) return IPCB_OK;
-  const int grid = 148 * 8;
-  if (fp64)
-    k_union_values<double><<<grid, 256, 0, (cudaStream_t)s>>>(nnz, capacity, src_a, (const double*)a_vals, src_b,
-                                                              (const double*)b_vals, b_scale, (double*)values);
-  else
-    k_union_values<float><<<grid, 256, 0, (cudaStream_t)s>>>(nnz, capacity, src_a, (const float*)a_vals, src_b,
-                                                             (const float*)b_vals, (float)b_scale, (float*)values);
+  auto run = [&](auto zero, auto index) {
+    using S = decltype(zero);
+    using I = decltype(index);
+    k_union_values<S, I><<<148 * 8, 256, 0, (cudaStream_t)s>>>(nnz, capacity, src_a, (const S*)a_vals, src_b,
+                                                               (const S*)b_vals, (S)b_scale, (S*)values);
+  };
+  with_index(fp64, capacity, run);
   return check_launch("ipcb_union_values");
 }
 

@@ -823,10 +823,25 @@ typedef struct {
   /* initial guess scalar[3n], or NULL for x = 0: ipcb_pcg_start copies it to
    * x and starts from r = b - A x0 (the stopping test stays relative to |b|) */
   const void* x0;
+  /* workspace of the sliced copy (ipcb_pcg_slice), or NULL; slice_nnz: blocks
+   * it is sized for (at least the matrix's) */
+  void* slice_ws;
+  size_t slice_bytes;
+  long long slice_nnz;
 } ipcb_pcg;
 
 int ipcb_pcg_start(const ipcb_pcg* P, double tol, int maxiter, ipcb_stream s);
 int ipcb_pcg_iterate(const ipcb_pcg* P, int k, ipcb_stream s);
+/* The same iterations on a copy of the matrix laid out for the product
+ * (slices of 32 rows sorted by length, one lane a row): between two iterations
+ * of a solve, ipcb_pcg_slice copies the matrix, the inverse diagonal blocks
+ * and the direction into slice_ws (ipcb_pcg_slice_workspace(n, slice_nnz)
+ * bytes); ipcb_pcg_iterate_slices then replaces ipcb_pcg_iterate for the rest
+ * of that solve.  The copy costs about three products: worth it for a solve
+ * that has not ended in its first batch of iterations. */
+size_t ipcb_pcg_slice_workspace(int n, long long nnz, int fp64);
+int ipcb_pcg_slice(const ipcb_pcg* P, ipcb_stream s);
+int ipcb_pcg_iterate_slices(const ipcb_pcg* P, int k, ipcb_stream s);
 /* Inverse diagonal blocks (diag may be NULL: found by a row scan). */
 int ipcb_block_jacobi(int n, const int* offsets, const int* columns, const int* diag, const void* values, int fp64,
                       void* dinv, int* status, ipcb_stream s);

@@ -89,7 +89,8 @@ class Pcg(ctypes.Structure):
     _fields_ = [("n", c_int), ("fp64", c_int), ("precond", c_int), ("offsets", P), ("columns", P), ("values", P),
                 ("dinv", P), ("g_offsets", P), ("g_columns", P), ("diag", P), ("g", P), ("scale", P), ("b", P),
                 ("x", P), ("r", P), ("z", P), ("p", P), ("q", P), ("t", P), ("state", P), ("n_point", c_int),
-                ("n_groups", c_int), ("dinv_group", P), ("x0", P)]
+                ("n_groups", c_int), ("dinv_group", P), ("x0", P), ("slice_ws", P), ("slice_bytes", c_size_t),
+                ("slice_nnz", ctypes.c_longlong)]
 
 
 SP, CP, BP = ctypes.POINTER(Soup), ctypes.POINTER(Contacts), ctypes.POINTER(Lbvh)
@@ -158,6 +159,9 @@ SIGNATURES = {
     "ipcb_adam": (c_int, [c_int, P, P, P, P, c_float, c_float, c_float, c_float, c_int, P]),
     "ipcb_fsai_apply": (c_int, [GP, P, P, c_int, P, P, P, P]),
     "ipcb_pcg_start": (c_int, [ctypes.POINTER(Pcg), c_double, c_int, P]),
+    "ipcb_pcg_slice_workspace": (c_size_t, [c_int, ctypes.c_longlong, c_int]),
+    "ipcb_pcg_slice": (c_int, [ctypes.POINTER(Pcg), P]),
+    "ipcb_pcg_iterate_slices": (c_int, [ctypes.POINTER(Pcg), c_int, P]),
     "ipcb_pcg_iterate": (c_int, [ctypes.POINTER(Pcg), c_int, P]),
     "ipcb_block_jacobi": (c_int, [c_int, P, P, P, P, c_int, P, P, P]),
     "ipcb_group_jacobi": (c_int, [c_int, c_int, P, P, P, c_int, P, P, P]),

@@ -16,6 +16,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "scan.cuh"
 
 namespace ipcb {
 int check_launch(const char* where);
@@ -413,18 +414,47 @@ __global__ void __launch_bounds__(kBlock) k_jacobi(int n, const T* __restrict__ 
   if (threadIdx.x == 0) atomicAdd(&st->rz_new, part);
 }
 
+// Where a sweep finds whether the solve has ended and adds r.z.
+struct StateCtl {
+  ipcb_pcg_state* st;
+  __device__ bool done() const { return st->done; }
+  __device__ double* rz_new() const { return &st->rz_new; }
+};
+
+// The scalars of a batch of iterations on the sliced copy: a slot for each
+// iteration's p.q, |r|^2 and r.z, so nothing is rotated between two kernels
+// (rotating them took the direction kernel a fence, an arrival count and its
+// last block's turn: 2 of its 6 us).  The direction kernel writes for the next
+// iteration whether the solve has ended; once it has, the kernels that follow
+// return on that word.  k_batch_end folds a batch into the state and clears
+// the slots.
+constexpr int kSlots = 32;
+struct Slots {
+  double pAp[kSlots], rr[kSlots], rz[kSlots + 1];
+  double bound;  // tol^2 |b|^2
+  int left;      // iterations the solve may still take
+  int ended[kSlots + 1];
+};
+
+struct SlotCtl {
+  Slots* s;
+  int j;  // iteration of the batch
+  __device__ bool done() const { return __ldcg(s->ended + j) != 0; }
+  __device__ double* rz_new() const { return s->rz + j + 1; }
+};
+
 // lanes per row of the factor sweeps: each reads half a row of the pattern
 // (measured on the wound rod bundle: 61.7 us an iteration with 4, 63.3 with
 // 8, 70.0 with 2)
 constexpr int kFsaiLanes = 4;
 
 // t = G_lower (S r)
-template <class T>
+template <class T, class C>
 __global__ void __launch_bounds__(kBlock) k_fsai_lower(int n, const int* __restrict__ off, const int* __restrict__ diag,
                                                        const int* __restrict__ cols, const bf16* __restrict__ g,
                                                        const float* __restrict__ scale, const T* __restrict__ r,
-                                                       T* __restrict__ t, ipcb_pcg_state* st) {
-  if (st->done) return;
+                                                       T* __restrict__ t, C ctl) {
+  if (ctl.done()) return;
   const int sub = threadIdx.x & (kFsaiLanes - 1);
   const int groups = (gridDim.x * blockDim.x) / kFsaiLanes;
   const int trips = (n + groups - 1) / groups;
@@ -443,13 +473,12 @@ __global__ void __launch_bounds__(kBlock) k_fsai_lower(int n, const int* __restr
 
 // z = S G_upper t (upper slots hold the transposed lower blocks; the diagonal
 // block is read transposed) ; state.rz_new += r.z
-template <class T>
+template <class T, class C>
 __global__ void __launch_bounds__(kBlock) k_fsai_upper(int n, const int* __restrict__ off, const int* __restrict__ diag,
                                                        const int* __restrict__ cols, const bf16* __restrict__ g,
                                                        const float* __restrict__ scale, const T* __restrict__ t,
-                                                       const T* __restrict__ r, T* __restrict__ z,
-                                                       ipcb_pcg_state* st) {
-  if (st->done) return;
+                                                       const T* __restrict__ r, T* __restrict__ z, C ctl) {
+  if (ctl.done()) return;
   const int sub = threadIdx.x & (kFsaiLanes - 1);
   const int groups = (gridDim.x * blockDim.x) / kFsaiLanes;
   const int trips = (n + groups - 1) / groups;
@@ -469,7 +498,7 @@ __global__ void __launch_bounds__(kBlock) k_fsai_upper(int n, const int* __restr
     }
   }
   part = block_sum(part);
-  if (threadIdx.x == 0) atomicAdd(&st->rz_new, part);
+  if (threadIdx.x == 0) atomicAdd(ctl.rz_new(), part);
 }
 
 // the end of an iteration (start: of the setup): rotate the scalars and
@@ -598,6 +627,345 @@ __global__ void k_fsai_mirror(int nnz, const int* __restrict__ rows, const int* 
     for (int c = 0; c < 3; ++c) g[9LL * e + 3 * r + c] = __float2bfloat16_rn(upper ? s[3 * c + r] : s[3 * r + c]);
 }
 
+// ---- iterations on a sliced copy of the matrix --------------------------
+// A solve that outlives its first batch copies the matrix once into slices of
+// 32 rows, one lane a row, the lanes' k-th blocks side by side (component-major,
+// 128-byte loads), rows sorted by length within windows of 256 so that a
+// slice pads little.  In block-row order a warp's nine loads of a 3x3 block
+// each span 1.1 KB (ten L1 lines); here each is one line, there is no
+// reduction over lanes, and the direction p lies in 16-byte records, so a
+// column's gather is one load.  Rod bundle (1.16M blocks, 46 MB, L2-resident):
+// product 14.5 -> 7.4 us, iteration 24.8 -> 14.5 us; the copy takes 36 us.  Rows above kLong blocks (an affine
+// body collects every contact of the body) stay in block-row order, a block
+// of threads a row.
+//
+// (Launching each kernel of an iteration with programmatic dependence on the
+// one before was measured slower, 4.98 against 4.66 ms a solve: blocks that
+// wait hold the slots of blocks that work.)
+constexpr int kLong = 64, kWindow = 256;
+
+// T x 4 records of the direction
+template <class T> struct P4;
+template <> struct P4<float> {
+  static __device__ __forceinline__ void load(const float* p, int i, float& a, float& b, float& c) {
+    const float4 v = reinterpret_cast<const float4*>(p)[i];
+    a = v.x;
+    b = v.y;
+    c = v.z;
+  }
+  static __device__ __forceinline__ void store(float* p, int i, float a, float b, float c) {
+    reinterpret_cast<float4*>(p)[i] = make_float4(a, b, c, 0.f);
+  }
+};
+template <> struct P4<double> {
+  static __device__ __forceinline__ void load(const double* p, int i, double& a, double& b, double& c) {
+    const double2 v = reinterpret_cast<const double2*>(p)[2 * i];
+    a = v.x;
+    b = v.y;
+    c = p[4 * (long long)i + 2];
+  }
+  static __device__ __forceinline__ void store(double* p, int i, double a, double b, double c) {
+    reinterpret_cast<double2*>(p)[2 * i] = make_double2(a, b);
+    p[4 * (long long)i + 2] = c;
+  }
+};
+
+// the rows of a window by length (longest first; the row breaks ties), the
+// widths of its slices, and the long rows
+__global__ void __launch_bounds__(kWindow) k_slice_shape(int n, const int* __restrict__ off, int* __restrict__ perm,
+                                                         int* __restrict__ width, int* __restrict__ n_long,
+                                                         int* __restrict__ long_rows) {
+  __shared__ int key[kWindow];
+  const int t = threadIdx.x, row = blockIdx.x * kWindow + t;
+  int len = row < n ? off[row + 1] - off[row] : -1;
+  if (len > kLong) {
+    long_rows[atomicAdd(n_long, 1)] = row;
+    len = -1;
+  }
+  key[t] = ((kLong - len) << 8) | t;
+  __syncthreads();
+  for (int sz = 2; sz <= kWindow; sz <<= 1)
+    for (int st = sz >> 1; st > 0; st >>= 1) {
+      const int l = t ^ st;
+      if (l > t) {
+        const int a = key[t], b = key[l];
+        if ((a > b) == ((t & sz) == 0)) {
+          key[t] = b;
+          key[l] = a;
+        }
+      }
+      __syncthreads();
+    }
+  const int k = key[t], w = kLong - (k >> 8);
+  perm[blockIdx.x * kWindow + t] = w >= 0 ? blockIdx.x * kWindow + (k & 255) : -1;
+  if ((t & 31) == 0) width[blockIdx.x * (kWindow / 32) + (t >> 5)] = w > 0 ? w : 0;
+}
+
+// a warp copies its slice; also the inverse diagonal blocks component by
+// component (when there are any) and p in records
+template <class T>
+__global__ void __launch_bounds__(256) k_slice_fill(int n, int slices, const int* __restrict__ off,
+                                                    const int* __restrict__ cols, const T* __restrict__ vals,
+                                                    const int* __restrict__ perm, const int* __restrict__ start,
+                                                    int capacity, int* __restrict__ scols, T* __restrict__ svals,
+                                                    const T* __restrict__ dinv, int n_dinv, T* __restrict__ sdinv,
+                                                    const T* __restrict__ p, T* __restrict__ p4,
+                                                    Slots* slots, const ipcb_pcg_state* st) {
+  if (blockIdx.x == 0 && threadIdx.x < kSlots) {
+    slots->pAp[threadIdx.x] = slots->rr[threadIdx.x] = slots->rz[threadIdx.x + 1] = 0.0;
+    if (threadIdx.x == 0) {
+      slots->rz[0] = st->rz;
+      slots->bound = st->tol2 * st->bb;
+      slots->left = st->maxiter - st->it;
+      slots->ended[0] = st->done;
+    }
+  }
+  const int lane = threadIdx.x & 31, sl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    P4<T>::store(p4, i, p[3 * i], p[3 * i + 1], p[3 * i + 2]);
+    if (i < n_dinv)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) sdinv[(long long)c * n + i] = dinv[9LL * i + c];
+  }
+  if (sl >= slices) return;
+  const int s0 = start[sl], w = start[sl + 1] - s0;
+  if ((s0 + w) * 32LL > capacity) return;  // never: sized for every order of lengths
+  const int row = perm[32 * sl + lane];
+  const int b = row >= 0 ? off[row] : 0, len = row >= 0 ? off[row + 1] - b : 0;
+  for (int k = 0; k < w; ++k) {
+    const bool in = k < len;
+    scols[32LL * (s0 + k) + lane] = in ? cols[b + k] : 0;
+    T* d = svals + 9 * 32LL * (s0 + k) + lane;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) d[32 * c] = in ? vals[9LL * (b + k) + c] : T(0);
+  }
+}
+
+// q = A p ; p.q
+template <class T>
+__global__ void __launch_bounds__(kBlock) k_slice_product(int slices, const int* __restrict__ perm,
+                                                          const int* __restrict__ start,
+                                                          const int* __restrict__ scols, const T* __restrict__ svals,
+                                                          const T* __restrict__ p, T* __restrict__ q,
+                                                          const int* __restrict__ off, const int* __restrict__ cols,
+                                                          const T* __restrict__ vals, const int* __restrict__ n_long,
+                                                          const int* __restrict__ long_rows, int slice_blocks,
+                                                          SlotCtl ctl) {
+  double part = 0.0;
+  if ((int)blockIdx.x < slice_blocks) {
+    const int lane = threadIdx.x & 31, sl = (blockIdx.x * kBlock + threadIdx.x) >> 5;
+    int row = -1, s0 = 0, w = 0;
+    if (sl < slices) {
+      row = __ldg(perm + 32 * sl + lane);
+      s0 = __ldg(start + sl);
+      w = __ldg(start + sl + 1) - s0;
+    }
+    const int* c = scols + 32LL * s0 + lane;
+    const T* m = svals + 9 * 32LL * s0 + lane;
+    constexpr int U = sizeof(T) == 4 ? 4 : 2;  // blocks in flight; the next ones are loaded before the sums
+    T a0 = 0, a1 = 0, a2 = 0;
+    int cc[U];
+    T v[U][9];
+    auto fetch = [&](int k) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = min(k + u, w - 1);
+        cc[u] = __ldg(c + 32 * j);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) v[u][e] = __ldg(m + 9 * 32 * j + 32 * e);
+      }
+    };
+    if (w > 0) fetch(0);
+    if (ctl.done()) return;
+    for (int k = 0; k < w; k += U) {
+      T x[U][3];
+#pragma unroll
+      for (int u = 0; u < U; ++u) P4<T>::load(p, cc[u], x[u][0], x[u][1], x[u][2]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (k + u < w) {
+          a0 += v[u][0] * x[u][0] + v[u][1] * x[u][1] + v[u][2] * x[u][2];
+          a1 += v[u][3] * x[u][0] + v[u][4] * x[u][1] + v[u][5] * x[u][2];
+          a2 += v[u][6] * x[u][0] + v[u][7] * x[u][1] + v[u][8] * x[u][2];
+        }
+      }
+      if (k + U < w) fetch(k + U);
+    }
+    if (row >= 0) {
+      T x0, x1, x2;
+      P4<T>::load(p, row, x0, x1, x2);
+      q[3 * row] = a0;
+      q[3 * row + 1] = a1;
+      q[3 * row + 2] = a2;
+      part = (double)x0 * a0 + (double)x1 * a1 + (double)x2 * a2;
+    }
+    part = block_sum(part);
+    if (threadIdx.x == 0) atomicAdd(ctl.s->pAp + ctl.j, part);
+    return;
+  }
+  __shared__ double srow[kBlock / 32][3];
+  const int n = *n_long, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  if (n == 0 || ctl.done()) return;
+  for (int r = blockIdx.x - slice_blocks; r < n; r += gridDim.x - slice_blocks) {
+    const int row = long_rows[r];
+    T a[3] = {0, 0, 0};
+    for (int k = off[row] + threadIdx.x; k < off[row + 1]; k += kBlock) {
+      const T* m = vals + 9LL * k;
+      T x0, x1, x2;
+      P4<T>::load(p, __ldg(cols + k), x0, x1, x2);
+#pragma unroll
+      for (int e = 0; e < 3; ++e) a[e] += __ldg(m + 3 * e) * x0 + __ldg(m + 3 * e + 1) * x1 + __ldg(m + 3 * e + 2) * x2;
+    }
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
+      if (lane == 0) srow[wp][e] = (double)a[e];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      T x[3];
+      P4<T>::load(p, row, x[0], x[1], x[2]);
+      for (int e = 0; e < 3; ++e) {
+        double sum = 0.0;
+        for (int k = 0; k < kBlock / 32; ++k) sum += srow[k][e];
+        q[3 * row + e] = (T)sum;
+        part += (double)x[e] * (double)(T)sum;
+      }
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && part != 0.0) atomicAdd(ctl.s->pAp + ctl.j, part);
+}
+
+// x += alpha p ; r -= alpha q, |r|^2 ; with JACOBI also z = D^-1 r and r.z, per
+// block row (component-major inverse blocks); groups as k_update_xr_groups.
+// The vectors of a thread's first row are loaded before the scalars are
+// tested, so that they arrive together: the kernel is a chain of latencies.
+template <class T, bool JACOBI>
+__global__ void __launch_bounds__(kBlock) k_slice_update(int n, int n_point, int n_groups, T* __restrict__ x,
+                                                         T* __restrict__ r, const T* __restrict__ p,
+                                                         const T* __restrict__ q, const T* __restrict__ sdinv,
+                                                         const T* __restrict__ dinv_group, T* __restrict__ z,
+                                                         SlotCtl ctl) {
+  const int base = group_base(n_point);
+  const long long total = JACOBI && n_groups > 0 ? group_items(n_point, n_groups) : n;
+  const int rows = JACOBI ? n_point : n;  // taken one a thread
+  const long long first = blockIdx.x * (long long)kBlock + threadIdx.x;
+  T d[9], pv[3], xv[3], rv[3], qv[3];
+  auto fetch = [&](long long i) {
+    if (JACOBI)
+#pragma unroll
+      for (int c = 0; c < 9; ++c) d[c] = __ldg(sdinv + (long long)c * n + i);
+    P4<T>::load(p, (int)i, pv[0], pv[1], pv[2]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      xv[c] = x[3 * i + c];
+      rv[c] = r[3 * i + c];
+      qv[c] = q[3 * i + c];
+    }
+  };
+  if (first < rows) fetch(first);
+  const double pAp = __ldcg(ctl.s->pAp + ctl.j), rz = __ldcg(ctl.s->rz + ctl.j);
+  if (ctl.done()) return;
+  const T alpha = (T)(pAp > 0.0 ? rz / pAp : 0.0);
+  double prr = 0.0, prz = 0.0;
+  for (long long i = first; i < total; i += (long long)gridDim.x * kBlock) {
+    if (i < rows) {
+      if (i != first) fetch(i);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        x[3 * i + c] = xv[c] + alpha * pv[c];
+        rv[c] -= alpha * qv[c];
+        r[3 * i + c] = rv[c];
+        prr += (double)rv[c] * rv[c];
+      }
+      if (JACOBI)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const T zc = d[3 * c] * rv[0] + d[3 * c + 1] * rv[1] + d[3 * c + 2] * rv[2];
+          z[3 * i + c] = zc;
+          prz += (double)rv[c] * zc;
+        }
+    } else if (JACOBI && i >= base) {  // whole warps only (base is a multiple of 32)
+      const long long j = i - base;
+      const int g = (int)(j >> 4), c = (int)(j & 15);
+      const bool on = g < n_groups && c < 12;
+      const long long o = 3LL * n_point + 12LL * g + c;
+      T rg = T(0);
+      if (on) {
+        x[o] += alpha * p[4 * (o / 3) + o % 3];
+        rg = r[o] - alpha * q[o];
+        r[o] = rg;
+        prr += (double)rg * rg;
+      }
+      const T* dg = dinv_group + 144LL * g + 12 * c;
+      T zc = T(0);
+#pragma unroll
+      for (int k = 0; k < 12; ++k) {
+        const T rk = __shfl_sync(0xffffffffu, rg, k, 16);
+        if (on) zc += dg[k] * rk;
+      }
+      if (on) {
+        z[o] = zc;
+        prz += (double)rg * zc;
+      }
+    }
+  }
+  block_sum2(prr, prz);
+  if (threadIdx.x == 0) {
+    atomicAdd(ctl.s->rr + ctl.j, prr);
+    if (JACOBI) atomicAdd(ctl.rz_new(), prz);
+  }
+}
+
+// p = z + beta p in records
+template <class T>
+__global__ void __launch_bounds__(kBlock) k_slice_direction(int n, const T* __restrict__ z, T* p, SlotCtl ctl) {
+  const int first = blockIdx.x * kBlock + threadIdx.x;
+  T a = 0, b = 0, c = 0, z0 = 0, z1 = 0, z2 = 0;
+  auto fetch = [&](int i) {
+    P4<T>::load(p, i, a, b, c);
+    z0 = z[3 * i];
+    z1 = z[3 * i + 1];
+    z2 = z[3 * i + 2];
+  };
+  if (first < n) fetch(first);
+  const double rz = __ldcg(ctl.s->rz + ctl.j), rz_new = __ldcg(ctl.rz_new());
+  const bool done = ctl.done();
+  if (first == 0)  // converged, broken down (p.q not positive), out of iterations, or before
+    ctl.s->ended[ctl.j + 1] = done || __ldcg(ctl.s->rr + ctl.j) <= ctl.s->bound ||
+                              !(__ldcg(ctl.s->pAp + ctl.j) > 0.0) || ctl.j + 1 >= ctl.s->left;
+  if (done) return;
+  const T beta = (T)(rz != 0.0 ? rz_new / rz : 0.0);
+  for (int i = first; i < n; i += gridDim.x * kBlock) {
+    if (i != first) fetch(i);
+    P4<T>::store(p, i, z0 + beta * a, z1 + beta * b, z2 + beta * c);
+  }
+}
+
+// a batch's slots into the state, and ready for the next batch: as
+// finish_state after each iteration
+__global__ void __launch_bounds__(32) k_batch_end(int k, Slots* s, ipcb_pcg_state* st) {
+  const int j = threadIdx.x;
+  const unsigned full = 0xffffffffu;
+  const double rr = s->rr[j], pAp = s->pAp[j], rz = s->rz[j + 1], bound = s->bound;
+  const int left = s->left, was = s->ended[0];
+  const bool breakdown = !(pAp > 0.0);  // the operator is not positive definite along p
+  const unsigned ends = __ballot_sync(full, j < k && (rr <= bound || breakdown || j + 1 >= left));
+  const int last = ends ? __ffs(ends) - 1 : k - 1;  // the batch's last iteration
+  __syncwarp();
+  s->pAp[j] = s->rr[j] = s->rz[j + 1] = 0.0;
+  if (j != last || was) return;
+  st->it += last + 1;
+  st->last_rr = rr;
+  if (breakdown) st->status |= 1;
+  if (ends) st->done = s->ended[0] = 1;
+  s->left = left - (last + 1);
+  s->rz[0] = st->rz = rz;
+}
+
 inline int gridn(long long n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
 // row-group kernels loop over rows: a fixed grid of 8 blocks per SM
@@ -621,6 +989,15 @@ int flat_grid(long long m) {
   return need < cap ? need : cap;
 }
 
+template <class T, class C>
+void sweeps(const ipcb_pcg* P, C ctl, cudaStream_t s) {
+  const int n = P->n;
+  k_fsai_lower<T><<<warp_grid(n), kBlock, 0, s>>>(n, P->g_offsets, P->diag, P->g_columns, (const bf16*)P->g, P->scale,
+                                                  (const T*)P->r, (T*)P->t, ctl);
+  k_fsai_upper<T><<<warp_grid(n), kBlock, 0, s>>>(n, P->g_offsets, P->diag, P->g_columns, (const bf16*)P->g, P->scale,
+                                                  (const T*)P->t, (const T*)P->r, (T*)P->z, ctl);
+}
+
 template <class T>
 int precond(const ipcb_pcg* P, cudaStream_t s) {
   const int n = P->n;
@@ -629,12 +1006,7 @@ int precond(const ipcb_pcg* P, cudaStream_t s) {
         P->n_point, P->n_groups, (const T*)P->dinv, (const T*)P->dinv_group, (const T*)P->r, (T*)P->z, P->state);
   else if (P->precond == 0)
     k_jacobi<T><<<flat_grid(n), kBlock, 0, s>>>(n, (const T*)P->dinv, (const T*)P->r, (T*)P->z, P->state);
-  else {
-    k_fsai_lower<T><<<warp_grid(n), kBlock, 0, s>>>(n, P->g_offsets, P->diag, P->g_columns, (const bf16*)P->g,
-                                                   P->scale, (const T*)P->r, (T*)P->t, P->state);
-    k_fsai_upper<T><<<warp_grid(n), kBlock, 0, s>>>(n, P->g_offsets, P->diag, P->g_columns, (const bf16*)P->g,
-                                                   P->scale, (const T*)P->t, (const T*)P->r, (T*)P->z, P->state);
-  }
+  else sweeps<T>(P, StateCtl{P->state}, s);
   return 0;
 }
 
@@ -679,6 +1051,97 @@ int iterate(const ipcb_pcg* P, int k, cudaStream_t s) {
   return 0;
 }
 
+inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
+
+// The sliced copy in its workspace (ipcb_pcg_slice_workspace).
+template <class T>
+struct Slices {
+  int windows, slices, capacity;  // capacity: blocks, padding included
+  int* n_long;
+  Slots* slots;
+  int* perm;
+  int* start;
+  int* long_rows;
+  int* scols;
+  T* svals;
+  T* sdinv;
+  T* p4;
+  void* scratch;
+};
+
+template <class T>
+size_t slice_layout(int n, long long nnz, char* p, Slices<T>* out) {
+  Slices<T> S;
+  S.windows = gridn(n, kWindow);
+  S.slices = S.windows * (kWindow / 32);
+  // a slice's width is at most the shortest row of the slice before it
+  const long long cap = nnz + 32LL * kLong * S.windows;
+  S.capacity = (int)cap;
+  char* p0 = p;
+  S.n_long = (int*)p; p += 256;
+  S.slots = (Slots*)p; p += al256(sizeof(Slots));
+  S.perm = (int*)p; p += al256(32LL * S.slices * 4);
+  S.start = (int*)p; p += al256((S.slices + 1LL) * 4);
+  S.long_rows = (int*)p; p += al256((size_t)n * 4);
+  S.scols = (int*)p; p += al256(cap * 4);
+  S.svals = (T*)p; p += al256(cap * 9 * sizeof(T));
+  S.sdinv = (T*)p; p += al256(9LL * n * sizeof(T));
+  S.p4 = (T*)p; p += al256(4LL * n * sizeof(T));
+  S.scratch = p; p += ipcb::scan::scratch_bytes(S.slices + 1);
+  if (out) *out = S;
+  return (size_t)(p - p0);
+}
+
+template <class T>
+void slice(const ipcb_pcg* P, cudaStream_t s) {
+  const int n = P->n;
+  Slices<T> S;
+  slice_layout<T>(n, P->slice_nnz, (char*)P->slice_ws, &S);
+  cudaMemsetAsync(S.n_long, 0, sizeof(int), s);
+  cudaMemsetAsync(S.start + S.slices, 0, sizeof(int), s);
+  k_slice_shape<<<S.windows, kWindow, 0, s>>>(n, P->offsets, S.perm, S.start, S.n_long, S.long_rows);
+  ipcb::scan::exclusive<int>(S.start, S.slices + 1, S.scratch, nullptr, s);
+  const int n_dinv = P->precond != 0 ? 0 : (P->n_groups > 0 ? P->n_point : n);
+  k_slice_fill<T><<<gridn(32LL * S.slices), 256, 0, s>>>(n, S.slices, P->offsets, P->columns, (const T*)P->values,
+                                                         S.perm, S.start, S.capacity, S.scols, S.svals,
+                                                         (const T*)P->dinv, n_dinv, S.sdinv, (const T*)P->p, S.p4,
+                                                         S.slots, P->state);
+}
+
+template <class T>
+int iterate_slices(const ipcb_pcg* P, int k, cudaStream_t s) {
+  const int n = P->n;
+  Slices<T> S;
+  slice_layout<T>(n, P->slice_nnz, (char*)P->slice_ws, &S);
+  const int slice_blocks = gridn(32LL * S.slices), long_blocks = 32;
+  const bool jacobi = P->precond == 0;
+  const int n_point = jacobi && P->n_groups > 0 ? P->n_point : n, n_groups = jacobi ? P->n_groups : 0;
+  const long long items = n_groups > 0 ? group_items(n_point, n_groups) : n;
+  // one row a thread up to 4 blocks a SM: few atomics on the scalars
+  auto grid = [](long long m) { return gridn(m) < 148 * 4 ? gridn(m) : 148 * 4; };
+  for (int first = 0; first < k; first += kSlots) {
+    const int batch = k - first < kSlots ? k - first : kSlots;
+    for (int j = 0; j < batch; ++j) {
+      const SlotCtl ctl{S.slots, j};
+      k_slice_product<T><<<slice_blocks + long_blocks, kBlock, 0, s>>>(
+          S.slices, S.perm, S.start, S.scols, S.svals, S.p4, (T*)P->q, P->offsets, P->columns, (const T*)P->values,
+          S.n_long, S.long_rows, slice_blocks, ctl);
+      if (jacobi) {
+        k_slice_update<T, true><<<grid(items), kBlock, 0, s>>>(n, n_point, n_groups, (T*)P->x, (T*)P->r, S.p4,
+                                                               (const T*)P->q, S.sdinv, (const T*)P->dinv_group,
+                                                               (T*)P->z, ctl);
+      } else {
+        k_slice_update<T, false><<<grid(n), kBlock, 0, s>>>(n, n, 0, (T*)P->x, (T*)P->r, S.p4, (const T*)P->q,
+                                                            S.sdinv, (const T*)nullptr, (T*)P->z, ctl);
+        sweeps<T>(P, ctl, s);
+      }
+      k_slice_direction<T><<<grid(n), kBlock, 0, s>>>(n, (const T*)P->z, S.p4, ctl);
+    }
+    k_batch_end<<<1, 32, 0, s>>>(batch, S.slots, P->state);
+  }
+  return 0;
+}
+
 bool pcg_ok(const ipcb_pcg* P) {
   if (!P || P->n <= 0 || !P->offsets || !P->columns || !P->values || !P->x || !P->r || !P->z || !P->p || !P->q ||
       !P->b || !P->state)
@@ -713,6 +1176,36 @@ int ipcb_pcg_iterate(const ipcb_pcg* P, int k, ipcb_stream s) {
   if (P->fp64) iterate<double>(P, k, (cudaStream_t)s);
   else iterate<float>(P, k, (cudaStream_t)s);
   return ipcb::check_launch("ipcb_pcg_iterate");
+}
+
+size_t ipcb_pcg_slice_workspace(int n, long long nnz, int fp64) {
+  if (n <= 0 || nnz < 0) return 0;
+  return fp64 ? slice_layout<double>(n, nnz, nullptr, nullptr) : slice_layout<float>(n, nnz, nullptr, nullptr);
+}
+
+static bool slice_ok(const ipcb_pcg* P) {
+  return pcg_ok(P) && P->slice_ws && P->slice_nnz >= 0 && P->slice_nnz + 32LL * kLong * gridn(P->n, kWindow) <= 0x7fffffff &&
+         P->slice_bytes >= ipcb_pcg_slice_workspace(P->n, P->slice_nnz, P->fp64);
+}
+
+int ipcb_pcg_slice(const ipcb_pcg* P, ipcb_stream s) {
+  if (!slice_ok(P)) {
+    ipcb::set_error_msg("pcg_slice: bad arguments");
+    return IPCB_E_ARG;
+  }
+  if (P->fp64) slice<double>(P, (cudaStream_t)s);
+  else slice<float>(P, (cudaStream_t)s);
+  return ipcb::check_launch("ipcb_pcg_slice");
+}
+
+int ipcb_pcg_iterate_slices(const ipcb_pcg* P, int k, ipcb_stream s) {
+  if (!slice_ok(P) || k < 0) {
+    ipcb::set_error_msg("pcg_iterate_slices: bad arguments");
+    return IPCB_E_ARG;
+  }
+  if (P->fp64) iterate_slices<double>(P, k, (cudaStream_t)s);
+  else iterate_slices<float>(P, k, (cudaStream_t)s);
+  return ipcb::check_launch("ipcb_pcg_iterate_slices");
 }
 
 int ipcb_block_jacobi(int n, const int* offsets, const int* columns, const int* diag, const void* values, int fp64,

@@ -80,7 +80,10 @@ class Pool:
     def get(self, name: str, shape, dtype, device) -> torch.Tensor:
         shape = tuple(int(v) for v in shape)
         t = self._bufs.get(name)
-        if t is None or t.dtype != dtype or t.device != torch.device(device) or t.numel() < math.prod(shape):
+        device = torch.device(device)
+        if device.index is None and device.type == "cuda":  # "cuda" is the current device, as for torch.empty
+            device = torch.device("cuda", torch.cuda.current_device())
+        if t is None or t.dtype != dtype or t.device != device or t.numel() < math.prod(shape):
             t = torch.empty(max(math.prod(shape), 1), dtype=dtype, device=device)
             self._bufs[name] = t
         return t[:math.prod(shape)].view(shape)

@@ -148,7 +148,9 @@ class JacobiPrecond:
 class DevicePcg:
     """PCG with device-resident scalars (ipcb_pcg_*): ``batch`` iterations
     per host check, replayed from a CUDA graph captured once per set of
-    buffers; one synchronisation per batch."""
+    buffers; one synchronisation per batch.  A solve that has not ended in its
+    first batch goes on with a copy of the matrix laid out for the product
+    (ipcb_pcg_slice)."""
 
     def __init__(self, batch: int = 16, use_graph: bool = True):
         self.batch = batch
@@ -156,14 +158,30 @@ class DevicePcg:
         self._bufs = None
         self._graph = None
         self._key = None
+        self._slice_graph = None
+        self._slice_key = None
+        self._slice_ws = None
+        self._slice_nnz = 0
 
     def _buffers(self, n, dtype, device):
         if self._bufs is None or self._bufs["n"] != n or self._bufs["dtype"] != dtype:
             z = lambda: torch.zeros((n, 3), dtype=dtype, device=device)
             self._bufs = dict(n=n, dtype=dtype, x=z(), r=z(), z=z(), p=z(), q=z(), t=z(), b=z(), x0=z(),
                               state=torch.zeros(ctypes.sizeof(N.PcgState), dtype=torch.uint8, device=device),
-                              host=torch.zeros(ctypes.sizeof(N.PcgState), dtype=torch.uint8).pin_memory())
+                              host=torch.zeros(ctypes.sizeof(N.PcgState), dtype=torch.uint8).pin_memory(),
+                              nnz=torch.zeros(1, dtype=torch.int32).pin_memory())
+            self._slice_ws = None
         return self._bufs
+
+    def _slice_room(self, P, nnz: int, device) -> None:
+        """P's workspace of the sliced copy, with room to spare: a Newton loop's
+        matrices differ a little in size, and the graph holds the addresses."""
+        if self._slice_ws is None or self._slice_nnz < nnz:
+            self._slice_nnz = nnz + nnz // 4 + 1024
+            self._slice_ws = None
+            nbytes = N.size("ipcb_pcg_slice_workspace", P.n, self._slice_nnz, P.fp64)
+            self._slice_ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        P.slice_ws, P.slice_bytes, P.slice_nnz = N.ptr(self._slice_ws), self._slice_ws.numel(), self._slice_nnz
 
     def solve(self, A: BsrMatrix, b: torch.Tensor, M, tol: float, maxiter: int, x0: torch.Tensor | None = None):
         """Returns (x, iterations, relative residual, status); x is a view of
@@ -184,27 +202,54 @@ class DevicePcg:
             P.x0 = N.ptr(B["x0"])
         self._P = P
         N.call("ipcb_pcg_start", ctypes.byref(P), float(tol), int(maxiter), N.stream_handle())
-        key = tuple(getattr(P, f) for f, _ in N.Pcg._fields_ if f != "x0")  # the loop never reads x0
+        key = self._fields(P)
         if self.use_graph and key != self._key:
-            self._graph = torch.cuda.CUDAGraph()
-            with N.no_collection(), torch.cuda.graph(self._graph):
-                N.call("ipcb_pcg_iterate", ctypes.byref(P), self.batch, N.stream_handle())
+            self._graph = self._capture("ipcb_pcg_iterate", P)
             self._key = key
-        st = N.PcgState()
-        while True:
-            if self.use_graph:
-                self._graph.replay()
-            else:
-                N.call("ipcb_pcg_iterate", ctypes.byref(P), self.batch, N.stream_handle())
-            B["host"].copy_(B["state"], non_blocking=True)
-            torch.cuda.current_stream().synchronize()
-            st = N.PcgState.from_buffer_copy(B["host"].numpy().tobytes())
-            if st.done:
-                break
+        self._batch(self._graph, "ipcb_pcg_iterate", P)
+        B["nnz"].copy_(A.offsets[n:n + 1], non_blocking=True)
+        st = self._read(B)
+        nnz = int(B["nnz"])
+        if not st.done and nnz + nnz // 4 + 8 * n + (1 << 14) > 0x7fffffff:  # past the copy's 32-bit slots
+            while not st.done:
+                self._batch(self._graph, "ipcb_pcg_iterate", P)
+                st = self._read(B)
+        if not st.done:
+            self._slice_room(P, nnz, A.device)
+            N.call("ipcb_pcg_slice", ctypes.byref(P), N.stream_handle())
+            key = self._fields(P)
+            if self.use_graph and key != self._slice_key:
+                self._slice_graph = self._capture("ipcb_pcg_iterate_slices", P, 2)
+                self._slice_key = key
+            while not st.done:  # the launches past the end cost less than the reads saved
+                self._batch(self._slice_graph, "ipcb_pcg_iterate_slices", P, 2)
+                st = self._read(B)
         if x0 is not None and not st.bb > 0:
             B["x"].zero_()  # b = 0: the solution is 0, whatever the guess
         rel = math.sqrt(st.last_rr / st.bb) if st.bb > 0 else 0.0
         return B["x"], st.it, rel, st.status
+
+    @staticmethod
+    def _fields(P):
+        return tuple(getattr(P, f) for f, _ in N.Pcg._fields_ if f != "x0")  # the loop never reads x0
+
+    def _capture(self, call, P, times: int = 1):
+        graph = torch.cuda.CUDAGraph()
+        with N.no_collection(), torch.cuda.graph(graph):
+            N.call(call, ctypes.byref(P), times * self.batch, N.stream_handle())
+        return graph
+
+    def _batch(self, graph, call, P, times: int = 1):
+        if self.use_graph:
+            graph.replay()
+        else:
+            N.call(call, ctypes.byref(P), times * self.batch, N.stream_handle())
+
+    @staticmethod
+    def _read(B):
+        B["host"].copy_(B["state"], non_blocking=True)
+        torch.cuda.current_stream().synchronize()
+        return N.PcgState.from_buffer_copy(B["host"].numpy().tobytes())
 
 
 def terms_candidates() -> list[tuple]:

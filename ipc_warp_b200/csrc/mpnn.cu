@@ -10,10 +10,11 @@
 // fused epilogue (bias, ReLU, residual, segmented message aggregation, head).
 // The message map is split by input block, [h_i | h_j | e] W1 = (h W1a)_i +
 // (h W1b)_j + e W1c: the two node projections are one node-sized product and
-// the edge product stages only the 128-byte edge state.  Weight
-// gradients use k_wgrad, which stages X^T and dY^T tiles (rows of the batch
-// along K) and keeps the [features x outputs] accumulator in TMEM across all
-// the row tiles a CTA visits, plus a bias row from a column of ones.
+// the edge product stages only the 128-byte edge state; the backward pass
+// splits it the same way (k_edge_grad).  Weight gradients use k_wgrad, which
+// reads row-major X and dY tiles as MN-major operands (rows of the batch along
+// K) and keeps the [features x outputs] accumulator in TMEM across all the
+// row tiles a CTA visits, plus a bias row from a column of ones.
 //
 // Storage: node/edge states and messages bf16, accumulation fp32, biases
 // fp32, G^ fp32 (the rounding points of oracle/mpnn.py).
@@ -125,6 +126,9 @@ __device__ __forceinline__ uint4 pack8(const float* f) {
   return u;
 }
 
+constexpr int kPieces = 3;               // bf16 pieces of an fp32 value
+constexpr int kSplit = kPieces * 2 * W;  // a row of split sums: pieces x [row | column] x 64
+
 // ------------------------------------------------------------ stages
 struct StageDense {  // row-major bf16 rows, columns >= kvalid read as zero
   const bf16* X;
@@ -141,6 +145,11 @@ struct StageNode {  // [h | a] of a node (a: mean message, from k_mean_messages)
   __device__ uint4 group(int row, int c, int g) const {
     return ld4((c == 0 ? h : a) + (size_t)row * W + g * 8);
   }
+};
+
+struct StageSplit {  // chunk c of a node's split sums
+  const bf16* s;
+  __device__ uint4 group(int row, int c, int g) const { return ld4(s + (size_t)row * kSplit + c * 64 + g * 8); }
 };
 
 struct StageGather {  // X[idx[row]] (64 wide)
@@ -303,22 +312,106 @@ struct EpiF32 {  // plain fp32 rows of width ld (lanes across the columns)
   }
 };
 
+__device__ __forceinline__ void st8f(float* p, const float (&f)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+
+struct EpiRows {  // out[idx[row]] = v (fp32, 64 columns)
+  float* out;
+  const int* idx;
+  __device__ void rows32(int grow0, int nvalid, const float* acc, int stride, const uint8_t*, int, int lane) const {
+    const int q = lane >> 3, cg = lane & 7;
+    const int mine = lane < nvalid ? __ldg(idx + grow0 + lane) : 0;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int r = 4 * it + q;
+      const int o = __shfl_sync(0xffffffffu, mine, r);
+      if (r >= nvalid) continue;
+      float v[8];
+      ld8s(acc + r * stride + 8 * cg, v);
+      st8f(out + (size_t)o * W + 8 * cg, v);
+    }
+  }
+};
+
+// d += v (fp32, 64 columns); with act also dy = bf16(d * (act > 0)), the
+// gradient below the activation that d has reached
+struct EpiAdd {
+  float* d;
+  const bf16* act;
+  bf16* dy;
+  __device__ void rows32(int grow0, int nvalid, const float* acc, int stride, const uint8_t*, int, int lane) const {
+    const int q = lane >> 3, cg = lane & 7;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int r = 4 * it + q;
+      if (r >= nvalid) continue;
+      const size_t o = (size_t)(grow0 + r) * W + 8 * cg;
+      float v[8], f[8];
+      ld8f(d + o, f);
+      ld8s(acc + r * stride + 8 * cg, v);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) f[t] += v[t];
+      st8f(d + o, f);
+      if (!act) continue;
+      float a[8];
+      unpack8(ld4(act + o), a);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) f[t] = a[t] > 0.f ? f[t] : 0.f;
+      *reinterpret_cast<uint4*>(dy + o) = pack8(f);
+    }
+  }
+};
+
+struct EpiUpdateGrad {  // [dh | dmean] of a node: dh += v[0:64], da = v[64:128] / degree
+  float *dh, *da;
+  const int* off;
+  __device__ void rows32(int grow0, int nvalid, const float* acc, int stride, const uint8_t*, int, int lane) const {
+    const int q = lane >> 4, cg = lane & 15;
+    const float mine = lane < nvalid ? (float)(__ldg(off + grow0 + lane + 1) - __ldg(off + grow0 + lane)) : 1.f;
+#pragma unroll 8
+    for (int it = 0; it < 16; ++it) {
+      const int r = 2 * it + q;
+      const float deg = __shfl_sync(0xffffffffu, mine, r);
+      if (r >= nvalid) continue;
+      float v[8];
+      ld8s(acc + r * stride + 8 * cg, v);
+      const size_t o = (size_t)(grow0 + r) * W + 8 * (cg & 7);
+      if (cg < 8) {
+        float f[8];
+        ld8f(dh + o, f);
+#pragma unroll
+        for (int t = 0; t < 8; ++t) f[t] += v[t];
+        st8f(dh + o, f);
+      } else {
+#pragma unroll
+        for (int t = 0; t < 8; ++t) v[t] /= deg;
+        st8f(da + o, v);
+      }
+    }
+  }
+};
+
 // ------------------------------------------------------------ k_mlp
 // Warp-specialised persistent product: D = A B^T + epilogue over 128-row
-// tiles of A.  Producer warps (0-3) gather tile k into shared stage k % 2
-// (thread t stages row t), then thread 0 issues the UMMAs into TMEM
-// accumulator k % 2 and commits to mma_done[k % 2]; epilogue warps (4-7) wait
+// tiles of A.  With S = 2 stages, producer warps (0-3) gather tile k into
+// shared stage k % 2, then thread 0 issues the UMMAs into TMEM accumulator
+// k % 2 and commits to mma_done[k % 2]; epilogue warps (4-7) wait
 // for it, read their 32 lanes each (and may read the staged tile) and arrive
 // on acc_free[k % 2].  Stage and accumulator k % 2 are reused for tile k + 2
 // only after that release, so tile k + 1 is gathered and multiplied while
 // tile k is drained.  Every wait is bounded; a wait that
 // gives up raises IPCB_STATUS_TIMEOUT and ends the CTA's loop.
-template <int N, int C>
+// S = 1 (one stage and accumulator, for the operand whose two stages exceed
+// shared memory) runs gather and drain in turn.  With CB < C the weights are
+// CB matrices [N][64] and chunk c of A is multiplied by matrix c % CB.
+template <int N, int C, int CB, int S>
 constexpr size_t mlp_smem() {
-  return 1024 + 2 * (size_t)C * 128 * 128 + (size_t)C * N * 128 + 128 * (size_t)(N + 1) * 4;
+  return 1024 + S * (size_t)C * 128 * 128 + (size_t)CB * N * 128 + 128 * (size_t)(N + 1) * 4;
 }
 
-template <int N, int C, class Stage, class Epi>
+template <int N, int C, int CB, int S, class Stage, class Epi>
 __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep, const bf16* __restrict__ Bw,
                                                      int* __restrict__ status) {
   extern __shared__ uint8_t dsmem[];
@@ -328,19 +421,21 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep,
   __shared__ int prod_abort, epi_abort;
   // accumulator stride: at least the 32 columns one tcgen05.ld reads
   constexpr int NA = N < 32 ? 32 : N;
-  constexpr uint32_t kCols = umma::tmem_cols(2 * NA);
-  static_assert(2 * NA <= 512, "two accumulators must fit the 512 TMEM columns");
+  constexpr uint32_t kCols = umma::tmem_cols(S * NA);
+  static_assert(C < 3 || C % 2 == 0, "chunks are staged in pairs");
+  static_assert(S * NA <= 512, "the accumulators must fit the 512 TMEM columns");
   constexpr int K = 64 * C;
   constexpr int kStage = C * 128 * 128;
   uint8_t* sA = align1024(dsmem);
-  uint8_t* sB = sA + 2 * kStage;
-  float* accs = reinterpret_cast<float*>(sB + C * N * 128);  // [128][N + 1]
+  uint8_t* sB = sA + S * kStage;
+  float* accs = reinterpret_cast<float*>(sB + CB * N * 128);  // [128][N + 1]
   constexpr int kStride = N + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  for (int idx = tid; idx < N * C * 8; idx += kMlpThreads) {
-    const int r = idx / (C * 8), c = (idx / 8) % C, g = idx % 8;
-    *reinterpret_cast<uint4*>(sB + umma::sw128_group(r, c, g, N)) = ld4(Bw + (size_t)r * K + c * 64 + g * 8);
+  for (int idx = tid; idx < N * CB * 8; idx += kMlpThreads) {
+    const int r = idx / (CB * 8), c = (idx / 8) % CB, g = idx % 8;
+    *reinterpret_cast<uint4*>(sB + umma::sw128_group(r, c, g, N)) =
+        ld4(Bw + (CB == C ? (size_t)r * K + c * 64 : ((size_t)c * N + r) * 64) + g * 8);
   }
   if (warp == 0) umma::tmem_alloc(&tslot, kCols);
   if (tid == 0) {
@@ -362,43 +457,47 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep,
 
   if (warp < 4) {
     for (int k = 0; k < mine; ++k) {
-      const int s = k & 1, use = k >> 1;
-      // stage s is free once the epilogue of tile k - 2 (which reads it) is done
-      if (k >= 2 && !umma::mbar_wait(&acc_free[s], (use - 1) & 1)) prod_abort = 1;
+      const int s = k % S, use = k / S;
+      // stage s is free once the epilogue of tile k - S (which reads it) is done
+      if (k >= S && !umma::mbar_wait(&acc_free[s], (use - 1) & 1)) prod_abort = 1;
       umma::named_sync(kProdBarrier, 128);
       if (prod_abort) break;  // uniform: read after the group barrier
       // warp w stages rows 32w..32w+31; lanes take consecutive 16-byte groups
       // of a row, so a warp reads contiguous row spans
       const int base = (blockIdx.x + k * gridDim.x) * 128 + 32 * warp;
       uint8_t* a = sA + s * kStage;
-      // all of the warp's loads first, then the shared stores
-      uint4 buf[C][8];
+      // the warp's loads of up to two chunks first, then their shared stores
+      constexpr int G = C < 2 ? C : 2;
 #pragma unroll
-      for (int c = 0; c < C; ++c)
+      for (int c0 = 0; c0 < C; c0 += G) {
+        uint4 buf[G][8];
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int item = it * 32 + lane, row = base + item / 8;
-          buf[c][it] = row < rows ? st.group(row, c, item % 8) : zero4();
-        }
+        for (int c = 0; c < G; ++c)
 #pragma unroll
-      for (int c = 0; c < C; ++c)
+          for (int it = 0; it < 8; ++it) {
+            const int item = it * 32 + lane, row = base + item / 8;
+            buf[c][it] = row < rows ? st.group(row, c0 + c, item % 8) : zero4();
+          }
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int item = it * 32 + lane;
-          *reinterpret_cast<uint4*>(a + umma::sw128_group(32 * warp + item / 8, c, item % 8, 128)) = buf[c][it];
-        }
+        for (int c = 0; c < G; ++c)
+#pragma unroll
+          for (int it = 0; it < 8; ++it) {
+            const int item = it * 32 + lane;
+            *reinterpret_cast<uint4*>(a + umma::sw128_group(32 * warp + item / 8, c0 + c, item % 8, 128)) = buf[c][it];
+          }
+      }
       umma::fence_async_smem();
       umma::named_sync(kProdBarrier, 128);
       if (tid == 0) {
         umma::fence_after();
-        umma::issue_tile<N, C>(tmem + s * NA, umma::smem_u32(a), umma::smem_u32(sB), false, &mma_done[s]);
+        umma::issue_tile<N, C, CB>(tmem + s * NA, umma::smem_u32(a), umma::smem_u32(sB), false, &mma_done[s]);
         issued = k + 1;
       }
     }
   } else {
     const int et = tid - 128;
     for (int k = 0; k < mine; ++k) {
-      const int s = k & 1, use = k >> 1;
+      const int s = k % S, use = k / S;
       if (!umma::mbar_wait(&mma_done[s], use & 1)) epi_abort = 1;
       umma::named_sync(kEpiBarrier, 128);
       if (epi_abort) break;  // uniform: read after the group barrier
@@ -428,7 +527,7 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep,
     if (tid == 0) {
       atomicOr(status, IPCB_STATUS_TIMEOUT);
       // let UMMAs still in flight finish (bounded) before the TMEM is freed
-      for (int k = issued > 2 ? issued - 2 : 0; k < issued; ++k) umma::mbar_wait(&mma_done[k & 1], (k >> 1) & 1);
+      for (int k = issued > S ? issued - S : 0; k < issued; ++k) umma::mbar_wait(&mma_done[k % S], (k / S) & 1);
     }
     __syncthreads();
   }
@@ -447,17 +546,17 @@ int sm_count() {
   return g_sms;
 }
 
-template <int N, int C, class Stage, class Epi>
+template <int N, int C, int CB = C, int S = 2, class Stage, class Epi>
 int launch_mlp(int rows, const Stage& st, const Epi& ep, const bf16* Bw, int* status, cudaStream_t s,
                const char* what) {
   if (rows <= 0) return 0;
-  constexpr size_t smem = mlp_smem<N, C>();
-  auto kern = k_mlp<N, C, Stage, Epi>;
+  constexpr size_t smem = mlp_smem<N, C, CB, S>();
+  auto kern = k_mlp<N, C, CB, S, Stage, Epi>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     ipcb::set_error_msg(what);
     return IPCB_E_CUDA;
   }
-  const int by_tmem = (int)(512 / umma::tmem_cols(2 * (N < 32 ? 32 : N)));
+  const int by_tmem = (int)(512 / umma::tmem_cols(S * (N < 32 ? 32 : N)));
   const int by_smem = (int)((227 * 1024) / (smem + 1024));
   const int per_sm = by_tmem < by_smem ? by_tmem : by_smem;
   const int tiles = (rows + 127) / 128;
@@ -467,137 +566,181 @@ int launch_mlp(int rows, const Stage& st, const Epi& ep, const bf16* Bw, int* st
 }
 
 // ------------------------------------------------------------ k_wgrad
-// dW[f][o] += sum_r X[r][f] dY[r][o] over all rows, plus the bias gradient in
-// row f = kx (a column of ones appended to X).  MT M-tiles of 128 features.
-struct EpiGrad {
-  float* dW;  // [kx][out]
-  float* db;  // [out]
-  int kx, out;
-  __device__ void add(int f, int col0, const float (&v)[32]) const {
-    if (f < kx) {
-      for (int i = 0; i < 32 && col0 + i < out; ++i) atomicAdd(dW + (size_t)f * out + col0 + i, v[i]);
-    } else if (f == kx) {
-      for (int i = 0; i < 32 && col0 + i < out; ++i) atomicAdd(db + col0 + i, v[i]);
-    }
-  }
+// All parameter gradients of a backward pass in one launch: a list of jobs
+// dW = X^T dY over batches of rows, every CTA a run of 128-row tiles of one
+// job, its products summed in TMEM and added to the gradient at the end.
+// Staging is the bound: both operands are row-major batches, and the UMMA
+// reads them MN-major, so a tile is staged by coalesced 16-byte loads and
+// 16-byte shared stores (the K-major form stored 2-byte elements transposed:
+// 77 us for an edge job of 91k rows and its 192 gathered features).  The
+// next tile's loads are in flight while the tensor core works on this one;
+// 80 KB and 128 TMEM columns a CTA leave two CTAs an SM.
+//
+// A's 128 columns are two staged chunks of 64, one of which can be the chunk
+// "ones" (column 0 ones), whose row of the product is the bias gradient:
+//   kBatch  [x0 | ones] x dY            columns 0..63 of the accumulator
+//   kPair   [x0 | x1] x dY, [ones | x1] x dY    columns 0..63 and 64..127
+//   kSums   [x0 | ones] x [s0 | s1], summed over the three bf16 pieces of s
+// Region r of the accumulator (columns 64 r ..) and half q of its rows go to
+// dst[r][q] (rows: how many of the 64 are written).
+enum { kBatch = 0, kPair = 1, kSums = 2 };
+struct WgradDst {
+  float* p;
+  int rows;
+};
+struct WgradJob {
+  const bf16 *x0, *x1;  // [rows][ldx], columns >= kx read as zero
+  const int* idx;       // rows of x0 (null: the batch rows)
+  const bf16* dy;       // [rows][64], or [rows][kSplit] split sums
+  int rows, mode, ldx, kx;
+  int ld, cols;         // row stride and written columns of dst
+  int first;            // first CTA of the job
+  WgradDst dst[2][2];
+};
+constexpr int kMaxJobs = 3 + 3 * LAYERS;
+struct WgradJobs {
+  WgradJob job[kMaxJobs];
+  int count, run;  // run: tiles a CTA takes
 };
 
-struct EpiGradHead {  // columns 0..8: the head
-  float *dW_off, *db_off;
-  __device__ void add(int f, int col0, const float (&v)[32]) const {
-    if (col0 != 0 || f > W) return;
-    for (int k = 0; k < 9; ++k) {
-      if (f < W) atomicAdd(dW_off + f * 9 + k, v[k]);
-      else atomicAdd(db_off + k, v[k]);
-    }
-  }
-};
+constexpr int kWgradThreads = 256;
+constexpr int kChunk = 128 * 128;  // bytes of a staged chunk
+constexpr size_t kWgradSmem = 1024 + 5 * kChunk;
 
-template <int MT, int N>
-constexpr size_t wgrad_smem() {
-  return 1024 + (size_t)MT * 2 * 128 * 128 + (size_t)2 * N * 128;
-}
-
-template <int MT, int N, class Epi>
-__global__ void __launch_bounds__(kThreads) k_wgrad(int R, const bf16* __restrict__ X, int ldx, int kx,
-                                                    const bf16* __restrict__ dY, int ldy, Epi ep,
-                                                    int* __restrict__ status) {
+__global__ void __launch_bounds__(kWgradThreads, 2) k_wgrad(const __grid_constant__ WgradJobs J,
+                                                            int* __restrict__ status) {
   extern __shared__ uint8_t dsmem[];
   __shared__ uint64_t mbar;
   __shared__ uint32_t tslot;
-  constexpr uint32_t kCols = umma::tmem_cols(MT * N);
-  uint8_t* sA = align1024(dsmem);                // MT x [128 features][128 rows]
-  uint8_t* sB = sA + MT * 2 * 128 * 128;         // [N outputs][128 rows]
-  const int tid = threadIdx.x, warp = tid >> 5;
-  if (warp == 0) umma::tmem_alloc(&tslot, kCols);
+  uint8_t* sx0 = align1024(dsmem);
+  uint8_t* sone = sx0 + kChunk;
+  uint8_t* sx1 = sone + kChunk;
+  uint8_t* sy = sx1 + kChunk;  // two chunks
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int j = 0;
+  while (j + 1 < J.count && (int)blockIdx.x >= J.job[j + 1].first) ++j;
+  const WgradJob& q = J.job[j];
+  const int mode = q.mode;
+  const int pieces = mode == kSums ? kPieces : 1;
+  const int tiles = (q.rows + 127) / 128 * pieces;
+  const int t0 = (blockIdx.x - q.first) * J.run, t1 = min(t0 + J.run, tiles);
+  const int g = tid & 7;
+  for (int i = tid; i < kChunk / 16; i += kWgradThreads) {
+    uint4 v = zero4();
+    if ((i & 7) == 0) v.x = 0x3f80u;  // bf16 1 in column 0
+    *reinterpret_cast<uint4*>(sone + umma::sw128_group(i >> 3, 0, i & 7, 128)) = v;
+  }
+  if (warp == 0) umma::tmem_alloc(&tslot, 128);
   if (tid == 0) umma::mbar_init(&mbar, 1);
   umma::fence_before();
   __syncthreads();
   umma::fence_after();
   const uint32_t tmem = tslot;
-  uint32_t phase = 0;
-  int ok = 1;
-  bool any = false;
-  const int ntiles = (R + 127) / 128;
-  const bf16 one = __float2bfloat16_rn(1.f), zero = __float2bfloat16_rn(0.f);
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int r = tile * 128 + tid;
-    const bool valid = r < R;
-    // X^T: element (feature f, k = tid)
-    for (int f0 = 0; f0 < MT * 128; f0 += 8) {
-      float xv[8];
-      if (valid && f0 + 8 <= kx) {
-        unpack8(ld4(X + (size_t)r * ldx + f0), xv);
+
+  uint4 bx[4], by[4], bz[4];
+  auto load = [&](int t) {
+    const int base = t / pieces * 128 + (tid >> 3), piece = t % pieces;
+#pragma unroll
+    for (int it = 0; it < 4; ++it) {
+      const int r = base + 32 * it;
+      bx[it] = by[it] = bz[it] = zero4();
+      if (r >= q.rows) continue;
+      if (8 * g < q.kx) bx[it] = ld4(q.x0 + (size_t)(q.idx ? __ldg(q.idx + r) : r) * q.ldx + 8 * g);
+      if (mode == kSums) {
+        const bf16* y = q.dy + (size_t)r * kSplit + piece * 2 * W + 8 * g;
+        by[it] = ld4(y);
+        bz[it] = ld4(y + W);
       } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) xv[i] = 0.f;
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int f = f0 + i;
-        bf16 val = f < kx ? __float2bfloat16_rn(xv[i]) : (f == kx && valid ? one : zero);
-        *reinterpret_cast<bf16*>(sA + (f >> 7) * (2 * 128 * 128) + umma::sw128_offset(f & 127, tid, 128)) = val;
+        by[it] = ld4(q.dy + (size_t)r * W + 8 * g);
+        if (mode == kPair) bz[it] = ld4(q.x1 + (size_t)r * q.ldx + 8 * g);
       }
     }
-    for (int o0 = 0; o0 < N; o0 += 8) {
-      float yv[8];
-      if (valid) unpack8(ld4(dY + (size_t)r * ldy + o0), yv);
-      else {
+  };
+  bool ok = true;
+  uint32_t phase = 0;
+  if (t0 < t1) load(t0);
+  for (int t = t0; t < t1; ++t) {
+    if (t > t0) {  // the tensor core has read the previous tile
+      ok = __syncthreads_and(umma::mbar_wait(&mbar, phase) ? 1 : 0);
+      if (!ok) break;
+      phase ^= 1;
+    }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) yv[i] = 0.f;
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        *reinterpret_cast<bf16*>(sB + umma::sw128_offset(o0 + i, tid, N)) = __float2bfloat16_rn(yv[i]);
+    for (int it = 0; it < 4; ++it) {
+      const uint32_t o = umma::sw128_group((tid >> 3) + 32 * it, 0, g, 128);
+      *reinterpret_cast<uint4*>(sx0 + o) = bx[it];
+      *reinterpret_cast<uint4*>(sy + o) = by[it];
+      if (mode != kBatch) *reinterpret_cast<uint4*>((mode == kPair ? sx1 : sy + kChunk) + o) = bz[it];
     }
     umma::fence_async_smem();
     __syncthreads();
+    if (t + 1 < t1) load(t + 1);
     if (tid == 0) {
       umma::fence_after();
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-        umma::issue<N, 2>(tmem + mt * N, umma::smem_u32(sA + mt * 2 * 128 * 128), umma::smem_u32(sB), any);
+      const uint32_t x0 = umma::smem_u32(sx0), one = umma::smem_u32(sone), y = umma::smem_u32(sy);
+      if (mode == kSums) {
+        umma::issue_mn<128>(tmem, x0, kChunk, y, kChunk, t > t0);
+      } else if (mode == kPair) {
+        umma::issue_mn<64>(tmem, x0, 2 * kChunk, y, kChunk, t > t0);
+        umma::issue_mn<64>(tmem + W, one, kChunk, y, kChunk, t > t0);
+      } else {
+        umma::issue_mn<64>(tmem, x0, kChunk, y, kChunk, t > t0);
+      }
       umma::commit(&mbar);
     }
-    ok = __syncthreads_and(umma::mbar_wait(&mbar, phase) ? 1 : 0);
-    phase ^= 1;
-    if (!ok) break;
-    any = true;
   }
+  if (ok && t0 < t1) ok = __syncthreads_and(umma::mbar_wait(&mbar, phase) ? 1 : 0);
   if (!ok) {
     if (tid == 0) atomicOr(status, IPCB_STATUS_TIMEOUT);
-    umma::mbar_wait(&mbar, phase);
-  } else if (any) {
+    umma::mbar_wait(&mbar, phase);  // the copies in flight, once more, before the TMEM is freed
+  } else if (t0 < t1) {
     umma::fence_after();
+    // warps 0-3 drain region 0, warps 4-7 region 1
+    const int region = warp >> 2, row = 32 * (warp & 3) + lane, half = row >> 6, f = row & 63;
+    const WgradDst d = q.dst[region][half];
+    if (q.dst[region][0].p) {  // uniform over the warp: the columns were written
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int col = 0; col < N; col += 32) {
+      for (int col = 0; col < W; col += 32) {
         float v[32];
-        umma::tmem_ld32(tmem + ((uint32_t)(32 * warp) << 16) + mt * N + col, v);
-        ep.add(mt * 128 + tid, col, v);
+        __syncwarp();
+        umma::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + region * W + col, v);
+        float* o = d.p + (size_t)f * q.ld + col;
+        if (!d.p || f >= d.rows) {
+        } else if (q.cols == W && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            atomicAdd(reinterpret_cast<float4*>(o + i), make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (col + i < q.cols) atomicAdd(o + i, v[i]);
+        }
       }
+    }
   }
   umma::fence_before();
   __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem, kCols);
+  if (warp == 0) umma::tmem_dealloc(tmem, 128);
 }
 
-template <int MT, int N, class Epi>
-int launch_wgrad(int R, const bf16* X, int ldx, int kx, const bf16* dY, int ldy, const Epi& ep, int* status,
-                 cudaStream_t s, const char* what) {
-  if (R <= 0) return 0;
-  constexpr size_t smem = wgrad_smem<MT, N>();
-  auto kern = k_wgrad<MT, N, Epi>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    ipcb::set_error_msg(what);
+int launch_wgrad(WgradJobs& J, int* status, cudaStream_t s) {
+  if (cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgradSmem) != cudaSuccess) {
+    ipcb::set_error_msg("mpnn wgrad");
     return IPCB_E_CUDA;
   }
-  const int tiles = (R + 127) / 128;
-  // few CTAs: each reduces many tiles in TMEM before its atomics
-  const int cap = sm_count();
-  kern<<<tiles < cap ? tiles : cap, kThreads, smem, s>>>(R, X, ldx, kx, dY, ldy, ep, status);
-  return ipcb::check_launch(what);
+  auto tiles = [](const WgradJob& q) { return (long long)((q.rows + 127) / 128) * (q.mode == kSums ? kPieces : 1); };
+  long long all = 0;
+  for (int j = 0; j < J.count; ++j) all += tiles(J.job[j]);
+  // one wave of two CTAs an SM: each reduces its run of tiles in TMEM before its atomics
+  const int cap = 2 * sm_count();
+  J.run = (int)((all + cap - 1) / cap);
+  int blocks = 0;
+  for (int j = 0; j < J.count; ++j) {
+    J.job[j].first = blocks;
+    blocks += (int)((tiles(J.job[j]) + J.run - 1) / J.run);
+  }
+  k_wgrad<<<blocks, kWgradThreads, kWgradSmem, s>>>(J, status);
+  return ipcb::check_launch("mpnn wgrad");
 }
 
 // ------------------------------------------------------------ graph
@@ -879,86 +1022,83 @@ __global__ void __launch_bounds__(256) k_mean_messages(int n, const int* __restr
 }
 
 // ------------------------------------------------------------ backward helpers
-__global__ void k_gather_rows(int R, const bf16* __restrict__ X, const int* __restrict__ idx, bf16* __restrict__ out) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;  // one 16-byte group
-  if (t >= R * 8) return;
-  const int r = t >> 3, g = t & 7;
-  reinterpret_cast<uint4*>(out)[t] = ld4(X + (size_t)idx[r] * W + g * 8);
+// Gradients through a message's two node inputs are linear in its gradient:
+// sum_e dY_e W1a^T over a row's edges is (sum_e dY_e) W1a^T.  So the backward
+// message product runs over the edges only for the edge input, and over the
+// nodes for the other two, on the sums of dY over a node's row and column.
+// The sums stay fp32: they are split into three bf16 pieces (8 significant
+// bits each, the rest of one piece exact in the next), and the products over
+// all pieces share one fp32 accumulator.
+__device__ __forceinline__ void store_split(bf16* s, const float (&v)[8]) {  // s: piece 0 of 8 columns
+  float r[8];
+#pragma unroll
+  for (int t = 0; t < 8; ++t) r[t] = v[t];
+#pragma unroll
+  for (int p = 0; p < kPieces; ++p) {
+    *reinterpret_cast<uint4*>(s + p * 2 * W) = pack8(r);
+#pragma unroll
+    for (int t = 0; t < 8; ++t) r[t] -= bfr(r[t]);
+  }
 }
 
-__global__ void k_edge_x(int nnz, const bf16* __restrict__ h, const bf16* __restrict__ e, const int* __restrict__ rows,
-                         const int* __restrict__ cols, bf16* __restrict__ X) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;  // 24 groups per edge
-  if (t >= nnz * 24) return;
-  const int k = t / 24, g = t % 24;
-  uint4 v;
-  if (g < 8) v = ld4(h + (size_t)rows[k] * W + g * 8);
-  else if (g < 16) v = ld4(h + (size_t)cols[k] * W + (g - 8) * 8);
-  else v = ld4(e + (size_t)k * W + (g - 16) * 8);
-  reinterpret_cast<uint4*>(X)[t] = v;
+// Per node: dY_e = bf16((de_e + da) * (m_e > 0)) over the row's edges and the
+// split sum of dY over the row.  A warp a row, 4 edges x 8 column groups a
+// step (as k_mean_messages): da is read once a row and de, m and dY move as
+// whole 256- and 128-byte rows.  Bound by those bytes; with the sum on board
+// it takes 10 us for 91k edges where a thread an element took 18.
+__global__ void __launch_bounds__(256) k_edge_grad(int n, const int* __restrict__ off, const float* __restrict__ de,
+                                                   const float* __restrict__ da, const bf16* __restrict__ m,
+                                                   bf16* __restrict__ dy, bf16* __restrict__ sums) {
+  const int lane = threadIdx.x & 31, slot = lane >> 3, g = lane & 7;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const int b = __ldg(off + i), e = __ldg(off + i + 1);
+    float d[8] = {0, 0, 0, 0, 0, 0, 0, 0}, acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (da) ld8f(da + (size_t)i * W + 8 * g, d);
+#pragma unroll 2
+    for (int k = b + slot; k < e; k += 4) {
+      float f[8], a[8];
+      ld8f(de + (size_t)k * W + 8 * g, f);
+      unpack8(ld4(m + (size_t)k * W + 8 * g), a);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        f[t] = a[t] > 0.f ? bfr(f[t] + d[t]) : 0.f;
+        acc[t] += f[t];
+      }
+      *reinterpret_cast<uint4*>(dy + (size_t)k * W + 8 * g) = pack8(f);
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 8);
+      acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 16);
+    }
+    if (slot == 0) store_split(sums + (size_t)i * kSplit + 8 * g, acc);
+  }
 }
 
-__global__ void k_node_x(int n, const bf16* __restrict__ h, const bf16* __restrict__ a, bf16* __restrict__ X) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;  // 16 groups per node
-  if (t >= n * 16) return;
-  const int i = t / 16, g = t % 16;
-  reinterpret_cast<uint4*>(X)[t] = g < 8 ? ld4(h + (size_t)i * W + g * 8) : ld4(a + (size_t)i * W + (g - 8) * 8);
-}
-
-// out = bf16(d * (act > 0)) over rows x 64
-__global__ void k_relu_grad(long long count, const float* __restrict__ d, const bf16* __restrict__ act,
-                            bf16* __restrict__ out) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  out[t] = __float2bfloat16_rn(__bfloat162float(act[t]) > 0.f ? d[t] : 0.f);
-}
-
-// dm = de + da[row]; out = bf16(dm * (m > 0))
-__global__ void k_edge_grad(int nnz, const float* __restrict__ de, const float* __restrict__ da,
-                            const int* __restrict__ rows, const bf16* __restrict__ m, bf16* __restrict__ out) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nnz * W) return;
-  const int e = (int)(t / W), c = (int)(t % W);
-  const float dm = de[t] + da[(size_t)rows[e] * W + c];
-  out[t] = __float2bfloat16_rn(__bfloat162float(m[t]) > 0.f ? dm : 0.f);
-}
-
-// dh += dXn[:, :64]; da = dXn[:, 64:] / deg
-__global__ void k_node_post(int n, const int* __restrict__ off, const float* __restrict__ dXn, float* __restrict__ dh,
-                            float* __restrict__ da) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n * W) return;
-  const int i = (int)(t / W), c = (int)(t % W);
-  const float deg = (float)(off[i + 1] - off[i]);
-  dh[t] += dXn[(size_t)i * 2 * W + c];
-  da[t] = dXn[(size_t)i * 2 * W + W + c] / deg;
-}
-
-// de += dX[:, 128:192]
-__global__ void k_edge_post_e(int nnz, const float* __restrict__ dX, float* __restrict__ de) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)nnz * W) return;
-  const int e = (int)(t / W), c = (int)(t % W);
-  de[t] += dX[(size_t)e * 3 * W + 2 * W + c];
-}
-
-// dh[i] += sum over row i of dX[e][0:64] + dX[rev e][64:128]
-__global__ void k_edge_post_h(int n, const int* __restrict__ off, const int* __restrict__ rev,
-                              const float* __restrict__ dX, float* __restrict__ dh) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)n * W) return;
-  const int i = (int)(t / W), c = (int)(t % W);
-  float s = 0.f;
-  for (int e = off[i]; e < off[i + 1]; ++e) s += dX[(size_t)e * 3 * W + c] + dX[(size_t)rev[e] * 3 * W + W + c];
-  dh[t] += s;
-}
-
-__global__ void k_scatter_rows(int R, const int* __restrict__ idx, const float* __restrict__ src,
-                               float* __restrict__ dst) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)R * W) return;
-  const int r = (int)(t / W), c = (int)(t % W);
-  dst[(size_t)idx[r] * W + c] = src[t];
+// The same sums over the node's column: the blocks (j, i) are the transposes
+// rev of row i's.
+__global__ void __launch_bounds__(256) k_column_sums(int n, const int* __restrict__ off, const int* __restrict__ rev,
+                                                     const bf16* __restrict__ dy, bf16* __restrict__ sums) {
+  const int lane = threadIdx.x & 31, slot = lane >> 3, g = lane & 7;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const int b = __ldg(off + i), e = __ldg(off + i + 1);
+    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
+    for (int k = b + slot; k < e; k += 4) {
+      float f[8];
+      unpack8(ld4(dy + (size_t)__ldg(rev + k) * W + 8 * g), f);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) acc[t] += f[t];
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 8);
+      acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], 16);
+    }
+    if (slot == 0) store_split(sums + (size_t)i * kSplit + W + 8 * g, acc);
+  }
 }
 
 __global__ void k_adam(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -1162,16 +1302,15 @@ int ipcb_mpnn_loss_grad(const ipcb_graph* g, const float* ahat, const void* x, c
 }
 
 size_t ipcb_mpnn_backward_workspace(int n, int nnz, int n_lower) {
-  const size_t big = (size_t)nnz * 3 * W > (size_t)n * 2 * W ? (size_t)nnz * 3 * W : (size_t)n * 2 * W;
-  const size_t rowsmax = (size_t)(nnz > n ? nnz : n);
+  (void)n_lower;
   size_t b = 0;
   auto add = [&](size_t bytes) { b += (bytes + 255) & ~(size_t)255; };
-  add(sizeof(float) * n * W);                 // dh
-  add(sizeof(float) * nnz * W);               // de
-  add(sizeof(float) * n * W);                 // da
-  add(sizeof(float) * (big > (size_t)n_lower * W ? big : (size_t)n_lower * W));  // dX
-  add(sizeof(bf16) * (big > (size_t)n_lower * W ? big : (size_t)n_lower * W));   // X
-  add(sizeof(bf16) * rowsmax * W);            // dY
+  add(sizeof(float) * n * W);                     // dh
+  add(sizeof(float) * nnz * W);                   // de
+  add(sizeof(float) * n * W);                     // da
+  add(sizeof(bf16) * LAYERS * n * W);             // dY of the node updates and of the node encoder
+  add(sizeof(bf16) * (LAYERS + 1) * nnz * W);     // dY of the messages and of the edge encoder
+  add(sizeof(bf16) * LAYERS * n * kSplit);        // split sums of the messages' dY
   return b + 256;
 }
 
@@ -1187,71 +1326,96 @@ int ipcb_mpnn_backward(const ipcb_graph* g, const void* packed, const float* par
   cudaStream_t st = (cudaStream_t)s;
   const bf16* P = (const bf16*)packed;
   const int n = g->n, nnz = g->nnz, L = g->n_lower;
-  const size_t big = (size_t)nnz * 3 * W > (size_t)n * 2 * W ? (size_t)nnz * 3 * W : (size_t)n * 2 * W;
-  const size_t bigl = big > (size_t)L * W ? big : (size_t)L * W;
   Carve c{(uint8_t*)ws, ws_bytes};
   float* dh = c.take<float>((size_t)n * W);
   float* de = c.take<float>((size_t)nnz * W);
   float* da = c.take<float>((size_t)n * W);
-  float* dX = c.take<float>(bigl);
-  bf16* X = c.take<bf16>(bigl);
-  bf16* dY = c.take<bf16>((size_t)(nnz > n ? nnz : n) * W);
+  bf16* dyn = c.take<bf16>((size_t)LAYERS * n * W);
+  bf16* dye = c.take<bf16>((size_t)(LAYERS + 1) * nnz * W);
+  bf16* sums = c.take<bf16>((size_t)LAYERS * n * kSplit);
+  // slot l: update l (l < LAYERS - 1) or message l; the last slot: the encoder
+  auto dY_node = [&](int l) { return dyn + (size_t)l * n * W; };
+  auto dY_edge = [&](int l) { return dye + (size_t)l * nnz * W; };
   const bf16* H = (const bf16*)tape->h;
   const bf16* E = (const bf16*)tape->e;
   const bf16* Mt = (const bf16*)tape->m;
   const bf16* At = (const bf16*)tape->a;
   const bf16* Ut = (const bf16*)tape->u;
   const bf16* dGb = (const bf16*)dG;
+  constexpr int kNodeEnc = LAYERS - 1, kEdgeEnc = LAYERS;
+  const long long need = ((long long)n * 32 + 255) / 256, most = 16LL * sm_count();
+  const int warp_rows = (int)(need < most ? need : most);
+  WgradJobs J{};
+  auto job = [&](int mode, int rows, const bf16* x0, const bf16* x1, const int* idx, int ldx, const bf16* dy,
+                 int ld) -> WgradJob& {
+    WgradJob& q = J.job[J.count++];
+    q.mode = mode; q.rows = rows; q.x0 = x0; q.x1 = x1; q.idx = idx; q.ldx = q.kx = ldx; q.dy = dy;
+    q.ld = q.cols = ld;
+    return q;
+  };
   int rc;
-  // head
-  k_gather_rows<<<grid_for((long long)L * 8), 256, 0, st>>>(L, E + (size_t)LAYERS * nnz * W, g->lower, X);
-  rc = launch_wgrad<1, 16>(L, X, W, W, dGb, 64, EpiGradHead{grad + P_WOFF, grad + P_BOFF}, status, st,
-                           "mpnn head wgrad");
-  if (rc) return rc;
-  rc = launch_mlp<64, 1>(L, StageDense{dGb, 64, 64}, EpiF32{dX, W}, P + K_HEAD, status, st, "mpnn head dx");
-  if (rc) return rc;
+  // head: it reads the edge states alone
   cudaMemsetAsync(de, 0, sizeof(float) * nnz * W, st);
   cudaMemsetAsync(dh, 0, sizeof(float) * n * W, st);
-  k_scatter_rows<<<grid_for((long long)L * W), 256, 0, st>>>(L, g->lower, dX, de);
+  rc = launch_mlp<64, 1>(L, StageDense{dGb, 64, 64}, EpiRows{de, g->lower}, P + K_HEAD, status, st, "mpnn head dx");
+  if (rc) return rc;
+  {
+    WgradJob& q = job(kBatch, L, E + (size_t)LAYERS * nnz * W, nullptr, g->lower, W, dGb, 9);
+    q.dst[0][0] = {grad + P_WOFF, W};
+    q.dst[0][1] = {grad + P_BOFF, 1};
+  }
   for (int l = LAYERS - 1; l >= 0; --l) {
     const bf16* h = H + (size_t)l * n * W;
     const bf16* e = E + (size_t)l * nnz * W;
     const bf16* m = Mt + (size_t)l * nnz * W;
     const bf16* a = At + (size_t)l * n * W;
-    const bf16* u = Ut + (size_t)l * n * W;
     float* gl = grad + P_LAYER0 + l * P_LAYER;
-    // node update: h_out = h + relu([h, a] W2 + b2)
-    k_relu_grad<<<grid_for((long long)n * W), 256, 0, st>>>((long long)n * W, dh, u, dY);
-    k_node_x<<<grid_for((long long)n * 16), 256, 0, st>>>(n, h, a, X);
-    rc = launch_wgrad<2, 64>(n, X, 2 * W, 2 * W, dY, W, EpiGrad{gl + O_W2, gl + O_B2, 2 * W, W}, status, st,
-                             "mpnn update wgrad");
-    if (rc) return rc;
-    rc = launch_mlp<128, 1>(n, StageDense{dY, W, W}, EpiF32{dX, 2 * W}, P + K_W2 + l * 2 * W * W, status, st,
-                            "mpnn update dx");
-    if (rc) return rc;
-    k_node_post<<<grid_for((long long)n * W), 256, 0, st>>>(n, g->offsets, dX, dh, da);
+    // node update: h_out = h + relu([h, a] W2 + b2).  Nothing reads the last
+    // layer's node states, so its update has no gradient.
+    const bool update = l + 1 < LAYERS;
+    if (update) {
+      rc = launch_mlp<128, 1>(n, StageDense{dY_node(l), W, W}, EpiUpdateGrad{dh, da, g->offsets},
+                              P + K_W2 + l * 2 * W * W, status, st, "mpnn update dx");
+      if (rc) return rc;
+      WgradJob& q = job(kPair, n, h, a, nullptr, W, dY_node(l), W);
+      q.dst[0][0] = {gl + O_W2, W};
+      q.dst[0][1] = {gl + O_W2 + W * W, W};
+      q.dst[1][0] = {gl + O_B2, 1};
+    }
     // message: e_out = e + m, m = relu([h_i, h_j, e] W1 + b1), a = mean m
-    k_edge_grad<<<grid_for((long long)nnz * W), 256, 0, st>>>(nnz, de, da, g->rows, m, dY);
-    k_edge_x<<<grid_for((long long)nnz * 24), 256, 0, st>>>(nnz, h, e, g->rows, g->columns, X);
-    rc = launch_wgrad<2, 64>(nnz, X, 3 * W, 3 * W, dY, W, EpiGrad{gl + O_W1, gl + O_B1, 3 * W, W}, status, st,
-                             "mpnn message wgrad");
+    bf16* sl = sums + (size_t)l * n * kSplit;
+    k_edge_grad<<<warp_rows, 256, 0, st>>>(n, g->offsets, de, update ? da : nullptr, m, dY_edge(l), sl);
+    k_column_sums<<<warp_rows, 256, 0, st>>>(n, g->offsets, g->rev, dY_edge(l), sl);
+    const bf16* w1 = P + K_W1 + l * 3 * W * W;
+    rc = launch_mlp<64, 1>(nnz, StageDense{dY_edge(l), W, W},
+                           EpiAdd{de, l ? nullptr : E, l ? nullptr : dY_edge(kEdgeEnc)}, w1 + 2 * W * W, status, st,
+                           "mpnn message dx");
     if (rc) return rc;
-    rc = launch_mlp<192, 1>(nnz, StageDense{dY, W, W}, EpiF32{dX, 3 * W}, P + K_W1 + l * 3 * W * W, status, st,
-                            "mpnn message dx");
+    rc = launch_mlp<64, 2 * kPieces, 2, 1>(
+        n, StageSplit{sl}, EpiAdd{dh, l ? Ut + (size_t)(l - 1) * n * W : H, dY_node(l ? l - 1 : kNodeEnc)}, w1, status,
+        st, "mpnn message dh");
     if (rc) return rc;
-    k_edge_post_e<<<grid_for((long long)nnz * W), 256, 0, st>>>(nnz, dX, de);
-    k_edge_post_h<<<grid_for((long long)n * W), 256, 0, st>>>(n, g->offsets, g->rev, dX, dh);
+    {
+      WgradJob& q = job(kBatch, nnz, e, nullptr, nullptr, W, dY_edge(l), W);
+      q.dst[0][0] = {gl + O_W1 + 2 * W * W, W};
+    }
+    WgradJob& q = job(kSums, n, h, nullptr, nullptr, W, sl, W);
+    q.dst[0][0] = {gl + O_W1, W};
+    q.dst[0][1] = {gl + O_B1, 1};
+    q.dst[1][0] = {gl + O_W1 + W * W, W};
   }
   // encoders
-  k_relu_grad<<<grid_for((long long)n * W), 256, 0, st>>>((long long)n * W, dh, H, dY);
-  rc = launch_wgrad<1, 64>(n, (const bf16*)x, IN, IN, dY, W, EpiGrad{grad + P_WHIN, grad + P_BHIN, IN, W}, status,
-                           st, "mpnn node encoder wgrad");
-  if (rc) return rc;
-  k_relu_grad<<<grid_for((long long)nnz * W), 256, 0, st>>>((long long)nnz * W, de, E, dY);
-  rc = launch_wgrad<1, 64>(nnz, (const bf16*)y, IN, IN, dY, W, EpiGrad{grad + P_WEIN, grad + P_BEIN, IN, W}, status,
-                           st, "mpnn edge encoder wgrad");
-  if (rc) return rc;
-  return ipcb::check_launch("ipcb_mpnn_backward");
+  {
+    WgradJob& q = job(kBatch, n, (const bf16*)x, nullptr, nullptr, IN, dY_node(kNodeEnc), W);
+    q.dst[0][0] = {grad + P_WHIN, IN};
+    q.dst[0][1] = {grad + P_BHIN, 1};
+  }
+  {
+    WgradJob& q = job(kBatch, nnz, (const bf16*)y, nullptr, nullptr, IN, dY_edge(kEdgeEnc), W);
+    q.dst[0][0] = {grad + P_WEIN, IN};
+    q.dst[0][1] = {grad + P_BEIN, 1};
+  }
+  return launch_wgrad(J, status, st);
 }
 
 int ipcb_adam(int n, float* params, const float* grad, float* m, float* v, float lr, float beta1, float beta2,

@@ -132,9 +132,10 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 }
 
 // D[128 x N] (+)= A[128 x 64C] * B[N x 64C]^T from SW128 K-major tiles at
-// shared addresses a_base (128 rows) and b_base (N rows).  Issued by one
-// thread; the caller commits to an mbarrier afterwards.
-template <int N, int C>
+// shared addresses a_base (128 rows) and b_base (N rows).  With CB < C, chunk
+// c of A meets chunk c % CB of B.  Issued by one thread; the caller commits
+// to an mbarrier afterwards.
+template <int N, int C, int CB = C>
 __device__ __forceinline__ void issue(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, bool accumulate) {
   constexpr uint32_t idesc = idesc_bf16_f32(N);
 #pragma unroll
@@ -142,16 +143,43 @@ __device__ __forceinline__ void issue(uint32_t tmem_d, uint32_t a_base, uint32_t
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       const uint64_t a = desc_sw128(a_base + c * 128 * 128 + s * 32);
-      const uint64_t b = desc_sw128(b_base + c * N * 128 + s * 32);
+      const uint64_t b = desc_sw128(b_base + (c % CB) * N * 128 + s * 32);
       mma_bf16(tmem_d, a, b, idesc, (accumulate || c > 0 || s > 0) ? 1u : 0u);
     }
 }
 
-template <int N, int C>
+template <int N, int C, int CB = C>
 __device__ __forceinline__ void issue_tile(uint32_t tmem_d, uint32_t a_base, uint32_t b_base, bool accumulate,
                                            uint64_t* mbar) {
-  issue<N, C>(tmem_d, a_base, b_base, accumulate);
+  issue<N, C, CB>(tmem_d, a_base, b_base, accumulate);
   commit(mbar);
+}
+
+// The same tile read the other way (MN-major): the chunk's 128 rows are the
+// K index and its 64 columns the M or N index, so a row-major batch staged
+// with sw128_group is the transposed operand as it lies.  Eight rows (1024
+// bytes) are one swizzle atom, SBO steps to the next eight rows, and LBO
+// steps to the next 64 columns (another chunk).
+__device__ __forceinline__ uint64_t desc_sw128_mn(uint32_t saddr, uint32_t lbo) {
+  uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)(1024u >> 4) << 32;
+  d |= (uint64_t)1u << 46;
+  d |= (uint64_t)2u << 61;
+  return d;
+}
+
+// D[128 x N] (+)= A^T B over the 128 rows of the staged chunks: A's 128
+// columns are the chunks at a_base and a_base + a_lbo, B's N columns the
+// chunks at b_base (and b_base + b_lbo for N > 64).
+template <int N>
+__device__ __forceinline__ void issue_mn(uint32_t tmem_d, uint32_t a_base, uint32_t a_lbo, uint32_t b_base,
+                                         uint32_t b_lbo, bool accumulate) {
+  constexpr uint32_t idesc = idesc_bf16_f32(N) | (1u << 15) | (1u << 16);  // both operands MN-major
+#pragma unroll
+  for (int s = 0; s < 8; ++s)
+    mma_bf16(tmem_d, desc_sw128_mn(a_base + s * 2048, a_lbo), desc_sw128_mn(b_base + s * 2048, b_lbo), idesc,
+             (accumulate || s > 0) ? 1u : 0u);
 }
 
 // TMEM columns to allocate for n accumulator columns (a power of two >= 32,

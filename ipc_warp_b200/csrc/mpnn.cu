@@ -301,21 +301,25 @@ struct EpiHead {
   }
 };
 
-struct EpiF32 {  // plain fp32 rows of width ld (lanes across the columns)
-  float* out;
-  int ld;
-  __device__ void rows32(int grow0, int nvalid, const float* acc, int stride, const uint8_t*, int, int lane) const {
-    for (int r = 0; r < nvalid; ++r) {
-      float* o = out + (size_t)(grow0 + r) * ld;
-      for (int c = lane; c < ld; c += 32) o[c] = acc[r * stride + c];
-    }
-  }
-};
-
 __device__ __forceinline__ void st8f(float* p, const float (&f)[8]) {
   reinterpret_cast<float4*>(p)[0] = make_float4(f[0], f[1], f[2], f[3]);
   reinterpret_cast<float4*>(p)[1] = make_float4(f[4], f[5], f[6], f[7]);
 }
+
+struct EpiPart {  // fp32 rows of 2 W columns, of which a part writes W
+  float* out;
+  __device__ void rows32(int grow0, int nvalid, const float* acc, int stride, const uint8_t*, int, int lane) const {
+    const int q = lane >> 3, cg = lane & 7;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int r = 4 * it + q;
+      if (r >= nvalid) continue;
+      float v[8];
+      ld8s(acc + r * stride + 8 * cg, v);
+      st8f(out + (size_t)(grow0 + r) * 2 * W + blockIdx.y * W + 8 * cg, v);
+    }
+  }
+};
 
 struct EpiRows {  // out[idx[row]] = v (fp32, 64 columns)
   float* out;
@@ -364,31 +368,27 @@ struct EpiAdd {
   }
 };
 
-struct EpiUpdateGrad {  // [dh | dmean] of a node: dh += v[0:64], da = v[64:128] / degree
+struct EpiUpdateGrad {  // [dh | dmean] of a node: part 0 dh += v, part 1 da = v / degree
   float *dh, *da;
   const int* off;
-  __device__ void rows32(int grow0, int nvalid, const float* acc, int stride, const uint8_t*, int, int lane) const {
-    const int q = lane >> 4, cg = lane & 15;
+  __device__ void rows32(int grow0, int nvalid, const float* acc, int stride, const uint8_t* tile, int r0,
+                         int lane) const {
+    if (blockIdx.y == 0) {
+      EpiAdd{dh, nullptr, nullptr}.rows32(grow0, nvalid, acc, stride, tile, r0, lane);
+      return;
+    }
+    const int q = lane >> 3, cg = lane & 7;
     const float mine = lane < nvalid ? (float)(__ldg(off + grow0 + lane + 1) - __ldg(off + grow0 + lane)) : 1.f;
-#pragma unroll 8
-    for (int it = 0; it < 16; ++it) {
-      const int r = 2 * it + q;
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int r = 4 * it + q;
       const float deg = __shfl_sync(0xffffffffu, mine, r);
       if (r >= nvalid) continue;
       float v[8];
       ld8s(acc + r * stride + 8 * cg, v);
-      const size_t o = (size_t)(grow0 + r) * W + 8 * (cg & 7);
-      if (cg < 8) {
-        float f[8];
-        ld8f(dh + o, f);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) f[t] += v[t];
-        st8f(dh + o, f);
-      } else {
-#pragma unroll
-        for (int t = 0; t < 8; ++t) v[t] /= deg;
-        st8f(da + o, v);
-      }
+      for (int t = 0; t < 8; ++t) v[t] /= deg;
+      st8f(da + (size_t)(grow0 + r) * W + 8 * cg, v);
     }
   }
 };
@@ -411,6 +411,11 @@ constexpr size_t mlp_smem() {
   return 1024 + S * (size_t)C * 128 * 128 + (size_t)CB * N * 128 + 128 * (size_t)(N + 1) * 4;
 }
 
+// Products wider than 64 columns run as gridDim.y column parts of N (the
+// epilogue's part): over the nodes there are fewer tiles than SMs, and a CTA's
+// time is the chain of its own loads, UMMAs and stores (projection and update
+// gradient of 6,500 nodes: 12.7 us a product with 128 columns at once, 8.4 in
+// two parts).
 template <int N, int C, int CB, int S, class Stage, class Epi>
 __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep, const bf16* __restrict__ Bw,
                                                      int* __restrict__ status) {
@@ -431,6 +436,7 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep,
   float* accs = reinterpret_cast<float*>(sB + CB * N * 128);  // [128][N + 1]
   constexpr int kStride = N + 1;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  Bw += (size_t)blockIdx.y * N * K;
 
   for (int idx = tid; idx < N * CB * 8; idx += kMlpThreads) {
     const int r = idx / (CB * 8), c = (idx / 8) % CB, g = idx % 8;
@@ -548,7 +554,7 @@ int sm_count() {
 
 template <int N, int C, int CB = C, int S = 2, class Stage, class Epi>
 int launch_mlp(int rows, const Stage& st, const Epi& ep, const bf16* Bw, int* status, cudaStream_t s,
-               const char* what) {
+               const char* what, int parts = 1) {
   if (rows <= 0) return 0;
   constexpr size_t smem = mlp_smem<N, C, CB, S>();
   auto kern = k_mlp<N, C, CB, S, Stage, Epi>;
@@ -561,7 +567,7 @@ int launch_mlp(int rows, const Stage& st, const Epi& ep, const bf16* Bw, int* st
   const int per_sm = by_tmem < by_smem ? by_tmem : by_smem;
   const int tiles = (rows + 127) / 128;
   const int cap = sm_count() * (per_sm > 0 ? per_sm : 1);
-  kern<<<tiles < cap ? tiles : cap, kMlpThreads, smem, s>>>(rows, st, ep, Bw, status);
+  kern<<<dim3(tiles < cap ? tiles : cap, parts), kMlpThreads, smem, s>>>(rows, st, ep, Bw, status);
   return ipcb::check_launch(what);
 }
 
@@ -1255,8 +1261,8 @@ int ipcb_mpnn_forward(const ipcb_graph* g, const void* packed, const float* para
     bf16* a = tr ? (bf16*)tape->a + (size_t)l * n * W : nullptr;
     bf16* u = tr ? (bf16*)tape->u + (size_t)l * n * W : nullptr;
     // per-node projections of both message endpoints, then the edge product
-    rc = launch_mlp<128, 1>(n, StageDense{hbuf(l), W, W}, EpiF32{tape->proj, 2 * W}, P + K_W1ABT + l * 2 * W * W,
-                            status, st, "mpnn message projection");
+    rc = launch_mlp<64, 1>(n, StageDense{hbuf(l), W, W}, EpiPart{tape->proj}, P + K_W1ABT + l * 2 * W * W, status, st,
+                           "mpnn message projection", 2);
     if (rc) return rc;
     rc = launch_mlp<64, 1>(nnz, StageDense{ebuf(l), W, W},
                            EpiEdge{pl + O_B1, tape->proj, ebuf(l + 1), m, g->rows, g->columns},
@@ -1374,8 +1380,8 @@ int ipcb_mpnn_backward(const ipcb_graph* g, const void* packed, const float* par
     // layer's node states, so its update has no gradient.
     const bool update = l + 1 < LAYERS;
     if (update) {
-      rc = launch_mlp<128, 1>(n, StageDense{dY_node(l), W, W}, EpiUpdateGrad{dh, da, g->offsets},
-                              P + K_W2 + l * 2 * W * W, status, st, "mpnn update dx");
+      rc = launch_mlp<64, 1>(n, StageDense{dY_node(l), W, W}, EpiUpdateGrad{dh, da, g->offsets},
+                             P + K_W2 + l * 2 * W * W, status, st, "mpnn update dx", 2);
       if (rc) return rc;
       WgradJob& q = job(kPair, n, h, a, nullptr, W, dY_node(l), W);
       q.dst[0][0] = {gl + O_W2, W};

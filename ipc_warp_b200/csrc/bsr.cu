@@ -42,24 +42,24 @@ IPCB_D bool valid_triplet(int t, const int* __restrict__ rows, const int* __rest
   return nz;
 }
 
+// place[t]: the triplet's place among its row's, -1 for a dropped one (the
+// blocks are read once, by this kernel; reading them again and a second round
+// of atomics took the scatter 25 us for 1.75M blocks, 8 without)
 template <class S>
 __global__ void k_row_count(int n, const int* __restrict__ rows, const int* __restrict__ cols,
-                            const S* __restrict__ vals, int nrow, int ncol, int* __restrict__ row_cnt) {
+                            const S* __restrict__ vals, int nrow, int ncol, int* __restrict__ row_cnt,
+                            int* __restrict__ place) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  if (valid_triplet(t, rows, cols, vals, nrow, ncol)) atomicAdd(row_cnt + rows[t], 1);
+  place[t] = valid_triplet(t, rows, cols, vals, nrow, ncol) ? atomicAdd(row_cnt + rows[t], 1) : -1;
 }
 
-template <class S>
-__global__ void k_row_scatter(int n, const int* __restrict__ rows, const int* __restrict__ cols,
-                              const S* __restrict__ vals, int nrow, int ncol, const int* __restrict__ row_start,
-                              int* __restrict__ cursor, int* __restrict__ bucket) {
+__global__ void k_row_scatter(int n, const int* __restrict__ rows, const int* __restrict__ place,
+                              const int* __restrict__ row_start, int* __restrict__ bucket) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
-  if (!valid_triplet(t, rows, cols, vals, nrow, ncol)) return;
-  int r = rows[t];
-  int pos = row_start[r] + atomicAdd(cursor + r, 1);
-  bucket[pos] = t;
+  const int k = place[t];
+  if (k >= 0) bucket[row_start[rows[t]] + k] = t;
 }
 
 // (col, id) as one 64-bit ordering key
@@ -67,63 +67,97 @@ IPCB_D unsigned long long ckey(const int* __restrict__ cols, int t) {
   return ((unsigned long long)(unsigned)cols[t] << 32) | (unsigned)t;
 }
 
-constexpr int kRowCap = 1024;      // entries a warp sorts in shared memory
-constexpr int kSortWarps = 4;      // warps (rows) per block in k_row_sort
+constexpr int kRowCap = 1024;  // entries a warp sorts in its registers
+constexpr int kSortWarps = 4;  // warps (rows) per block in k_row_sort
 
-// Warp per row: sort the row's bucket by (col, id), keys distinct, then count
-// distinct columns.  Rows up to kRowCap entries use a bitonic network in
-// shared memory; longer rows are appended to long_rows for k_row_sort_long.
-__global__ void __launch_bounds__(kSortWarps * 32) k_row_sort(int nrow, const int* __restrict__ cols,
-                                                              const int* __restrict__ row_start,
-                                                              int* __restrict__ bucket, int* __restrict__ tmp,
-                                                              int* __restrict__ row_nnz, int* __restrict__ long_rows,
-                                                              int* __restrict__ n_long) {
-  __shared__ unsigned long long sk[kSortWarps][kRowCap];
-  const int wib = threadIdx.x >> 5;
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (warp >= nrow) return;
-  int b = row_start[warp], e = row_start[warp + 1], L = e - b;
-  if (L <= kRowCap) {
-    int P = 1;
-    while (P < L) P <<= 1;
-    unsigned long long* k = sk[wib];
-    for (int i = lane; i < P; i += 32) k[i] = i < L ? ckey(cols, bucket[b + i]) : ~0ULL;
-    __syncwarp();
-    for (int sz = 2; sz <= P; sz <<= 1) {
-      for (int st = sz >> 1; st > 0; st >>= 1) {
-        for (int i = lane; i < P; i += 32) {
-          int l = i ^ st;
-          if (l > i) {
-            unsigned long long a = k[i], c = k[l];
-            bool up = (i & sz) == 0;
-            if ((a > c) == up) {
-              k[i] = c;
-              k[l] = a;
-            }
-          }
-        }
-        __syncwarp();
+// compare-exchange of entries 32 D apart (the registers' index stays static)
+template <int K, int D>
+IPCB_D void cas_registers(unsigned long long (&k)[K], int sz) {
+  if constexpr (D < K) {
+#pragma unroll
+    for (int r = 0; r < K; ++r) {
+      if (r & D) continue;
+      const unsigned long long a = k[r], c = k[r | D];
+      const bool swap = (a > c) == (((32 * r) & sz) == 0);
+      k[r] = swap ? c : a;
+      k[r | D] = swap ? a : c;
+    }
+  }
+}
+
+// Sorts one row: entry i of the network is register i / 32 of lane i % 32, so
+// distances below 32 are shuffles and the others register pairs.  Then the
+// ids go back in order; returns the number of distinct columns.
+template <int K>
+IPCB_D int sort_row(int L, const int* __restrict__ cols, int* __restrict__ bucket, int lane) {
+  unsigned long long k[K];
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    const int i = 32 * r + lane;
+    k[r] = i < L ? ckey(cols, bucket[i]) : ~0ULL;
+  }
+  for (int sz = 2; sz <= 32 * K; sz <<= 1) {
+    if (sz >= 1024) cas_registers<K, 16>(k, sz);
+    if (sz >= 512) cas_registers<K, 8>(k, sz);
+    if (sz >= 256) cas_registers<K, 4>(k, sz);
+    if (sz >= 128) cas_registers<K, 2>(k, sz);
+    if (sz >= 64) cas_registers<K, 1>(k, sz);
+    for (int st = sz >> 1 < 16 ? sz >> 1 : 16; st > 0; st >>= 1) {
+#pragma unroll
+      for (int r = 0; r < K; ++r) {
+        const unsigned long long o = __shfl_xor_sync(0xffffffffu, k[r], st);
+        const bool up = ((32 * r + lane) & sz) == 0, low = (lane & st) == 0;
+        k[r] = ((o < k[r]) == (up == low)) ? o : k[r];
       }
     }
-    for (int i = lane; i < L; i += 32) tmp[b + i] = (int)(unsigned)(k[i] & 0xffffffffULL);
-  } else {  // a long row: sorted and counted by k_row_sort_long
-    if (lane == 0) {
-      long_rows[atomicAdd(n_long, 1)] = warp;
-      row_nnz[warp] = 0;
-    }
-    return;
   }
-  __syncwarp();
-  int distinct = 0;
-  for (int i = lane; i < L; i += 32) {
-    int t = tmp[b + i];
-    bucket[b + i] = t;
-    distinct += (i == 0 || cols[tmp[b + i - 1]] != cols[t]) ? 1 : 0;
-  }
+  int n = 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) distinct += __shfl_xor_sync(0xffffffffu, distinct, o);
-  if (lane == 0) row_nnz[warp] = distinct;
+  for (int r = 0; r < K; ++r) {
+    const int i = 32 * r + lane;
+    unsigned long long before = __shfl_up_sync(0xffffffffu, k[r], 1);
+    const unsigned long long last = r ? __shfl_sync(0xffffffffu, k[r ? r - 1 : 0], 31) : 0;
+    if (lane == 0) before = last;
+    const bool head = i < L && (i == 0 || (before >> 32) != (k[r] >> 32));
+    if (i < L) bucket[i] = (int)(unsigned)(k[r] & 0xffffffffULL);
+    n += __popc(__ballot_sync(0xffffffffu, head));
+  }
+  return n;
+}
+
+// Warp per row: sort the row's bucket by (col, id), keys distinct, then count
+// the distinct columns.  The network runs in registers of the smallest power
+// of two that holds the row: through shared memory a stage was a chain of
+// loads, compares and stores per 32 entries (277 us for the 8.8k rows and 1.75M
+// blocks of 16 balls on stacked cubes, 111 in registers).  Rows above
+// kRowCap are appended to long_rows for k_row_sort_long.
+__global__ void __launch_bounds__(kSortWarps * 32) k_row_sort(int nrow, const int* __restrict__ cols,
+                                                              const int* __restrict__ row_start,
+                                                              int* __restrict__ bucket, int* __restrict__ row_nnz,
+                                                              int* __restrict__ long_rows, int* __restrict__ n_long) {
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (row >= nrow) return;
+  const int b = row_start[row], L = row_start[row + 1] - b;
+  bucket += b;
+  int n = 0;
+  if (L == 0) {
+  } else if (L <= 32) {
+    n = sort_row<1>(L, cols, bucket, lane);
+  } else if (L <= 64) {
+    n = sort_row<2>(L, cols, bucket, lane);
+  } else if (L <= 128) {
+    n = sort_row<4>(L, cols, bucket, lane);
+  } else if (L <= 256) {
+    n = sort_row<8>(L, cols, bucket, lane);
+  } else if (L <= 512) {
+    n = sort_row<16>(L, cols, bucket, lane);
+  } else if (L <= kRowCap) {
+    n = sort_row<32>(L, cols, bucket, lane);
+  } else if (lane == 0) {  // sorted and counted by k_row_sort_long
+    long_rows[atomicAdd(n_long, 1)] = row;
+  }
+  if (lane == 0) row_nnz[row] = n;
 }
 
 // Warp per row over the sorted bucket, 32 entries at a time: a segmented
@@ -409,22 +443,20 @@ int assemble(int nrow, int ncol, int n, const int* rows, const int* cols, const 
   size_t R = (size_t)nrow + 1, N = (size_t)n;
   char* p = (char*)ws;
   int* row_start = (int*)p; p += al(R * 4);
-  int* cursor = (int*)p; p += al(R * 4);
   int* total = (int*)p; p += 256;
   int* bucket = (int*)p; p += al(N * 4);
-  int* tmp = (int*)p; p += al(N * 4);
+  int* place = (int*)p; p += al(N * 4);
   int* long_rows = (int*)p; p += al(R * 4);
   int* n_long = (int*)p; p += 256;
   unsigned long long* lkeys = (unsigned long long*)p; p += al(2 * N * 8);
   void* scratch = p;
   cudaMemsetAsync(n_long, 0, sizeof(int), st);
   cudaMemsetAsync(row_start, 0, R * sizeof(int), st);
-  cudaMemsetAsync(cursor, 0, R * sizeof(int), st);
   int g = div_up(n, 256);
-  k_row_count<S><<<g, 256, 0, st>>>(n, rows, cols, vals, nrow, ncol, row_start);
+  k_row_count<S><<<g, 256, 0, st>>>(n, rows, cols, vals, nrow, ncol, row_start, place);
   scan::exclusive<int>(row_start, (int)R, scratch, total, st);  // row_start[nrow] = valid count
-  k_row_scatter<S><<<g, 256, 0, st>>>(n, rows, cols, vals, nrow, ncol, row_start, cursor, bucket);
-  k_row_sort<<<div_up(nrow, kSortWarps), kSortWarps * 32, 0, st>>>(nrow, cols, row_start, bucket, tmp, offsets,
+  k_row_scatter<<<g, 256, 0, st>>>(n, rows, place, row_start, bucket);
+  k_row_sort<<<div_up(nrow, kSortWarps), kSortWarps * 32, 0, st>>>(nrow, cols, row_start, bucket, offsets,
                                                                      long_rows, n_long);
   const int g_long = nrow < kLongGrid ? nrow : kLongGrid;
   k_row_sort_long<<<g_long, kLongThreads, 0, st>>>(long_rows, n_long, cols, row_start, bucket, lkeys, offsets);
@@ -447,7 +479,7 @@ extern "C" {
 size_t ipcb_bsr_workspace(int n_trip, int nrow, int ncol) {
   (void)ncol;
   size_t R = (size_t)(nrow > 0 ? nrow : 0) + 1, N = (size_t)(n_trip > 0 ? n_trip : 1);
-  return 3 * al(R * 4) + 512 + 2 * al(N * 4) + al(2 * N * 8) + scan::scratch_bytes((int)R);
+  return 2 * al(R * 4) + 512 + 2 * al(N * 4) + al(2 * N * 8) + scan::scratch_bytes((int)R);
 }
 
 int ipcb_bsr_from_triplets(int nrow, int ncol, int n_trip, const int* rows, const int* cols, const void* vals,

@@ -184,6 +184,10 @@ int ipcb_iteration_begin(const ipcb_soup* soup, const void* dx, void* x1, void* 
 int ipcb_iteration_results(int fp64, const int* ee_cnt, const int* pt_cnt, const int* bsr_status, const int* status,
                            const double* energy, const void* toi, int* counts_out, double* energy_out, void* toi_out,
                            ipcb_stream s);
+/* Up to 8 32-bit words in one launch: *dst[i] = *src[i], or 0 where src[i] is
+ * null.  dst and src are host arrays of addresses the device can reach (device
+ * memory or pinned host memory). */
+int ipcb_words(int n, void* const* dst, const void* const* src, ipcb_stream s);
 
 /* ---- narrow phase (dynamic_contacts.py:152-246 contact_hessian_ee/pt, 375-398 energy) ----
  * kind 0 = EE list, 1 = PT list.  n >= 0: number of records; n < 0: read

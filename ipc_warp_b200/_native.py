@@ -224,6 +224,7 @@ SIGNATURES = {
     "ipcb_union_values": (c_int, [c_int, P, c_int, P, P, P, P, c_double, P, P]),
     "ipcb_newton_rhs": (c_int, [c_int, c_int, P, P, P, P, P, c_double, P, P, P, c_double, P, P]),
     "ipcb_iteration_begin": (c_int, [SP, P, P, P, P, P, P, P, P, P, P]),
+    "ipcb_words": (c_int, [c_int, ctypes.POINTER(P), ctypes.POINTER(P), P]),
     "ipcb_iteration_results": (c_int, [c_int, P, P, P, P, P, P, P, P, P, P]),
     "ipcb_contact_bsr_rows": (c_int, [CP, c_int, CP, c_int, c_int, P, c_size_t, P]),
     "ipcb_contact_bsr_blocks": (c_int, [CP, c_int, CP, c_int, c_int, P, P, c_int, P, P, P, P, P, P, c_size_t, P]),
@@ -286,6 +287,14 @@ def call(name: str, *args):
         msg = lib().ipcb_last_error()
         raise NativeError(f"{name} returned {rc}: {msg.decode() if msg else ''}")
     return rc
+
+
+def words(*moves):
+    """Moves (dst, src) of 32-bit words in one launch, addresses of device or
+    pinned host memory; src None writes 0."""
+    n = len(moves)
+    arr = P * n
+    call("ipcb_words", n, arr(*[d for d, _ in moves]), arr(*[v for _, v in moves]), stream_handle())
 
 
 def size(name: str, *args) -> int:

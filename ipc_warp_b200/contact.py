@@ -168,7 +168,8 @@ class ContactSolverBase:
         # CCD candidate staging (a query that overflows it is redone inline)
         cap = max(1 << 20, 4 * max(n_edges, n_nodes))
         self._toi_ws = torch.empty(N.size("ipcb_toi_workspace", cap), dtype=torch.uint8, device=dev)
-        self._counts_host = torch.zeros(3, dtype=torch.int32).pin_memory() if dev.type == "cuda" else None
+        # both counts and the status; then the TOI (two words) and the status
+        self._counts_host = torch.zeros(6, dtype=torch.int32).pin_memory() if dev.type == "cuda" else None
 
     # ------------------------------------------------------------- branches
     @contextmanager
@@ -276,12 +277,10 @@ class ContactSolverBase:
         """One host read of both list counts and the query status word (kept
         in ``query_status``)."""
         h = self._counts_host
-        h[0:1].copy_(self.contacts_new.cnt, non_blocking=True)
-        if self.has_triangles:
-            h[1:2].copy_(self.contacts_pt.cnt, non_blocking=True)
-        else:
-            h[1] = 0
-        h[2:3].copy_(self._status, non_blocking=True)
+        to = N.ptr(h)
+        N.words((to, N.ptr(self.contacts_new.cnt)),
+                (to + 4, N.ptr(self.contacts_pt.cnt) if self.has_triangles else None),
+                (to + 8, N.ptr(self._status)))
         torch.cuda.current_stream().synchronize()
         self.query_status = int(h[2])
         return int(h[0]), int(h[1])
@@ -331,8 +330,12 @@ class ContactSolverBase:
         set IPCB_STATUS_STACK or IPCB_STATUS_ROOT_ITERS: such a query may have
         missed an earlier impact, so its TOI is no bound.  Refusals are
         counted in ``ccd_refusals``."""
-        toi, status = torch.cat([self.ccd_toi.double(), self._status.double()]).tolist()
-        return self._bound_from(toi, int(status))
+        h = self._counts_host
+        toi, to, src = h[4:6] if self.ccd_toi.dtype == torch.float64 else h[4:5], N.ptr(h), N.ptr(self.ccd_toi)
+        moves = [(to + 16 + 4 * k, src + 4 * k) for k in range(toi.numel())]
+        N.words((to + 12, N.ptr(self._status)), *moves)
+        torch.cuda.current_stream().synchronize()
+        return self._bound_from(float(toi.view(self.ccd_toi.dtype)), int(h[3]))
 
     def _bound_from(self, toi: float, status: int) -> float:
         self.query_status = status

@@ -91,6 +91,8 @@ class FixedBodyContactSolver(ContactSolverBase):
         self.fixed_body_pairs = torch.zeros((cap, 2), **i32)
         self.fixed_body_pair_count = torch.zeros(1, **i32)
         self._fixed_status = torch.zeros(1, **i32)
+        self._pairs_host = torch.zeros(2, dtype=torch.int32).pin_memory()
+        self._toi_one = torch.ones(1, dtype=self.ccd_toi.dtype, device=dev)
         # the reference's mode switches; one implementation serves all modes
         self.fixed_pair_cull_mode = "kernel"
         self.fixed_query_mode = "scalar"
@@ -109,17 +111,13 @@ class FixedBodyContactSolver(ContactSolverBase):
         self._ccd_ws_fixed = torch.empty(N.size("ipcb_toi_workspace", max(1 << 20, 4 * soup.n_edges)),
                                          dtype=torch.uint8, device=dev)
 
-    def _read(self, *tensors):
-        out = torch.cat([t.reshape(-1).to(torch.int64) for t in tensors]).cpu()
-        return [int(v) for v in out]
-
     def _pairs(self, swept_dq=None):
         """(n_pairs, singular) after the (swept) body cull."""
         q = self.affine_q
         fp64 = int(q.dtype == torch.float64)
+        count, status, to = N.ptr(self.fixed_body_pair_count), N.ptr(self._fixed_status), N.ptr(self._pairs_host)
         while True:
-            self.fixed_body_pair_count.zero_()
-            self._fixed_status.zero_()
+            N.words((count, None), (status, None))
             cap = self.fixed_body_pairs.shape[0]
             if swept_dq is None:
                 N.call("ipcb_body_pairs", ctypes.byref(self._bodies), fp64, N.ptr(q),
@@ -129,7 +127,9 @@ class FixedBodyContactSolver(ContactSolverBase):
                 N.call("ipcb_body_pairs_swept", ctypes.byref(self._bodies), fp64, N.ptr(q), N.ptr(swept_dq), 1.0e-7,
                        N.ptr(self.fixed_body_pairs), cap, N.ptr(self.fixed_body_pair_count),
                        N.ptr(self._fixed_status), N.stream_handle())
-            n, st = self._read(self.fixed_body_pair_count, self._fixed_status)
+            N.words((to, count), (to + 4, status))
+            torch.cuda.current_stream().synchronize()
+            n, st = self._pairs_host.tolist()
             if n <= cap:
                 return n, bool(st & STATUS_SINGULAR)
             self.fixed_body_pairs = torch.zeros((1 << (n - 1).bit_length(), 2), dtype=torch.int32,
@@ -153,9 +153,8 @@ class FixedBodyContactSolver(ContactSolverBase):
         s = N.stream_handle()
         th = float(contact_mod._thickness)
         while True:
-            self.contacts_new.cnt.zero_()
-            self.contacts_pt.cnt.zero_()
-            self._status.zero_()
+            N.words((N.ptr(self.contacts_new.cnt), None), (N.ptr(self.contacts_pt.cnt), None),
+                    (N.ptr(self._status), None))
             if n_pairs:
                 N.call("ipcb_fixed_dcd_ee", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self._bodies),
                        N.ptr(self.fixed_body_pairs), n_pairs, th, ctypes.byref(self.contacts_new.c_struct()),
@@ -188,8 +187,8 @@ class FixedBodyContactSolver(ContactSolverBase):
         n_pairs, singular = self._pairs(abd.dx)
         if singular:
             return ContactSolverBase.collision_free_step(self, dx)
-        self.ccd_toi.fill_(1.0)
-        self._status.zero_()
+        toi, one = N.ptr(self.ccd_toi), N.ptr(self._toi_one)
+        N.words((N.ptr(self._status), None), *((toi + k, one + k) for k in range(0, self.ccd_toi.element_size(), 4)))
         if n_pairs:
             ws = self._ccd_ws_fixed
             N.call("ipcb_fixed_edge_edge_toi", ctypes.byref(soup), N.ptr(self.ccd_x1), ctypes.byref(self._bodies),

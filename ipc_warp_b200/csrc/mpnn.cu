@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep,
   // accumulator stride: at least the 32 columns one tcgen05.ld reads
   constexpr int NA = N < 32 ? 32 : N;
   constexpr uint32_t kCols = umma::tmem_cols(S * NA);
-  static_assert(C < 3 || C % 2 == 0, "chunks are staged in pairs");
+  static_assert(C < 3 || C % 2 == 0 || C % 3 == 0, "chunks are staged two or three at a time");
   static_assert(S * NA <= 512, "the accumulators must fit the 512 TMEM columns");
   constexpr int K = 64 * C;
   constexpr int kStage = C * 128 * 128;
@@ -472,8 +472,8 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp(int rows, Stage st, Epi ep,
       // of a row, so a warp reads contiguous row spans
       const int base = (blockIdx.x + k * gridDim.x) * 128 + 32 * warp;
       uint8_t* a = sA + s * kStage;
-      // the warp's loads of up to two chunks first, then their shared stores
-      constexpr int G = C < 2 ? C : 2;
+      // the warp's loads of up to three chunks first, then their shared stores
+      constexpr int G = C < 2 ? C : C % 3 ? 2 : 3;
 #pragma unroll
       for (int c0 = 0; c0 < C; c0 += G) {
         uint4 buf[G][8];
@@ -579,8 +579,9 @@ int launch_mlp(int rows, const Stage& st, const Epi& ep, const bf16* Bw, int* st
 // reads them MN-major, so a tile is staged by coalesced 16-byte loads and
 // 16-byte shared stores (the K-major form stored 2-byte elements transposed:
 // 77 us for an edge job of 91k rows and its 192 gathered features).  The
-// next tile's loads are in flight while the tensor core works on this one;
-// 80 KB and 128 TMEM columns a CTA leave two CTAs an SM.
+// next tile's loads are in flight while the tensor core works on this one, and
+// 65 KB and 128 TMEM columns a CTA leave three CTAs an SM: a CTA waits for its
+// loads most of the time (all jobs of a pass over 71,500 edges: 61 us with two, 44 with three).
 //
 // A's 128 columns are two staged chunks of 64, one of which can be the chunk
 // "ones" (column 0 ones), whose row of the product is the bias gradient:
@@ -611,17 +612,17 @@ struct WgradJobs {
 
 constexpr int kWgradThreads = 256;
 constexpr int kChunk = 128 * 128;  // bytes of a staged chunk
-constexpr size_t kWgradSmem = 1024 + 5 * kChunk;
+constexpr size_t kWgradSmem = 1024 + 4 * kChunk;
 
-__global__ void __launch_bounds__(kWgradThreads, 2) k_wgrad(const __grid_constant__ WgradJobs J,
+__global__ void __launch_bounds__(kWgradThreads, 3) k_wgrad(const __grid_constant__ WgradJobs J,
                                                             int* __restrict__ status) {
   extern __shared__ uint8_t dsmem[];
   __shared__ uint64_t mbar;
   __shared__ uint32_t tslot;
   uint8_t* sx0 = align1024(dsmem);
   uint8_t* sone = sx0 + kChunk;
-  uint8_t* sx1 = sone + kChunk;
-  uint8_t* sy = sx1 + kChunk;  // two chunks
+  uint8_t* sy = sone + kChunk;
+  uint8_t* sz = sy + kChunk;  // x1, or the second half of the split sums
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   int j = 0;
   while (j + 1 < J.count && (int)blockIdx.x >= J.job[j + 1].first) ++j;
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(kWgradThreads, 2) k_wgrad(const __grid_constan
       const uint32_t o = umma::sw128_group((tid >> 3) + 32 * it, 0, g, 128);
       *reinterpret_cast<uint4*>(sx0 + o) = bx[it];
       *reinterpret_cast<uint4*>(sy + o) = by[it];
-      if (mode != kBatch) *reinterpret_cast<uint4*>((mode == kPair ? sx1 : sy + kChunk) + o) = bz[it];
+      if (mode != kBatch) *reinterpret_cast<uint4*>(sz + o) = bz[it];
     }
     umma::fence_async_smem();
     __syncthreads();
@@ -687,8 +688,8 @@ __global__ void __launch_bounds__(kWgradThreads, 2) k_wgrad(const __grid_constan
       if (mode == kSums) {
         umma::issue_mn<128>(tmem, x0, kChunk, y, kChunk, t > t0);
       } else if (mode == kPair) {
-        umma::issue_mn<64>(tmem, x0, 2 * kChunk, y, kChunk, t > t0);
-        umma::issue_mn<64>(tmem + W, one, kChunk, y, kChunk, t > t0);
+        umma::issue_mn<64>(tmem, x0, 3 * kChunk, y, kChunk, t > t0);
+        umma::issue_mn<64>(tmem + W, one, 2 * kChunk, y, kChunk, t > t0);
       } else {
         umma::issue_mn<64>(tmem, x0, kChunk, y, kChunk, t > t0);
       }
@@ -737,14 +738,18 @@ int launch_wgrad(WgradJobs& J, int* status, cudaStream_t s) {
   auto tiles = [](const WgradJob& q) { return (long long)((q.rows + 127) / 128) * (q.mode == kSums ? kPieces : 1); };
   long long all = 0;
   for (int j = 0; j < J.count; ++j) all += tiles(J.job[j]);
-  // one wave of two CTAs an SM: each reduces its run of tiles in TMEM before its atomics
-  const int cap = 2 * sm_count();
-  J.run = (int)((all + cap - 1) / cap);
-  int blocks = 0;
-  for (int j = 0; j < J.count; ++j) {
-    J.job[j].first = blocks;
-    blocks += (int)((tiles(J.job[j]) + J.run - 1) / J.run);
-  }
+  // one wave of three CTAs an SM: each reduces its run of tiles in TMEM before its atomics
+  const int cap = 3 * sm_count();
+  J.run = (int)((all + cap - 1) / cap) - 1;
+  int blocks;
+  do {  // every job rounds up: the smallest run whose CTAs fit the wave
+    ++J.run;
+    blocks = 0;
+    for (int j = 0; j < J.count; ++j) {
+      J.job[j].first = blocks;
+      blocks += (int)((tiles(J.job[j]) + J.run - 1) / J.run);
+    }
+  } while (blocks > cap && J.run < all);
   k_wgrad<<<blocks, kWgradThreads, kWgradSmem, s>>>(J, status);
   return ipcb::check_launch("mpnn wgrad");
 }
@@ -903,15 +908,19 @@ __global__ void k_fsai_T(int n_lower, const int* __restrict__ lower, const int* 
 
 // Per row: M_i = sum_j T_ij H_ij^T, Cholesky M_i = C C^T, G^_ij = C^-1 H_ij;
 // acc[0] += log det M_i, minv_i = M_i^-1.  A row whose M_i is not positive
-// definite keeps G^ = H and raises IPCB_STATUS_PATTERN.
-__global__ void k_fsai_rows(int n, const int* __restrict__ off, const int* __restrict__ diag,
-                            const float* __restrict__ H, const float* __restrict__ T, float* __restrict__ minv,
-                            float* __restrict__ G, double* __restrict__ acc, int* __restrict__ status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// definite keeps G^ = H and raises IPCB_STATUS_PATTERN.  Eight lanes a row:
+// the blocks of a row lie together, and a thread a row read them one by one
+// (6,500 rows: 21 us, now 7).
+__global__ void __launch_bounds__(256) k_fsai_rows(int n, const int* __restrict__ off, const int* __restrict__ diag,
+                                                   const float* __restrict__ H, const float* __restrict__ T,
+                                                   float* __restrict__ minv, float* __restrict__ G,
+                                                   double* __restrict__ acc, int* __restrict__ status) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(t >> 3), sub = (int)(t & 7);
   double part = 0.0;
+  double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   if (i < n) {
-    double M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int e = off[i]; e <= diag[i]; ++e) {
+    for (int e = off[i] + sub; e <= diag[i]; e += 8) {
       const float* t = T + (size_t)e * 9;
       const float* h = H + (size_t)e * 9;
 #pragma unroll
@@ -921,6 +930,12 @@ __global__ void k_fsai_rows(int n, const int* __restrict__ off, const int* __res
           M[3 * r + c] += (double)t[3 * r] * h[3 * c] + (double)t[3 * r + 1] * h[3 * c + 1] +
                           (double)t[3 * r + 2] * h[3 * c + 2];
     }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < 9; ++q) M[q] += __shfl_xor_sync(0xffffffffu, M[q], o);
+  if (i < n) {
     // symmetrise, Cholesky
     const double m00 = M[0], m10 = 0.5 * (M[3] + M[1]), m11 = M[4], m20 = 0.5 * (M[6] + M[2]),
                  m21 = 0.5 * (M[7] + M[5]), m22 = M[8];
@@ -939,17 +954,19 @@ __global__ void k_fsai_rows(int n, const int* __restrict__ off, const int* __res
     L[4] = 1.0 / c11; L[3] = -c10 * L[0] / c11; L[5] = 0.0;
     L[8] = 1.0 / c22; L[6] = -(c20 * L[0] + c21 * L[3]) / c22; L[7] = -c21 * L[4] / c22;
     if (!ok) {
-      atomicOr(status, IPCB_STATUS_PATTERN);
+      if (sub == 0) atomicOr(status, IPCB_STATUS_PATTERN);
       for (int q = 0; q < 9; ++q) L[q] = (q % 4) == 0 ? 1.0 : 0.0;
     }
     // M^-1 = L^T L
+    if (sub == 0) {
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+      for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
-        minv[(size_t)i * 9 + 3 * r + c] = (float)(L[r] * L[c] + L[3 + r] * L[3 + c] + L[6 + r] * L[6 + c]);
-    part = ok ? 2.0 * log(c00 * c11 * c22) : 0.0;
-    for (int e = off[i]; e <= diag[i]; ++e) {
+        for (int c = 0; c < 3; ++c)
+          minv[(size_t)i * 9 + 3 * r + c] = (float)(L[r] * L[c] + L[3 + r] * L[3 + c] + L[6 + r] * L[6 + c]);
+      part = ok ? 2.0 * log(c00 * c11 * c22) : 0.0;
+    }
+    for (int e = off[i] + sub; e <= diag[i]; e += 8) {
       const float* h = H + (size_t)e * 9;
       float* g = G + (size_t)e * 9;
 #pragma unroll
@@ -959,8 +976,14 @@ __global__ void k_fsai_rows(int n, const int* __restrict__ off, const int* __res
           g[3 * r + c] = (float)(L[3 * r] * h[c] + L[3 * r + 1] * h[3 + c] + L[3 * r + 2] * h[6 + c]);
     }
   }
+  __shared__ double parts[8];  // one atomic for the block's 32 rows
   part = warp_sum(part);
-  if ((threadIdx.x & 31) == 0 && part != 0.0) atomicAdd(acc, part);
+  if ((threadIdx.x & 31) == 0) parts[threadIdx.x >> 5] = part;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) part += parts[w];
+    if (part != 0.0) atomicAdd(acc, part);
+  }
 }
 
 // gradient of weight * (1/N) sum_i log det M_i w.r.t. the head outputs:
@@ -1292,7 +1315,7 @@ int ipcb_fsai_normalize(const ipcb_graph* g, const float* ahat, const float* H, 
   cudaStream_t st = (cudaStream_t)s;
   k_fsai_T<<<grid_for(g->n_lower), 256, 0, st>>>(g->n_lower, g->lower, g->rows, g->columns, g->offsets, g->diag, ahat,
                                                  H, T);
-  k_fsai_rows<<<grid_for(g->n), 256, 0, st>>>(g->n, g->offsets, g->diag, H, T, minv, G, acc, status);
+  k_fsai_rows<<<grid_for((long long)g->n * 8), 256, 0, st>>>(g->n, g->offsets, g->diag, H, T, minv, G, acc, status);
   return ipcb::check_launch("ipcb_fsai_normalize");
 }
 

@@ -246,6 +246,28 @@ def no_collection():
             gc.enable()
 
 
+@contextlib.contextmanager
+def capture(graph, owner):
+    """Captures the launches inside into ``graph`` on a side stream that
+    ``owner`` keeps.  torch.cuda.graph() also waits for the whole device and
+    returns the allocator's cached memory to the driver, which a solver's
+    first call then allocates again (the first solve on 102,800 rows: 43 ms,
+    5.5 without)."""
+    import torch
+
+    side = owner.__dict__.get("_capture_stream")
+    if side is None:
+        side = owner.__dict__["_capture_stream"] = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with no_collection(), torch.cuda.stream(side):
+        graph.capture_begin()
+        try:
+            yield
+        finally:
+            graph.capture_end()
+    torch.cuda.current_stream().wait_stream(side)
+
+
 class NativeError(RuntimeError):
     pass
 

@@ -147,8 +147,10 @@ class JacobiPrecond:
 
 class DevicePcg:
     """PCG with device-resident scalars (ipcb_pcg_*): ``batch`` iterations
-    per host check, replayed from a CUDA graph captured once per set of
-    buffers; one synchronisation per batch.  A solve that has not ended in its
+    per host check, replayed from a CUDA graph once a set of buffers comes
+    back (the first solve on them launches plainly: capturing costs about a
+    millisecond a graph, the launches less than the iterations take); one
+    synchronisation per batch.  A solve that has not ended in its
     first batch goes on with a copy of the matrix laid out for the product
     (ipcb_pcg_slice)."""
 
@@ -156,10 +158,7 @@ class DevicePcg:
         self.batch = batch
         self.use_graph = use_graph
         self._bufs = None
-        self._graph = None
-        self._key = None
-        self._slice_graph = None
-        self._slice_key = None
+        self._graphs = {}  # C call -> (buffers, graph or None while they were seen once)
         self._slice_ws = None
         self._slice_nnz = 0
 
@@ -202,27 +201,21 @@ class DevicePcg:
             P.x0 = N.ptr(B["x0"])
         self._P = P
         N.call("ipcb_pcg_start", ctypes.byref(P), float(tol), int(maxiter), N.stream_handle())
-        key = self._fields(P)
-        if self.use_graph and key != self._key:
-            self._graph = self._capture("ipcb_pcg_iterate", P)
-            self._key = key
-        self._batch(self._graph, "ipcb_pcg_iterate", P)
+        graph = self._graph_of("ipcb_pcg_iterate", P)
+        self._batch(graph, "ipcb_pcg_iterate", P)
         B["nnz"].copy_(A.offsets[n:n + 1], non_blocking=True)
         st = self._read(B)
         nnz = int(B["nnz"])
         if not st.done and nnz + nnz // 4 + 8 * n + (1 << 14) > 0x7fffffff:  # past the copy's 32-bit slots
             while not st.done:
-                self._batch(self._graph, "ipcb_pcg_iterate", P)
+                self._batch(graph, "ipcb_pcg_iterate", P)
                 st = self._read(B)
         if not st.done:
             self._slice_room(P, nnz, A.device)
             N.call("ipcb_pcg_slice", ctypes.byref(P), N.stream_handle())
-            key = self._fields(P)
-            if self.use_graph and key != self._slice_key:
-                self._slice_graph = self._capture("ipcb_pcg_iterate_slices", P, 2)
-                self._slice_key = key
+            graph = self._graph_of("ipcb_pcg_iterate_slices", P, 2)
             while not st.done:  # the launches past the end cost less than the reads saved
-                self._batch(self._slice_graph, "ipcb_pcg_iterate_slices", P, 2)
+                self._batch(graph, "ipcb_pcg_iterate_slices", P, 2)
                 st = self._read(B)
         if x0 is not None and not st.bb > 0:
             B["x"].zero_()  # b = 0: the solution is 0, whatever the guess
@@ -233,14 +226,24 @@ class DevicePcg:
     def _fields(P):
         return tuple(getattr(P, f) for f, _ in N.Pcg._fields_ if f != "x0")  # the loop never reads x0
 
-    def _capture(self, call, P, times: int = 1):
-        graph = torch.cuda.CUDAGraph()
-        with N.no_collection(), torch.cuda.graph(graph):
-            N.call(call, ctypes.byref(P), times * self.batch, N.stream_handle())
+    def _graph_of(self, call, P, times: int = 1):
+        """The batch's graph for P's buffers: None for buffers not seen in the
+        solve before."""
+        if not self.use_graph:
+            return None
+        key = self._fields(P)
+        seen, graph = self._graphs.get(call, (None, None))
+        if seen != key:
+            graph = None
+        elif graph is None:
+            graph = torch.cuda.CUDAGraph()
+            with N.capture(graph, self):
+                N.call(call, ctypes.byref(P), times * self.batch, N.stream_handle())
+        self._graphs[call] = (key, graph)
         return graph
 
     def _batch(self, graph, call, P, times: int = 1):
-        if self.use_graph:
+        if graph is not None:
             graph.replay()
         else:
             N.call(call, ctypes.byref(P), times * self.batch, N.stream_handle())
@@ -538,8 +541,7 @@ class FEMContactSolver(ContactBarrierMixin):
             return A
         cap = self._graph_buffers()
         graph = torch.cuda.CUDAGraph()
-        torch.cuda.synchronize()
-        with N.no_collection(), torch.cuda.graph(graph):
+        with N.capture(graph, self):
             self._enqueue_A(cfg, cap)
         self._A_graph = (self._A_graph_key(), graph, cfg)
         # the capture recorded the launches without running them: run them now
@@ -939,7 +941,7 @@ class FEMContactSolver(ContactBarrierMixin):
             self._ls_prelude_launches(mode)
             return
         graph = torch.cuda.CUDAGraph()
-        with N.no_collection(), torch.cuda.graph(graph):
+        with N.capture(graph, self):
             self._ls_prelude_launches(mode)
         graphs[key] = graph
         graph.replay()

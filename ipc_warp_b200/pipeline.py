@@ -158,8 +158,7 @@ class ContactPipeline(ContactBarrierMixin):
         if key[-1]:  # periodic rebuilds alternate with refits: not one fixed sequence
             return
         g = torch.cuda.CUDAGraph()
-        torch.cuda.synchronize()
-        with N.no_collection(), torch.cuda.graph(g):
+        with N.capture(g, self):
             self._enqueue()
         self._graph = (key, g)
 

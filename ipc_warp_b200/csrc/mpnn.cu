@@ -36,7 +36,6 @@ using bf16 = __nv_bfloat16;
 constexpr int W = IPCB_MPNN_WIDTH;  // 64
 constexpr int IN = IPCB_MPNN_IN;    // 16
 constexpr int LAYERS = IPCB_MPNN_LAYERS;
-constexpr int kThreads = 128;
 // k_mlp: warps 0-3 produce (stage tiles, issue the UMMAs), warps 4-7 drain the
 // accumulators; hardware barrier ids 1 and 2 synchronise each group
 constexpr int kMlpThreads = 256;

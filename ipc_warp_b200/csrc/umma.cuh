@@ -21,12 +21,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// byte offset of element (r, k) in an SW128 K-major tile of R rows
-__host__ __device__ __forceinline__ uint32_t sw128_offset(int r, int k, int R) {
-  const int c = k >> 6, kk = k & 63;
-  return (uint32_t)(c * R * 128 + r * 128 + ((((kk >> 3) ^ (r & 7)) & 7) << 4) + ((kk & 7) << 1));
-}
-
 // byte offset of the 16-byte group g (elements 8g..8g+7 of the 64-wide chunk
 // c) of row r
 __host__ __device__ __forceinline__ uint32_t sw128_group(int r, int c, int g, int R) {

@@ -193,15 +193,19 @@ struct BoxArray {  // boxes given as float[3n] lower / upper
 
 // ------------------------------------------------------------- traversal
 // Calls pair(tb) for every leaf block tb whose box overlaps [glo, ghi] (SELF:
-// and tb >= qb, so a block pair is met once).  The whole warp runs it; `turn`
-// counts the pairs, of which this warp takes every nsub-th (nsub a power of
-// two): several warps can share one query block when there are too few.
+// and tb >= qb, so a block pair is met once).  The whole warp runs it.  Several
+// warps can share one query block when there are too few: warp sub of nsub (a
+// power of two, at most 32) takes the leaf blocks sub, sub + nsub, ..  Whose a
+// block is depends on the block alone: the warps may walk with different boxes
+// (a point query's reach up to the TOI stored when its warp starts), so what
+// one of them meets says nothing about what the others meet.
 template <bool SELF, class Pair>
 IPCB_D void for_block_pairs(const View& v, f3 glo, f3 ghi, int qb, int sub, int nsub, unsigned* stack, Pair&& pair) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  int sp = 0, lev = v.top, first = 0, turn = 0;
+  int sp = 0, lev = v.top, first = 0;  // first: a multiple of 32
   if (v.n <= 0) return;
+  const unsigned own = __ballot_sync(0xffffffffu, (lane & (nsub - 1)) == sub);
   for (;;) {
     const int c = first + lane;
     bool hit = false;
@@ -213,11 +217,7 @@ IPCB_D void for_block_pairs(const View& v, f3 glo, f3 ghi, int qb, int sub, int 
     }
     unsigned m = __ballot_sync(0xffffffffu, hit);
     if (lev == 1) {
-      while (m) {
-        const int tb = first + __ffs(m) - 1;
-        m &= m - 1;
-        if ((turn++ & (nsub - 1)) == sub) pair(tb);
-      }
+      for (m &= own; m; m &= m - 1) pair(first + __ffs(m) - 1);
     } else {
       if (hit) stack[sp + __popc(m & below)] = ((unsigned)(lev - 1) << 28) | (unsigned)c;
       sp += __popc(m);

@@ -94,3 +94,36 @@ def test_both_queries_with_a_small_staging_list(cuda):
         pipe._toi_ws_pt = torch.empty_like(pipe._toi_ws)
         small = pipe.iteration(dx)
         assert (small.n_ee, small.n_pt, small.alpha, small.status) == (full.n_ee, full.n_pt, full.alpha, 0)
+
+
+@pytest.mark.parametrize("n", [40, 342, 4700, 9400, 18000])
+def test_point_walk_from_any_stored_toi(cuda, n):
+    """The point walks form their boxes up to the TOI stored when a warp
+    starts; with 16, 16, 8, 4 and 2 warps a query block the records and the
+    minimum are the oracle's from whatever word they start."""
+    sc = loose_triangles(n, seed=n)
+    pipe = ContactPipeline.from_scene(sc, dtype=torch.float32, device=cuda)
+    rng = np.random.default_rng(n)
+    dx = torch.tensor(rng.normal(scale=0.02, size=sc.x.shape), dtype=torch.float32, device=cuda)
+    x0 = pipe.soup.x_transformed.cpu().numpy()
+    pt = sort_records(po.dcd_pt(x0, sc.triangles, sc.body, np.float32(sc.thickness)))
+    toi, _ = po.scene_toi(x0, x0 - dx.cpu().numpy(), np.zeros(0, np.int32), sc.triangles, sc.body)
+    pipe.collision_free_step(dx)  # ccd_x1
+
+    def check(start, found):
+        got = float(pipe.ccd_toi.item())
+        assert got <= min(start, toi) and min(start, toi) - got <= 1e-6
+        if found is not None:
+            assert len(found) == len(pt) and np.array_equal(sort_records(found), pt)
+
+    for start in (1.0, 0.6, 0.5 * (toi + 1.0), toi, 0.5 * toi, 0.0):
+        start = float(np.float32(start))
+        pipe.ccd_toi.fill_(start)
+        pipe.contacts_pt.cnt.zero_()
+        pipe._both_queries("pt", pipe._toi_ws_pt)
+        found = pipe.contacts_pt.records(int(pipe.contacts_pt.cnt.item())).cpu().numpy()
+        pipe._solve_staged("pt", pipe._toi_ws_pt)
+        check(start, found)
+        pipe.ccd_toi.fill_(start)
+        pipe._ccd_query("pt", 0, pipe.soup.n_verts, pipe._toi_ws_pt)
+        check(start, None)

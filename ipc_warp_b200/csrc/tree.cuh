@@ -303,18 +303,24 @@ IPCB_D void block_pair(const View& v, Block& B, int qb, int tb, bool qactive, f3
 // than the rest of the kernel).  The block is taken in segments: [s0, end)
 // with end the lane after which the boxes' areas, weighted by their lanes,
 // fall below a quarter of the whole segment's (a plain patch cut in two keeps
-// half), again until no cut pays.  Returns the segment's end.
+// half), again until no cut pays.  Returns the segment's end.  Every turn but
+// the last shortens the segment.  The areas are of extents over the segment's,
+// so they stay finite while those do (a diverged step's boxes reach 1e19, whose
+// squares do not); a segment of infinite extent is not cut.
 IPCB_D int segment_end(int s0, int end, f3 lo, f3 hi) {
   const int lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu;
   while (end - s0 > 1) {
     const bool in = lane >= s0 && lane < end;
+    float unit;
     {  // a cut that pays needs a step between neighbours of the order of the segment
       const f3 c = mk3(lo.x + hi.x, lo.y + hi.y, lo.z + hi.z);
       const f3 d = mk3(__shfl_down_sync(full, c.x, 1), __shfl_down_sync(full, c.y, 1), __shfl_down_sync(full, c.z, 1));
       const float step = in && lane < end - 1 ? fabsf(d.x - c.x) + fabsf(d.y - c.y) + fabsf(d.z - c.z) : 0.f;
       const f3 l = warp_min3(in ? lo : mk3(kBig, kBig, kBig)), h = warp_max3(in ? hi : mk3(-kBig, -kBig, -kBig));
-      if (!(warp_max(step) > 0.8f * ((h.x - l.x) + (h.y - l.y) + (h.z - l.z)))) break;
+      const float size = (h.x - l.x) + (h.y - l.y) + (h.z - l.z);
+      if (!(warp_max(step) > 0.8f * size)) break;
+      unit = 1.0f / size;
     }
     f3 al = in ? lo : mk3(kBig, kBig, kBig), ah = in ? hi : mk3(-kBig, -kBig, -kBig);
     f3 bl = al, bh = ah;  // al, ah: lanes up to this one; bl, bh: from the next one on
@@ -335,8 +341,9 @@ IPCB_D int segment_end(int s0, int end, f3 lo, f3 hi) {
         bh = mk3(fmaxf(bh.x, dh.x), fmaxf(bh.y, dh.y), fmaxf(bh.z, dh.z));
       }
     }
-    auto area = [](f3 l, f3 h) {
-      const float x = fmaxf(h.x - l.x, 0.f), y = fmaxf(h.y - l.y, 0.f), z = fmaxf(h.z - l.z, 0.f);
+    auto area = [unit](f3 l, f3 h) {
+      const float x = fmaxf((h.x - l.x) * unit, 0.f), y = fmaxf((h.y - l.y) * unit, 0.f),
+                  z = fmaxf((h.z - l.z) * unit, 0.f);
       return x * y + y * z + z * x;
     };
     const float whole = __shfl_sync(full, area(al, ah), end - 1) * (float)(end - s0);
@@ -345,8 +352,9 @@ IPCB_D int segment_end(int s0, int end, f3 lo, f3 hi) {
                            ? area(al, ah) * (float)(lane + 1 - s0) + right * (float)(end - 1 - lane)
                            : kBig;
     const float best = warp_min(cost);
-    if (!(best < 0.25f * whole)) break;
-    end = s0 + max(1, __ffs(__ballot_sync(full, cost == best) >> s0));
+    const int cut = s0 + max(1, __ffs(__ballot_sync(full, cost == best) >> s0));
+    if (!(best < 0.25f * whole) || cut >= end) break;
+    end = cut;
   }
   return end;
 }

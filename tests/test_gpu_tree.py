@@ -127,3 +127,19 @@ def test_point_walk_from_any_stored_toi(cuda, n):
         pipe.ccd_toi.fill_(start)
         pipe._ccd_query("pt", 0, pipe.soup.n_verts, pipe._toi_ws_pt)
         check(start, None)
+
+
+@pytest.mark.parametrize("far", [1e17, 3e19, 1e30])
+def test_step_far_beyond_the_scene(cuda, far):
+    """A diverged direction: boxes whose areas exceed float32."""
+    sc = loose_triangles(342, seed=7)
+    pipe = ContactPipeline.from_scene(sc, dtype=torch.float32, device=cuda)
+    rng = np.random.default_rng(8)
+    dx = rng.normal(scale=0.001, size=sc.x.shape).astype(np.float32)
+    dx[[5, 600]] = far * rng.normal(size=(2, 3))
+    x0 = pipe.soup.x_transformed.cpu().numpy()
+    toi, _ = po.scene_toi(x0, x0 - dx, sc.edges, sc.triangles, sc.body)
+    dev = torch.tensor(dx, device=cuda)
+    for bound in (pipe.collision_free_step(dev), pipe.iteration(dev).alpha):
+        got = float(pipe.ccd_toi.item())
+        assert got <= toi and toi - got <= 1e-6 and bound == (0.9 * got if got < 1.0 else 1.0)

@@ -1,7 +1,7 @@
-"""The packed tree's walk (csrc/tree.cuh) on the CPU: the warps that share a
-query block find every pair once, whatever boxes each of them walks with (a
-warp forms its boxes from the time of impact stored when it starts, which
-another query lowers meanwhile)."""
+"""The packed tree's walk (csrc/tree.cuh) on the CPU: its segments end for
+every box, and the warps that share a query block find every pair once,
+whatever boxes each of them walks with (a warp forms its boxes from the time
+of impact stored when it starts, which another query lowers meanwhile)."""
 import ctypes
 import os
 import re
@@ -34,6 +34,30 @@ def walk(tmp_path_factory):
     lib.segments.argtypes = [f, f, ctypes.c_long, i]
     lib.pairs.argtypes = [ctypes.c_int, f, f, ctypes.c_int, f, f, ctypes.c_long, i, ctypes.c_int]
     return lib
+
+
+def _row(rng):
+    lo = np.arange(32)[:, None] * np.float32([0.1, 0, 0]) + rng.uniform(0, 0.05, (32, 3))
+    return lo.astype(np.float32), (lo + 0.1).astype(np.float32)
+
+
+@pytest.mark.parametrize("size", [0.0, 1.0, 1e3, 1e18, 3e19, 1e20, 1e30, 3e38, np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["one", "apart", "scattered"])
+def test_segments_end(walk, size, kind):
+    rng = np.random.default_rng(1)
+    lo, hi = _row(rng)
+    if kind == "one":  # one primitive swept far
+        hi[7] = size
+    elif kind == "apart":  # neighbours on both sides of the origin
+        lo[1::2], hi[1::2] = -size, 0.0
+        lo[::2], hi[::2] = 0.0, size
+    else:
+        c = (rng.uniform(-0.5, 0.5, (32, 3)) * size).astype(np.float32)
+        lo, hi = lo + c, hi + c
+    ends = np.zeros(64, np.int32)
+    n = walk.segments(lo, hi, LIMIT, ends)
+    assert 1 <= n <= 32
+    assert (np.diff(np.concatenate([[0], ends[:n]])) > 0).all() and ends[n - 1] == 32
 
 
 @pytest.mark.parametrize("nsub", [1, 2, 4, 8, 16])

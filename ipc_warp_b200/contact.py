@@ -188,6 +188,12 @@ class ContactSolverBase:
         for k in ks:
             torch.cuda.current_stream().wait_stream(self._branches[k])
 
+    def _captured(self) -> tuple:
+        """What a captured sequence holds by value, or by an address a caller
+        may replace: part of the key of every graph, so that all of a
+        solver's graphs follow a change at the same call."""
+        return (_thickness, buffer, bool(self.disable_self_collision), float(self.contact_stiffness), float(self.h))
+
     # --------------------------------------------------------------- hooks
     def profile_timer(self, name):
         return nullcontext()

@@ -546,12 +546,14 @@ class MixedSolver(ContactBarrierMixin):
     def _ls_key(self):
         ee, pt = self.contacts_new, self.contacts_pt
         return (self.q.data_ptr(), self.q_start.data_ptr(), self.dq.data_ptr(), self.x.data_ptr(),
-                ee.a1a2b1b2.data_ptr(), ee.capacity, pt.a1a2b1b2.data_ptr(), pt.capacity)
+                ee.a1a2b1b2.data_ptr(), ee.capacity, pt.a1a2b1b2.data_ptr(), pt.capacity, self._captured())
+
+    def _captured(self):
+        return (*super()._captured(), self.material, self.mu, self.lam)
 
     def _ls_graph(self):
         """The WHILE graph of one trial (q = q_start - alpha dq, x = J q, the
-        energy, the accept test), captured once per buffer set on a side
-        stream."""
+        energy, the accept test), captured once per key on a side stream."""
         ls = self._ls
         key = self._ls_key()
         if ls["graph"] is not None and ls["key"] == key:

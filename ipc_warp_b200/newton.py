@@ -521,6 +521,7 @@ class FEMContactSolver(ContactBarrierMixin):
         st = self._static
         g = getattr(self, "_A_graph", None)
         if g is not None and g[0] == self._A_graph_key():
+            self._diagonal()
             g[1].replay()
             torch.cuda.current_stream().synchronize()
             n_ee, n_pt, bst, qst = (int(v) for v in st["graph_read"])
@@ -552,15 +553,21 @@ class FEMContactSolver(ContactBarrierMixin):
         return self.A
 
     def _A_graph_key(self):
-        """The buffers a captured compute_A reads and writes (the schedule is
-        kept as captured while they stay: a later workload bucket's choice
-        would cost a recapture per change of bucket)."""
+        """The buffers a captured compute_A reads and writes and the scalars
+        it holds (the schedule is kept as captured while they stay: a later
+        workload bucket's choice would cost a recapture per change of
+        bucket)."""
         st = self._static
         ee, pt, t = self.contacts_new, self.contacts_pt, self.collision_triplets
         return (ee.a1a2b1b2.data_ptr(), ee.capacity, pt.a1a2b1b2.data_ptr(), pt.capacity,
                 None if t is None else t.rows.data_ptr(), None if self.A is None else self.A.values.data_ptr(),
                 None if getattr(self, "_C", None) is None else self._C.values.data_ptr(),
-                st.get("a_rows").data_ptr() if "a_rows" in st else None, self.states.x.data_ptr())
+                st.get("a_rows").data_ptr() if "a_rows" in st else None, self.states.x.data_ptr(), self._captured())
+
+    def _captured(self):
+        return (*super()._captured(), self.material, self.mu, self.lam, self.k_att, self.tets.data_ptr(),
+                self.Bm.data_ptr(), self.W.data_ptr(), self.mass.data_ptr(), self.b.data_ptr(),
+                self.soup.xcs.data_ptr())
 
     def _compute_A_generic(self) -> BsrMatrix:
         """Per-term kernels, then one sort-based assembly of every triplet."""
@@ -607,9 +614,8 @@ class FEMContactSolver(ContactBarrierMixin):
         g_idx = torch.argsort(sl, stable=True).to(torch.int32)
         g_off = torch.zeros(nnz + 1, dtype=torch.int32, device=dev)
         g_off[1:] = torch.cumsum(torch.bincount(sl, minlength=nnz), 0).to(torch.int32)
-        h2 = self.h * self.h
-        diag = (self.mass + (h2 * self.k_att) * self.fixed.double()).to(self.dtype)
-        self._static = dict(S=S, nnz=nnz, g_off=g_off, g_idx=g_idx, diag=diag, rows_t=rows_t, cols_t=cols_t,
+        self._static = dict(S=S, nnz=nnz, g_off=g_off, g_idx=g_idx, rows_t=rows_t, cols_t=cols_t,
+                            diag=torch.empty(V, dtype=self.dtype, device=dev), diag_of=None,
                             tet_vals=torch.empty((16 * nt, 3, 3), dtype=self.dtype, device=dev),
                             queue=torch.zeros(1, dtype=torch.int32, device=dev),
                             status=torch.zeros(1, dtype=torch.int32, device=dev),
@@ -624,6 +630,13 @@ class FEMContactSolver(ContactBarrierMixin):
         n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
         self._n_sm = n_sm
         self._tuner = Autotuner("terms", terms_candidates())
+
+    def _diagonal(self):
+        """M + h^2 k_att of the fixed vertices, into the buffer the graphs hold."""
+        st, of = self._static, (self.h, self.k_att)
+        if st["diag_of"] != of:
+            st["diag"].copy_(self.mass + (self.h * self.h * self.k_att) * self.fixed.double())
+            st["diag_of"] = of
 
     def _sorted_workspaces(self):
         """Device workspaces of the class-sorted narrow phase, one per list."""
@@ -656,6 +669,7 @@ class FEMContactSolver(ContactBarrierMixin):
         union with the fixed elastic pattern with gathered values."""
         if self._static is None:
             self._static_pattern()
+        self._diagonal()
         st = self._static
         h2 = self.h * self.h
         V = self.soup.n_verts
@@ -868,11 +882,12 @@ class FEMContactSolver(ContactBarrierMixin):
     def _ls_key(self):
         return (self.states.x.data_ptr(), self.states.dx.data_ptr(), self.states.x0.data_ptr(),
                 self.states.xdot.data_ptr(), self.contacts_new.a1a2b1b2.data_ptr(), self.contacts_new.capacity,
-                self.contacts_pt.a1a2b1b2.data_ptr(), self.contacts_pt.capacity, self.x_target.data_ptr())
+                self.contacts_pt.a1a2b1b2.data_ptr(), self.contacts_pt.capacity, self.x_target.data_ptr(),
+                self._captured())
 
     def _ls_graph(self):
-        """The WHILE graph of one trial, captured once per buffer set (on a
-        side stream: the legacy default stream cannot be captured)."""
+        """The WHILE graph of one trial, captured once per key (on a side
+        stream: the legacy default stream cannot be captured)."""
         ls = self._ls
         key = self._ls_key()
         if ls["graph"] is not None and ls["key"] == key:
@@ -924,11 +939,9 @@ class FEMContactSolver(ContactBarrierMixin):
     def _ls_prelude(self, mode: str):
         """Everything before the trials: x kept, E0, the CCD bound, the search
         state.  Replayed from a graph from the second search on (per mode and
-        buffer set): the launches alone take the host longer than the GPU."""
+        key): the launches alone take the host longer than the GPU."""
         ls = self._ls
-        key = (mode, self._ls_key(), self._toi_ws.data_ptr(), self.ccd_toi.data_ptr(), contact_mod._thickness,
-               contact_mod.buffer, self.disable_self_collision, float(self.contact_stiffness), self.h, self.material,
-               self.mu, self.lam, self.k_att)
+        key = (mode, self._ls_key(), self._toi_ws.data_ptr(), self.ccd_toi.data_ptr())
         graphs = ls.setdefault("prelude", {})
         if len(graphs) > 8:  # buffers that came and went
             graphs.clear()

@@ -94,7 +94,7 @@ class ContactPipeline(ContactBarrierMixin):
         list capacities) and the counts, the BSR status, the energy and the
         TOI come back in one read at the end.  After one such iteration the
         whole sequence is captured in a CUDA graph and replayed (recaptured
-        when a buffer is reallocated).  A list that overflowed or a BSR row
+        when a buffer is reallocated or a scalar it holds changes).  A list that overflowed or a BSR row
         with too many columns sends the iteration through the step-by-step
         calls, which grow the lists and pick the generic assembly."""
         if dx is not None:
@@ -130,7 +130,8 @@ class ContactPipeline(ContactBarrierMixin):
         io = None if self._host_io is None else tuple(a.data_ptr() for a in self._host_io)
         return (ee.a1a2b1b2.data_ptr(), ee.capacity, pt.a1a2b1b2.data_ptr(), pt.capacity,
                 None if t is None else t.rows.data_ptr(), None if H is None else H.values.data_ptr(),
-                None if H is None else H._ws.data_ptr(), ws, io, getattr(self, "bvh_rebuild_interval", 0))
+                None if H is None else H._ws.data_ptr(), ws, io, self._captured(),
+                getattr(self, "bvh_rebuild_interval", 0))
 
     def iteration_host(self, x: torch.Tensor, dx: torch.Tensor, b: torch.Tensor) -> IterationResult:
         """iteration() from host memory: positions x and direction dx (V, 3)

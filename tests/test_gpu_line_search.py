@@ -117,3 +117,42 @@ def test_newton_iteration_reuses_detection_for_e0(cuda):
     alpha2 = s.line_search()  # direct call: detects at x0 again, same direction
     assert s.stats.energies[-1][0] == pytest.approx(e0_reused, rel=1e-12)
     assert alpha2 == alpha and torch.equal(s.states.x, x1)
+
+
+@pytest.mark.parametrize("change", ["contact_stiffness", "h", "k_att", "mu"])
+def test_graphs_follow_a_changed_scalar(cuda, change):
+    """Every graph holds the scalars by value: after a change on a solver
+    whose graphs are captured, matrix and energies are those of a solver that
+    had the value from the start."""
+    s, fresh = _solver(torch.float64, "device"), _solver(torch.float64, "device")
+    x0 = s.states.x.clone()
+    dx = torch.tensor(np.random.default_rng(3).normal(scale=1e-5, size=tuple(x0.shape)), device=cuda)
+    s.states.dx.copy_(dx)
+    for _ in range(3):  # step by step, captured, replayed
+        s.compute_A()
+        s.line_search()
+        s.states.x.copy_(x0)
+    value = 1.5 * getattr(s, change)
+    for k in (s, fresh):
+        setattr(k, change, value)
+        k.states.dx.copy_(dx)
+        A = k.compute_A()
+        k.dense = (A.nnz_sync(), A.values[:A.nnz_sync()].clone(), k.line_search(), k.stats.energies[-1])
+    n, values, alpha, energies = s.dense
+    assert n == fresh.dense[0] and alpha == fresh.dense[2]
+    # the sums' order differs between instances: a few roundings
+    assert torch.allclose(values, fresh.dense[1], rtol=1e-12, atol=1e-12 * float(values.abs().max()))
+    assert energies == pytest.approx(fresh.dense[3], rel=1e-12)
+
+
+def test_pipeline_graph_follows_a_changed_stiffness(cuda):
+    from ipc_warp_b200.pipeline import ContactPipeline
+
+    sc = two_cubes(n=3, gap=4e-4, angle_deg=15.0, jitter=0.0, seed=0, dhat=1e-3, kappa=1e6)
+    pipe = ContactPipeline.from_scene(sc, dtype=torch.float64, device=cuda)
+    dx = torch.zeros_like(pipe.states.x)
+    for _ in range(3):
+        e = pipe.iteration(dx).energy
+    pipe.contact_stiffness *= 3.0
+    assert pipe.iteration(dx).energy == pytest.approx(3.0 * e, rel=1e-12)
+    assert pipe.iteration(dx).energy == pytest.approx(3.0 * e, rel=1e-12)

@@ -720,9 +720,32 @@ class FEMContactSolver(ContactBarrierMixin):
         self.collision_hessian = C
         return A
 
+    def _readable(self, dtype, shape, *tensors) -> bool:
+        """Whether the tensors (which a caller may have replaced) are laid out
+        as the kernels read them."""
+        dev = self.b.device
+        return all(t.dtype == dtype and t.shape == shape and t.is_contiguous() and t.device == dev for t in tensors)
+
+    def _plain_states(self, *more) -> bool:
+        st, V = self.states, self.soup.n_verts
+        return self._readable(torch.float64, (V,), self.mass) and \
+            self._readable(self.dtype, (V, 3), st.x0, st.xdot, self.x_target, *more)
+
     def compute_rhs(self) -> torch.Tensor:
-        """time_integrator_base.py:82-91,428-438: gradient of the total energy."""
+        """time_integrator_base.py:82-91,428-438: gradient of the total
+        energy, in one launch; from tensors of any type and stride, or with a
+        subclass's x_tilde, as a sum of tensors."""
         st = self.states
+        if not (self._plain_states(self.b, st.x) and self._readable(torch.bool, (self.soup.n_verts,), self.fixed) and
+                self._readable(torch.float64, (3,), self.gravity) and
+                type(self).x_tilde is FEMContactSolver.x_tilde):
+            h2 = self.h * self.h
+            x = st.x.double()
+            g = -h2 * self.b.double() + self.mass[:, None] * (x - self.x_tilde())
+            if bool(self.fixed.any()):
+                g = g + (h2 * self.k_att) * self.fixed.double()[:, None] * (x - self.x_target.double())
+            self.rhs = g.to(self.dtype)
+            return self.rhs
         self.rhs = torch.empty_like(self.b)
         N.call("ipcb_newton_rhs", int(self.dtype == torch.float64), self.soup.n_verts, N.ptr(self.b), N.ptr(st.x),
                N.ptr(st.x0), N.ptr(st.xdot), N.ptr(self.gravity), self.h, N.ptr(self.mass), N.ptr(self.fixed),
@@ -786,8 +809,9 @@ class FEMContactSolver(ContactBarrierMixin):
         return self.states.dx
 
     def line_search(self) -> float:
-        """time_integrator_base.py:514-546 with the CCD bound."""
-        if self.line_search_mode == "device":
+        """time_integrator_base.py:514-546 with the CCD bound (the host loop
+        also where the device's kernels cannot read the states)."""
+        if self.line_search_mode == "device" and self._plain_states():
             return self._line_search_device()
         return self._line_search_host()
 
@@ -885,11 +909,10 @@ class FEMContactSolver(ContactBarrierMixin):
                 self.contacts_pt.a1a2b1b2.data_ptr(), self.contacts_pt.capacity, self.x_target.data_ptr(),
                 self._captured())
 
-    def _ls_graph(self):
-        """The WHILE graph of one trial, captured once per key (on a side
-        stream: the legacy default stream cannot be captured)."""
+    def _ls_graph(self, key: tuple):
+        """The WHILE graph of one trial, captured once per _ls_key() (on a
+        side stream: the legacy default stream cannot be captured)."""
         ls = self._ls
-        key = self._ls_key()
         if ls["graph"] is not None and ls["key"] == key:
             return ls["graph"]
         if ls["graph"] is not None:
@@ -936,12 +959,12 @@ class FEMContactSolver(ContactBarrierMixin):
             if end_rc != 0:
                 raise N.NativeError("ipcb_graph_while_end failed: " + (N.lib().ipcb_last_error() or b"").decode())
 
-    def _ls_prelude(self, mode: str):
+    def _ls_prelude(self, mode: str, key: tuple):
         """Everything before the trials: x kept, E0, the CCD bound, the search
         state.  Replayed from a graph from the second search on (per mode and
-        key): the launches alone take the host longer than the GPU."""
+        _ls_key()): the launches alone take the host longer than the GPU."""
         ls = self._ls
-        key = (mode, self._ls_key(), self._toi_ws.data_ptr(), self.ccd_toi.data_ptr())
+        key = (mode, key, self._toi_ws.data_ptr(), self.ccd_toi.data_ptr())
         graphs = ls.setdefault("prelude", {})
         if len(graphs) > 8:  # buffers that came and went
             graphs.clear()
@@ -991,8 +1014,9 @@ class FEMContactSolver(ContactBarrierMixin):
         mode = "cached" if getattr(self, "_ls_cache", False) else \
             ("fresh" if getattr(self, "_lists_at_x", False) else "detect")
         self._lists_at_x = False
-        self._ls_prelude(mode)
-        graph = self._ls_graph()
+        key = self._ls_key()
+        self._ls_prelude(mode, key)
+        graph = self._ls_graph(key)
         N.call("ipcb_graph_launch", graph, s)
         N.call("ipcb_ls_finish", N.ptr(ls["state"]), fp64, self.soup.n_verts, N.ptr(ls["x_tmp"]),
                N.ptr(self.states.x), s)

@@ -183,3 +183,41 @@ def test_direct_solver_step_matches_pcg_step(cuda):
     assert np.abs(out["direct"][0] - out["pcg"][0]).max() <= 1e-9
     assert np.abs(out["direct"][0] - out["fallback"][0]).max() <= 1e-12
     assert out["fallback"][1] == 1 and out["pcg"][1] == 0
+
+
+@pytest.mark.parametrize("odd", ["xdot", "x0", "x_target", "fixed", "gravity", "strided", "x_tilde"])
+def test_rhs_of_any_type_and_stride(cuda, odd):
+    """States of another type or stride and a subclass's x_tilde, as the sum
+    of tensors took them."""
+    class Pulled(FEMContactSolver):
+        def x_tilde(self):
+            return super().x_tilde() + 1e-3
+
+    sc = _scene(4e-4)
+    s = _solver(sc, torch.float64, "stvk")
+    if odd == "x_tilde":
+        s.__class__ = Pulled
+    x, xdot = _state(sc)
+    s.states.x.copy_(torch.tensor(x))
+    s.states.xdot.copy_(torch.tensor(xdot))
+    s.compute_A()
+    if odd in ("xdot", "x0"):
+        setattr(s.states, odd, getattr(s.states, odd).float())
+    elif odd == "x_target":
+        s.x_target = s.x_target.float()
+    elif odd == "fixed":
+        s.fixed = s.fixed.to(torch.int32)
+    elif odd == "gravity":
+        s.gravity = s.gravity.float()
+    elif odd == "strided":
+        s.states.xdot = s.states.xdot.t().contiguous().t()
+    got = s.compute_rhs()
+    h2, st = s.h * s.h, s.states
+    xt = st.x0.double() + s.h * st.xdot.double() + h2 * s.gravity + (1e-3 if odd == "x_tilde" else 0.0)
+    ref = -h2 * s.b + s.mass[:, None] * (st.x - xt) + \
+        h2 * s.k_att * s.fixed.double()[:, None] * (st.x - s.x_target.double())
+    assert got.dtype == torch.float64
+    assert torch.allclose(got, ref, rtol=1e-12, atol=1e-14 * float(ref.abs().max()))
+    s.states.dx.copy_(1e-3 * torch.tensor(xdot))
+    alpha, x0 = s.line_search(), s.states.x.clone()
+    assert np.isfinite(s.stats.energies[-1][0]) and 0.0 <= alpha <= 1.0 and bool(torch.isfinite(x0).all())

@@ -818,6 +818,7 @@ class FEMContactSolver(ContactBarrierMixin):
     def _line_search_host(self) -> float:
         """The reference's loop: energies and the accept test on the host."""
         self._lists_at_x = False
+        self._ls_cache = False  # the device search's terms are of another point from here on
         x_tmp = self.states.x.clone()
         E0 = self.total_energy()
         refusals = self.ccd_refusals

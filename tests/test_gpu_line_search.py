@@ -156,3 +156,20 @@ def test_pipeline_graph_follows_a_changed_stiffness(cuda):
     pipe.contact_stiffness *= 3.0
     assert pipe.iteration(dx).energy == pytest.approx(3.0 * e, rel=1e-12)
     assert pipe.iteration(dx).energy == pytest.approx(3.0 * e, rel=1e-12)
+
+
+def test_overflowed_search_leaves_no_cached_energy(cuda):
+    """Inside a step a search starts from the terms its predecessor accepted;
+    one that the host finished leaves none."""
+    s = _solver(torch.float64, "device")
+    _direction(s)
+    s._in_step = True
+    assert s.line_search() > 0 and s._ls_cache
+    _direction(s)
+    s.contacts_new.grow(1)
+    s.contacts_list_new = s.contacts_new
+    s.line_search()
+    _direction(s)
+    at = s.total_energy()
+    s.line_search()
+    assert s.stats.energies[-1][0] == pytest.approx(at, rel=1e-12)

@@ -176,11 +176,11 @@ int ipcb_dcd_pt_range(const ipcb_soup* soup, const float* x4, const ipcb_lbvh* t
 
 /* The two ends of a contact iteration, one launch each.  begin: b = 0, x1 =
  * x - dx (dx may be null: x1 untouched), both list counts, both status words
- * and the energy 0, toi 1.  results: the counts, the two status words
+ * and the energy 0, toi 1, and x4 the packed positions (ipcb_pack_positions).  results: the counts, the two status words
  * (counts_out[0..3]), the energy and the TOI written to memory the device can
  * reach (pinned host memory). */
 int ipcb_iteration_begin(const ipcb_soup* soup, const void* dx, void* x1, void* b, int* ee_cnt, int* pt_cnt,
-                         int* status, int* bsr_status, double* energy, void* toi, ipcb_stream s);
+                         int* status, int* bsr_status, double* energy, void* toi, float* x4, ipcb_stream s);
 int ipcb_iteration_results(int fp64, const int* ee_cnt, const int* pt_cnt, const int* bsr_status, const int* status,
                            const double* energy, const void* toi, int* counts_out, double* energy_out, void* toi_out,
                            ipcb_stream s);

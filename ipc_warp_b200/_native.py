@@ -223,7 +223,7 @@ SIGNATURES = {
     "ipcb_contact_bsr_workspace": (c_size_t, [c_int, c_int]),
     "ipcb_union_values": (c_int, [c_int, P, c_int, P, P, P, P, c_double, P, P]),
     "ipcb_newton_rhs": (c_int, [c_int, c_int, P, P, P, P, P, c_double, P, P, P, c_double, P, P]),
-    "ipcb_iteration_begin": (c_int, [SP, P, P, P, P, P, P, P, P, P, P]),
+    "ipcb_iteration_begin": (c_int, [SP, P, P, P, P, P, P, P, P, P, P, P]),
     "ipcb_words": (c_int, [c_int, ctypes.POINTER(P), ctypes.POINTER(P), P]),
     "ipcb_iteration_results": (c_int, [c_int, P, P, P, P, P, P, P, P, P, P]),
     "ipcb_contact_bsr_rows": (c_int, [CP, c_int, CP, c_int, c_int, P, c_size_t, P]),

@@ -21,6 +21,7 @@ import ctypes
 import warnings
 from contextlib import contextmanager, nullcontext
 from dataclasses import dataclass
+from functools import partial
 
 import torch
 
@@ -116,6 +117,16 @@ class Contacts:
         return torch.cat([self.a1a2b1b2[:n], self.e0e1[:n]], dim=1)
 
 
+def _edge_aabbs(soup: Soup, x4, pad: float, lower, upper):
+    N.call("ipcb_edge_aabbs", ctypes.byref(soup.c_struct()), N.ptr(x4), pad, N.ptr(lower), N.ptr(upper),
+           N.stream_handle())
+
+
+def _triangle_aabbs(soup: Soup, x4, lower, upper):
+    N.call("ipcb_triangle_aabbs", ctypes.byref(soup.c_struct()), N.ptr(x4), 0.0, N.ptr(lower), N.ptr(upper),
+           N.stream_handle())
+
+
 def _next_pow2(n: int) -> int:
     return 1 << (max(n, 1) - 1).bit_length()
 
@@ -132,10 +143,10 @@ class ContactSolverBase:
         n_edges, n_nodes, n_tris = soup.n_edges, soup.n_verts, soup.n_tris
         f32 = dict(dtype=torch.float32, device=dev)
         self.x4 = torch.zeros((n_nodes, 4), **f32)  # float32 mesh copy (contact.py:476, x_mesh)
-        self.bvh_edges_lower = torch.zeros((n_edges, 3), **f32)
-        self.bvh_edges_upper = torch.zeros((n_edges, 3), **f32)
+        self.bvh_edges = None
+        self._edge_boxes = torch.zeros((n_edges, 3), **f32), torch.zeros((n_edges, 3), **f32)
         self.compute_edge_aabbs()
-        self.bvh_edges = Bvh(self.bvh_edges_lower, self.bvh_edges_upper)
+        self.bvh_edges = Bvh(*self._edge_boxes)
         # CCD boxes are refit into the DCD hierarchies (same primitives, same
         # topology); detect_collision refits them back before every query.
         self.ccd_edge_lower = torch.zeros((n_edges, 3), **f32)
@@ -145,10 +156,10 @@ class ContactSolverBase:
         self.ccd_x1 = torch.zeros_like(soup.x_transformed)
         self.has_triangles = n_tris > 0
         if self.has_triangles:
-            self.tri_lower = torch.zeros((n_tris, 3), **f32)
-            self.tri_upper = torch.zeros((n_tris, 3), **f32)
+            self.tri_mesh = None
+            self._tri_boxes = torch.zeros((n_tris, 3), **f32), torch.zeros((n_tris, 3), **f32)
             self._triangle_aabbs()
-            self.tri_mesh = Bvh(self.tri_lower, self.tri_upper)
+            self.tri_mesh = Bvh(*self._tri_boxes)
             self.ccd_triangle_lower = torch.zeros((n_tris, 3), **f32)
             self.ccd_triangle_upper = torch.zeros((n_tris, 3), **f32)
             self.ccd_triangle_bvh = self.tri_mesh
@@ -208,12 +219,27 @@ class ContactSolverBase:
     def compute_edge_aabbs(self):
         """contact.py:679-681: edge boxes padded by _thickness + buffer."""
         self._pack()
-        N.call("ipcb_edge_aabbs", ctypes.byref(self.soup.c_struct()), N.ptr(self.x4), float(_thickness + buffer),
-               N.ptr(self.bvh_edges_lower), N.ptr(self.bvh_edges_upper), N.stream_handle())
+        boxes = self._edge_boxes if self.bvh_edges is None else self.bvh_edges.rewrite()
+        _edge_aabbs(self.soup, self.x4, float(_thickness + buffer), *boxes)
 
     def _triangle_aabbs(self):
-        N.call("ipcb_triangle_aabbs", ctypes.byref(self.soup.c_struct()), N.ptr(self.x4), 0.0,
-               N.ptr(self.tri_lower), N.ptr(self.tri_upper), N.stream_handle())
+        _triangle_aabbs(self.soup, self.x4, *(self._tri_boxes if self.tri_mesh is None else self.tri_mesh.rewrite()))
+
+    @property
+    def bvh_edges_lower(self) -> torch.Tensor:
+        return self.bvh_edges.lower
+
+    @property
+    def bvh_edges_upper(self) -> torch.Tensor:
+        return self.bvh_edges.upper
+
+    @property
+    def tri_lower(self) -> torch.Tensor:
+        return self.tri_mesh.lower
+
+    @property
+    def tri_upper(self) -> torch.Tensor:
+        return self.tri_mesh.upper
 
     def update_bvh(self):
         """contact.py:672-677: edge boxes + refit, float32 mesh copy + refit.
@@ -237,22 +263,39 @@ class ContactSolverBase:
     def _refit_edges(self):
         """The boxes the edge query reads, from x4 (after _pack)."""
         N.call("ipcb_lbvh_refit_edges", ctypes.byref(self.soup.c_struct()), N.ptr(self.x4),
-               float(_thickness + buffer), ctypes.byref(self.bvh_edges.c), N.stream_handle())
+               float(_thickness + buffer), ctypes.byref(self.bvh_edges._c), N.stream_handle())
 
     def _refit_triangles(self):
         """The boxes the point-triangle query reads, from x4 (after _pack)."""
         N.call("ipcb_lbvh_refit_triangles", ctypes.byref(self.soup.c_struct()), N.ptr(self.x4), 0.0,
-               ctypes.byref(self.tri_mesh.c), N.stream_handle())
+               ctypes.byref(self.tri_mesh._c), N.stream_handle())
+
+    def _refits_packed(self) -> bool:
+        """Whether the packed boxes are all a detection has to form: not where
+        update_bvh rebuilds or a subclass has its own boxes."""
+        own = type(self).update_bvh is not ContactSolverBase.update_bvh or \
+            type(self).compute_edge_aabbs is not ContactSolverBase.compute_edge_aabbs
+        return not (own or getattr(self, "bvh_rebuild_interval", 0))
 
     def _refit_queries(self):
-        """What the queries need of update_bvh: the packed boxes only (the
-        binary nodes and the box arrays keep update_bvh's last values)."""
-        if getattr(self, "bvh_rebuild_interval", 0):
+        """What the queries need of update_bvh: the packed boxes."""
+        if not self._refits_packed():
             return self.update_bvh()
         self._pack()
         self._refit_edges()
         if self.has_triangles:
             self._refit_triangles()
+        self._follow_x4()
+
+    def _follow_x4(self):
+        """After a detection (or a replay of one) that formed the packed boxes
+        alone: box arrays and nodes follow from x4, as update_bvh forms them,
+        when they are read."""
+        if not self._refits_packed():
+            return
+        self.bvh_edges.follow(partial(_edge_aabbs, self.soup, self.x4, float(_thickness + buffer)))
+        if self.has_triangles:
+            self.tri_mesh.follow(partial(_triangle_aabbs, self.soup, self.x4))
 
     # ----------------------------------------------------------------- DCD
     def _grow_contact_list(self, contacts: Contacts, required: int, point_triangle: bool = False):
@@ -270,12 +313,12 @@ class ContactSolverBase:
         s = N.stream_handle()
         if which == "ee":
             self.contacts_new.cnt.zero_()
-            N.call("ipcb_dcd_ee", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.bvh_edges.c),
+            N.call("ipcb_dcd_ee", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.bvh_edges._c),
                    float(_thickness), float(_thickness + buffer), int(self.disable_self_collision),
                    ctypes.byref(self.contacts_new.c_struct()), N.ptr(self._status), s)
         else:
             self.contacts_pt.cnt.zero_()
-            N.call("ipcb_dcd_pt", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.tri_mesh.c),
+            N.call("ipcb_dcd_pt", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.tri_mesh._c),
                    float(_thickness), float(2.0 * (_thickness + buffer)), int(self.disable_self_collision),
                    N.ptr(self._point_order), ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self._status), s)
 
@@ -326,8 +369,17 @@ class ContactSolverBase:
     # ----------------------------------------------------------------- CCD
     def collision_free_step(self, dx: torch.Tensor) -> float:
         """contact.py:539-585: conservative CCD bound for x -= alpha * dx;
-        returns 0.9 * toi if toi < 1 else 1."""
+        returns 0.9 * toi if toi < 1 else 1.  Leaves the swept boxes of the
+        whole step in ccd_edge_lower / _upper and ccd_triangle_lower / _upper."""
         self._launch_ccd(dx)
+        soup, s, x1 = ctypes.byref(self.soup.c_struct()), N.stream_handle(), N.ptr(self.ccd_x1)
+        boxes = self.ccd_edge_lower, self.ccd_edge_upper
+        N.call("ipcb_swept_edge_aabbs", soup, x1, 1e-7, *map(N.ptr, boxes), s)
+        self.ccd_edge_bvh.follow(nodes=boxes)
+        if self.has_triangles:
+            boxes = self.ccd_triangle_lower, self.ccd_triangle_upper
+            N.call("ipcb_swept_triangle_aabbs", soup, x1, 1e-7, *map(N.ptr, boxes), s)
+            self.ccd_triangle_bvh.follow(nodes=boxes)
         return self._step_bound()
 
     def _step_bound(self) -> float:
@@ -380,11 +432,11 @@ class ContactSolverBase:
         s = N.stream_handle()
         if which == "ee":
             N.call("ipcb_edge_edge_step", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   ctypes.byref(self.ccd_edge_bvh.c), ctypes.byref(self.contacts_new.c_struct()), excl, first, count,
+                   ctypes.byref(self.ccd_edge_bvh._c), ctypes.byref(self.contacts_new.c_struct()), excl, first, count,
                    N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(ws), ws.numel(), s)
         else:
             N.call("ipcb_point_triangle_step", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   ctypes.byref(self.ccd_triangle_bvh.c), N.ptr(self._point_order),
+                   ctypes.byref(self.ccd_triangle_bvh._c), N.ptr(self._point_order),
                    ctypes.byref(self.contacts_pt.c_struct()), excl, first, count, N.ptr(self.ccd_toi),
                    N.ptr(self._status), N.ptr(ws), ws.numel(), s)
 
@@ -398,12 +450,12 @@ class ContactSolverBase:
         excl = int(self.disable_self_collision)
         s = N.stream_handle()
         if which == "ee":
-            N.call("ipcb_edge_edge_both", ctypes.byref(soup), N.ptr(self.ccd_x1), pad, ctypes.byref(self.bvh_edges.c),
+            N.call("ipcb_edge_edge_both", ctypes.byref(soup), N.ptr(self.ccd_x1), pad, ctypes.byref(self.bvh_edges._c),
                    float(_thickness), float(_thickness + buffer), excl, ctypes.byref(self.contacts_new.c_struct()),
                    N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(ws), ws.numel(), s)
         else:
             N.call("ipcb_point_triangle_both", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   ctypes.byref(self.tri_mesh.c), float(_thickness), float(2.0 * (_thickness + buffer)),
+                   ctypes.byref(self.tri_mesh._c), float(_thickness), float(2.0 * (_thickness + buffer)),
                    N.ptr(self._point_order), excl, ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self.ccd_toi),
                    N.ptr(self._status), N.ptr(ws), ws.numel(), s)
 
@@ -415,10 +467,10 @@ class ContactSolverBase:
         tail = (excl, N.ptr(self.ccd_toi), N.ptr(self._status), N.ptr(ws), ws.numel(), N.stream_handle())
         if which == "ee":
             N.call("ipcb_edge_edge_solve", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   ctypes.byref(self.ccd_edge_bvh.c), *tail)
+                   ctypes.byref(self.ccd_edge_bvh._c), *tail)
         else:
             N.call("ipcb_point_triangle_solve", ctypes.byref(soup), N.ptr(self.ccd_x1), pad,
-                   ctypes.byref(self.ccd_triangle_bvh.c), N.ptr(self._point_order), *tail)
+                   ctypes.byref(self.ccd_triangle_bvh._c), N.ptr(self._point_order), *tail)
 
     def new_intersections(self, x0: torch.Tensor, x1: torch.Tensor) -> float:
         """contact.py:587-670 (the augmented-Lagrangian solver's CCD): every
@@ -439,7 +491,7 @@ class ContactSolverBase:
         def edges():
             self.contacts_new.cnt.zero_()
             self.ccd_toi.fill_(1.0)
-            N.call("ipcb_edge_edge_intersections", ctypes.byref(soup), N.ptr(x1), ctypes.byref(self.ccd_edge_bvh.c),
+            N.call("ipcb_edge_edge_intersections", ctypes.byref(soup), N.ptr(x1), ctypes.byref(self.ccd_edge_bvh._c),
                    N.ptr(self.ccd_edge_lower), N.ptr(self.ccd_edge_upper), excl, th, N.ptr(self.ccd_toi),
                    ctypes.byref(self.contacts_new.c_struct()), N.ptr(self._status), N.ptr(self._toi_ws),
                    self._toi_ws.numel(), s)
@@ -458,7 +510,7 @@ class ContactSolverBase:
             def points():
                 self.contacts_pt.cnt.zero_()
                 N.call("ipcb_point_triangle_intersections", ctypes.byref(soup), N.ptr(x1),
-                       ctypes.byref(self.ccd_triangle_bvh.c), pad, excl, th, N.ptr(self.ccd_toi),
+                       ctypes.byref(self.ccd_triangle_bvh._c), pad, excl, th, N.ptr(self.ccd_toi),
                        ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self._status), N.ptr(self._toi_ws),
                        self._toi_ws.numel(), s)
                 return int(self.contacts_pt.cnt.item())

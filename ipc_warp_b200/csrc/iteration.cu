@@ -11,12 +11,14 @@ namespace {
 
 template <class S>
 __global__ void k_begin(const S* __restrict__ x, const S* __restrict__ dx, S* __restrict__ x1, S* __restrict__ b,
-                        int n3, int* ee_cnt, int* pt_cnt, int* status, int* bsr_status, double* energy, S* toi) {
+                        int n3, int* ee_cnt, int* pt_cnt, int* status, int* bsr_status, double* energy, S* toi,
+                        float4* __restrict__ x4) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n3) {
     b[i] = S(0);
     if (dx) x1[i] = xsub(x[i], dx[i]);
   }
+  if (3 * i < n3) x4[i] = make_float4((float)x[3 * i], (float)x[3 * i + 1], (float)x[3 * i + 2], 0.f);
   if (i == 0) {
     *ee_cnt = *pt_cnt = *status = *bsr_status = 0;
     *energy = 0.0;
@@ -54,16 +56,18 @@ using namespace ipcb;
 extern "C" {
 
 int ipcb_iteration_begin(const ipcb_soup* soup, const void* dx, void* x1, void* b, int* ee_cnt, int* pt_cnt,
-                         int* status, int* bsr_status, double* energy, void* toi, ipcb_stream s) {
-  if (!soup || !b || (dx && !x1) || !ee_cnt || !pt_cnt || !status || !bsr_status || !energy || !toi) return IPCB_E_ARG;
+                         int* status, int* bsr_status, double* energy, void* toi, float* x4, ipcb_stream s) {
+  if (!soup || !b || (dx && !x1) || !ee_cnt || !pt_cnt || !status || !bsr_status || !energy || !toi || !x4)
+    return IPCB_E_ARG;
   const int n3 = 3 * soup->n_verts, grid = div_up(n3 > 0 ? n3 : 1, 256);
   if (soup->fp64)
     k_begin<double><<<grid, 256, 0, (cudaStream_t)s>>>((const double*)soup->x, (const double*)dx, (double*)x1,
                                                        (double*)b, n3, ee_cnt, pt_cnt, status, bsr_status, energy,
-                                                       (double*)toi);
+                                                       (double*)toi, (float4*)x4);
   else
     k_begin<float><<<grid, 256, 0, (cudaStream_t)s>>>((const float*)soup->x, (const float*)dx, (float*)x1, (float*)b,
-                                                      n3, ee_cnt, pt_cnt, status, bsr_status, energy, (float*)toi);
+                                                      n3, ee_cnt, pt_cnt, status, bsr_status, energy, (float*)toi,
+                                                      (float4*)x4);
   return check_launch("ipcb_iteration_begin");
 }
 

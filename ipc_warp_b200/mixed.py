@@ -609,6 +609,7 @@ class MixedSolver(ContactBarrierMixin):
                N.ptr(ls["acc0"]), h2, eps, 64, ctypes.byref(self.contacts_new.c_struct()),
                ctypes.byref(self.contacts_pt.c_struct()), s)
         N.call("ipcb_graph_launch", self._ls_graph(), s)
+        self._follow_x4()
         N.call("ipcb_ls_finish", N.ptr(ls["state"]), self.fp64, self.nq, N.ptr(self.q_start), N.ptr(self.q), s)
         self._sync()
         ls["host"].copy_(ls["state"], non_blocking=True)

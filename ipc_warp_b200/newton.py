@@ -470,14 +470,20 @@ class FEMContactSolver(ContactBarrierMixin):
                        N.ptr(self.Bm), N.ptr(self.W), self.mu, self.lam, None, None, N.ptr(st["tet_vals"]),
                        N.ptr(self.b), N.stream_handle())
                 elastic_values()
-        self._pack()
+        packed = self._refits_packed()
+        if packed:
+            self._pack()
+        else:
+            self.update_bvh()
         with self._branch(0):
             if self.has_triangles:
-                self._refit_triangles()
+                if packed:
+                    self._refit_triangles()
                 self._launch_dcd("pt")
             else:
                 pt.cnt.zero_()
-        self._refit_edges()
+        if packed:
+            self._refit_edges()
         self._launch_dcd("ee")
         self._join(0)
         with self._branch(2):  # of the lists only
@@ -523,6 +529,7 @@ class FEMContactSolver(ContactBarrierMixin):
         if g is not None and g[0] == self._A_graph_key():
             self._diagonal()
             g[1].replay()
+            self._follow_x4()
             torch.cuda.current_stream().synchronize()
             n_ee, n_pt, bst, qst = (int(v) for v in st["graph_read"])
             ee, pt = self.contacts_new, self.contacts_pt
@@ -867,22 +874,22 @@ class FEMContactSolver(ContactBarrierMixin):
             N.call("ipcb_ls_inertia", fp64, self.soup.n_verts, N.ptr(self.states.x), N.ptr(self.states.x0),
                    N.ptr(self.states.xdot), ls["gravity"], self.h, N.ptr(self.mass),
                    N.ptr(ls["fixed"]) if ls["any_fixed"] else None, N.ptr(self.x_target), self.k_att, base + 16, s)
-        rebuild = getattr(self, "bvh_rebuild_interval", 0)
+        packed = self._refits_packed()
         if detect:
-            if rebuild:
-                self.update_bvh()
-            else:
+            if packed:
                 self._pack()
+            else:
+                self.update_bvh()
         if self.has_triangles:
             with self._branch(0):
                 if detect:
-                    if not rebuild:
+                    if packed:
                         self._refit_triangles()
                     self._launch_dcd("pt")
                 N.call("ipcb_contact_energy", 1, ctypes.byref(soup), ctypes.byref(self.contacts_pt.c_struct()), -1,
                        kappa, base + 8, N.stream_handle())
         if detect:
-            if not rebuild:
+            if packed:
                 self._refit_edges()
             self._launch_dcd("ee")
         N.call("ipcb_contact_energy", 0, ctypes.byref(soup), ctypes.byref(self.contacts_new.c_struct()), -1, kappa,
@@ -1019,6 +1026,7 @@ class FEMContactSolver(ContactBarrierMixin):
         self._ls_prelude(mode, key)
         graph = self._ls_graph(key)
         N.call("ipcb_graph_launch", graph, s)
+        self._follow_x4()
         N.call("ipcb_ls_finish", N.ptr(ls["state"]), fp64, self.soup.n_verts, N.ptr(ls["x_tmp"]),
                N.ptr(self.states.x), s)
         ls["host"].copy_(ls["state"], non_blocking=True)

@@ -108,6 +108,7 @@ class ContactPipeline(ContactBarrierMixin):
             self._graph[1].replay()
         else:
             self._enqueue()
+        self._follow_x4()
         torch.cuda.current_stream().synchronize()
         h = self._readback
         ee, pt = self.contacts_new, self.contacts_pt
@@ -198,7 +199,7 @@ class ContactPipeline(ContactBarrierMixin):
         self.compute_V(ret=False)
         N.call("ipcb_iteration_begin", soup, N.ptr(self._dx_buf) if io is None else None, N.ptr(self.ccd_x1),
                N.ptr(self.b), N.ptr(ee.cnt), N.ptr(pt.cnt), N.ptr(self._status), N.ptr(self._bsr_status),
-               N.ptr(self._energy), N.ptr(self.ccd_toi), N.stream_handle())
+               N.ptr(self._energy), N.ptr(self.ccd_toi), N.ptr(self.x4), N.stream_handle())
         if io is not None:  # the direction crosses the bus beside the discrete queries
             cin = self._copy_in
             cin.wait_stream(main)
@@ -206,7 +207,6 @@ class ContactPipeline(ContactBarrierMixin):
                 self._dx_buf.copy_(io[1], non_blocking=True)
                 N.call("ipcb_add_dx", soup, N.ptr(self._dx_buf), N.ptr(self.ccd_x1), N.stream_handle())
                 self._x1_done.record(cin)
-            self._pack()
         side.wait_stream(main)
         with torch.cuda.stream(side):
             if io is None:

@@ -110,13 +110,13 @@ class ShardedContactPipeline(ContactBarrierMixin):
         if which == "ee":
             self.contacts_new.cnt.zero_()
             first, count = self.ee_range
-            N.call("ipcb_dcd_ee_range", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.bvh_edges.c), th,
+            N.call("ipcb_dcd_ee_range", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.bvh_edges._c), th,
                    float(contact._thickness + contact.buffer), int(self.disable_self_collision), first, count,
                    ctypes.byref(self.contacts_new.c_struct()), N.ptr(self._status), s)
         else:
             self.contacts_pt.cnt.zero_()
             first, count = self.pt_range
-            N.call("ipcb_dcd_pt_range", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.tri_mesh.c), th,
+            N.call("ipcb_dcd_pt_range", ctypes.byref(soup), N.ptr(self.x4), ctypes.byref(self.tri_mesh._c), th,
                    float(2.0 * (contact._thickness + contact.buffer)), int(self.disable_self_collision), N.ptr(self._point_order), first,
                    count, ctypes.byref(self.contacts_pt.c_struct()), N.ptr(self._status), s)
 

@@ -235,7 +235,7 @@ int ipcb_edge_triangle_crossings(const ipcb_soup* soup, const ipcb_lbvh* tri_bvh
 
 /* ---- CCD (ccd/ccd.py:360-427 point_triangle_toi / edge_edge_toi) ----
  * Cubic coplanarity TOI in double for every candidate whose swept boxes
- * overlap; toi (scalar[1], caller sets 1) gets the minimum root < 1,
+ * overlap (the caller's; the points' are formed here, padded by pad); toi (scalar[1], caller sets 1) gets the minimum root < 1,
  * rounded toward zero when stored as float.  The workspace stages candidate
  * pairs (ipcb_toi_workspace(capacity) bytes, int32 count first); pairs that
  * do not fit are solved during traversal, so any capacity >= 0 is correct. */

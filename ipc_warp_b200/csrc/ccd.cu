@@ -706,7 +706,7 @@ enum Mode {
 // staged or solved.
 template <class S, int KIND, int MODE>
 IPCB_D void take_pairs(const S* __restrict__ x0, const S* __restrict__ x1, const int* __restrict__ prims, bool has,
-                       int2 pr, double pad, float l0f, S l0, const ipcb_contacts& out, const CandList& cand,
+                       int2 pr, double pair_pad, float l0f, S l0, const ipcb_contacts& out, const CandList& cand,
                        const CandOrder& o, int* hist, S* toi, const Sink& sink, int& st) {
   const unsigned lane = threadIdx.x & 31;
   bool want = false, accept = false;
@@ -733,7 +733,7 @@ IPCB_D void take_pairs(const S* __restrict__ x0, const S* __restrict__ x1, const
     }
   }
   if (MODE == kInline) {
-    if (want && (pad < 0.0 || swept_boxes_meet<S, KIND>(x0, x1, ids, pad))) {
+    if (want && (pair_pad < 0.0 || swept_boxes_meet<S, KIND>(x0, x1, ids, pair_pad))) {
       const d3 p0[4] = {ld(x0, ids.x), ld(x0, ids.y), ld(x0, ids.z), ld(x0, ids.w)};
       const d3 p1[4] = {ld(x1, ids.x), ld(x1, ids.y), ld(x1, ids.z), ld(x1, ids.w)};
       const double tt = collision_time<KIND>(p0, p1, st);
@@ -774,7 +774,7 @@ template <class S, int MODE>
 __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_ee_collect(
     const S* __restrict__ x0, const S* __restrict__ x1, const int* __restrict__ edges, const int* __restrict__ body,
     const __grid_constant__ tree::View v, const int* __restrict__ order, int first, int count, int nsub, int items,
-    const float* __restrict__ lo, const float* __restrict__ hi, double pad, int exclude, float thickness,
+    const float* __restrict__ lo, const float* __restrict__ hi, double pair_pad, int exclude, float thickness,
     ipcb_contacts out, CandList cand, CandOrder o, S* toi, int* status, Sink sink, const int* gate) {
   __shared__ tree::Block blocks[tree::kWarps];
   __shared__ int hist[kBuckets];
@@ -816,7 +816,7 @@ __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_
       const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);
       const int a = __float_as_int(B.qlo[pr.x].w);
       // the reference's (lower id, higher id) pair
-      take_pairs<S, 0, MODE>(x0, x1, edges, has, make_int2(min(a, pr.y), max(a, pr.y)), pad, l0f, l0, out, cand, o,
+      take_pairs<S, 0, MODE>(x0, x1, edges, has, make_int2(min(a, pr.y), max(a, pr.y)), pair_pad, l0f, l0, out, cand, o,
                              hist, toi, sink, st);
     };
     tree::for_segments(active, qlo, qhi, [&](bool in, f3 glo, f3 ghi) {
@@ -853,8 +853,8 @@ template <class S, int MODE>
 __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_pt_collect(
     const S* __restrict__ x0, const S* __restrict__ x1, const int* __restrict__ tris, const int* __restrict__ body,
     const __grid_constant__ tree::View v, const int* __restrict__ order, int first, int count, int nsub, int items,
-    double pad, float qpad, int exclude, float thickness, ipcb_contacts out, CandList cand, CandOrder o, S* toi,
-    int* status, Sink sink, const int* gate) {
+    double pad, double pair_pad, float qpad, int exclude, float thickness, ipcb_contacts out, CandList cand,
+    CandOrder o, S* toi, int* status, Sink sink, const int* gate) {
   __shared__ tree::Block blocks[tree::kWarps];
   __shared__ int hist[kBuckets];
   if (MODE == kInline && *gate == 0) return;
@@ -865,8 +865,9 @@ __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_
   const float l0f = xmul(thickness, 2.0f);
   const S l0 = S(thickness) * S(2.0);
   int st = 0;
-  // boxes up to the TOI stored so far (see swept_box)
-  const double t_end = sink.on ? 1.0 : dmin(1.0, current_toi(toi));
+  // boxes up to the TOI stored so far (see swept_box), against the caller's
+  // boxes those of the whole step
+  const double t_end = sink.on || pair_pad < 0.0 ? 1.0 : dmin(1.0, current_toi(toi));
   for (int item = blockIdx.x * tree::kWarps + (threadIdx.x >> 5); item < items; item += gridDim.x * tree::kWarps) {
     const int sub = item % nsub;
     // queries: the vertices first .. first + count - 1 of the visiting order
@@ -892,7 +893,7 @@ __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_
       const bool has = lane < n;
       const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);
       const int a = __float_as_int(B.qlo[pr.x].w);
-      take_pairs<S, 1, MODE>(x0, x1, tris, has, make_int2(a, pr.y), pad, l0f, l0, out, cand, o, hist, toi, sink, st);
+      take_pairs<S, 1, MODE>(x0, x1, tris, has, make_int2(a, pr.y), pair_pad, l0f, l0, out, cand, o, hist, toi, sink, st);
     };
     tree::for_segments(active, qlo, qhi, [&](bool in, f3 glo, f3 ghi) {
     tree::for_block_pairs<false>(v, glo, ghi, 0, sub, nsub, B.stack, [&](int tb) {
@@ -1030,7 +1031,7 @@ __global__ void __launch_bounds__(256) k_cand_bucket(CandList cand, CandOrder o,
 
 template <class S, int KIND>
 __global__ void __launch_bounds__(128) k_cand_solve(const S* __restrict__ x0, const S* __restrict__ x1,
-                                                    const int* __restrict__ prims, double pad, CandList cand,
+                                                    const int* __restrict__ prims, double pair_pad, CandList cand,
                                                     CandOrder o, S* toi, int* status, const int* skip_if) {
   if (skip_if && *skip_if) return;
   int total = 0;
@@ -1055,7 +1056,7 @@ __global__ void __launch_bounds__(128) k_cand_solve(const S* __restrict__ x0, co
     if (k < 0 || (double)tl >= cur) continue;
     const int2 pr = cand.pairs[k];
     const int4 ids = pair_ids<KIND>(prims, pr);
-    if (pad >= 0.0 && !swept_boxes_meet<S, KIND>(x0, x1, ids, pad)) continue;
+    if (pair_pad >= 0.0 && !swept_boxes_meet<S, KIND>(x0, x1, ids, pair_pad)) continue;
     d3 p0[4] = {ld(x0, ids.x), ld(x0, ids.y), ld(x0, ids.z), ld(x0, ids.w)};
     d3 p1[4] = {ld(x1, ids.x), ld(x1, ids.y), ld(x1, ids.z), ld(x1, ids.w)};
     const double tt = collision_time<KIND>(p0, p1, st);
@@ -1329,7 +1330,8 @@ struct Query {
   const S* x1;
   const ipcb_lbvh* bvh;
   const float *lower, *upper;  // EE: query boxes (null: the tree's leaf boxes)
-  double pad;                  // of the swept boxes; < 0: the caller's boxes decide
+  double pad;                  // of the swept boxes formed here
+  double pair_pad;             // of the pairs' own box test; < 0: the caller's boxes decide
   float reach, thickness;      // kBoth: the discrete query's
   const int* order;            // PT: visiting order or null
   int exclude, first, count;
@@ -1357,11 +1359,11 @@ void collect(const Query<S>& q) {
   if (KIND == 0)
     k_ee_collect<S, MODE><<<grid, 32 * tree::kWarps, 0, q.st>>>(
         x0, q.x1, q.soup->edges, q.soup->body, v, q.bvh->sorted, q.first, q.count, nsub, items, q.lower, q.upper,
-        q.pad, q.exclude, q.thickness, q.out, q.cand, o, q.toi, q.status, q.sink, gate);
+        q.pair_pad, q.exclude, q.thickness, q.out, q.cand, o, q.toi, q.status, q.sink, gate);
   else
     k_pt_collect<S, MODE><<<grid, 32 * tree::kWarps, 0, q.st>>>(
-        x0, q.x1, q.soup->triangles, q.soup->body, v, q.order, q.first, q.count, nsub, items, q.pad, q.reach,
-        q.exclude, q.thickness, q.out, q.cand, o, q.toi, q.status, q.sink, gate);
+        x0, q.x1, q.soup->triangles, q.soup->body, v, q.order, q.first, q.count, nsub, items, q.pad, q.pair_pad,
+        q.reach, q.exclude, q.thickness, q.out, q.cand, o, q.toi, q.status, q.sink, gate);
 }
 
 constexpr int kHeaderWords = 2 + 2 * kBuckets + 1;  // zero when a query starts staging
@@ -1379,14 +1381,16 @@ void solve(const Query<S>& q) {
   } else if (c.capacity) {
     const CandOrder o = cand_order(q.ws, c);
     k_cand_bucket<<<min(div_up(c.capacity, 256), 148 * 4), 256, 0, q.st>>>(c, o, c.overflow);
-    k_cand_solve<S, KIND><<<148 * 3, 128, 0, q.st>>>(x0, q.x1, prims, q.pad, c, o, q.toi, q.status, c.overflow);
+    k_cand_solve<S, KIND><<<148 * 3, 128, 0, q.st>>>(x0, q.x1, prims, q.pair_pad, c, o, q.toi, q.status, c.overflow);
   }
   collect<S, KIND, kInline>(q);
 }
 
-// Boxes given (EE: also the query boxes): stage and solve.
+// Boxes given (EE: also the query boxes), and with them what a pair is: stage
+// and solve.
 template <class S, int KIND>
-void run_boxes(const Query<S>& q) {
+void run_boxes(Query<S> q) {
+  q.pair_pad = -1.0;
   cudaMemsetAsync(q.ws, 0, kHeaderWords * sizeof(int), q.st);
   collect<S, KIND, kStage>(q);
   solve<S, KIND>(q);
@@ -1425,7 +1429,7 @@ Query<S> make_query(const ipcb_soup* soup, const void* x1, const ipcb_lbvh* bvh,
   q.soup = soup;
   q.x1 = (const S*)x1;
   q.bvh = bvh;
-  q.pad = pad;
+  q.pad = q.pair_pad = pad;
   q.exclude = exclude;
   q.first = first;
   q.count = count;
@@ -1513,7 +1517,7 @@ int ipcb_edge_edge_toi_range(const ipcb_soup* soup, const void* x1, const ipcb_l
   if (count == 0) return IPCB_OK;
   in_scalar(soup, [&](auto* scalar) {
     using S = std::remove_pointer_t<decltype(scalar)>;
-    Query<S> q = make_query<S>(soup, x1, bvh, -1.0, exclude_same_body, first, count, toi, status, ws, ws_bytes, s);
+    Query<S> q = make_query<S>(soup, x1, bvh, 0.0, exclude_same_body, first, count, toi, status, ws, ws_bytes, s);
     q.lower = lower;
     q.upper = upper;
     run_boxes<S, 0>(q);
@@ -1658,7 +1662,7 @@ int ipcb_edge_edge_intersections(const ipcb_soup* soup, const void* x1, const ip
   if (soup->n_edges == 0) return IPCB_OK;
   in_scalar(soup, [&](auto* scalar) {
     using S = std::remove_pointer_t<decltype(scalar)>;
-    Query<S> q = make_query<S>(soup, x1, bvh, -1.0, exclude_same_body, 0, soup->n_edges, toi, status, ws, ws_bytes, s);
+    Query<S> q = make_query<S>(soup, x1, bvh, 0.0, exclude_same_body, 0, soup->n_edges, toi, status, ws, ws_bytes, s);
     q.lower = lower;
     q.upper = upper;
     q.sink = Sink{*out, thickness * 2.0, 1};

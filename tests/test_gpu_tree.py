@@ -143,3 +143,57 @@ def test_step_far_beyond_the_scene(cuda, far):
     for bound in (pipe.collision_free_step(dev), pipe.iteration(dev).alpha):
         got = float(pipe.ccd_toi.item())
         assert got <= toi and toi - got <= 1e-6 and bound == (0.9 * got if got < 1.0 else 1.0)
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("cap", [1 << 16, 40, 0])
+def test_toi_of_given_boxes_equals_the_step(cuda, fp64, cap):
+    """The CCD queries on boxes the caller formed (whole, and in ranges off the
+    32-query blocks; a staging list that fits, overflows, or is none) give the
+    TOI of the queries that form their own, also where the caller's triangle
+    boxes are wider than the points'."""
+    import ctypes
+
+    from ipc_warp_b200 import _native as N
+
+    sc = loose_triangles(342, seed=9)
+    dtype = torch.float64 if fp64 else torch.float32
+    pipe = ContactPipeline.from_scene(sc, dtype=dtype, device=cuda)
+    dx = torch.tensor(np.random.default_rng(10).normal(scale=0.02, size=sc.x.shape), dtype=dtype, device=cuda)
+    pipe.collision_free_step(dx)  # ccd_x1
+    soup, x1, toi, st = ctypes.byref(pipe.soup.c_struct()), N.ptr(pipe.ccd_x1), pipe.ccd_toi, pipe._status
+    ws = torch.empty(N.size("ipcb_toi_workspace", cap), dtype=torch.uint8, device=cuda)
+
+    def value(calls):
+        toi.fill_(1.0)
+        st.zero_()
+        for c in calls:
+            c()
+        assert int(st.item()) == 0
+        return float(toi.item())
+
+    s = N.stream_handle()
+    tail = (N.ptr(toi), N.ptr(st), N.ptr(ws), ws.numel(), s)
+    cuts = {"ee": (0, 7, 33, 500, pipe.soup.n_edges), "pt": (0, 31, 64, 333, pipe.soup.n_verts)}
+    for which, step in (("ee", pipe._toi_ws), ("pt", pipe._toi_ws_pt)):
+        n = cuts[which][-1]
+        ref = value([lambda: pipe._ccd_query(which, 0, n, step)])
+        assert ref < 1.0
+        assert value([lambda a=a, b=b: pipe._ccd_query(which, a, b - a, ws)
+                      for a, b in zip(cuts[which], cuts[which][1:])]) == ref
+        for pad in (1e-7, 0.03):
+            if which == "ee":
+                lo, hi, bvh = pipe.ccd_edge_lower, pipe.ccd_edge_upper, pipe.ccd_edge_bvh
+                N.call("ipcb_swept_edge_aabbs", soup, x1, pad, N.ptr(lo), N.ptr(hi), s)
+                bvh.refit(lo, hi)
+                head = (soup, x1, ctypes.byref(bvh.c), N.ptr(lo), N.ptr(hi), 0)
+                name = "ipcb_edge_edge_toi"
+            else:
+                lo, hi, bvh = pipe.ccd_triangle_lower, pipe.ccd_triangle_upper, pipe.ccd_triangle_bvh
+                N.call("ipcb_swept_triangle_aabbs", soup, x1, pad, N.ptr(lo), N.ptr(hi), s)
+                bvh.refit(lo, hi)
+                head = (soup, x1, ctypes.byref(bvh.c), 1e-7, 0)
+                name = "ipcb_point_triangle_toi"
+            assert value([lambda: N.call(name, *head, *tail)]) == ref
+            assert value([lambda a=a, b=b: N.call(name + "_range", *head, a, b - a, *tail)
+                          for a, b in zip(cuts[which], cuts[which][1:])]) == ref

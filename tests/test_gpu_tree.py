@@ -197,3 +197,23 @@ def test_toi_of_given_boxes_equals_the_step(cuda, fp64, cap):
             assert value([lambda: N.call(name, *head, *tail)]) == ref
             assert value([lambda a=a, b=b: N.call(name + "_range", *head, a, b - a, *tail)
                           for a, b in zip(cuts[which], cuts[which][1:])]) == ref
+
+
+@pytest.mark.parametrize("fp64", [False, True])
+@pytest.mark.parametrize("offset", [0.0, 30.0, 1000.0])
+def test_touch_bound_keeps_the_minimum_far_from_the_origin(cuda, fp64, offset):
+    """The pairs are bounded in float before the double solve; the margin
+    covers the rounding of positions far from the origin (the oracle solves
+    every pair whose boxes meet)."""
+    sc = loose_triangles(200, seed=11)
+    sc.x = sc.x + offset * np.array([1.0, -0.7, 0.4])
+    dtype = torch.float64 if fp64 else torch.float32
+    pipe = ContactPipeline.from_scene(sc, dtype=dtype, device=cuda)
+    for seed, scale in ((1, 0.01), (2, 0.1), (3, 1.0)):
+        dx = torch.tensor(np.random.default_rng(seed).normal(scale=scale, size=sc.x.shape), dtype=dtype, device=cuda)
+        x0 = pipe.soup.x_transformed.cpu().numpy()
+        toi, _ = po.scene_toi(x0, x0 - dx.cpu().numpy(), sc.edges, sc.triangles, sc.body, fp64=fp64)
+        for run in (pipe.collision_free_step, pipe.iteration):
+            run(dx)
+            got = float(pipe.ccd_toi.item())
+            assert got <= toi and toi - got <= 1e-6

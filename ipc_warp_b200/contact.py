@@ -203,7 +203,8 @@ class ContactSolverBase:
         """What a captured sequence holds by value, or by an address a caller
         may replace: part of the key of every graph, so that all of a
         solver's graphs follow a change at the same call."""
-        return (_thickness, buffer, bool(self.disable_self_collision), float(self.contact_stiffness), float(self.h))
+        return (_thickness, buffer, bool(self.disable_self_collision), float(self.contact_stiffness), float(self.h),
+                getattr(self, "bvh_rebuild_interval", 0))
 
     # --------------------------------------------------------------- hooks
     def profile_timer(self, name):

@@ -173,3 +173,16 @@ def test_overflowed_search_leaves_no_cached_energy(cuda):
     at = s.total_energy()
     s.line_search()
     assert s.stats.energies[-1][0] == pytest.approx(at, rel=1e-12)
+
+
+def test_search_follows_a_rebuild_interval(cuda):
+    """Rebuilds asked for once the search's start is a captured graph."""
+    s = _solver(torch.float64, "device")
+    _direction(s)
+    x0 = s.states.x.clone()
+    for _ in range(3):
+        alpha = s.line_search()
+        s.states.x.copy_(x0)
+    s.bvh_rebuild_interval = 1
+    calls = getattr(s, "_bvh_calls", 0)
+    assert s.line_search() == alpha and s._bvh_calls > calls + 1  # E0's detection, and the trial's capture

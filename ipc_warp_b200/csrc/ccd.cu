@@ -334,11 +334,10 @@ __global__ void k_swept(const S* __restrict__ x0, const S* __restrict__ x1, cons
 }
 
 // Candidate pairs are staged in a list so the cubic solves run one pair per
-// thread (balanced) instead of inside divergent traversal loops.  Workspace:
-// [count int32 | overflow int32 | pad to 256 B | int2 pairs[capacity]].  When
-// a pair finds the list full the overflow flag is raised and an inline pass
-// solves every pair of the query during traversal, so the result never
-// depends on the capacity.
+// thread (balanced) instead of inside divergent traversal loops (layout of the
+// workspace: cand_list, cand_order).  When a pair finds the list full the
+// overflow flag is raised and an inline pass solves every pair of the query
+// during traversal, so the result never depends on the capacity.
 struct CandList {
   int* count;
   int* overflow;  // set by a collect pass that dropped pairs (the inline pass then redoes the query)
@@ -766,9 +765,9 @@ IPCB_D void take_pairs(const S* __restrict__ x0, const S* __restrict__ x1, const
 // topology tests are bounded on full warps and staged.  kInline (run only when
 // *gate is set: the staging list overflowed) solves every pair in place.
 // lo / hi: the queries' boxes, or null for the tree's own leaf boxes.
-// 64 registers (8 blocks a SM; 96 unbounded): the walk issues about 5,000
-// instructions a block in short dependent runs, and the spills (72 B, around
-// the flush) cost less than the missing warps (screw and nut iteration 1.59 ->
+// 64 registers (8 blocks a SM; 96 unbounded): the walk issues about 7,900
+// instructions a block in short dependent runs, and the spills (around the
+// flush) cost less than the missing warps (screw and nut iteration 1.59 ->
 // 1.45 ms, from 3.37 with a traversal per thread).
 template <class S, int MODE>
 __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_ee_collect(
@@ -810,7 +809,7 @@ __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_
     B.qhi[lane] = make_float4(qhi.x, qhi.y, qhi.z, __int_as_float(bi));
     B.ev[lane] = ea;
     __syncwarp();
-      int nq = 0;
+    int nq = 0;
     auto flush = [&](int n) {
       const bool has = lane < n;
       const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);
@@ -888,7 +887,7 @@ __global__ void __launch_bounds__(32 * tree::kWarps, MODE == kInline ? 1 : 8) k_
     B.qlo[lane] = make_float4(qlo.x, qlo.y, qlo.z, __int_as_float(i));
     B.qhi[lane] = make_float4(qhi.x, qhi.y, qhi.z, __int_as_float(bi));
     __syncwarp();
-      int nq = 0;
+    int nq = 0;
     auto flush = [&](int n) {
       const bool has = lane < n;
       const int2 pr = has ? B.queue[nq - n + lane] : make_int2(0, 0);

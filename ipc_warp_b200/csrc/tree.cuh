@@ -7,7 +7,8 @@
 // that forms every leaf box from the positions, reduces 32 at a time and
 // writes 33 bytes a leaf, where the binary tree's climb (k_refit) pays a chain
 // of fences and atomics per level and writes 192 bytes a node: 1.49M edges
-// 31 us against 211 us, and the box kernel before it is gone too.
+// 39 us (ncu, cold; 30 MB of DRAM) against 211 us, and the box kernel before it
+// is gone too.
 //
 // A query is a block of 32 primitives in Morton order (one lane each), and a
 // warp walks the tree once for the whole block: 32 children are loaded as one
@@ -16,9 +17,12 @@
 // are read from shared memory (broadcast), so a block pair costs at most 32
 // uniform box tests, all lanes busy, instead of 32 private traversals that
 // diverge (14 of 32 lanes active) over dependent 128-byte loads.  On the screw
-// and nut (1.49M edges) a block opens 10 tree nodes and meets 10 blocks, 7 of
-// them with a live pair; 74 box tests and 37 queue rounds a block.  Bound by
-// instruction issue.
+// and nut the joined edge walk (46,566 blocks) issues 367M instructions, 7,900 a
+// block, 27 of 32 lanes active, and takes 0.54 ms: the issue slots are 64% busy
+// with the 48% of the warp slots its 64 registers leave; 91 MB of DRAM.  So it
+// is bound by issue and by the latency of its short dependent runs, not by
+// memory; a smaller scene leaves warps waiting for the last of their CTA (a
+// sixth of the mesh: 53% issue, 39% of the warp slots, barrier 1.7 a issue).
 #pragma once
 #include "common.cuh"
 

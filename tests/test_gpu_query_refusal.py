@@ -31,10 +31,6 @@ class _FailingCcd:
         super()._launch_ccd(dx, reset_status)
         self._status.fill_(self.fail_bits)
 
-    def _ccd_launches(self, dx):
-        super()._ccd_launches(dx)
-        self._status.fill_(self.fail_bits)
-
 
 class FailingSolver(_FailingCcd, FEMContactSolver):
     pass

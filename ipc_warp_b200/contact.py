@@ -109,6 +109,17 @@ class Contacts:
         return N.Contacts(N.ptr(self.a1a2b1b2), N.ptr(self.e0e1), N.ptr(self.l0), N.ptr(self.alpha),
                           N.ptr(self.lam), N.ptr(self.cnt), self.capacity)
 
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        self.__dict__["_addresses"] = None  # of the columns as they were
+
+    def addresses(self) -> tuple:
+        """What a captured sequence holds of the list (part of its key)."""
+        if self._addresses is None:
+            self.__dict__["_addresses"] = (self.capacity, *(c.data_ptr() for c in (
+                self.a1a2b1b2, self.e0e1, self.l0, self.alpha, self.lam, self.cnt)))
+        return self._addresses
+
     def grow(self, capacity: int) -> None:
         self.__init__(capacity, self.dtype, self.device)
 
@@ -204,7 +215,8 @@ class ContactSolverBase:
         may replace: part of the key of every graph, so that all of a
         solver's graphs follow a change at the same call."""
         return (_thickness, buffer, bool(self.disable_self_collision), float(self.contact_stiffness), float(self.h),
-                getattr(self, "bvh_rebuild_interval", 0))
+                getattr(self, "bvh_rebuild_interval", 0), self.soup.x_transformed.data_ptr(), self.soup.xcs.data_ptr(),
+                self.contacts_new.addresses(), self.contacts_pt.addresses())
 
     # --------------------------------------------------------------- hooks
     def profile_timer(self, name):

@@ -544,9 +544,7 @@ class MixedSolver(ContactBarrierMixin):
         N.call("ipcb_acc_fold", base + 16, eb, 4, s)
 
     def _ls_key(self):
-        ee, pt = self.contacts_new, self.contacts_pt
-        return (self.q.data_ptr(), self.q_start.data_ptr(), self.dq.data_ptr(), self.x.data_ptr(),
-                ee.a1a2b1b2.data_ptr(), ee.capacity, pt.a1a2b1b2.data_ptr(), pt.capacity, self._captured())
+        return (self.q.data_ptr(), self.q_start.data_ptr(), self.dq.data_ptr(), self.x.data_ptr(), *self._captured())
 
     def _captured(self):
         return (*super()._captured(), self.material, self.mu, self.lam)

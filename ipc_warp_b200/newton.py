@@ -565,16 +565,14 @@ class FEMContactSolver(ContactBarrierMixin):
         workload bucket's choice would cost a recapture per change of
         bucket)."""
         st = self._static
-        ee, pt, t = self.contacts_new, self.contacts_pt, self.collision_triplets
-        return (ee.a1a2b1b2.data_ptr(), ee.capacity, pt.a1a2b1b2.data_ptr(), pt.capacity,
-                None if t is None else t.rows.data_ptr(), None if self.A is None else self.A.values.data_ptr(),
+        t = self.collision_triplets
+        return (None if t is None else t.rows.data_ptr(), None if self.A is None else self.A.values.data_ptr(),
                 None if getattr(self, "_C", None) is None else self._C.values.data_ptr(),
-                st.get("a_rows").data_ptr() if "a_rows" in st else None, self.states.x.data_ptr(), self._captured())
+                st.get("a_rows").data_ptr() if "a_rows" in st else None, self.states.x.data_ptr(), *self._captured())
 
     def _captured(self):
         return (*super()._captured(), self.material, self.mu, self.lam, self.k_att, self.tets.data_ptr(),
-                self.Bm.data_ptr(), self.W.data_ptr(), self.mass.data_ptr(), self.b.data_ptr(),
-                self.soup.xcs.data_ptr())
+                self.Bm.data_ptr(), self.W.data_ptr(), self.mass.data_ptr(), self.b.data_ptr())
 
     def _compute_A_generic(self) -> BsrMatrix:
         """Per-term kernels, then one sort-based assembly of every triplet."""
@@ -913,9 +911,7 @@ class FEMContactSolver(ContactBarrierMixin):
 
     def _ls_key(self):
         return (self.states.x.data_ptr(), self.states.dx.data_ptr(), self.states.x0.data_ptr(),
-                self.states.xdot.data_ptr(), self.contacts_new.a1a2b1b2.data_ptr(), self.contacts_new.capacity,
-                self.contacts_pt.a1a2b1b2.data_ptr(), self.contacts_pt.capacity, self.x_target.data_ptr(),
-                self._captured())
+                self.states.xdot.data_ptr(), self.x_target.data_ptr(), *self._captured())
 
     def _ls_graph(self, key: tuple):
         """The WHILE graph of one trial, captured once per _ls_key() (on a

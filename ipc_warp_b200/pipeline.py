@@ -125,13 +125,12 @@ class ContactPipeline(ContactBarrierMixin):
         return IterationResult(n_ee, n_pt, float(h["energy"][0]) * self.h * self.h, alpha, qst)
 
     def _graph_key(self):
-        ee, pt, t, H = self.contacts_new, self.contacts_pt, self.collision_triplets, self.collision_hessian
+        t, H = self.collision_triplets, self.collision_hessian
         ws = tuple(None if getattr(self, a, None) is None else getattr(self, a).data_ptr()
                    for a in ("_ws_ee", "_ws_pt"))
         io = None if self._host_io is None else tuple(a.data_ptr() for a in self._host_io)
-        return (ee.a1a2b1b2.data_ptr(), ee.capacity, pt.a1a2b1b2.data_ptr(), pt.capacity,
-                None if t is None else t.rows.data_ptr(), None if H is None else H.values.data_ptr(),
-                None if H is None else H._ws.data_ptr(), ws, io, self._captured(),
+        return (None if t is None else t.rows.data_ptr(), None if H is None else H.values.data_ptr(),
+                None if H is None else H._ws.data_ptr(), ws, io, *self._captured(),
                 getattr(self, "bvh_rebuild_interval", 0))
 
     def iteration_host(self, x: torch.Tensor, dx: torch.Tensor, b: torch.Tensor) -> IterationResult:

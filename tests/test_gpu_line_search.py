@@ -186,3 +186,49 @@ def test_search_follows_a_rebuild_interval(cuda):
     s.bvh_rebuild_interval = 1
     calls = getattr(s, "_bvh_calls", 0)
     assert s.line_search() == alpha and s._bvh_calls > calls + 1  # E0's detection, and the trial's capture
+
+
+@pytest.mark.parametrize("column", ["cnt", "e0e1", "a1a2b1b2", "l0"])
+def test_graphs_follow_a_replaced_column(cuda, column):
+    """A list column in other memory: every graph that holds the list is
+    captured again."""
+    from ipc_warp_b200.pipeline import ContactPipeline
+
+    s = _solver(torch.float64, "device")
+    _direction(s)
+    x0 = s.states.x.clone()
+    sc = two_cubes(n=3, gap=4e-4, angle_deg=15.0, jitter=0.0, seed=0, dhat=1e-3, kappa=1e6)
+    pipe = ContactPipeline.from_scene(sc, dtype=torch.float64, device=cuda)
+    dx = torch.zeros_like(pipe.states.x)
+    kept = []  # the old columns stay allocated: nothing is written to freed memory
+
+    def passes():
+        out = []
+        for _ in range(3):  # launched, captured, replayed
+            s.states.x.copy_(x0)
+            nnz, lists = s.compute_A().nnz_sync(), [s.contacts_new, s.contacts_pt, pipe.contacts_new, pipe.contacts_pt]
+            alpha = s.line_search()
+            pipe.iteration(dx)
+            out.append((nnz, alpha, s.n_contacts, *(int(c.cnt) for c in lists),
+                        *(c.records(int(c.cnt)).sum(0).tolist() for c in lists), *(float(c.l0[0]) for c in lists)))
+        return out
+
+    want = passes()
+    assert want[0] == want[1] == want[2]
+    for lst in (s.contacts_new, s.contacts_pt, pipe.contacts_new, pipe.contacts_pt):
+        old = getattr(lst, column)
+        kept.append(old)
+        setattr(lst, column, torch.zeros_like(old))
+    assert passes() == want
+
+
+def test_pipeline_graph_follows_other_positions(cuda):
+    from ipc_warp_b200.pipeline import ContactPipeline
+
+    sc = two_cubes(n=3, gap=4e-4, angle_deg=15.0, jitter=0.0, seed=0, dhat=1e-3, kappa=1e6)
+    pipe = ContactPipeline.from_scene(sc, dtype=torch.float64, device=cuda)
+    dx = torch.zeros_like(pipe.states.x)
+    for _ in range(3):
+        assert pipe.iteration(dx).n_ee > 0
+    pipe.soup.x_transformed = torch.where(torch.tensor(sc.body, device=cuda)[:, None] == 1, 1.0, 0.0) + pipe.soup.x_transformed
+    assert pipe.iteration(dx).n_ee == 0

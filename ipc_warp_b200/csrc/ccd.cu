@@ -1023,7 +1023,8 @@ __global__ void __launch_bounds__(256) k_cand_bucket(CandList cand, CandOrder o,
       sbase[q] = sb[q] ? start + atomicAdd(o.bcursor + q, sb[q]) : 0;
     }
     __syncthreads();
-    if (b >= 0) o.order[sbase[b] + local] = k;
+    // (a second solve of the same list finds the cursors at its end)
+    if (b >= 0 && sbase[b] + local < cand.capacity) o.order[sbase[b] + local] = k;
     __syncthreads();
   }
 }

@@ -217,3 +217,28 @@ def test_touch_bound_keeps_the_minimum_far_from_the_origin(cuda, fp64, offset):
             run(dx)
             got = float(pipe.ccd_toi.item())
             assert got <= toi and toi - got <= 1e-6
+
+
+def test_solving_a_staged_list_twice(cuda):
+    """The second call of a solve stays inside the list and finds nothing new."""
+    from ipc_warp_b200 import _native as N
+
+    sc = loose_triangles(342, seed=12)
+    pipe = ContactPipeline.from_scene(sc, dtype=torch.float32, device=cuda)
+    dx = torch.tensor(np.random.default_rng(13).normal(scale=0.02, size=sc.x.shape), dtype=torch.float32, device=cuda)
+    bound = pipe.collision_free_step(dx)
+    for which in ("ee", "pt"):
+        pipe.ccd_toi.fill_(1.0)
+        pipe._both_queries(which, pipe._toi_ws)
+        n = int(pipe._toi_ws[:4].view(torch.int32))  # a list that just holds them
+        ws = torch.empty(N.size("ipcb_toi_workspace", n) + 4096, dtype=torch.uint8, device=cuda)
+        guard = ws[-4096:]
+        guard.fill_(0x5A)
+        ws = ws[:-4096]
+        pipe._both_queries(which, ws)
+        assert int(ws[:4].view(torch.int32)) == n > 0
+        pipe._solve_staged(which, ws)
+        toi = float(pipe.ccd_toi.item())
+        pipe._solve_staged(which, ws)
+        assert float(pipe.ccd_toi.item()) == toi and bool((guard == 0x5A).all())
+        assert bound <= (0.9 * toi if toi < 1.0 else 1.0)
